@@ -46,8 +46,20 @@ SGMEV_API int sgmev_fma_peak(int precision, double* flops_per_second, int* sm_cl
 #define SGMEV_KERNEL_MULTT_MAT16 16 /* multTranspose streaming it */
 #define SGMEV_KERNEL_BLOCK_MULT 17  /* B [a_1 .. a_16], BF16 tensor-core tiles */
 #define SGMEV_KERNEL_BLOCK_MULTT 18 /* B^T [v_1 .. v_16], BF16 tensor-core tiles */
+#define SGMEV_KERNEL_MULT_NEST64 19  /* FP64 mult, nested subspace products */
+#define SGMEV_KERNEL_MULTT_NEST64 20 /* FP64 multTranspose, nested subspace products */
 SGMEV_API int sgmev_profile(sgmev_op* op, int enable);
 SGMEV_API int sgmev_profile_read(sgmev_op* op, int kind, int64_t* launches, double* seconds);
+
+/*
+ * Host evaluation (no GPU) of the nested subspace plan's two programs on finite data, coefficients
+ * and sources: mult_out [n_data] = B alpha, multt_out [n_grid] = B^T source, every array access
+ * checked. 0: done, 1: not a grid that the nested kernels take, 2: an index left its array.
+ */
+SGMEV_API int sgmev_nest_host(int dim, int64_t n_grid, const double* level_pow2,
+                              const double* index, int modlinear, int64_t n_data,
+                              const double* data, const double* alpha, const double* source,
+                              double* mult_out, double* multt_out);
 
 #ifdef __cplusplus
 }

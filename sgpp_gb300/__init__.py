@@ -66,7 +66,7 @@ EXPORTED_SYMBOLS = (
     "sgmev_batch_info", "sgdata_size", "sgdata_read", "sgfit_config_defaults", "sgfit_create",
     "sgfit_destroy", "sgfit_fit", "sgfit_adapt", "sgfit_update", "sgfit_evaluate", "sgfit_grid",
     "sgfit_alpha", "sgfit_stats", "sgmev_mult_block", "sgmev_mult_transpose_block",
-    "sgmev_fit_block", "sgmev_fit_block_device", "sgmev_set_params",
+    "sgmev_fit_block", "sgmev_fit_block_device", "sgmev_set_params", "sgmev_nest_host",
 )
 
 SGMEV_KERNEL_MULT_FP32 = 0
@@ -88,6 +88,8 @@ SGMEV_KERNEL_MULT_MAT16 = 15
 SGMEV_KERNEL_MULTT_MAT16 = 16
 SGMEV_KERNEL_BLOCK_MULT = 17
 SGMEV_KERNEL_BLOCK_MULTT = 18
+SGMEV_KERNEL_MULT_NEST64 = 19
+SGMEV_KERNEL_MULTT_NEST64 = 20
 SGMEV_BLOCK_RHS = 16
 
 
@@ -189,6 +191,7 @@ def load_library(path: str = LIBRARY_PATH):
         "sgmev_batch_info": (c_int, [vp, pi64, pi64, ctypes.POINTER(c_int)]),
         "sgmev_profile": (c_int, [vp, c_int]),
         "sgmev_profile_read": (c_int, [vp, c_int, pi64, pdbl]),
+        "sgmev_nest_host": (c_int, [c_int, i64, vp, vp, c_int, i64, vp, vp, vp, vp, vp]),
         "sgdata_size": (c_int, [c_int, ctypes.c_char_p, i64, c_int, c_int, vp, c_int, pi64, pi64]),
         "sgdata_read": (c_int, [c_int, ctypes.c_char_p, i64, c_int, c_int, i64, vp, c_int, vp,
                                 c_int, vp, vp, i64, pi64, pi64]),

@@ -26,8 +26,8 @@ CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wall",
              "-I" + os.path.join(ROOT, "include")]
 
 CU_SOURCES = ["sgmev.cu", "dense_mod.cu", "peak.cu", "noalloc.cu", "batch.cu", "subspace.cu",
-              "subspace_mat.cu", "devmem.cu", "fitter.cu", "block_tc.cu"]
-CPP_SOURCES = ["grid.cpp", "datasets.cpp"]
+              "subspace_mat.cu", "nest.cu", "devmem.cu", "fitter.cu", "block_tc.cu"]
+CPP_SOURCES = ["grid.cpp", "datasets.cpp", "nest_plan.cpp"]
 
 
 def _nvcc() -> str:

@@ -23,6 +23,7 @@
 #include "dense.h"
 #include "kernels.cuh"
 #include "devmem.h"
+#include "nest.h"
 #include "subspace.h"
 #include "block_tc.h"
 
@@ -135,6 +136,10 @@ struct sgmev_op {
   int algo = 2;          // FP32 products: 0 dense, 1 subspace, 2 auto (params "algo")
   SubPlan sub;           // subspace tables of the current grid
   bool sub_ok = false;   // sub is built and chosen for the FP32 products
+  // nested subspace plan of the FP64 products, built on the first of them from the eval arrays
+  sgmev::NestPlan nest;
+  bool nest_failed = false;  // the current grid is not one the nested kernels take
+  std::vector<double> h_level_pow2, h_index;
   // BF16 tensor-core products with 16 right-hand sides (built on the first block call)
   sgmev::BlockPlan blk;
   bool blk_ok = false;
@@ -157,8 +162,8 @@ struct sgmev_op {
   std::vector<cudaEvent_t> prof_events;  // pool, 2 per launch
   std::vector<int> prof_kind;            // kind of launch i
   size_t prof_used = 0;                  // launches recorded since the last reset
-  int64_t prof_count[19] = {0};
-  double prof_seconds[19] = {0.0};
+  int64_t prof_count[21] = {0};
+  double prof_seconds[21] = {0.0};
 };
 
 namespace sgmev {
@@ -183,9 +188,11 @@ enum {
   KIND_MULT_MAT16 = 15,
   KIND_MULTT_MAT16 = 16,
   KIND_BLOCK_MULT = 17,
-  KIND_BLOCK_MULTT = 18
+  KIND_BLOCK_MULTT = 18,
+  KIND_MULT_NEST64 = 19,
+  KIND_MULTT_NEST64 = 20
 };
-constexpr int kKinds = 19;
+constexpr int kKinds = 21;
 
 template <typename T>
 static const T* gscale(const sgmev_op* op);
@@ -852,6 +859,24 @@ static bool mat_ready(sgmev_op* op) {
   return true;
 }
 
+// The nested subspace kernels serve the FP64 products of every grid whose plan they take, unless
+// "algo" is "dense" (they cost about 1.3 FP64 instructions per subspace and data point, the dense
+// kernels 3 d per grid point and data point, and a subspace has at least one grid point; smallest
+// measured, 351 points and 3,000 data points: a host system product 279 -> 113 us). ModLinear
+// data outside the cube stays on the dense kernels, which extrapolate.
+static bool nest_ready(sgmev_op* op) {
+  using namespace sgmev;
+  if (op->nest.ok) return true;
+  if (op->algo == 0 || op->nest_failed || op->n < 1 || (op->mod && !op->in_cube)) return false;
+  std::string why;
+  if (!nest_build(&op->nest, op->dim, op->n, op->h_level_pow2.data(), op->h_index.data(), op->mod,
+                  op->num_sms, op->stream, &why)) {
+    op->nest_failed = true;
+    return false;
+  }
+  return true;
+}
+
 // Inputs per precision: FP64 a64; FP32 a32; DF64 (a32, a32lo) — all padded to npad.
 // out64 / out32 [mpad] (zero beyond m) = B a over data range [j_begin, j_end).
 static int dev_mult(sgmev_op* op, int prec, const double* a64, const float* a32,
@@ -861,7 +886,15 @@ static int dev_mult(sgmev_op* op, int prec, const double* a64, const float* a32,
   Plan p;
   const int64_t total = j_end;
   const int64_t valid = std::min(op->m, total);
-  if (prec == SGMEV_FP64) {
+  if (prec == SGMEV_FP64 && out64 && !out32 && nest_ready(op)) {
+    int launches = 0;
+    const long ev = prof_begin(op, KIND_MULT_NEST64);
+    SGMEV_CUDA(nest_mult64(op->nest, op->stream, NestDense{op->xt64, op->li64, op->mpad}, op->m, a64,
+                           out64, j_begin, j_end, static_cast<double*>(op->part), op->part_elems,
+                           op->num_sms, &launches));
+    prof_end(op, ev);
+    op->launches += launches;
+  } else if (prec == SGMEV_FP64) {
     SGMEV_TRY(run_mult<double>(op, op->xt64, op->li64, a64, j_begin, j_end, &p));
     if (out64) SGMEV_TRY((run_reduce<double, double>(op, (int)p.nsplit, op->mpad, j_begin, valid, total, out64, nullptr, 0.0)));
     if (out32) SGMEV_TRY((run_reduce<double, float>(op, (int)p.nsplit, op->mpad, j_begin, valid, total, out32, nullptr, 0.0)));
@@ -909,7 +942,14 @@ static int dev_multt(sgmev_op* op, int prec, const double* v64, const float* v32
   if (g_end <= g_begin) return SGMEV_OK;
   Plan p;
   const int64_t valid = std::min(op->n, g_end);
-  if (prec == SGMEV_FP64) {
+  if (prec == SGMEV_FP64 && nest_ready(op)) {
+    int launches = 0;
+    const long ev = prof_begin(op, KIND_MULTT_NEST64);
+    SGMEV_CUDA(nest_multt64(op->nest, op->stream, NestDense{op->xt64, op->li64, op->mpad}, op->m, v64,
+                            op->npad, out64, add, scale, op->num_sms, &launches));
+    prof_end(op, ev);
+    op->launches += launches;
+  } else if (prec == SGMEV_FP64) {
     SGMEV_TRY(run_multt<double>(op, op->xt64, v64, op->li64, g_begin, g_end, &p));
     SGMEV_TRY((run_reduce<double, double>(op, (int)p.nsplit, op->npad, g_begin, valid, g_end, out64, add, scale)));
   } else if (prec == SGMEV_DF64 && op->sub_ok && op->mat_multt && mat_ready(op) &&
@@ -1111,6 +1151,10 @@ static int stage_grid(sgmev_op* op, int64_t n, const double* level_pow2, const d
   op->blk_ok = false;
   op->blk_failed = false;
   subspace_free(&op->sub);
+  nest_free(&op->nest);
+  op->nest_failed = false;
+  op->h_level_pow2.assign(level_pow2, level_pow2 + n * op->dim);
+  op->h_index.assign(index, index + n * op->dim);
   if (op->algo != 0 && n > 0) {
     std::string why;
     if (subspace_build(&op->sub, op->dim, n, level_pow2, index, op->stream, &why)) {
@@ -1151,6 +1195,7 @@ static void release(sgmev_op* op) {
   if (op->own_stream && op->own_stream != op->stream) cudaStreamSynchronize(op->own_stream);
   block_free(&op->blk);
   subspace_free(&op->sub);
+  nest_free(&op->nest);
   void* ptrs[] = {op->xt64, op->xt32, op->xt32lo, op->li64, op->li32, op->gq, op->gs64, op->gs32, op->a64,
                   op->a32,  op->a32lo, op->v64,   op->v32,  op->v32lo, op->out64, op->part,
                   op->cg,   op->dot_part, op->dot_out, op->scal};

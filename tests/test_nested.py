@@ -1,0 +1,170 @@
+"""The nested subspace products: the plan's two programs on the host (every index checked) against
+the dense evaluation, and the FP64 kernels against the dense ones on the GPU."""
+import numpy as np
+import pytest
+
+import sgpp_gb300 as sg
+
+EPS = 2.0 ** -52
+
+
+def _grid(dim, level, basis="linear", rounds=0, seed=0):
+    make = sg.Grid.createModLinearGrid if basis == "modlinear" else sg.Grid.createLinearGrid
+    grid = make(dim)
+    grid.getGenerator().regular(level)
+    rng = np.random.default_rng(seed)
+    for _ in range(rounds):
+        alpha = rng.standard_normal(grid.getSize())
+        grid.getGenerator().refine(sg.SurplusRefinementFunctor(alpha, 7, 0.0))
+    return grid
+
+
+def _points(rng, m, dim, level):
+    """Interior points, dyadic points of the finest cells, faces and corners of the cube."""
+    x = rng.random((m, dim))
+    x[1::5] = np.round(x[1::5] * 2 ** level) / 2 ** level
+    x[2::7, 0] = 0.0
+    x[3::7, dim - 1] = 1.0
+    x[4::11, 0] = 2.0 ** -60
+    return x
+
+
+def _dense(grid, x, alpha, v):
+    """(B alpha, B^T v) in FP64, every grid point for every data point, and the norms' scale."""
+    st = grid.getStorage()
+    lev, idx = st.level.astype(np.float64), st.index.astype(np.float64)
+    mod = grid.getType() == sg.GridType.ModLinear
+    b = np.ones((x.shape[0], grid.getSize()))
+    for t in range(x.shape[1]):
+        L, i, xt = 2.0 ** lev[:, t], idx[:, t], x[:, t][:, None]
+        h = 1.0 - np.abs(L * xt - i)
+        if mod:
+            h = np.where(i == 1, 2.0 - L * xt, h)
+            h = np.where(i == L - 1, L * xt - i + 1.0, h)
+            h = np.where(L == 2, 1.0, h)
+        b *= np.maximum(h, 0.0)
+    return b @ alpha, b.T @ v, np.abs(b) @ np.abs(alpha), np.abs(b).T @ np.abs(v)
+
+
+# regular grids from one dimension to many, level 1 (one subspace) to subspaces of 512 cells,
+# grids with holes and levels of their own per dimension (refined), more subspaces than a chunk
+GRIDS = [(1, 1, 0), (1, 10, 0), (2, 1, 0), (2, 9, 0), (3, 6, 0), (4, 4, 9), (5, 6, 0), (6, 3, 25),
+         (9, 4, 3), (12, 3, 0), (17, 2, 2), (30, 2, 0)]
+
+
+@pytest.mark.parametrize("basis", ["linear", "modlinear"])
+@pytest.mark.parametrize("dim,level,rounds", GRIDS)
+def test_programs_on_the_host_match_the_dense_form(lib, dim, level, rounds, basis):
+    grid = _grid(dim, level, basis, rounds)
+    lp, ix = grid.getStorage().getLevelIndexArraysForEval()
+    rng = np.random.default_rng(dim * 10 + level)
+    m, n = 48, grid.getSize()
+    x = np.ascontiguousarray(_points(rng, m, dim, level + 1))
+    alpha, v = rng.standard_normal(n), rng.standard_normal(m)
+    out, outt = np.full(m, np.nan), np.full(n, np.nan)
+    rc = lib.sgmev_nest_host(dim, n, lp.ctypes.data, ix.ctypes.data, int(basis == "modlinear"), m,
+                             x.ctypes.data, alpha.ctypes.data, v.ctypes.data, out.ctypes.data,
+                             outt.ctypes.data)
+    assert rc == 0
+    ref, reft, mag, magt = _dense(grid, x, alpha, v)
+    # per product 3 roundings a dimension on either side, per sum one an addend
+    tol = (6 * dim + n + m) * EPS
+    assert np.all(np.abs(out - ref) <= tol * (mag + 2.0 ** dim))
+    assert np.all(np.abs(outt - reft) <= tol * (magt + 2.0 ** dim))
+
+
+def test_grids_without_their_ancestors(lib):
+    """Level vectors whose parents are missing (a storage need not be closed), shuffled points."""
+    level = np.array([[3, 1, 2], [1, 1, 1], [2, 4, 1], [3, 1, 2], [1, 3, 3]], np.int32)
+    index = np.array([[5, 1, 3], [1, 1, 1], [1, 9, 1], [1, 1, 1], [1, 7, 5]], np.int32)
+    grid = sg.Grid.fromArrays(level, index)
+    lp, ix = grid.getStorage().getLevelIndexArraysForEval()
+    rng = np.random.default_rng(5)
+    x = np.ascontiguousarray(_points(rng, 60, 3, 4))
+    alpha, v = rng.standard_normal(5), rng.standard_normal(60)
+    out, outt = np.zeros(60), np.zeros(5)
+    assert lib.sgmev_nest_host(3, 5, lp.ctypes.data, ix.ctypes.data, 0, 60, x.ctypes.data,
+                               alpha.ctypes.data, v.ctypes.data, out.ctypes.data,
+                               outt.ctypes.data) == 0
+    ref, reft, _, _ = _dense(grid, x, alpha, v)
+    np.testing.assert_allclose(out, ref, atol=100 * EPS)
+    np.testing.assert_allclose(outt, reft, atol=100 * EPS)
+
+
+def test_grids_the_plan_does_not_take(lib):
+    """Subspaces of more than 512 cells stay on the dense kernels."""
+    level, index = np.array([[11]], np.int32), np.array([[3]], np.int32)
+    lp, ix = sg.Grid.fromArrays(level, index).getStorage().getLevelIndexArraysForEval()
+    x, one = np.array([[0.5]]), np.ones(1)
+    assert lib.sgmev_nest_host(1, 1, lp.ctypes.data, ix.ctypes.data, 0, 1, x.ctypes.data,
+                               one.ctypes.data, one.ctypes.data, np.zeros(1).ctypes.data,
+                               np.zeros(1).ctypes.data) == 1
+
+
+# ---- GPU -------------------------------------------------------------------------------------------
+def _op(grid, x, algo, precision="double"):
+    cfg = sg.OperationMultipleEvalConfiguration(
+        sg.OperationMultipleEvalType.STREAMING, sg.OperationMultipleEvalSubType.CUDA,
+        parameters={"precision": precision, "algo": algo})
+    return sg.createOperationMultipleEval(grid, x, cfg)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("basis", ["linear", "modlinear"])
+@pytest.mark.parametrize("m", [1, 63, 64, 65, 1025, 40000])
+@pytest.mark.parametrize("dim,level,rounds", [(1, 1, 0), (1, 10, 0), (3, 6, 0), (5, 5, 0),
+                                              (6, 3, 25), (9, 4, 3), (17, 2, 2)])
+def test_fp64_products_match_the_dense_kernels(dim, level, rounds, m, basis):
+    grid = _grid(dim, level, basis, rounds)
+    n = grid.getSize()
+    rng = np.random.default_rng(m + dim)
+    x = _points(rng, m, dim, level + 1)
+    alpha, v = rng.standard_normal(n), rng.standard_normal(m)
+    op, ref = _op(grid, x, "auto"), _op(grid, x, "dense")
+    op.profile(True)
+    out, outr, outt, outtr = np.zeros(m), np.zeros(m), np.zeros(n), np.zeros(n)
+    op.mult(alpha, out)
+    op.multTranspose(v, outt)
+    assert op.profileRead(sg.SGMEV_KERNEL_MULT_NEST64)[0] == 1
+    assert op.profileRead(sg.SGMEV_KERNEL_MULTT_NEST64)[0] == 1
+    ref.mult(alpha, outr)
+    ref.multTranspose(v, outtr)
+    # 3 roundings a dimension in each product on either side, one an addend in each sum; the
+    # magnitudes are those of sums of |alpha| (or |v|) over hats, at most 2^dim for ModLinear ramps
+    big = 1.0 if basis == "linear" else 2.0 ** min(dim, level)
+    assert np.abs(out - outr).max() <= (6 * dim + n) * EPS * big * np.abs(alpha).sum()
+    assert np.abs(outt - outtr).max() <= (6 * dim + m) * EPS * big * np.abs(v).sum()
+    # a range gives the bits of the full product, and a second product the same bits
+    lo, hi = m // 3, m - m // 4
+    part = np.full(m, -7.0)
+    op.mult(alpha, part, lo, hi)
+    np.testing.assert_array_equal(part[lo:hi], out[lo:hi])
+    assert np.all(part[:lo] == -7.0) and np.all(part[hi:] == -7.0)
+    again = np.zeros(n)
+    op.multTranspose(v, again)
+    np.testing.assert_array_equal(again, outt)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+def test_values_that_are_not_finite_spread_as_in_the_dense_kernels(value):
+    grid = _grid(4, 4)
+    n, m = grid.getSize(), 500
+    rng = np.random.default_rng(3)
+    x = _points(rng, m, 4, 3)
+    x[7, 2] = np.nan
+    x[9, 1] = -0.5
+    for single in (True, False):
+        alpha, v = rng.standard_normal(n), rng.standard_normal(m)
+        alpha[0 if single else 5] = value
+        v[11 if single else 9] = value
+        got, want = [], []
+        for algo, into in (("auto", got), ("dense", want)):
+            op = _op(grid, x, algo)
+            a, b = np.zeros(m), np.zeros(n)
+            op.mult(alpha, a)
+            op.multTranspose(v, b)
+            into += [a, b]
+        for a, b in zip(got, want):
+            np.testing.assert_array_equal(np.isnan(a), np.isnan(b))
+            np.testing.assert_array_equal(np.isinf(a), np.isinf(b))
