@@ -48,6 +48,8 @@ SGMEV_API int sgmev_fma_peak(int precision, double* flops_per_second, int* sm_cl
 #define SGMEV_KERNEL_BLOCK_MULTT 18 /* B^T [v_1 .. v_16], BF16 tensor-core tiles */
 #define SGMEV_KERNEL_MULT_NEST64 19  /* FP64 mult, nested subspace products */
 #define SGMEV_KERNEL_MULTT_NEST64 20 /* FP64 multTranspose, nested subspace products */
+#define SGMEV_KERNEL_MULT_NEST32 21  /* FP32 mult, nested subspace products */
+#define SGMEV_KERNEL_MULT_NESTDF 22  /* df64 mult, nested subspace products */
 SGMEV_API int sgmev_profile(sgmev_op* op, int enable);
 SGMEV_API int sgmev_profile_read(sgmev_op* op, int kind, int64_t* launches, double* seconds);
 

@@ -90,6 +90,8 @@ SGMEV_KERNEL_BLOCK_MULT = 17
 SGMEV_KERNEL_BLOCK_MULTT = 18
 SGMEV_KERNEL_MULT_NEST64 = 19
 SGMEV_KERNEL_MULTT_NEST64 = 20
+SGMEV_KERNEL_MULT_NEST32 = 21
+SGMEV_KERNEL_MULT_NESTDF = 22
 SGMEV_BLOCK_RHS = 16
 
 

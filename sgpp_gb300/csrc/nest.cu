@@ -1,30 +1,37 @@
-// Nested subspace products in FP64.
+// Nested subspace products.
 //
-// The dense kernels evaluate every grid point's basis function for every data point: 3 d FP64
-// instructions per pair, and GB300's FP64 rate is 1/62 of FP32's. Exactly one function per
-// subspace can be non-zero at a point (the reference's DEFAULT operator evaluates only those,
-// base/src/sgpp/base/algorithm/AlgorithmEvaluation.hpp:129-179), and the functions of subspaces
-// that share active dimensions share factors. So the subspaces form a tree (nest.h), a point's
-// one-dimensional factors are tabulated once per data set, and
+// The dense kernels evaluate every grid point's basis function for every data point (in FP64 3 d
+// instructions per pair, at 1/62 of FP32's rate); the materialised ones stream a product per subspace
+// and point from HBM. Exactly one function per subspace can be non-zero at a point (the reference's
+// DEFAULT operator evaluates only those, base/src/sgpp/base/algorithm/AlgorithmEvaluation.hpp:129-179),
+// and the functions of subspaces that share active dimensions share factors. So the subspaces form a
+// tree (nest_plan.h), a point's one-dimensional factors are tabulated once per data set, and
 //   mult   nests the sum: result = H_1 sum over the tree, each node costing one multiply-add,
 //              sum_r P_r sum_{q below r} T_q (a_q + sum_{leaf c below q} T_c a_c)
 //          with groups r (their product P_r is formed once), inner nodes q (children of r that have
-//          children) and the leaves below q;
+//          children) and the leaves below q; whole subtrees of up to three more levels, which is most
+//          of a regular grid, run as unrolled code on registers;
 //   multT  forms v_j P_q for the inner nodes of a tile of points in shared memory and then, one
 //          thread per subspace, adds (v_j P_q) T into the thread's own cells: one multiply-add per
 //          subspace and point, in a fixed order.
-// Bound: the FP64 pipe (2 lanes per clock and SM), at about 1.3 instructions per subspace and
-// point against 3 d per grid point and point of the dense kernels. d=5 level 6 (5,503 points, 252
-// subspaces), 65,536 data points: mult 10,791 -> 43 us, multTranspose 10,895 -> 60 us; B^T(B a) on an
-// adaptive d=8 grid (4,024 points), 2^19 data points: 199.1 -> 1.46 ms. The error against 64-bit
-// sums is that of the dense kernels (mult 6.0e-16 against 5.9e-16, multTranspose 4.0e-16 against
-// 5.6e-16 of the result's norm).
+// Bound: FP64 the FP64 pipe (2 lanes per clock and SM), at about 1.3 instructions per subspace and
+// point; FP32 and float-float instruction issue (7 instructions per subspace and point in FP32, 28 in
+// float-float, at 0.55 of the issue rate with the 12 to 14 warps per SM that the tables leave room
+// for). Measured before and after:
+//   FP64, d=5 level 6 (252 subspaces), 65,536 points: mult 10,791 -> 36 us, multT 10,895 -> 60 us
+//   FP64, adaptive d=8 grid (4,024 points), 2^19 data points: B^T (B a) 199.1 -> 1.22 ms
+//   FP32, d=10 level 5 (1,001 subspaces), 262,147 points: mult 168 -> 92 us (materialised before)
+//   float-float, d=9 level 6 (2,002 subspaces), 40,961 points: mult 583 -> 109 us (hats on the fly)
+// The errors against 64-bit results, relative to their norm: FP64 mult 6.1e-16 before and after,
+// multT 6.2e-16 -> 4.4e-16; FP32 mult 1.2e-7 before and after; float-float 1.5e-13 -> 8e-15.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <utility>
 
+#include "../../include/sgmev.h"
 #include "devmem.h"
 #include "kernels.cuh"
 #include "nest.h"
@@ -33,20 +40,27 @@
 namespace sgmev {
 namespace {
 
-constexpr int kMultThreads = kNestMultThreads, kTile = kNestTile;
-constexpr int kBadBlocks = 32;  // blocks of the coefficient gather
-
+constexpr int kTile = kNestTile;
 // ---- tables -----------------------------------------------------------------------------------
 // One thread per data point. The hats of a dimension follow one another by the tent map,
 // h_{l+1} = 2 min(h_l, 1 - h_l), which is exact in floating point (the smaller side is h_l itself or
 // an exact difference by Sterbenz's lemma), from h_1 = 2 min(x, 1 - x). A point outside (0, 1)^d
 // (or closer to a face than 2^-1000) has H_1 = 0 and the table of the cube's centre.
-template <bool MOD>
+template <bool MOD, bool F64, bool F32>
 __global__ void nest_table_kernel(const double* __restrict__ xt, int64_t mpad, int64_t m, int dim,
-                                  const int* __restrict__ lmax, double* __restrict__ tab,
+                                  const int* __restrict__ lmax, double* __restrict__ tab64,
+                                  float* __restrict__ tab_hi, float* __restrict__ tab_lo,
                                   uint32_t* __restrict__ xcell) {
   const int64_t j = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (j >= mpad) return;
+  auto put = [&](int e, double v) {
+    if constexpr (F64) tab64[e * mpad + j] = v;
+    if constexpr (F32) {
+      const float hi = static_cast<float>(v);
+      tab_hi[e * mpad + j] = hi;
+      tab_lo[e * mpad + j] = static_cast<float>(v - static_cast<double>(hi));
+    }
+  };
   bool inside = j < m;
   for (int t = 0; t < dim; ++t) {
     const double x = xt[t * mpad + j];
@@ -68,7 +82,7 @@ __global__ void nest_table_kernel(const double* __restrict__ xt, int64_t mpad, i
         if (k == 0u) h = 2.0 - y;
         else if (k == top) h = y - (L - 2.0);
         else h = 1.0 - fabs(y - static_cast<double>(2u * k + 1u));
-        tab[e * mpad + j] = h;
+        put(e, h);
       }
     } else {
       double h = 2.0 * (x > 0.5 ? 1.0 - x : x);
@@ -76,27 +90,87 @@ __global__ void nest_table_kernel(const double* __restrict__ xt, int64_t mpad, i
       const double r = 1.0 / h;
       for (int l = 2; l <= bits + 1; ++l, ++e) {
         h = 2.0 * (h > 0.5 ? 1.0 - h : h);
-        tab[e * mpad + j] = h * r;
+        put(e, h * r);
       }
     }
   }
-  tab[j] = h1p;
+  put(0, h1p);
 }
 
 // ---- mult ----------------------------------------------------------------------------------------
-// coefficients into position order; bad[block] = a coefficient that is not finite was seen
+// The three arithmetics. A value of the float-float one is (h, l) as in kernels.cuh.
+__device__ __forceinline__ void set_val(float& r, double v) { r = static_cast<float>(v); }
+__device__ __forceinline__ void set_val(double& r, double v) { r = v; }
+__device__ __forceinline__ void set_val(ff& r, double v) {
+  r.h = static_cast<float>(v);
+  r.l = static_cast<float>(v - static_cast<double>(r.h));
+}
+// s += t * a
+__device__ __forceinline__ void mac(float& s, float t, float a) { s = fmaf(t, a, s); }
+__device__ __forceinline__ void mac(double& s, double t, double a) { s = fma(t, a, s); }
+__device__ __forceinline__ void mac(ff& s, ff t, ff a) { add_ff(s, mul_ff(t, a)); }
+template <typename V, int R>
+__device__ __forceinline__ void mac_all(V (&s)[R], const V (&t)[R], const V (&a)[R]) {
+#pragma unroll
+  for (int r = 0; r < R; ++r) mac(s[r], t[r], a[r]);
+}
+// two FP32 multiply-adds in one instruction
+__device__ __forceinline__ void mac_all(float (&s)[2], const float (&t)[2], const float (&a)[2]) {
+  asm("{\n\t.reg .b64 vs, vt, va;\n\tmov.b64 vs, {%0, %1};\n\tmov.b64 vt, {%2, %3};\n\tmov.b64 va, {%4, %5};\n\t"
+      "fma.rn.f32x2 vs, vt, va, vs;\n\tmov.b64 {%0, %1}, vs;\n\t}"
+      : "+f"(s[0]), "+f"(s[1]) : "f"(t[0]), "f"(t[1]), "f"(a[0]), "f"(a[1]));
+}
+__device__ __forceinline__ float mul(float a, float b) { return a * b; }
+__device__ __forceinline__ double mul(double a, double b) { return a * b; }
+__device__ __forceinline__ ff mul(ff a, ff b) {
+  ff r = mul_ff(a, b);
+  renorm_ff(r);
+  return r;
+}
+// a finished sum, before it becomes a factor (mul_ff drops the product of the low parts)
+__device__ __forceinline__ void settle(float&) {}
+__device__ __forceinline__ void settle(double&) {}
+__device__ __forceinline__ void settle(ff& s) { renorm_ff(s); }
+__device__ __forceinline__ double to_double(float v) { return static_cast<double>(v); }
+__device__ __forceinline__ double to_double(double v) { return v; }
+__device__ __forceinline__ double to_double(ff v) {
+  return static_cast<double>(v.h) + static_cast<double>(v.l);
+}
+// asynchronous copies into shared memory: `bytes` (4 or 8) of a thread's own column
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                   static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src), "n"(BYTES) : "memory");
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+template <typename V>
+__device__ __forceinline__ void prefetch_entry(const float* hi, const float* lo, const double* d, int64_t k) {
+  if constexpr (std::is_same<V, double>::value) {
+    prefetch_l2(d + k);
+  } else {
+    prefetch_l2(hi + k);
+    if constexpr (sizeof(V) == 8) prefetch_l2(lo + k);
+  }
+}
+// table entries of R adjacent points (k: the first one's index)
+__device__ __forceinline__ void load_entry(float (&r)[2], const float* hi, const float*, const double*, int64_t k) { copy_async<8>(r, hi + k); }
+__device__ __forceinline__ void load_entry(double (&r)[1], const float*, const float*, const double* d, int64_t k) { copy_async<8>(r, d + k); }
+__device__ __forceinline__ void load_entry(ff (&r)[1], const float* hi, const float* lo, const double*, int64_t k) {
+  copy_async<4>(&r[0].h, hi + k);
+  copy_async<4>(&r[0].l, lo + k);
+}
+
+// coefficients into position order (launches that stage them more than once)
+template <typename V>
 __global__ void nest_coef_kernel(const double* __restrict__ alpha, const int* __restrict__ inv,
-                                 int64_t total, double* __restrict__ coef, int* __restrict__ bad) {
-  bool b = false;
+                                 int64_t total, V* __restrict__ coef) {
   for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < total;
        p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int g = inv[p];
-    const double a = g >= 0 ? alpha[g] : 0.0;
-    coef[p] = a;
-    b = b || !isfinite(a);
+    set_val(coef[p], g >= 0 ? alpha[g] : 0.0);
   }
-  const int any = __syncthreads_or(b);
-  if (threadIdx.x == 0) bad[blockIdx.x] = any;
 }
 
 // the dense value of grid point g's function at point j (0 exactly outside its support)
@@ -119,57 +193,297 @@ __device__ __noinline__ double mult_poison(const NestDense& d, int dim, int64_t 
   return r;
 }
 
-// One thread per data point; its table row and cells in shared memory ([entry][thread], private to
-// the thread). The program is the same for all threads, so its loads are broadcasts; the
-// coefficients are gathered through L1 (a subspace's cells are contiguous). blockIdx.y takes the
-// groups [cuts[y], cuts[y + 1]) and writes its own row of `out`.
-template <bool MOD>
-__global__ void __launch_bounds__(kMultThreads) nest_mult64_kernel(
-    const NestOp4* __restrict__ rops, const int* __restrict__ facs, const NestOp4* __restrict__ qops,
-    const NestOp2* __restrict__ lops, const int* __restrict__ cuts, const double* __restrict__ coef,
-    const double* __restrict__ tab, const uint32_t* __restrict__ xcell, int n_ent, int dim,
-    int64_t m, int64_t j_begin, int64_t out_stride, double* __restrict__ out,
-    const int* __restrict__ bad, NestDense dense, const double* __restrict__ alpha, int64_t n) {
+// R adjacent data points per thread (two in FP32, one in the wider arithmetics), a warp at a time over
+// a contiguous range of 32 R-point tiles; the points' table rows and cells in shared memory
+// ([entry][thread][R], private to the thread, copied asynchronously), their level-2 and level-3
+// factors and cells in registers for the runs and trees (MD = dim, or 0 for more dimensions than
+// kNestMacroDim: then the plan has none). A window's coefficients and program are staged in shared
+// memory: a warp's 32 gathers from one row hit different banks or the same word, and the program's
+// loads are broadcasts (read through L1 they missed half the time beside this much shared memory,
+// and the FP32 kernel took 203 us instead of 128). blockIdx.y takes windows
+// [y windows / splits, (y + 1) windows / splits) of the list and, with several splits, writes its own
+// row of partial sums.
+template <typename V>
+constexpr int kPts = sizeof(V) == 4 ? 2 : 1;
+constexpr int kMultMaxThreads = 448;
+
+struct NestMultArgs {
+  const NestOp4 *windows, *prog;
+  int n_windows, words;  // windows of the list, words of the longest program
+  int n_ent, dim;
+  int entry[32], lmax[32];  // first table entry (level 2) and finest level of each dimension
+  const float *tab_hi, *tab_lo;
+  const double* tab64;
+  const uint32_t* xcell;
+  int64_t m, j_begin, n_tiles;
+  float* out32;
+  double* out64;
+  void* part;
+  int64_t out_end;  // outputs are written for j < out_end, zero beyond m
+  NestDense dense;
+  const int* inv;
+  const double* alpha;
+  int64_t n;
+  const void* coef;  // coefficients in position order, or nullptr: gathered while they are staged
+  int warps;         // warps of a CTA that take tiles; the others only help to stage
+};
+
+template <typename V, int MD, bool MOD>
+__global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
+    nest_mult_kernel(const __grid_constant__ NestMultArgs a) {
+  constexpr int D = MD > 0 ? MD : 1, kV = sizeof(V), R = kPts<V>;
   extern __shared__ __align__(16) unsigned char smem[];
-  const int tid = threadIdx.x;
-  const int64_t mpad = dense.mpad;
-  const int64_t j = j_begin + static_cast<int64_t>(blockIdx.x) * kMultThreads + tid;
-  double* s_tab = reinterpret_cast<double*>(smem) + tid;
-  uint32_t* s_x = reinterpret_cast<uint32_t*>(smem + sizeof(double) * n_ent * kMultThreads) + tid;
-#pragma unroll 8
-  for (int e = 0; e < n_ent; ++e) s_tab[e * kMultThreads] = tab[e * mpad + j];
+  const int tid = threadIdx.x, all = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = a.warps;
+  const int nth = 32 * nw;
+  const int64_t mpad = a.dense.mpad;
+  using Col = V[R];
+  using ColX = uint32_t[R];
+  NestOp4* s_prog = reinterpret_cast<NestOp4*>(smem);
+  Col* s_tab = reinterpret_cast<Col*>(s_prog + a.words) + tid;
+  ColX* s_x = reinterpret_cast<ColX*>(s_tab - tid + a.n_ent * nth) + tid;
+  V* s_coef = reinterpret_cast<V*>(s_x - tid + a.dim * nth);
+  const int w_begin = blockIdx.y * a.n_windows / gridDim.y;
+  const int w_end = (blockIdx.y + 1) * a.n_windows / gridDim.y;
+  bool poison = false;  // FP64: a coefficient that is not finite (the same in every thread)
+  auto stage = [&](const NestOp4& w) {
+    for (int k = w.x + tid; k < w.y; k += all) s_prog[k - w.x] = a.prog[k];
+    bool finite = true;
+    if (a.coef) {
 #pragma unroll 4
-  for (int t = 0; t < dim; ++t) s_x[t * kMultThreads] = xcell[t * mpad + j];
-  double acc = 0.0;
-  const int r_end = cuts[blockIdx.y + 1];
-  for (int r = cuts[blockIdx.y]; r < r_end; ++r) {
-    const NestOp4 ro = rops[r];
-    double pr = 1.0;
-    uint32_t cr = 0;
-    for (int i = ro.z; i < ro.w; ++i) {
-      const int f = facs[i];
-      pr *= s_tab[fac_e(f) * kMultThreads];
-      cr = (cr << fac_k(f)) | (s_x[fac_t(f) * kMultThreads] >> fac_shift(f));
-    }
-    double ar = 0.0;
-    for (int q = ro.x; q < ro.y; ++q) {
-      const NestOp4 qo = qops[q];
-      const uint32_t c = (cr << fac_k(qo.w)) | (s_x[fac_t(qo.w) * kMultThreads] >> fac_shift(qo.w));
-      double sum = qo.x >= 0 ? __ldg(coef + qo.x + c) : 0.0;
-#pragma unroll 4
-      for (int i = qo.y; i < qo.z; ++i) {
-        const NestOp2 lo = lops[i];
-        const uint32_t cl =
-            (c << fac_k(lo.y)) | (s_x[fac_t(lo.y) * kMultThreads] >> fac_shift(lo.y));
-        sum = fma(s_tab[fac_e(lo.y) * kMultThreads], __ldg(coef + lo.x + cl), sum);
+      for (int k = w.z + tid; k < w.w; k += all) {
+        const V v = static_cast<const V*>(a.coef)[k];
+        finite = finite && isfinite(to_double(v));
+        s_coef[k - w.z] = v;
       }
-      ar = fma(s_tab[fac_e(qo.w) * kMultThreads], sum, ar);
+    } else {
+#pragma unroll 4
+      for (int k = w.z + tid; k < w.w; k += all) {
+        const int g = a.inv[k];
+        const double v = g >= 0 ? a.alpha[g] : 0.0;
+        finite = finite && isfinite(v);
+        set_val(s_coef[k - w.z], v);
+      }
     }
-    acc = fma(pr, ar, acc);
+    if constexpr (std::is_same<V, double>::value) poison = __syncthreads_or(!finite) || poison;
+    else __syncthreads();
+  };
+  // the warps' tile ranges are contiguous and as equal as can be; every warp of the CTA runs the same
+  // number of rounds (the barriers of several windows), some of them on no tile
+  const int64_t warps = static_cast<int64_t>(gridDim.x) * nw, gw = static_cast<int64_t>(blockIdx.x) * nw + warp;
+  const int64_t t_begin = warp < nw ? gw * a.n_tiles / warps : 0;
+  const int64_t t_end = warp < nw ? (gw + 1) * a.n_tiles / warps : 0;
+  const int64_t rounds = (a.n_tiles + warps - 1) / warps;
+  const bool one = w_end - w_begin == 1;
+  if (one) stage(a.windows[w_begin]);
+  for (int64_t round = 0; round < rounds; ++round) {
+    const bool live = t_begin + round < t_end;
+    if (one && !live) break;
+    const int64_t j = a.j_begin + ((t_begin + round) * 32 + lane) * R;
+    V T2[D][R], T3[D][R];
+    uint32_t B2[D][R], B3[D][R];  // byte offsets of the points' cells of levels 2 and 3
+    if (live) {
+#pragma unroll 4
+      for (int t = 0; t < a.dim; ++t) copy_async<4 * R>(s_x[t * nth], a.xcell + t * mpad + j);
+#pragma unroll 4
+      for (int e = 0; e < a.n_ent; ++e)
+        load_entry(s_tab[e * nth], a.tab_hi, a.tab_lo, a.tab64, e * mpad + j);
+      // the warp's next tile into L2: it streams from HBM otherwise, a full latency per tile
+      if (t_begin + round + 1 < t_end && (lane & 15) == 0) {
+        const int64_t jn = j + 32 * R;
+        for (int e = 0; e < a.n_ent; ++e) prefetch_entry<V>(a.tab_hi, a.tab_lo, a.tab64, e * mpad + jn);
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      if constexpr (MD > 0) {
+#pragma unroll
+        for (int t = 0; t < MD; ++t) {
+          const int bits = a.lmax[t] - 1;
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const uint32_t x = s_x[t * nth][r];
+            T2[t][r] = bits >= 1 ? s_tab[a.entry[t] * nth][r] : V{};
+            B2[t][r] = bits >= 1 ? (x >> (bits - 1)) * kV : 0u;
+            T3[t][r] = bits >= 2 ? s_tab[(a.entry[t] + 1) * nth][r] : V{};
+            B3[t][r] = bits >= 2 ? (x >> (bits - 2)) * kV : 0u;
+          }
+        }
+      }
+    }
+    V acc[R] = {};
+    for (int w = w_begin; w < w_end; ++w) {
+      const NestOp4 win = a.windows[w];
+      if (!one) {
+        __syncthreads();  // the previous window is no longer read
+        stage(win);
+      }
+      if (!live) continue;
+      const NestOp4* op = s_prog;
+      const NestOp4* const op_end = op + (win.y - win.x);
+      while (op < op_end) {
+        const NestOp4 head = *op++;
+        V pr[R], ar[R] = {};
+        uint32_t cr[R] = {};
+#pragma unroll
+        for (int r = 0; r < R; ++r) set_val(pr[r], 1.0);
+        const int* facs = reinterpret_cast<const int*>(op);
+        for (int i = 0; i < head.y; ++i) {
+          const int f = facs[i];
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            pr[r] = mul(pr[r], s_tab[fac_e(f) * nth][r]);
+            cr[r] = (cr[r] << fac_k(f)) | (s_x[fac_t(f) * nth][r] >> fac_shift(f));
+          }
+        }
+        op += (head.y + 3) / 4;
+        for (int q = 0; q < head.x; ++q) {
+          const NestOp4 qo = op[0], qf = op[1];
+          op += 2;
+          uint32_t c[R];
+          V tq[R], sum[R] = {};
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            tq[r] = s_tab[qf.x * nth][r];
+            c[r] = (cr[r] << qf.z) | (s_x[qf.y * nth][r] >> qf.w);
+          }
+          if (MD == 0 || qo.y >= 0) {
+            if (qo.x >= 0) {
+#pragma unroll
+              for (int r = 0; r < R; ++r) sum[r] = s_coef[qo.x + c[r]];
+            }
+            const NestOp4* const leaf_end = op + qo.y;
+#pragma unroll 2
+            for (; op < leaf_end; ++op) {
+              const NestOp4 lo = *op;
+              const int e = lo.y & 0xFFFF, t = lo.y >> 16;
+#pragma unroll
+              for (int r = 0; r < R; ++r)
+                mac(sum[r], s_tab[e * nth][r],
+                    s_coef[lo.x + ((c[r] << lo.z) | (s_x[t * nth][r] >> lo.w))]);
+            }
+          } else if constexpr (MD > 0) {
+            const int kind = -qo.y - 1, t0 = kind >> 2;
+            auto ld = [](const char* p) { return *reinterpret_cast<const V*>(p); };
+            // the value of a run and of a tree whose dimensions begin at t1, from their rows
+            auto run = [&](const char* (&row)[R], int t1, V (&sr)[R]) {
+#pragma unroll
+              for (int r = 0; r < R; ++r) sr[r] = ld(row[r]);
+#pragma unroll
+              for (int t = MD - 1; t >= 0; --t) {
+                if (t < t1) break;
+                V v[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) v[r] = ld(row[r] + B2[t][r] + kV * (1 + 2 * (MD - 1 - t)));
+                mac_all(sr, T2[t], v);
+              }
+            };
+            auto tree = [&](const char* (&row)[R], int t1, V (&st)[R]) {
+#pragma unroll
+              for (int r = 0; r < R; ++r) st[r] = ld(row[r]);
+#pragma unroll
+              for (int t = MD - 1; t >= 0; --t) {
+                if (t < t1) break;
+                const int kt = MD - 1 - t, sec = kV * nest_tree_at(kt);
+                V sq[R], v[R];
+                const char* rq[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                  rq[r] = row[r] + B2[t][r] * static_cast<uint32_t>(nest_run_row(kt));
+                  sq[r] = ld(rq[r] + sec);
+                  v[r] = ld(row[r] + B3[t][r] + (sec + kV * 2 * nest_run_row(kt)));
+                }
+                mac_all(st, T3[t], v);
+#pragma unroll
+                for (int u = MD - 1; u > t; --u) {
+#pragma unroll
+                  for (int r = 0; r < R; ++r) v[r] = ld(rq[r] + B2[u][r] + (sec + kV * (1 + 2 * (MD - 1 - u))));
+                  mac_all(sq, T2[u], v);
+                }
+#pragma unroll
+                for (int r = 0; r < R; ++r) settle(sq[r]);
+                mac_all(st, T2[t], sq);
+              }
+            };
+            const char* row[R];
+            if ((kind & 3) < 2) {
+#pragma unroll
+              for (int r = 0; r < R; ++r) row[r] = reinterpret_cast<const char*>(s_coef + qo.x + c[r] * qo.z);
+              if ((kind & 3) == 0) run(row, t0, sum);
+              else tree(row, t0, sum);
+            } else {
+              const V* cells = s_coef + qo.x;
+#pragma unroll
+              for (int r = 0; r < R; ++r) sum[r] = cells[c[r]];
+              cells += ((1 << qo.z) + 3) & ~3;
+              int tree_row = nest_tree_row(0), run_row = nest_run_row(0), tree_end = nest_tree_at(0);
+              for (int t = MD - 1; t >= t0; --t) {
+                const int bits = a.lmax[t] - 1;
+                const Col* te = s_tab + a.entry[t] * nth;
+                V v[R], tl[R];
+                uint32_t x[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                  x[r] = s_x[t * nth][r];
+                  row[r] = reinterpret_cast<const char*>(cells + ((c[r] << 1) | (x[r] >> (bits - 1))) * tree_row);
+                  tl[r] = te[0][r];
+                }
+                tree(row, t + 1, v);
+#pragma unroll
+                for (int r = 0; r < R; ++r) settle(v[r]);
+                mac_all(sum, tl, v);
+                cells += (2 * tree_row) << qo.z;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                  row[r] = reinterpret_cast<const char*>(cells + ((c[r] << 2) | (x[r] >> (bits - 2))) * run_row);
+                  tl[r] = te[nth][r];
+                }
+                run(row, t + 1, v);
+#pragma unroll
+                for (int r = 0; r < R; ++r) settle(v[r]);
+                mac_all(sum, tl, v);
+                cells += (4 * run_row) << qo.z;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                  v[r] = cells[(c[r] << 3) | (x[r] >> (bits - 3))];
+                  tl[r] = te[2 * nth][r];
+                }
+                mac_all(sum, tl, v);
+                cells += 8 << qo.z;
+                // the next dimension's row lengths (nest_tree_at, nest_tree_row and nest_run_row of k + 1)
+                tree_end += 2 * run_row + 4;
+                tree_row = ((tree_end + 3) & ~7) + 4;
+                const int k = MD - t;
+                run_row = 2 * k + ((k & 1) == 0 ? 2 : 4);
+              }
+            }
+          }
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            settle(sum[r]);
+            mac(ar[r], tq[r], sum[r]);
+          }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          settle(ar[r]);
+          mac(acc[r], pr[r], ar[r]);
+        }
+      }
+    }
+    if (!live) continue;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int64_t k = j + r;
+      const bool real = k < a.m;
+      if constexpr (std::is_same<V, double>::value) {
+        if (poison && real) acc[r] += mult_poison<MOD>(a.dense, a.dim, a.n, a.alpha, k);
+      }
+      if (gridDim.y > 1) {
+        reinterpret_cast<V*>(a.part)[blockIdx.y * mpad + k] = acc[r];
+      } else {
+        if (a.out32 && k < a.out_end) a.out32[k] = real ? static_cast<float>(to_double(acc[r])) : 0.0f;
+        if (a.out64 && k < a.out_end) a.out64[k] = real ? to_double(acc[r]) : 0.0;
+      }
+    }
   }
-  if (blockIdx.y == 0 && __syncthreads_or(tid < kBadBlocks && bad[tid] != 0) && j < m)
-    acc += mult_poison<MOD>(dense, dim, n, alpha, j);
-  out[blockIdx.y * out_stride + j] = j < m ? acc : 0.0;
 }
 
 // ---- multTranspose -----------------------------------------------------------------------------
@@ -292,10 +606,17 @@ bool nest_build(NestPlan* p, int dim, int64_t n, const double* level_pow2, const
   p->mod = mod;
   p->n_sub = h.n_sub;
   p->n_ent = h.n_ent;
-  p->n_r = static_cast<int>(h.rops.size());
+  p->lists = h.list_begin;
+  p->list_cells = h.list_cells;
+  p->list_words = h.list_words;
+  for (int t = 0, e = 1; t < dim; ++t) {
+    p->h_entry[t] = e;
+    p->h_lmax[t] = h.lmax[t];
+    e += h.lmax[t] - 1;
+  }
   p->total = static_cast<int64_t>(h.inv.size());
   p->classes = h.classes;
-  int flags = std::max(kBadBlocks, 4 * num_sms);
+  int flags = 4 * num_sms;
   for (const NestClass& c : h.classes) flags = std::max(flags, c.chunks);
   // one allocation and one copy for the whole plan: the operator may live for a single product
   std::vector<unsigned char> host;
@@ -307,11 +628,8 @@ bool nest_build(NestPlan* p, int dim, int64_t n, const double* level_pow2, const
     at.emplace_back(reinterpret_cast<void**>(dst), o);
   };
   put(&p->lmax, h.lmax);
-  put(&p->rops, h.rops);
-  put(&p->facs, h.facs);
-  put(&p->qops, h.qops);
-  put(&p->lops, h.lops);
-  put(&p->cuts, h.cuts);
+  put(&p->windows, h.windows);
+  put(&p->prog, h.prog);
   put(&p->inv, h.inv);
   put(&p->chunks, h.chunks);
   put(&p->cq, h.cq);
@@ -330,71 +648,205 @@ bool nest_build(NestPlan* p, int dim, int64_t n, const double* level_pow2, const
     return false;
   }
   for (const auto& k : at) *k.first = p->block + k.second;
-  p->coef = reinterpret_cast<double*>(p->block + o_coef);
+  p->coef = p->block + o_coef;
   p->bad = reinterpret_cast<int*>(p->block + o_bad);
   p->ok = true;
   return true;
 }
 
 void nest_free(NestPlan* p) {
-  void* ptrs[] = {p->block, p->rows, p->tab64, p->xcell};
+  void* ptrs[] = {p->block, p->rows, p->tab64, p->tab_hi, p->xcell};
   for (void* q : ptrs) dev_free(q, p->stream);
   *p = NestPlan{};
 }
 
 namespace {
-cudaError_t tables(NestPlan& p, cudaStream_t s, const NestDense& d, int64_t m, int* launches) {
-  if (p.tab64) return cudaSuccess;
+// the tables that the precision reads, built on its first product
+cudaError_t tables(NestPlan& p, cudaStream_t s, const NestDense& d, int64_t m, bool f64,
+                   int* launches) {
+  if (f64 ? p.tab64 != nullptr : p.tab_hi != nullptr) return cudaSuccess;
   cudaError_t e = cudaSuccess;
   if (!p.xcell) e = dev_malloc(&p.xcell, sizeof(uint32_t) * p.dim * d.mpad, s);
-  if (e == cudaSuccess) e = dev_malloc(&p.tab64, sizeof(double) * p.n_ent * d.mpad, s);
+  if (e != cudaSuccess) return e;
+  const int64_t n = p.n_ent * d.mpad;
+  if (f64) e = dev_malloc(&p.tab64, sizeof(double) * n, s);
+  else e = dev_malloc(&p.tab_hi, 2 * sizeof(float) * n, s);
   if (e != cudaSuccess) return e;
   const unsigned blocks = static_cast<unsigned>((d.mpad + 127) / 128);
-  auto kern = p.mod ? nest_table_kernel<true> : nest_table_kernel<false>;
-  kern<<<blocks, 128, 0, s>>>(d.xt, d.mpad, m, p.dim, p.lmax, p.tab64, p.xcell);
+  auto kern = f64 ? (p.mod ? nest_table_kernel<true, true, false> : nest_table_kernel<false, true, false>)
+                  : (p.mod ? nest_table_kernel<true, false, true> : nest_table_kernel<false, false, true>);
+  kern<<<blocks, 128, 0, s>>>(d.xt, d.mpad, m, p.dim, p.lmax, p.tab64, p.tab_hi,
+                              p.tab_hi ? p.tab_hi + n : nullptr, p.xcell);
   ++*launches;
+  return cudaGetLastError();
+}
+
+// Threads per CTA, the window list and the CTAs that share a tile of points, once per operator (m
+// does not change). A CTA has as many warps as its shared memory holds table rows for (one CTA per
+// SM), or fewer when the tiles would not reach every SM. Of the lists, the one with the least cycles
+// by a model of the measured kernels: a round of a warp costs about 2,500 cycles for its table rows
+// and 75 (FP32, two points a thread), 150 (float-float) or 21 a warp of the SM (FP64, whose pipe the
+// warps share) per subspace; staging a window about 1,500 and a cycle per 40 bytes; several CTAs per
+// tile pay about 5,000 for the partial sums' pass.
+template <typename V, typename Kern>
+cudaError_t mult_config(const NestPlan& p, NestConfig* c, Kern kern, int64_t m, int64_t mpad,
+                        int64_t part_bytes, int num_sms) {
+  constexpr int64_t kV = sizeof(V), R = kPts<V>;
+  const int caps = kV == 4 ? 0 : kNestLists / 2;
+  const int64_t tiles = std::max<int64_t>(1, (m + 32 * R - 1) / (32 * R));
+  const int64_t row = 32 * R * (kV * p.n_ent + 4 * p.dim);  // table rows of a warp
+  const int64_t most = (kV == 4 ? 384 : kMultMaxThreads) / 32;
+  double best = 0.0;
+  int64_t warps = 1, window = 0;
+  for (int k = 0; k < kNestLists / 2; ++k) {
+    const int list = caps + k, n_windows = p.lists[list + 1] - p.lists[list];
+    const int64_t ctas = nest_list_ctas(list);
+    if (k > 0 && (n_windows < ctas || part_bytes < ctas * mpad * kV)) break;
+    const int64_t w = kV * p.list_cells[list] + static_cast<int64_t>(sizeof(NestOp4)) * p.list_words[list];
+    const int64_t fit = std::max<int64_t>(1, std::min<int64_t>({most, (static_cast<int64_t>(kNestMultSmem) - w) / row,
+                                                                std::max<int64_t>(2, (tiles * ctas + num_sms - 1) / num_sms)}));
+    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((tiles + fit - 1) / fit, num_sms / ctas));
+    const int64_t rounds = (tiles + blocks * fit - 1) / (blocks * fit);
+    const double per_sub = std::is_same<V, double>::value ? 21.0 * static_cast<double>(fit) : kV == 4 ? 75.0 : 150.0;
+    const double staged = 1500.0 + static_cast<double>(kV * p.list_cells[list]) / 40.0;
+    const int64_t per_cta = (n_windows + ctas - 1) / ctas;
+    const double cost = static_cast<double>(rounds) * (2500.0 + 20.0 * p.n_ent + per_sub * p.n_sub / static_cast<double>(ctas)) +
+                        static_cast<double>(per_cta > 1 ? rounds * per_cta : 1) * staged + (ctas > 1 ? 5000.0 : 0.0);
+    if (k == 0 || cost < best) {
+      best = cost;
+      c->list = list;
+      c->splits = static_cast<int>(ctas);
+      c->restage = per_cta > 1 && rounds > 1;
+      warps = fit;
+      window = w;
+    }
+  }
+  c->warps = static_cast<int>(warps);
+  c->threads = 32 * std::max(8, c->warps);
+  c->smem = static_cast<size_t>(window + row * warps);
+  cudaError_t e = set_smem_cap(kern, c->smem);
+  int per_sm = 0;
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, c->threads, c->smem);
+  if (e != cudaSuccess) return e;
+  c->ctas = std::max(1, per_sm) * num_sms;
+  return cudaSuccess;
+}
+
+template <typename V, int MD, bool MOD>
+cudaError_t launch_mult(NestPlan& p, cudaStream_t s, NestConfig& c, NestMultArgs& a, int64_t mpad,
+                        int64_t part_bytes, int64_t tiles, int num_sms) {
+  auto kern = nest_mult_kernel<V, MD, MOD>;
+  if (c.threads == 0) {
+    const cudaError_t e = mult_config<V>(p, &c, kern, a.m, mpad, part_bytes, num_sms);
+    if (e != cudaSuccess) {
+      c.threads = 0;
+      return e;
+    }
+  }
+  a.windows = p.windows + p.lists[c.list];
+  a.n_windows = p.lists[c.list + 1] - p.lists[c.list];
+  a.words = p.list_words[c.list];
+  a.warps = c.warps;
+  a.coef = nullptr;
+  if (c.restage) {
+    nest_coef_kernel<V><<<32, 512, 0, s>>>(a.alpha, p.inv, p.total, static_cast<V*>(p.coef));
+    a.coef = p.coef;
+  }
+  const int nw = c.warps;
+  const int64_t blocks = std::max<int64_t>(
+      1, std::min<int64_t>((tiles + nw - 1) / nw, c.ctas / c.splits));
+  kern<<<dim3(static_cast<unsigned>(blocks), static_cast<unsigned>(c.splits)), c.threads, c.smem, s>>>(a);
+  return cudaGetLastError();
+}
+
+template <typename V, bool MOD>
+cudaError_t launch_mult_dim(NestPlan& p, cudaStream_t s, NestConfig& c, NestMultArgs& a,
+                            int64_t mpad, int64_t part_bytes, int64_t tiles, int num_sms) {
+  switch (p.dim) {
+#define F(D) \
+  case D:    \
+    return launch_mult<V, D, MOD>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
+    F(1) F(2) F(3) F(4) F(5) F(6) F(7) F(8) F(9) F(10) F(11) F(12) F(13) F(14) F(15) F(16)
+#undef F
+    default:
+      return launch_mult<V, 0, MOD>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
+  }
+}
+
+template <typename V, typename TP>
+cudaError_t mult(NestPlan& p, cudaStream_t s, NestConfig& c, const NestDense& dense, int64_t m,
+                 const double* alpha, float* out32, double* out64, int64_t j_begin, int64_t j_end,
+                 int64_t out_end, void* part, int64_t part_bytes, int num_sms, int* launches) {
+  constexpr bool kF64 = std::is_same<V, double>::value;
+  cudaError_t e = tables(p, s, dense, m, kF64, launches);
+  if (e != cudaSuccess) return e;
+  constexpr int64_t kTilePts = 32 * kPts<V>;
+  j_begin = j_begin / kTilePts * kTilePts;  // mpad is a multiple of 1024
+  j_end = (j_end + kTilePts - 1) / kTilePts * kTilePts;
+  NestMultArgs a;
+  a.prog = p.prog;
+  a.n_ent = p.n_ent;
+  a.dim = p.dim;
+  for (int t = 0; t < 32; ++t) {
+    a.entry[t] = t < p.dim ? p.h_entry[t] : 0;
+    a.lmax[t] = t < p.dim ? p.h_lmax[t] : 1;
+  }
+  a.tab_hi = p.tab_hi;
+  a.tab_lo = p.tab_hi ? p.tab_hi + p.n_ent * dense.mpad : nullptr;
+  a.tab64 = p.tab64;
+  a.xcell = p.xcell;
+  a.m = m;
+  a.j_begin = j_begin;
+  a.n_tiles = (j_end - j_begin) / kTilePts;
+  a.out32 = out32;
+  a.out64 = out64;
+  a.part = part;
+  a.out_end = out_end;
+  a.dense = dense;
+  a.inv = p.inv;
+  a.alpha = alpha;
+  a.n = p.n;
+  // (MOD only changes the dense form that non-finite FP64 coefficients are checked against)
+  if constexpr (kF64)
+    e = p.mod ? launch_mult_dim<V, true>(p, s, c, a, dense.mpad, part_bytes, a.n_tiles, num_sms)
+              : launch_mult_dim<V, false>(p, s, c, a, dense.mpad, part_bytes, a.n_tiles, num_sms);
+  else
+    e = launch_mult_dim<V, false>(p, s, c, a, dense.mpad, part_bytes, a.n_tiles, num_sms);
+  if (e != cudaSuccess) return e;
+  *launches += c.restage ? 2 : 1;
+  if (c.splits > 1) {
+    const unsigned blocks = static_cast<unsigned>((j_end - j_begin + 255) / 256);
+    if (out64)
+      reduce_splits_kernel<TP, double><<<blocks, 256, 0, s>>>(static_cast<const TP*>(part), c.splits, dense.mpad, j_begin,
+                                                              std::min(m, j_end), std::min(out_end, j_end), out64, nullptr, 0.0);
+    if (out32)
+      reduce_splits_kernel<TP, float><<<blocks, 256, 0, s>>>(static_cast<const TP*>(part), c.splits, dense.mpad, j_begin,
+                                                             std::min(m, j_end), std::min(out_end, j_end), out32, nullptr, 0.0);
+    ++*launches;
+  }
   return cudaGetLastError();
 }
 }  // namespace
 
-cudaError_t nest_mult64(NestPlan& p, cudaStream_t s, const NestDense& dense, int64_t m,
-                        const double* alpha, double* out, int64_t j_begin, int64_t j_end,
-                        double* part, int64_t part_elems, int num_sms, int* launches) {
-  cudaError_t e = tables(p, s, dense, m, launches);
-  if (e != cudaSuccess) return e;
-  j_begin = j_begin / kMultThreads * kMultThreads;  // whole tiles; mpad is a multiple of them
-  j_end = (j_end + kMultThreads - 1) / kMultThreads * kMultThreads;
-  nest_coef_kernel<<<kBadBlocks, 512, 0, s>>>(alpha, p.inv, p.total, p.coef, p.bad);
-  const size_t sm = (sizeof(double) * p.n_ent + sizeof(uint32_t) * p.dim) * kMultThreads;
-  auto kern = p.mod ? nest_mult64_kernel<true> : nest_mult64_kernel<false>;
-  e = set_smem_cap(kern, sm);
-  if (e != cudaSuccess) return e;
-  // few tiles of points: several CTAs share the groups of one tile, so that every SM has work. The
-  // count comes from the whole data set, so that a range gives the bits of the full product.
-  const int64_t tiles_all = (m + kMultThreads - 1) / kMultThreads;
-  int64_t splits = std::min<int64_t>({kNestSplits, 4 * num_sms / std::max<int64_t>(tiles_all, 1),
-                                      p.n_sub / 32, p.n_r, part_elems / dense.mpad});
-  splits = std::max<int64_t>(1, splits);
-  const dim3 grid(static_cast<unsigned>((j_end - j_begin) / kMultThreads),
-                  static_cast<unsigned>(splits));
-  kern<<<grid, kMultThreads, sm, s>>>(
-      p.rops, p.facs, p.qops, p.lops, p.cuts + (splits - 1) * (kNestSplits + 1), p.coef, p.tab64,
-      p.xcell, p.n_ent, p.dim, m, j_begin, dense.mpad, splits > 1 ? part : out, p.bad, dense, alpha,
-      p.n);
-  *launches += 2;
-  if (splits > 1) {
-    const unsigned blocks = static_cast<unsigned>((j_end - j_begin + 255) / 256);
-    reduce_splits_kernel<double, double><<<blocks, 256, 0, s>>>(
-        part, static_cast<int>(splits), dense.mpad, j_begin, std::min(m, j_end), j_end, out, nullptr, 0.0);
-    ++*launches;
+cudaError_t nest_mult(NestPlan& p, cudaStream_t s, int precision, const NestDense& dense, int64_t m,
+                      const double* alpha, float* out32, double* out64, int64_t j_begin,
+                      int64_t j_end, int64_t out_end, void* part, int64_t part_bytes, int num_sms,
+                      int* launches) {
+  NestConfig& c = p.config[precision];
+  switch (precision) {
+    case SGMEV_FP64:
+      return mult<double, double>(p, s, c, dense, m, alpha, out32, out64, j_begin, j_end, out_end, part, part_bytes, num_sms, launches);
+    case SGMEV_FP32:
+      return mult<float, float>(p, s, c, dense, m, alpha, out32, out64, j_begin, j_end, out_end, part, part_bytes, num_sms, launches);
+    default:
+      return mult<ff, float2>(p, s, c, dense, m, alpha, out32, out64, j_begin, j_end, out_end, part, part_bytes, num_sms, launches);
   }
-  return cudaGetLastError();
 }
 
 cudaError_t nest_multt64(NestPlan& p, cudaStream_t s, const NestDense& dense, int64_t m,
                          const double* v, int64_t npad, double* out, const double* add,
                          double scale, int num_sms, int* launches) {
-  cudaError_t e = tables(p, s, dense, m, launches);
+  cudaError_t e = tables(p, s, dense, m, true, launches);
   if (e != cudaSuccess) return e;
   const int64_t n_tiles = std::max<int64_t>(1, (m + kTile - 1) / kTile);
   if (!p.rows) {

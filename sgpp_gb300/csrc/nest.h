@@ -13,23 +13,32 @@
 
 namespace sgmev {
 
+struct NestConfig {  // launch of the mult in one precision, fixed on its first product
+  int threads = 0, warps = 0, list = 0, splits = 1, ctas = 0;
+  bool restage = false;  // coefficients in position order first: they are staged several times
+  size_t smem = 0;
+};
+
 struct NestPlan {
   bool ok = false;
   bool mod = false;
-  int dim = 0, n_sub = 0, n_ent = 0, n_r = 0;
+  int dim = 0, n_sub = 0, n_ent = 0;
   int64_t n = 0, total = 0;
   std::vector<NestClass> classes;
+  std::vector<int> lists, list_cells, list_words;  // see NestTables
+  int h_entry[32] = {0}, h_lmax[32] = {0};
+  NestConfig config[3];  // by precision (SGMEV_FP64, SGMEV_FP32, SGMEV_DF64)
   unsigned char* block = nullptr;  // device memory of the plan
   // device copies of NestTables
-  int *lmax = nullptr, *facs = nullptr, *cuts = nullptr, *inv = nullptr, *clev = nullptr,
-      *ccell = nullptr, *tinv = nullptr;
-  NestOp4 *rops = nullptr, *qops = nullptr, *chunks = nullptr;
-  NestOp2 *lops = nullptr, *cq = nullptr, *cs = nullptr;
+  int *lmax = nullptr, *inv = nullptr, *clev = nullptr, *ccell = nullptr, *tinv = nullptr;
+  NestOp4 *windows = nullptr, *prog = nullptr, *chunks = nullptr;
+  NestOp2 *cq = nullptr, *cs = nullptr;
   double* rows = nullptr;  // multTranspose: partial rows, per class [streams][row_len]
+  void* coef = nullptr;    // [total] coefficients in position order, in the product's precision
   int* bad = nullptr;      // flags of values that are not finite, one per block
-  double* coef = nullptr;  // [total] coefficients in position order
   // tables of the data, built on the first product
-  double* tab64 = nullptr;    // [n_ent][mpad]
+  double* tab64 = nullptr;    // [n_ent][mpad], FP64 products
+  float* tab_hi = nullptr;    // [2][n_ent][mpad], high and low parts, FP32 and float-float products
   uint32_t* xcell = nullptr;  // [dim][mpad]
   cudaStream_t stream = nullptr;
 };
@@ -47,11 +56,14 @@ struct NestDense {
   int64_t mpad;
 };
 
-// out[j] = sum_g alpha_g phi_g(x_j), j in [j_begin, j_end) and the rest of their 64-point tiles,
-// 0 beyond m; `part` holds part_elems partial sums
-cudaError_t nest_mult64(NestPlan& p, cudaStream_t s, const NestDense& dense, int64_t m,
-                        const double* alpha, double* out, int64_t j_begin, int64_t j_end,
-                        double* part, int64_t part_elems, int num_sms, int* launches);
+// out32[j] and / or out64[j] = sum_g alpha_g phi_g(x_j) in the given precision (SGMEV_FP64, SGMEV_FP32,
+// SGMEV_DF64), j in [j_begin, j_end) and the rest of their tiles (32 points, 64 in FP32) up to
+// out_end, 0 beyond m; alpha [n] FP64;
+// `part` holds part_bytes of partial sums
+cudaError_t nest_mult(NestPlan& p, cudaStream_t s, int precision, const NestDense& dense, int64_t m,
+                      const double* alpha, float* out32, double* out64, int64_t j_begin,
+                      int64_t j_end, int64_t out_end, void* part, int64_t part_bytes, int num_sms,
+                      int* launches);
 
 // out[g] (g < n; zero in [n, npad)) = sum_j v_j phi_g(x_j) (+ scale * add[g])
 cudaError_t nest_multt64(NestPlan& p, cudaStream_t s, const NestDense& dense, int64_t m,

@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <numeric>
 
 #include "../../include/sgmev_tools.h"
 
@@ -78,8 +79,7 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
   std::vector<int> parent, fac, last, excess, ent(dim + 1, 1);
   for (int t = 0; t < dim; ++t) ent[t + 1] = ent[t] + p->lmax[t] - 1;
   p->n_ent = ent[dim];
-  if (p->n_ent > 1000 || sizeof(double) * kNestMultThreads * p->n_ent +
-                                 sizeof(uint32_t) * kNestMultThreads * dim > kNestSmem) {
+  if (p->n_ent > 1000 || 64 * (8 * p->n_ent + 4 * dim) > 128 * 1024) {
     *err = "nested kernels: the table of a data point is too long";
     return false;
   }
@@ -113,30 +113,6 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
     std::sort(k.begin(), k.end(), [&](int a, int b) { return fac_e(fac[a]) < fac_e(fac[b]); });
   auto inner = [&](int id) { return id == root || !kids[id].empty(); };
   // ---- mult program ----
-  std::vector<NestOp4> rops, qops;
-  std::vector<NestOp2> lops;
-  std::vector<int> facs, base(n_nodes, -1), work;
-  int64_t total = 0;
-  auto place = [&](int id) {
-    if (real[id]) {
-      base[id] = static_cast<int>(total);
-      total += int64_t(1) << excess[id];
-    }
-    return base[id];
-  };
-  auto add_q = [&](int id, int& units) {
-    const int b = place(id), l0 = static_cast<int>(lops.size());
-    for (int c : kids[id])
-      if (!inner(c)) lops.push_back(NestOp2{place(c), fac[c]});
-    qops.push_back(NestOp4{b, l0, static_cast<int>(lops.size()), fac[id]});
-    units += 3 + static_cast<int>(lops.size()) - l0;
-  };
-  {
-    int units = 0;
-    add_q(root, units);  // the root by itself: its factor is H_1
-    rops.push_back(NestOp4{0, 1, 0, 0});
-    work.push_back(units);
-  }
   std::vector<int> dfs{root}, order;
   while (!dfs.empty()) {
     const int id = dfs.back();
@@ -144,29 +120,203 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
     order.push_back(id);
     for (size_t k = kids[id].size(); k-- > 0;) dfs.push_back(kids[id][k]);
   }
+  // a node of budget b has in every later dimension, and no others, children of levels 2 .. b + 1, that
+  // of level l of budget b + 1 - l (in the last dimension: a leaf). The kernels evaluate budgets 1
+  // (run), 2 (tree) and 3 (forest) whole (nest_plan.h).
+  std::vector<int> budget(n_nodes, 0);
+  auto block_of = [&](int id, int b) -> int64_t {
+    const int k = dim - 1 - last[id];
+    const int64_t c = int64_t(1) << excess[id];
+    return b == 1 ? c * nest_run_row(k) : b == 2 ? c * nest_tree_row(k) : (c + 3) / 4 * 4 + c * nest_forest_at(k);
+  };
+  if (dim <= kNestMacroDim) {
+    for (size_t at = order.size(); at-- > 0;) {  // children before parents
+      const int id = order[at], k = dim - 1 - last[id], nk = static_cast<int>(kids[id].size());
+      if (k == 0 || nk % k != 0 || nk / k < 1 || nk / k > 3) continue;
+      const int b = nk / k;
+      bool all = block_of(id, b) <= kNestBlockCells;
+      for (int i = 0; i < nk; ++i) {  // ordered by (dimension, level)
+        const int c = kids[id][i], t = last[id] + 1 + i / b, l = 2 + i % b;
+        all = all && last[c] == t && fac_k(fac[c]) == l - 1 &&
+              (l == b + 1 || t == dim - 1 ? kids[c].empty() : budget[c] == b + 1 - l);
+      }
+      if (all) budget[id] = b;
+    }
+  }
+  // where the coefficient of cell c of a node lies: base + (c >> hs) hi + ((c >> ms) & mm) mid + (c & lm)
+  struct Place { int64_t base = -1, hi = 0; int hs = 31, ms = 31, mm = 0, mid = 0, lm = 0; };
+  std::vector<Place> place(n_nodes);
+  std::vector<NestOp4> qops;
+  std::vector<NestOp2> lops;
+  std::vector<int> facs, q_work, q_group;
+  std::vector<int64_t> q_coef;  // first position of an inner node's coefficients
+  std::vector<NestOp2> groups;  // first and end factor
+  int64_t total = 0;
+  auto plain = [&](int id) {  // cells in order
+    place[id].base = total;
+    place[id].lm = (1 << excess[id]) - 1;
+    total += int64_t(1) << excess[id];
+  };
+  auto add_q = [&](int id) {
+    q_coef.push_back(total);
+    q_group.push_back(static_cast<int>(groups.size()) - 1);
+    const int k = dim - 1 - last[id], t0 = last[id] + 1;
+    if (budget[id] > 0) {
+      const int64_t b = total;
+      auto put = [&](int c, int64_t base, int64_t hi, int hs, int ms, int mm, int mid, int lm) {
+        place[c].base = base;
+        place[c].hi = hi;
+        place[c].hs = hs;
+        place[c].ms = ms;
+        place[c].mm = mm;
+        place[c].mid = mid;
+        place[c].lm = lm;
+      };
+      auto run = [&](int n, int64_t at) {  // the node's rows from `at` on
+        const int row = nest_run_row(dim - 1 - last[n]);
+        put(n, at, row, 0, 31, 0, 0, 0);
+        for (int c : kids[n]) put(c, at + 1 + 2 * (dim - 1 - last[c]), row, 1, 31, 0, 0, 1);
+      };
+      auto tree = [&](int n, int64_t at) {
+        const int row = nest_tree_row(dim - 1 - last[n]);
+        put(n, at, row, 0, 31, 0, 0, 0);
+        for (int c : kids[n]) {
+          const int kt = dim - 1 - last[c], rr = nest_run_row(kt);
+          const int64_t sec = at + nest_tree_at(kt);
+          if (fac_k(fac[c]) == 2) {  // the level-3 leaf
+            put(c, sec + 2 * rr, row, 2, 31, 0, 0, 3);
+          } else {
+            put(c, sec, row, 1, 0, 1, rr, 0);
+            for (int g : kids[c]) put(g, sec + 1 + 2 * (dim - 1 - last[g]), row, 2, 1, 1, rr, 1);
+          }
+        }
+      };
+      int param = budget[id] == 1 ? nest_run_row(k) : nest_tree_row(k);
+      if (budget[id] == 1) {
+        run(id, b);
+      } else if (budget[id] == 2) {
+        tree(id, b);
+      } else {
+        const int64_t c0 = int64_t(1) << excess[id], b0 = b + (c0 + 3) / 4 * 4;
+        param = excess[id];
+        put(id, b, 0, 31, 31, 0, 0, (1 << excess[id]) - 1);
+        for (int c : kids[id]) {
+          const int kt = dim - 1 - last[c], l = fac_k(fac[c]) + 1;
+          const int64_t at = b0 + c0 * nest_forest_at(kt);
+          if (l == 2) tree(c, at);
+          else if (l == 3) run(c, at + 2 * c0 * nest_tree_row(kt));
+          else put(c, at + 2 * c0 * nest_tree_row(kt) + 4 * c0 * nest_run_row(kt), 0, 31, 31, 0, 0, (1 << excess[c]) - 1);
+        }
+      }
+      qops.push_back(NestOp4{static_cast<int>(b), -(1 + 4 * t0 + (budget[id] - 1)), param, fac[id]});
+      int units = 6 + 2 * k;
+      if (budget[id] == 2) units = 8 + k * (k + 5);
+      if (budget[id] == 3)
+        for (int i = 0; i < k; ++i) units += 14 + i * (i + 5);
+      q_work.push_back(units);
+      total += (block_of(id, budget[id]) + 3) / 4 * 4;
+      return;
+    }
+    int b = -1, l0 = static_cast<int>(lops.size());
+    if (real[id]) {
+      b = static_cast<int>(total);
+      plain(id);
+    }
+    auto flush = [&] {
+      const int l1 = static_cast<int>(lops.size());
+      qops.push_back(NestOp4{b, l0, l1, fac[id]});
+      q_work.push_back(6 + 3 * (l1 - l0));
+      l0 = l1;
+      b = -1;
+    };
+    for (int c : kids[id]) {
+      if (inner(c)) continue;
+      if (total - q_coef.back() + (int64_t(1) << excess[c]) > kNestBlockCells ||
+          static_cast<int>(lops.size()) - l0 == kNestLeaves) {
+        flush();  // the rest of the leaves under the same node, in a window of their own if need be
+        q_coef.push_back(total);
+        q_group.push_back(q_group.back());
+      }
+      lops.push_back(NestOp2{static_cast<int>(total), fac[c]});
+      plain(c);
+    }
+    flush();
+  };
+  groups.push_back(NestOp2{0, 0});
+  add_q(root);  // the root by itself: its factor is H_1
   for (int id : order) {
-    const int q0 = static_cast<int>(qops.size()), f0 = static_cast<int>(facs.size());
-    int units = 2 + excess[id];
-    for (int c : kids[id])
-      if (inner(c)) add_q(c, units);
-    if (static_cast<int>(qops.size()) == q0) continue;
+    if (budget[id] > 0) continue;
+    const int f0 = static_cast<int>(facs.size());
+    bool any = false;
+    for (int c : kids[id]) any = any || inner(c);
+    if (!any) continue;
     facs.push_back(kFacH1);
     for (int a = id; a != root; a = parent[a]) facs.push_back(fac[a]);
     std::reverse(facs.begin() + f0 + 1, facs.end());  // cells are built from the first dimension on
-    rops.push_back(NestOp4{q0, static_cast<int>(qops.size()), f0, static_cast<int>(facs.size())});
-    work.push_back(units);
+    groups.push_back(NestOp2{f0, static_cast<int>(facs.size())});
+    for (int c : kids[id])
+      if (inner(c)) add_q(c);
   }
-  if (lops.empty()) lops.push_back(NestOp2{0, kFacH1});
-  if (facs.empty()) facs.push_back(kFacH1);
-  const int n_r = static_cast<int>(rops.size());
-  // group boundaries for 1 .. kNestSplits CTAs per tile, by work
-  std::vector<int64_t> cum(n_r + 1, 0);
-  for (int r = 0; r < n_r; ++r) cum[r + 1] = cum[r] + work[r];
-  p->cuts.assign(kNestSplits * (kNestSplits + 1), n_r);
-  for (int s = 1; s <= kNestSplits; ++s)
-    for (int k = 0; k < s; ++k)
-      p->cuts[(s - 1) * (kNestSplits + 1) + k] = static_cast<int>(
-          std::lower_bound(cum.begin(), cum.end(), cum.back() * k / s) - cum.begin());
+  q_coef.push_back(total);
+  // windows: runs of inner nodes whose coefficients and program fit shared memory together; a list
+  // for S CTAs per tile of points has a multiple of S of them, with about the same work each
+  const int n_q = static_cast<int>(qops.size());
+  const int64_t all_work = std::accumulate(q_work.begin(), q_work.end(), int64_t(0));
+  for (int list = 0; list < kNestLists; ++list) {
+    const int64_t cap = nest_list_cap(list), ctas = nest_list_ctas(list);
+    const size_t prog0 = p->prog.size(), win0 = p->windows.size();
+    int64_t widest = 0, longest = 0;
+    for (int64_t want = ctas;; want += ctas) {
+      p->prog.resize(prog0);
+      p->windows.resize(win0);
+      widest = longest = 0;
+      int64_t done = 0, made = 0;
+      for (int q = 0; q < n_q;) {
+        const int p0 = static_cast<int>(p->prog.size()), q0 = q;
+        size_t header = 0;
+        for (; q < n_q; ++q) {
+          const NestOp4& o = qops[q];
+          const NestOp2& g = groups[q_group[q]];
+          const int nf = g.y - g.x, nl = o.y >= 0 ? o.z - o.y : 0;
+          const bool open = q == q0 || q_group[q - 1] != q_group[q];
+          const int64_t words = static_cast<int64_t>(p->prog.size()) - p0 +
+                                (open ? 1 + (nf + 3) / 4 : 0) + 2 + nl;
+          // (a window ends where the work so far, with half of the next node's, passes its share)
+          if (q > q0 && (q_coef[q + 1] - q_coef[q0] > cap || words > kNestProgram ||
+                         (2 * done + q_work[q]) * want >= 2 * all_work * (made + 1)))
+            break;
+          done += q_work[q];
+          if (open) {
+            header = p->prog.size();
+            p->prog.push_back(NestOp4{0, nf, 0, 0});
+            for (int i = g.x; i < g.y; i += 4) {
+              auto f = [&](int k) { return k < g.y ? facs[k] : 0; };
+              p->prog.push_back(NestOp4{f(i), f(i + 1), f(i + 2), f(i + 3)});
+            }
+          }
+          ++p->prog[header].x;
+          const int c0 = static_cast<int>(q_coef[q0]);
+          p->prog.push_back(NestOp4{o.x >= 0 ? o.x - c0 : -1, o.y >= 0 ? nl : o.y, o.z, 0});
+          p->prog.push_back(NestOp4{fac_e(o.w), fac_t(o.w), fac_k(o.w), fac_shift(o.w)});
+          for (int i = 0; i < nl; ++i) {
+            const NestOp2& u = lops[o.y + i];
+            p->prog.push_back(NestOp4{u.x - c0, fac_e(u.y) | (fac_t(u.y) << 16), fac_k(u.y), fac_shift(u.y)});
+          }
+        }
+        ++made;
+        const int p1 = static_cast<int>(p->prog.size());
+        widest = std::max(widest, q_coef[q] - q_coef[q0]);
+        longest = std::max<int64_t>(longest, p1 - p0);
+        p->windows.push_back(NestOp4{p0, p1, static_cast<int>(q_coef[q0]), static_cast<int>(q_coef[q])});
+      }
+      // enough windows were asked for, or there are no more nodes to divide
+      if (made <= want || want >= 2 * n_q) break;
+    }
+    p->list_begin.push_back(static_cast<int>(win0));
+    p->list_cells.push_back(static_cast<int>(widest));
+    p->list_words.push_back(static_cast<int>(longest));
+  }
+  p->list_begin.push_back(static_cast<int>(p->windows.size()));
   std::vector<int> inv(static_cast<size_t>(total), -1);
   std::vector<int> cell_of(static_cast<size_t>(n));
   for (int64_t g = 0; g < n; ++g) {
@@ -175,7 +325,8 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
     for (int t = 0; t < dim; ++t)
       if (l[t] > 1) c = (c << (l[t] - 1)) | ((static_cast<int>(index[g * dim + t]) - 1) / 2);
     cell_of[g] = c;
-    inv[base[node_of[g]] + c] = static_cast<int>(g);
+    const Place& pl = place[node_of[g]];
+    inv[pl.base + (c >> pl.hs) * pl.hi + ((c >> pl.ms) & pl.mm) * pl.mid + (c & pl.lm)] = static_cast<int>(g);
   }
   // ---- multTranspose program: subspaces by cell count, then tree order, in chunks ----
   std::vector<int> subs;
@@ -263,10 +414,6 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
     tinv[tpos[node_of[g]] + static_cast<int64_t>(cell_of[g]) * tstep[node_of[g]]] = static_cast<int>(g);
   p->dim = dim;
   p->n = n;
-  p->rops = std::move(rops);
-  p->qops = std::move(qops);
-  p->lops = std::move(lops);
-  p->facs = std::move(facs);
   p->inv = std::move(inv);
   p->chunks = std::move(chunks);
   p->cq = std::move(cq);
@@ -299,7 +446,6 @@ extern "C" SGMEV_API int sgmev_nest_host(int dim, int64_t n_grid, const double* 
     }
     return v[static_cast<size_t>(i)];
   };
-  const int n_r = static_cast<int>(p.rops.size());
   std::vector<double> coef(p.inv.size(), 0.0);
   for (size_t k = 0; k < p.inv.size(); ++k)
     if (p.inv[k] >= 0) coef[k] = alpha[p.inv[k]];
@@ -333,35 +479,87 @@ extern "C" SGMEV_API int sgmev_nest_host(int dim, int64_t n_grid, const double* 
     auto step = [&](uint32_t c, int f) {
       return (c << fac_k(f)) | (at(xc, fac_t(f)) >> fac_shift(f));
     };
-    // mult: the groups of every split, and the whole program the same whatever the split
+    // mult: the windows of a list, another list for another point
     double acc = 0.0;
-    const int splits = 1 + static_cast<int>(j % kNestSplits);
-    for (int y = 0; y < splits; ++y) {
-      const int r_end = at(p.cuts, (splits - 1) * (kNestSplits + 1) + y + 1);
-      for (int r = at(p.cuts, (splits - 1) * (kNestSplits + 1) + y); r < r_end; ++r) {
-        const NestOp4 ro = at(p.rops, r);
+    const int list = static_cast<int>(j % kNestLists);
+    for (int w = at(p.list_begin, list); w < at(p.list_begin, list + 1); ++w) {
+      const NestOp4 win = at(p.windows, w);
+      if (win.w - win.z > p.list_cells[list] || win.w - win.z > nest_list_cap(list) ||
+          win.y - win.x > p.list_words[list] || win.y - win.x > kNestProgram)
+        bad = true;
+      auto co = [&](int64_t i) {  // a window's coefficients only
+        if (i < 0 || i >= win.w - win.z) bad = true;
+        return at(coef, win.z + i);
+      };
+      for (int at_op = win.x; at_op < win.y && !bad;) {
+        const NestOp4 head = at(p.prog, at_op++);
         double pr = 1.0, ar = 0.0;
         uint32_t cr = 0;
-        for (int i = ro.z; i < ro.w; ++i) {
-          pr *= at(tab, fac_e(at(p.facs, i)));
-          cr = step(cr, at(p.facs, i));
+        for (int i = 0; i < head.y; ++i) {
+          const NestOp4 f4 = at(p.prog, at_op + i / 4);
+          const int f = i % 4 == 0 ? f4.x : i % 4 == 1 ? f4.y : i % 4 == 2 ? f4.z : f4.w;
+          pr *= at(tab, fac_e(f));
+          cr = step(cr, f);
         }
-        for (int q = ro.x; q < ro.y; ++q) {
-          const NestOp4 qo = at(p.qops, q);
-          const uint32_t c = step(cr, qo.w);
-          double sum = qo.x >= 0 ? at(coef, static_cast<int64_t>(qo.x) + c) : 0.0;
-          for (int i = qo.y; i < qo.z; ++i) {
-            const NestOp2 lo = at(p.lops, i);
-            sum += at(tab, fac_e(lo.y)) * at(coef, static_cast<int64_t>(lo.x) + step(c, lo.y));
+        at_op += (head.y + 3) / 4;
+        for (int q = 0; q < head.x; ++q) {
+          const NestOp4 qo = at(p.prog, at_op++), qf = at(p.prog, at_op++);
+          const int qfac = make_fac(qf.x, qf.y, qf.z, qf.w);
+          const uint32_t c = step(cr, qfac);
+          double sum = 0.0;
+          if (qo.y >= 0) {
+            sum = qo.x >= 0 ? co(static_cast<int64_t>(qo.x) + c) : 0.0;
+            for (int i = 0; i < qo.y; ++i) {
+              const NestOp4 l4 = at(p.prog, at_op++);
+              const NestOp2 lo{l4.x, make_fac(l4.y & 0xFFFF, l4.y >> 16, l4.z, l4.w)};
+              sum += at(tab, fac_e(lo.y)) * co(static_cast<int64_t>(lo.x) + step(c, lo.y));
+            }
+          } else {
+            const int kind = -qo.y - 1, t0 = kind >> 2;
+            auto cell_at = [&](int t, int l) { return xc[t] >> (p.lmax[t] - l); };
+            auto entry = [&](int t, int l) {
+              int e0 = 1;
+              for (int u = 0; u < t; ++u) e0 += p.lmax[u] - 1;
+              return at(tab, e0 + l - 2);
+            };
+            auto run = [&](int64_t r0, int t1) {
+              double sr = co(r0);
+              for (int t = t1; t < dim; ++t)
+                sr += entry(t, 2) * co(r0 + 1 + 2 * (dim - 1 - t) + cell_at(t, 2));
+              return sr;
+            };
+            auto tree = [&](int64_t row, int t1) {
+              double st = co(row);
+              for (int t = t1; t < dim; ++t) {
+                const int kt = dim - 1 - t;
+                const int64_t sec = row + nest_tree_at(kt);
+                st += entry(t, 2) * run(sec + static_cast<int64_t>(cell_at(t, 2)) * nest_run_row(kt), t + 1);
+                st += entry(t, 3) * co(sec + 2 * nest_run_row(kt) + cell_at(t, 3));
+              }
+              return st;
+            };
+            if ((kind & 3) == 0) {
+              sum = run(qo.x + static_cast<int64_t>(c) * qo.z, t0);
+            } else if ((kind & 3) == 1) {
+              sum = tree(qo.x + static_cast<int64_t>(c) * qo.z, t0);
+            } else {
+              const int64_t c0 = int64_t(1) << qo.z, b0 = qo.x + (c0 + 3) / 4 * 4;
+              sum = co(qo.x + c);
+              for (int t = t0; t < dim; ++t) {
+                const int kt = dim - 1 - t;
+                const int64_t at_t = b0 + c0 * nest_forest_at(kt), at_r = at_t + 2 * c0 * nest_tree_row(kt),
+                              at_l = at_r + 4 * c0 * nest_run_row(kt);
+                sum += entry(t, 2) * tree(at_t + static_cast<int64_t>((c << 1) | cell_at(t, 2)) * nest_tree_row(kt), t + 1);
+                sum += entry(t, 3) * run(at_r + static_cast<int64_t>((c << 2) | cell_at(t, 3)) * nest_run_row(kt), t + 1);
+                sum += entry(t, 4) * co(at_l + ((c << 3) | cell_at(t, 4)));
+              }
+            }
           }
-          ar += at(tab, fac_e(qo.w)) * sum;
+          ar += at(tab, fac_e(qfac)) * sum;
         }
         acc += pr * ar;
       }
     }
-    if (at(p.cuts, (splits - 1) * (kNestSplits + 1)) != 0 ||
-        at(p.cuts, (splits - 1) * (kNestSplits + 1) + splits) != n_r)
-      bad = true;
     mult_out[j] = acc;
     // multTranspose
     int64_t cs_at = 0;

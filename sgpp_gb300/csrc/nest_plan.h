@@ -32,10 +32,47 @@ constexpr int kFacH1 = make_fac(0, 0, 0, 31);  // entry 0; a shift of 31 gives c
 struct alignas(8) NestOp2 { int x, y; };
 struct alignas(16) NestOp4 { int x, y, z, w; };
 
-constexpr int kNestMultThreads = 64;  // points per CTA of the mult
+// The mult evaluates three common kinds of subtrees whole, with the factors of levels 2 and 3 in
+// registers. For runs and trees, per cell of a node whose last active dimension is t, with k = dim - 1 - t dimensions
+// after it, the coefficients lie in one row:
+//   run  (the node and its level-2 leaves): the node, then the two cells of the leaf of dimension
+//        t' at 1 + 2 (dim - 1 - t')
+//   tree (the node, its level-2 children with their runs, its level-3 leaves): the node, then per
+//        dimension t' from the last to the first, at nest_tree_at(dim - 1 - t'), the two run rows
+//        of the level-2 child and the four cells of the level-3 leaf
+// A section's place does not depend on t. Run rows are 2 mod 4 long and tree rows 4 mod 8: a warp's
+// gathers at one place of a tree (row c, run row b, cell b': c rows + b run rows + b') then hit
+// different banks for up to 8 rows (odd lengths gave 1.9 wavefronts a gather on the regression
+// workload's grid).
+NEST_HD constexpr int nest_run_row(int k) { return 2 * k + (k % 2 == 0 ? 2 : 4); }
+NEST_HD constexpr int nest_tree_at(int k) {
+  int r = 4;
+  for (int i = 0; i < k; ++i) r += 2 * nest_run_row(i) + 4;
+  return r;
+}
+NEST_HD constexpr int nest_tree_row(int k) { return (nest_tree_at(k) + 3) / 8 * 8 + 4; }
+// A forest (the node, and per later dimension t' its level-2 child with its tree, its level-3 child
+// with its run and its level-4 leaf) holds the node's cells (a multiple of 4) and then, per dimension
+// from the last to the first, at C nest_forest_at(dim - 1 - t') for C cells of the node: the child's
+// 2 C tree rows, 4 C run rows and 8 C cells.
+NEST_HD constexpr int nest_forest_step(int k) { return 2 * nest_tree_row(k) + 4 * nest_run_row(k) + 8; }
+NEST_HD constexpr int nest_forest_at(int k) {
+  int r = 0;
+  for (int i = 0; i < k; ++i) r += nest_forest_step(i);
+  return r;
+}
+constexpr int kNestMacroDim = 16;
+constexpr int kNestBlockCells = 6144;  // most coefficients of one inner node's block
+constexpr int kNestLeaves = 256;       // most leaves of one inner node's record
+constexpr int kNestProgram = 640;      // most words (16 bytes) of a window's program
+// window lists: at most cap coefficients per window, for so many CTAs sharing a tile of points
+constexpr int kNestLists = 10;
+NEST_HD constexpr int nest_list_cap(int list) { return list < kNestLists / 2 ? 18432 : 6144; }
+NEST_HD constexpr int nest_list_ctas(int list) { return 1 << (list % (kNestLists / 2)); }
+
 constexpr int kNestTile = 32;         // points per tile of the multTranspose (a warp's lanes)
-constexpr int kNestSplits = 16;       // most CTAs that share the groups of one tile of points
 constexpr size_t kNestSmem = 200 * 1024;
+constexpr size_t kNestMultSmem = 220 * 1024;  // the mult runs one CTA per SM
 constexpr size_t kNestAccBudget = 64 * 1024;  // cell sums of a multTranspose CTA (two CTAs per SM)
 
 // shared memory of a multTranspose CTA behind its [cells][threads] sums: per point of the tile the
@@ -65,12 +102,15 @@ struct NestTables {
   int dim = 0, n_sub = 0, n_ent = 0;
   int64_t n = 0;
   std::vector<int> lmax;  // [dim] finest level per dimension
-  // mult: groups (first and end inner node, first and end factor of the group's product), inner
-  // nodes (position or -1, first and end leaf, factor) and leaves (position, factor)
-  std::vector<NestOp4> rops, qops;
-  std::vector<NestOp2> lops;
-  std::vector<int> facs;
-  std::vector<int> cuts;  // row s - 1 of kNestSplits + 1: boundaries of the groups among s CTAs
+  // mult: per window list, windows (first and end word of the program, first and end position). The
+  // program is a sequence of groups: a header (inner nodes, factors), the factors of the group's
+  // product (four a word), and per inner node two words: position in the window or -1, leaves, -, -;
+  // or for runs and trees position, -(1 + 4 (first dimension) + (0 run, 1 tree, 2 forest)), row length
+  // (forest: log2 of the node's cells), -;
+  // and the node's factor unpacked: e, t, l - 1, shift. Then the leaves, a word each: position,
+  // e | t << 16, l - 1, shift.
+  std::vector<NestOp4> windows, prog;
+  std::vector<int> list_begin, list_cells, list_words;  // first window, widest, longest program
   std::vector<int> inv;   // grid point of a position or -1
   // multTranspose: chunks (first inner node, inner nodes, first depth boundary, depths), their inner
   // nodes (local parent, factor), depth boundaries, subspaces by thread (local parent, factor) and

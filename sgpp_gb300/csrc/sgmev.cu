@@ -162,8 +162,8 @@ struct sgmev_op {
   std::vector<cudaEvent_t> prof_events;  // pool, 2 per launch
   std::vector<int> prof_kind;            // kind of launch i
   size_t prof_used = 0;                  // launches recorded since the last reset
-  int64_t prof_count[21] = {0};
-  double prof_seconds[21] = {0.0};
+  int64_t prof_count[23] = {0};
+  double prof_seconds[23] = {0.0};
 };
 
 namespace sgmev {
@@ -190,9 +190,11 @@ enum {
   KIND_BLOCK_MULT = 17,
   KIND_BLOCK_MULTT = 18,
   KIND_MULT_NEST64 = 19,
-  KIND_MULTT_NEST64 = 20
+  KIND_MULTT_NEST64 = 20,
+  KIND_MULT_NEST32 = 21,
+  KIND_MULT_NESTDF = 22
 };
-constexpr int kKinds = 21;
+constexpr int kKinds = 23;
 
 template <typename T>
 static const T* gscale(const sgmev_op* op);
@@ -859,11 +861,15 @@ static bool mat_ready(sgmev_op* op) {
   return true;
 }
 
-// The nested subspace kernels serve the FP64 products of every grid whose plan they take, unless
-// "algo" is "dense" (they cost about 1.3 FP64 instructions per subspace and data point, the dense
-// kernels 3 d per grid point and data point, and a subspace has at least one grid point; smallest
-// measured, 351 points and 3,000 data points: a host system product 279 -> 113 us). ModLinear
-// data outside the cube stays on the dense kernels, which extrapolate.
+// The nested subspace kernels serve the FP64 products, and the FP32 and float-float mult, of every grid
+// whose plan they take, unless "algo" is "dense" or, for the latter two, "materialize" is "on" (which
+// asks for the materialised products). FP64: about 1.3 instructions of the FP64 pipe per subspace and
+// data point against 3 d per grid point and data point, and a subspace has at least one grid point;
+// smallest measured, 351 points and 3,000 data points: a host system product 279 -> 97 us. FP32 and
+// float-float mult against the materialised ones, d = 3..10, level 5..7, 1,000 to 256,000 points:
+// 13-103 against 24-143 us (FP16 products) and 15-240 against 31-371 us; equal at d=10 level 5 and
+// 64,000 points (56 us), whose FP16 products stay in L2. ModLinear data outside the cube stays on the
+// dense kernels, which extrapolate.
 static bool nest_ready(sgmev_op* op) {
   using namespace sgmev;
   if (op->nest.ok) return true;
@@ -877,21 +883,29 @@ static bool nest_ready(sgmev_op* op) {
   return true;
 }
 
-// Inputs per precision: FP64 a64; FP32 a32; DF64 (a32, a32lo) — all padded to npad.
+static bool nest_mults(sgmev_op* op, int prec) {
+  return (prec == SGMEV_FP64 || op->mat_mode != 2) && nest_ready(op);
+}
+
+// Inputs: a64 [n] where nest_mults(); otherwise per precision FP64 a64; FP32 a32; DF64 (a32, a32lo) —
+// all padded to npad.
 // out64 / out32 [mpad] (zero beyond m) = B a over data range [j_begin, j_end).
+// out_end (nest_mults() only): the end of the outputs, when they are not padded to mpad.
 static int dev_mult(sgmev_op* op, int prec, const double* a64, const float* a32,
                     const float* a32lo, double* out64, float* out32, int64_t j_begin,
-                    int64_t j_end) {
+                    int64_t j_end, int64_t out_end = INT64_MAX) {
   if (j_end <= j_begin) return SGMEV_OK;
   Plan p;
   const int64_t total = j_end;
   const int64_t valid = std::min(op->m, total);
-  if (prec == SGMEV_FP64 && out64 && !out32 && nest_ready(op)) {
+  if (nest_mults(op, prec)) {
     int launches = 0;
-    const long ev = prof_begin(op, KIND_MULT_NEST64);
-    SGMEV_CUDA(nest_mult64(op->nest, op->stream, NestDense{op->xt64, op->li64, op->mpad}, op->m, a64,
-                           out64, j_begin, j_end, static_cast<double*>(op->part), op->part_elems,
-                           op->num_sms, &launches));
+    const long ev = prof_begin(op, prec == SGMEV_FP64   ? KIND_MULT_NEST64
+                                   : prec == SGMEV_FP32 ? KIND_MULT_NEST32
+                                                        : KIND_MULT_NESTDF);
+    SGMEV_CUDA(nest_mult(op->nest, op->stream, prec, NestDense{op->xt64, op->li64, op->mpad}, op->m,
+                         a64, out32, out64, j_begin, j_end, std::min(out_end, op->mpad), op->part,
+                         static_cast<int64_t>(op->part_bytes), op->num_sms, &launches));
     prof_end(op, ev);
     op->launches += launches;
   } else if (prec == SGMEV_FP64) {
@@ -1001,10 +1015,13 @@ static int dev_convert(sgmev_op* op, const double* in, int64_t n, int64_t npad, 
 
 // out64[npad] = B^T (B a) + lm * a, a given as padded FP64 device vector [npad]
 static int dev_system(sgmev_op* op, int prec, const double* a64, double* out64, double lm) {
+  const bool nested = nest_mults(op, prec);
   if (prec == SGMEV_FP32) {
-    SGMEV_TRY(dev_convert(op, a64, op->npad, op->npad, nullptr, op->a32, nullptr));
-    if (op->fused_system && !op->use_half && op->sub_ok && op->mat_multt && mat_ready(op) &&
-        subspace_system_mat_fits(op->sub)) {
+    const bool fused = op->fused_system && !op->use_half && op->sub_ok && op->mat_multt &&
+                       mat_ready(op) && subspace_system_mat_fits(op->sub);
+    if (fused || !nested)
+      SGMEV_TRY(dev_convert(op, a64, op->npad, op->npad, nullptr, op->a32, nullptr));
+    if (fused) {
       // one pass over the materialised products for B^T (B a)
       const long ev = prof_begin(op, KIND_SYSTEM_MAT32);
       SGMEV_CUDA(subspace_system_mat(op->sub, op->stream, op->mpad, op->a32, op->npad, out64, a64,
@@ -1013,11 +1030,11 @@ static int dev_system(sgmev_op* op, int prec, const double* a64, double* out64, 
       op->launches += 4;
       return SGMEV_OK;
     }
-    SGMEV_TRY(dev_mult(op, prec, nullptr, op->a32, nullptr, nullptr, op->v32, 0, op->mpad));
+    SGMEV_TRY(dev_mult(op, prec, a64, op->a32, nullptr, nullptr, op->v32, 0, op->mpad));
     SGMEV_TRY(dev_multt(op, prec, nullptr, op->v32, nullptr, out64, 0, op->npad, a64, lm));
   } else if (prec == SGMEV_DF64) {
-    SGMEV_TRY(dev_convert(op, a64, op->npad, op->npad, nullptr, op->a32, op->a32lo));
-    SGMEV_TRY(dev_mult(op, prec, nullptr, op->a32, op->a32lo, op->v64, nullptr, 0, op->mpad));
+    if (!nested) SGMEV_TRY(dev_convert(op, a64, op->npad, op->npad, nullptr, op->a32, op->a32lo));
+    SGMEV_TRY(dev_mult(op, prec, a64, op->a32, op->a32lo, op->v64, nullptr, 0, op->mpad));
     SGMEV_TRY(dev_convert(op, op->v64, op->mpad, op->mpad, nullptr, op->v32, op->v32lo));
     SGMEV_TRY(dev_multt(op, prec, nullptr, op->v32, op->v32lo, out64, 0, op->npad, a64, lm));
   } else {
@@ -1626,15 +1643,22 @@ static int mult_common(sgmev_op* op, const double* alpha_dev_or_null, const doub
                                  cudaMemcpyHostToDevice, op->stream));
     src = op->out64;
   }
-  SGMEV_TRY(dev_convert(op, src, op->n, op->npad, prec == SGMEV_FP64 ? op->a64 : nullptr,
-                        prec == SGMEV_FP64 ? nullptr : op->a32,
-                        prec == SGMEV_DF64 ? op->a32lo : nullptr));
+  const bool nested = nest_mults(op, prec);
+  if (!nested)
+    SGMEV_TRY(dev_convert(op, src, op->n, op->npad, prec == SGMEV_FP64 ? op->a64 : nullptr,
+                          prec == SGMEV_FP64 ? nullptr : op->a32,
+                          prec == SGMEV_DF64 ? op->a32lo : nullptr));
   // tile-aligned data range covering [start, end)
   const int64_t tile_pts = mult_tile_pts(op, prec);
   const int64_t jb = (start / tile_pts) * tile_pts;
   const int64_t je = std::min(op->mpad, round_up(end, tile_pts));
-  SGMEV_TRY(dev_mult(op, prec, op->a64, op->a32, op->a32lo, op->v64, nullptr, jb, je));
-  if (result_host) {
+  // the nested kernels write a whole product into the caller's device vector themselves
+  const bool direct = nested && result_dev && start == 0 && end == op->m;
+  SGMEV_TRY(dev_mult(op, prec, nested ? src : op->a64, op->a32, op->a32lo, direct ? result_dev : op->v64,
+                     nullptr, jb, je, direct ? op->m : INT64_MAX));
+  if (direct) {
+    // nothing to copy
+  } else if (result_host) {
     if (end > start)
       SGMEV_CUDA(cudaMemcpyAsync(result_host + start, op->v64 + start,
                                  sizeof(double) * (end - start), cudaMemcpyDeviceToHost,

@@ -168,3 +168,31 @@ def test_values_that_are_not_finite_spread_as_in_the_dense_kernels(value):
         for a, b in zip(got, want):
             np.testing.assert_array_equal(np.isnan(a), np.isnan(b))
             np.testing.assert_array_equal(np.isinf(a), np.isinf(b))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("basis", ["linear", "modlinear"])
+@pytest.mark.parametrize("precision,unit", [("float", 2.0 ** -24), ("df64", 2.0 ** -44)])
+@pytest.mark.parametrize("m", [1, 33, 2000, 70001])
+@pytest.mark.parametrize("dim,level,rounds", [(1, 1, 0), (1, 10, 0), (2, 9, 0), (3, 6, 0), (4, 3, 25),
+                                              (7, 5, 0), (9, 6, 0), (12, 3, 0), (16, 3, 0), (17, 2, 2)])
+def test_fp32_and_df64_mult_match_fp64(dim, level, rounds, m, precision, unit, basis):
+    """One window and several (9 dimensions, level 6: more coefficients than shared memory), points
+    split over warps and subspaces over CTAs (small m), runs and trees of every first dimension."""
+    grid = _grid(dim, level, basis, rounds)
+    n = grid.getSize()
+    rng = np.random.default_rng(m + dim)
+    x = _points(rng, m, dim, level + 1)
+    alpha = rng.standard_normal(n)
+    op, ref = _op(grid, x, "auto", precision), _op(grid, x, "auto", "double")
+    op.profile(True)
+    out, outr, part = np.zeros(m), np.zeros(m), np.full(m, -7.0)
+    op.mult(alpha, out)
+    kind = sg.SGMEV_KERNEL_MULT_NEST32 if precision == "float" else sg.SGMEV_KERNEL_MULT_NESTDF
+    assert op.profileRead(kind)[0] == 1
+    ref.mult(alpha, outr)
+    # two roundings a factor (table entry and product), one an addend
+    big = 1.0 if basis == "linear" else 2.0 ** min(dim, level)
+    assert np.abs(out - outr).max() <= (4 * dim + n) * unit * big * np.abs(alpha).sum()
+    op.mult(alpha, part, m // 3, m - m // 4)
+    np.testing.assert_array_equal(part[m // 3:m - m // 4], out[m // 3:m - m // 4])
