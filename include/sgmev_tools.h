@@ -50,6 +50,8 @@ SGMEV_API int sgmev_fma_peak(int precision, double* flops_per_second, int* sm_cl
 #define SGMEV_KERNEL_MULTT_NEST64 20 /* FP64 multTranspose, nested subspace products */
 #define SGMEV_KERNEL_MULT_NEST32 21  /* FP32 mult, nested subspace products */
 #define SGMEV_KERNEL_MULT_NESTDF 22  /* df64 mult, nested subspace products */
+#define SGMEV_KERNEL_MULTT_NEST32 23 /* FP32 multTranspose, nested subspace products */
+#define SGMEV_KERNEL_MULTT_NESTDF 24 /* df64 multTranspose, nested subspace products */
 SGMEV_API int sgmev_profile(sgmev_op* op, int enable);
 SGMEV_API int sgmev_profile_read(sgmev_op* op, int kind, int64_t* launches, double* seconds);
 

@@ -92,6 +92,8 @@ SGMEV_KERNEL_MULT_NEST64 = 19
 SGMEV_KERNEL_MULTT_NEST64 = 20
 SGMEV_KERNEL_MULT_NEST32 = 21
 SGMEV_KERNEL_MULT_NESTDF = 22
+SGMEV_KERNEL_MULTT_NEST32 = 23
+SGMEV_KERNEL_MULTT_NESTDF = 24
 SGMEV_BLOCK_RHS = 16
 
 

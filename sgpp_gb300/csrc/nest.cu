@@ -490,47 +490,65 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
 // CTA (stream, chunk): chunk's subspaces over the stream's contiguous range of tiles. Phase A: lane
 // = point, a warp per inner node, one depth of the tree after the other. Phase B: thread =
 // subspace, points in order, sums in the thread's own cells.
-__global__ void __launch_bounds__(256) nest_multt64_kernel(
-    const NestOp4* __restrict__ chunks, const NestOp2* __restrict__ cq, const int* __restrict__ clev,
-    const NestOp2* __restrict__ cs, const int* __restrict__ ccell, const double* __restrict__ tab,
-    const uint32_t* __restrict__ xcell, int64_t mpad, int64_t m, int n_ent, int dim, int nq_max,
-    int cells, const double* __restrict__ v, int64_t n_tiles, int streams, int64_t row_len,
-    double* __restrict__ rows, int* __restrict__ bad) {
+struct NestMulttArgs {
+  const NestOp4* chunks;
+  const NestOp2 *cq, *cs, *cwarp;
+  const int *clev, *ccell;
+  const float *tab_hi, *tab_lo;
+  const double* tab64;
+  const uint32_t* xcell;
+  int64_t mpad, m, n_tiles, row_len;
+  int n_ent, dim, nq_max, sums, streams;
+  double* rows;
+  int* bad;
+};
+__device__ __forceinline__ void read_entry(float& r, const NestMulttArgs& a, int64_t k) { r = a.tab_hi[k]; }
+__device__ __forceinline__ void read_entry(double& r, const NestMulttArgs& a, int64_t k) { r = a.tab64[k]; }
+__device__ __forceinline__ void read_entry(ff& r, const NestMulttArgs& a, int64_t k) { r = ff{a.tab_hi[k], a.tab_lo[k]}; }
+
+template <typename V, typename VIN>
+__global__ void __launch_bounds__(256) nest_multt_kernel(const __grid_constant__ NestMulttArgs a,
+                                                         const VIN* __restrict__ v) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nth >> 5;
-  const int chunk = blockIdx.x / streams, stream = blockIdx.x - chunk * streams;
-  const NestTileLayout lay(nq_max, n_ent, dim);
-  double* s_acc = reinterpret_cast<double*>(smem);
-  double* s_p = s_acc + static_cast<size_t>(cells) * nth;
-  double* s_t = s_p + kTile * lay.qs;
+  const int chunk = blockIdx.x / a.streams, stream = blockIdx.x - chunk * a.streams;
+  const NestTileLayout lay(a.nq_max, a.n_ent, a.dim);
+  V* s_acc = reinterpret_cast<V*>(smem);
+  V* s_p = s_acc + a.sums;
+  V* s_t = s_p + kTile * lay.qs;
   uint32_t* s_x = reinterpret_cast<uint32_t*>(s_t + kTile * lay.es);
   uint16_t* s_c = reinterpret_cast<uint16_t*>(s_x + kTile * lay.xs);
-  const NestOp4 ch = chunks[chunk];
-  const NestOp2 own = cs[chunk * nth + tid];
-  const int own_cells = ccell[chunk * nth + tid];
+  const NestOp4 ch = a.chunks[chunk];
+  const NestOp2 own = a.cs[chunk * nth + tid];
+  const int own_cells = a.ccell[chunk * nth + tid];
   const int own_e = fac_e(own.y), own_t = fac_t(own.y), own_k = fac_k(own.y),
             own_s = fac_shift(own.y);
-  for (int c = 0; c < own_cells; ++c) s_acc[c * nth + tid] = 0.0;
+  const NestOp2 at = a.cwarp[chunk * nw + warp];
+  V* const own_acc = s_acc + at.x + lane;  // cell c at 32 c
+  for (int c = 0; c < own_cells; ++c) own_acc[32 * c] = V{};
   bool nonfinite = false;
-  const int64_t t_end = (stream + 1) * n_tiles / streams;
-  for (int64_t tile = stream * n_tiles / streams; tile < t_end; ++tile) {
+  const int64_t t_begin = stream * a.n_tiles / a.streams, t_end = (stream + 1) * a.n_tiles / a.streams;
+  for (int64_t tile = t_begin; tile < t_end; ++tile) {
     const int64_t j0 = tile * kTile;
     __syncthreads();  // phase B of the previous tile is done
-    for (int e = warp; e < n_ent; e += nw) s_t[lane * lay.es + e] = tab[e * mpad + j0 + lane];
-    for (int t = warp; t < dim; t += nw) s_x[lane * lay.xs + t] = xcell[t * mpad + j0 + lane];
+    for (int e = warp; e < a.n_ent; e += nw) read_entry(s_t[lane * lay.es + e], a, e * a.mpad + j0 + lane);
+    for (int t = warp; t < a.dim; t += nw) s_x[lane * lay.xs + t] = a.xcell[t * a.mpad + j0 + lane];
     if (warp == nw - 1) {  // the root: v_j H_1 (the same warp reads H_1 itself)
-      const double vj = j0 + lane < m ? v[j0 + lane] : 0.0;
+      const double vj = j0 + lane < a.m ? static_cast<double>(v[j0 + lane]) : 0.0;
       nonfinite = nonfinite || !isfinite(vj);
-      s_p[lane * lay.qs] = vj * tab[j0 + lane];
+      V h1, vv;
+      read_entry(h1, a, j0 + lane);
+      set_val(vv, vj);
+      s_p[lane * lay.qs] = mul(vv, h1);
       s_c[lane * lay.cs] = 0;
-      s_t[lane * lay.es + n_ent] = 1.0;
+      set_val(s_t[lane * lay.es + a.n_ent], 1.0);
     }
     __syncthreads();
     for (int d = 0; d < ch.w; ++d) {
-      const int q_end = clev[ch.z + d + 1];
-      for (int q = clev[ch.z + d] + warp; q < q_end; q += nw) {
-        const NestOp2 o = cq[ch.x + q];
-        s_p[lane * lay.qs + q] = s_p[lane * lay.qs + o.x] * s_t[lane * lay.es + fac_e(o.y)];
+      const int q_end = a.clev[ch.z + d + 1];
+      for (int q = a.clev[ch.z + d] + warp; q < q_end; q += nw) {
+        const NestOp2 o = a.cq[ch.x + q];
+        s_p[lane * lay.qs + q] = mul(s_p[lane * lay.qs + o.x], s_t[lane * lay.es + fac_e(o.y)]);
         s_c[lane * lay.cs + q] = static_cast<uint16_t>(
             (static_cast<uint32_t>(s_c[lane * lay.cs + o.x]) << fac_k(o.y)) |
             (s_x[lane * lay.xs + fac_t(o.y)] >> fac_shift(o.y)));
@@ -542,15 +560,20 @@ __global__ void __launch_bounds__(256) nest_multt64_kernel(
       for (int i = 0; i < kTile; ++i) {
         const uint32_t c = (static_cast<uint32_t>(s_c[i * lay.cs + own.x]) << own_k) |
                            (s_x[i * lay.xs + own_t] >> own_s);
-        double* a = s_acc + c * nth + tid;
-        *a = fma(s_p[i * lay.qs + own.x], s_t[i * lay.es + own_e], *a);
+        V* acc = own_acc + 32 * c;
+        V r = *acc;
+        mac(r, s_p[i * lay.qs + own.x], s_t[i * lay.es + own_e]);
+        *acc = r;
       }
+      // float-float sums are settled every 1,024 points
+      if (std::is_same<V, ff>::value && ((tile - t_begin) & 31) == 31)
+        for (int c = 0; c < own_cells; ++c) settle(own_acc[32 * c]);
     }
   }
-  double* row = rows + stream * row_len + static_cast<int64_t>(chunk) * cells * nth;
-  for (int c = 0; c < own_cells; ++c) row[c * nth + tid] = s_acc[c * nth + tid];
-  const int any = __syncthreads_or(nonfinite);
-  if (tid == 0) bad[blockIdx.x] = any;
+  double* row = a.rows + stream * a.row_len + at.y + lane;
+  for (int c = 0; c < own_cells; ++c) row[32 * c] = to_double(own_acc[32 * c]);
+  const int any = __syncthreads_or(std::is_same<V, double>::value && nonfinite);
+  if (tid == 0) a.bad[blockIdx.x] = any;
 }
 
 // NaN when a non-finite v_j meets a hat of 0 of grid point g, else 0
@@ -635,6 +658,7 @@ bool nest_build(NestPlan* p, int dim, int64_t n, const double* level_pow2, const
   put(&p->cq, h.cq);
   put(&p->clev, h.clev);
   put(&p->cs, h.cs);
+  put(&p->cwarp, h.cwarp);
   put(&p->ccell, h.ccell);
   put(&p->tinv, h.tinv);
   const size_t o_coef = (host.size() + 255) / 256 * 256,
@@ -843,48 +867,95 @@ cudaError_t nest_mult(NestPlan& p, cudaStream_t s, int precision, const NestDens
   }
 }
 
-cudaError_t nest_multt64(NestPlan& p, cudaStream_t s, const NestDense& dense, int64_t m,
-                         const double* v, int64_t npad, double* out, const double* add,
-                         double scale, int num_sms, int* launches) {
-  cudaError_t e = tables(p, s, dense, m, true, launches);
+namespace {
+template <typename V, typename VIN>
+cudaError_t multt(NestPlan& p, cudaStream_t s, std::vector<int>& streams, const NestDense& dense,
+                  int64_t m, const VIN* v, int64_t npad, double* out, const double* add, double scale,
+                  int num_sms, int* launches) {
+  constexpr bool kF64 = std::is_same<V, double>::value;
+  cudaError_t e = tables(p, s, dense, m, kF64, launches);
   if (e != cudaSuccess) return e;
+  auto kern = nest_multt_kernel<V, VIN>;
   const int64_t n_tiles = std::max<int64_t>(1, (m + kTile - 1) / kTile);
-  if (!p.rows) {
+  if (streams.empty()) {
     // as many streams as fit the SMs at once (at most 256 MB of rows); fixed from here on, and
     // with them the order of every sum
+    std::vector<int> st;
     int64_t elems = 0;
-    for (NestClass& c : p.classes) {
-      e = set_smem_cap(nest_multt64_kernel, c.smem);
+    for (const NestClass& c : p.classes) {
+      const size_t sm = c.smem(sizeof(V), p.n_ent, p.dim);
+      e = set_smem_cap(kern, sm);
       int per_sm = 0;
-      if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, nest_multt64_kernel, c.threads, c.smem);
+      if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, c.threads, sm);
       if (e != cudaSuccess) return e;
       const int64_t resident = std::min<int64_t>(4, std::max(1, per_sm)) * num_sms;
-      c.streams = static_cast<int>(std::max<int64_t>(
-          1, std::min<int64_t>({resident / c.chunks, n_tiles, (int64_t(1) << 25) / c.row_len})));
-      elems += c.streams * c.row_len;
+      st.push_back(static_cast<int>(std::max<int64_t>(
+          1, std::min<int64_t>({resident / c.chunks, n_tiles, (int64_t(1) << 25) / c.row_len}))));
+      elems += st.back() * c.row_len;
     }
-    e = dev_malloc(&p.rows, sizeof(double) * elems, s);
-    if (e != cudaSuccess) return e;
+    if (elems > p.row_elems) {
+      dev_free(p.rows, s);
+      p.rows = nullptr;
+      p.row_elems = 0;
+      e = dev_malloc(&p.rows, sizeof(double) * elems, s);
+      if (e != cudaSuccess) return e;
+      p.row_elems = elems;
+    }
+    streams = st;
   }
   if (npad > p.n) {
     e = cudaMemsetAsync(out + p.n, 0, sizeof(double) * (npad - p.n), s);
     if (e != cudaSuccess) return e;
   }
-  double* rows = p.rows;
+  NestMulttArgs a;
+  a.cq = p.cq;
+  a.clev = p.clev;
+  a.tab_hi = p.tab_hi;
+  a.tab_lo = p.tab_hi ? p.tab_hi + p.n_ent * dense.mpad : nullptr;
+  a.tab64 = p.tab64;
+  a.xcell = p.xcell;
+  a.mpad = dense.mpad;
+  a.m = m;
+  a.n_tiles = n_tiles;
+  a.n_ent = p.n_ent;
+  a.dim = p.dim;
+  a.bad = p.bad;
+  a.rows = p.rows;
   int64_t cs_at = 0;
-  for (const NestClass& c : p.classes) {
-    nest_multt64_kernel<<<static_cast<unsigned>(c.streams * c.chunks), c.threads, c.smem, s>>>(
-        p.chunks + c.chunk_begin, p.cq, p.clev, p.cs + cs_at, p.ccell + cs_at, p.tab64, p.xcell,
-        dense.mpad, m, p.n_ent, p.dim, c.nq, c.cells, v, n_tiles, c.streams, c.row_len, rows, p.bad);
+  for (size_t k = 0; k < p.classes.size(); ++k) {
+    const NestClass& c = p.classes[k];
+    a.chunks = p.chunks + c.chunk_begin;
+    a.cs = p.cs + cs_at;
+    a.ccell = p.ccell + cs_at;
+    a.nq_max = c.nq;
+    a.cwarp = p.cwarp + cs_at / 32;
+    a.sums = c.sums;
+    a.streams = streams[k];
+    a.row_len = c.row_len;
+    kern<<<static_cast<unsigned>(streams[k] * c.chunks), c.threads, c.smem(sizeof(V), p.n_ent, p.dim), s>>>(a, v);
+    // (non-finite values are looked after in FP64 only, and only there the basis matters)
+    const double* v64 = kF64 ? reinterpret_cast<const double*>(v) : nullptr;
     auto fin = p.mod ? nest_finish_kernel<true> : nest_finish_kernel<false>;
     fin<<<static_cast<unsigned>((c.row_len + 31) / 32), dim3(32, kSumGroups), 0, s>>>(
-        rows, c.streams, c.row_len, p.tinv + c.row_begin, add, scale, out, p.bad, dense, p.dim, m, v);
-    rows += c.streams * c.row_len;
+        a.rows, streams[k], c.row_len, p.tinv + c.row_begin, add, scale, out, p.bad, dense, p.dim, m, v64);
+    a.rows += streams[k] * c.row_len;
     cs_at += static_cast<int64_t>(c.chunks) * c.threads;
     *launches += 2;
   }
   return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t nest_multt(NestPlan& p, cudaStream_t s, int precision, const NestDense& dense, int64_t m,
+                       const double* v64, const float* v32, int64_t npad, double* out,
+                       const double* add, double scale, int num_sms, int* launches) {
+  std::vector<int>& st = p.streams[precision];
+  if (precision == SGMEV_FP64)
+    return multt<double>(p, s, st, dense, m, v64, npad, out, add, scale, num_sms, launches);
+  if (precision == SGMEV_DF64)
+    return multt<ff>(p, s, st, dense, m, v64, npad, out, add, scale, num_sms, launches);
+  if (v32) return multt<float>(p, s, st, dense, m, v32, npad, out, add, scale, num_sms, launches);
+  return multt<float>(p, s, st, dense, m, v64, npad, out, add, scale, num_sms, launches);
 }
 
 }  // namespace sgmev

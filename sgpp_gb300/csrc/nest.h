@@ -28,12 +28,14 @@ struct NestPlan {
   std::vector<int> lists, list_cells, list_words;  // see NestTables
   int h_entry[32] = {0}, h_lmax[32] = {0};
   NestConfig config[3];  // by precision (SGMEV_FP64, SGMEV_FP32, SGMEV_DF64)
+  std::vector<int> streams[3];  // multTranspose: tile streams (rows of partial sums) of each class
   unsigned char* block = nullptr;  // device memory of the plan
   // device copies of NestTables
   int *lmax = nullptr, *inv = nullptr, *clev = nullptr, *ccell = nullptr, *tinv = nullptr;
   NestOp4 *windows = nullptr, *prog = nullptr, *chunks = nullptr;
-  NestOp2 *cq = nullptr, *cs = nullptr;
+  NestOp2 *cq = nullptr, *cs = nullptr, *cwarp = nullptr;
   double* rows = nullptr;  // multTranspose: partial rows, per class [streams][row_len]
+  int64_t row_elems = 0;
   void* coef = nullptr;    // [total] coefficients in position order, in the product's precision
   int* bad = nullptr;      // flags of values that are not finite, one per block
   // tables of the data, built on the first product
@@ -65,9 +67,10 @@ cudaError_t nest_mult(NestPlan& p, cudaStream_t s, int precision, const NestDens
                       int64_t j_end, int64_t out_end, void* part, int64_t part_bytes, int num_sms,
                       int* launches);
 
-// out[g] (g < n; zero in [n, npad)) = sum_j v_j phi_g(x_j) (+ scale * add[g])
-cudaError_t nest_multt64(NestPlan& p, cudaStream_t s, const NestDense& dense, int64_t m,
-                         const double* v, int64_t npad, double* out, const double* add,
-                         double scale, int num_sms, int* launches);
+// out[g] (g < n; zero in [n, npad)) = sum_j v_j phi_g(x_j) (+ scale * add[g]) in the given precision;
+// v64 [m], or v32 [m] (nullptr: v64) for SGMEV_FP32
+cudaError_t nest_multt(NestPlan& p, cudaStream_t s, int precision, const NestDense& dense, int64_t m,
+                       const double* v64, const float* v32, int64_t npad, double* out,
+                       const double* add, double scale, int num_sms, int* launches);
 
 }  // namespace sgmev

@@ -334,11 +334,10 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
     if (real[id]) subs.push_back(id);
   std::stable_sort(subs.begin(), subs.end(), [&](int a, int b) { return excess[a] > excess[b]; });
   std::vector<NestOp4> chunks;
-  std::vector<NestOp2> cq, cs;
+  std::vector<NestOp2> cq, cs, cwarp;
   std::vector<int> clev, ccell, local(n_nodes, -1), depth(n_nodes, 0);
   for (int id : order) depth[id] = parent[id] < 0 ? 0 : depth[parent[id]] + 1;
   std::vector<int64_t> tpos(n_nodes, -1);
-  std::vector<int> tstep(n_nodes, 0);
   int64_t row_total = 0;
   for (size_t at = 0; at < subs.size();) {
     const int cells = 1 << excess[subs[at]];
@@ -349,7 +348,6 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
     // their own would run blocks of four times the threads
     NestClass c;
     c.threads = threads;
-    c.cells = cells;
     c.chunk_begin = static_cast<int>(chunks.size());
     c.row_begin = row_total;
     while (at < subs.size()) {
@@ -391,18 +389,26 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
         cs.push_back(id == root ? NestOp2{0, make_fac(p->n_ent, 0, 0, 31)}
                                 : NestOp2{local[parent[id]], fac[id]});
         ccell.push_back(1 << excess[id]);
-        tpos[id] = row_total + static_cast<int64_t>(chunks.size() - 1 - c.chunk_begin) * cells * threads + k;
-        tstep[id] = threads;
       }
+      // a warp's sums: [most cells of its subspaces][32], in the chunk's shared memory and in the rows
+      int sums = 0;
+      for (int w = 0; w < threads / 32; ++w) {
+        int most = 0;
+        for (int k = 32 * w; k < std::min(cnt, 32 * w + 32); ++k) {
+          most = std::max(most, 1 << excess[subs[at + k]]);
+          tpos[subs[at + k]] = row_total + c.row_len + sums + (k - 32 * w);
+        }
+        cwarp.push_back(NestOp2{sums, static_cast<int>(c.row_len) + sums});
+        sums += 32 * most;
+      }
+      c.sums = std::max(c.sums, sums);
+      c.row_len += sums;
       c.nq = std::max(c.nq, static_cast<int>(need.size()));
       for (int a : need) local[a] = -1;
       at += cnt;
     }
     c.chunks = static_cast<int>(chunks.size()) - c.chunk_begin;
-    c.row_len = static_cast<int64_t>(c.chunks) * cells * threads;
-    c.smem = sizeof(double) * static_cast<size_t>(cells) * threads +
-             NestTileLayout(c.nq, p->n_ent, dim).bytes();
-    if (c.smem > kNestSmem) {
+    if (c.smem(sizeof(double), p->n_ent, dim) > kNestSmem) {
       *err = "nested kernels: a chunk of subspaces does not fit shared memory";
       return false;
     }
@@ -411,13 +417,14 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
   }
   std::vector<int> tinv(static_cast<size_t>(row_total), -1);
   for (int64_t g = 0; g < n; ++g)
-    tinv[tpos[node_of[g]] + static_cast<int64_t>(cell_of[g]) * tstep[node_of[g]]] = static_cast<int>(g);
+    tinv[tpos[node_of[g]] + static_cast<int64_t>(cell_of[g]) * 32] = static_cast<int>(g);
   p->dim = dim;
   p->n = n;
   p->inv = std::move(inv);
   p->chunks = std::move(chunks);
   p->cq = std::move(cq);
   p->cs = std::move(cs);
+  p->cwarp = std::move(cwarp);
   p->clev = std::move(clev);
   p->ccell = std::move(ccell);
   p->tinv = std::move(tinv);
@@ -564,7 +571,7 @@ extern "C" SGMEV_API int sgmev_nest_host(int dim, int64_t n_grid, const double* 
     // multTranspose
     int64_t cs_at = 0;
     for (const NestClass& c : p.classes) {
-      if (c.threads < 32 || c.threads > 256 || c.threads % 32 || c.smem > kNestSmem) bad = true;
+      if (c.threads < 32 || c.threads > 256 || c.threads % 32 || c.smem(8, p.n_ent, dim) > kNestSmem) bad = true;
       for (int k = 0; k < c.chunks; ++k) {
         const NestOp4 ch = at(p.chunks, c.chunk_begin + k);
         if (ch.y > c.nq || at(p.clev, ch.z + ch.w) != ch.y) bad = true;
@@ -586,8 +593,10 @@ extern "C" SGMEV_API int sgmev_nest_host(int dim, int64_t n_grid, const double* 
           if (cells == 0) continue;
           const NestOp2 o = at(p.cs, cs_at + static_cast<int64_t>(k) * c.threads + t);
           const uint32_t cl = step(at(cell, o.x), o.y);
-          if (cl >= static_cast<uint32_t>(cells) || cells > c.cells) bad = true;
-          const int64_t pos = c.row_begin + (static_cast<int64_t>(k) * c.cells + cl) * c.threads + t;
+          const NestOp2 wp = at(p.cwarp, cs_at / 32 + (k * c.threads + t) / 32);
+          const int64_t in_chunk = wp.x + static_cast<int64_t>(cl) * 32 + t % 32;
+          if (cl >= static_cast<uint32_t>(cells) || in_chunk >= c.sums) bad = true;
+          const int64_t pos = c.row_begin + wp.y + static_cast<int64_t>(cl) * 32 + t % 32;
           if (pos >= c.row_begin + c.row_len || pos >= static_cast<int64_t>(sums.size())) bad = true;
           else sums[pos] += at(prod, o.x) * at(tab, fac_e(o.y));
         }

@@ -75,27 +75,28 @@ constexpr size_t kNestSmem = 200 * 1024;
 constexpr size_t kNestMultSmem = 220 * 1024;  // the mult runs one CTA per SM
 constexpr size_t kNestAccBudget = 64 * 1024;  // cell sums of a multTranspose CTA (two CTAs per SM)
 
-// shared memory of a multTranspose CTA behind its [cells][threads] sums: per point of the tile the
+// shared memory of a multTranspose CTA behind its cell sums: per point of the tile the
 // inner products, the table row (with a 1 behind it), the inner cells and the coordinates' cells; odd
-// row lengths keep a warp's 32 points in different banks
+// row lengths keep a warp's 32 points in different banks (bytes: with values of `value` bytes)
 struct NestTileLayout {
-  int qs, es, cs, xs;  // row lengths: doubles, doubles, uint16, uint32
+  int qs, es, cs, xs;  // row lengths: values, values, uint16, uint32
   NEST_HD NestTileLayout(int nq, int n_ent, int dim)
       : qs(nq | 1), es((n_ent + 1) | 1), cs(((nq + 1) / 2 | 1) * 2), xs(dim | 1) {}
-  NEST_HD size_t bytes() const {
-    return static_cast<size_t>(kNestTile) * (8 * qs + 8 * es + 2 * cs + 4 * xs);
+  NEST_HD size_t bytes(int value) const {
+    return static_cast<size_t>(kNestTile) * (value * (qs + es) + 2 * cs + 4 * xs);
   }
 };
 
 // multTranspose launches: chunks of one block size
 struct NestClass {
   int threads = 0;  // subspaces per chunk, one per thread
-  int cells = 0;    // most cells of a subspace
+  int sums = 0;     // most cell sums of a chunk
   int chunk_begin = 0, chunks = 0;
   int nq = 0;       // most inner nodes of a chunk
-  size_t smem = 0;
+  size_t smem(int value, int n_ent, int dim) const {
+    return static_cast<size_t>(value) * sums + NestTileLayout(nq, n_ent, dim).bytes(value);
+  }
   int64_t row_begin = 0, row_len = 0;  // positions of the class in the transposed layout
-  int streams = 0;  // tile streams (rows of partial sums)
 };
 
 struct NestTables {
@@ -114,10 +115,11 @@ struct NestTables {
   std::vector<int> inv;   // grid point of a position or -1
   // multTranspose: chunks (first inner node, inner nodes, first depth boundary, depths), their inner
   // nodes (local parent, factor), depth boundaries, subspaces by thread (local parent, factor) and
-  // their cell counts (0: none), grid point of a transposed position
+  // their cell counts (0: none), where a warp's sums begin in shared memory and in a row (thread's
+  // cell c at 32 c + lane), grid point of a transposed position
   std::vector<NestClass> classes;
   std::vector<NestOp4> chunks;
-  std::vector<NestOp2> cq, cs;
+  std::vector<NestOp2> cq, cs, cwarp;
   std::vector<int> clev, ccell, tinv;
 };
 

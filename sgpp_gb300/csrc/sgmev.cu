@@ -162,8 +162,8 @@ struct sgmev_op {
   std::vector<cudaEvent_t> prof_events;  // pool, 2 per launch
   std::vector<int> prof_kind;            // kind of launch i
   size_t prof_used = 0;                  // launches recorded since the last reset
-  int64_t prof_count[23] = {0};
-  double prof_seconds[23] = {0.0};
+  int64_t prof_count[25] = {0};
+  double prof_seconds[25] = {0.0};
 };
 
 namespace sgmev {
@@ -192,9 +192,11 @@ enum {
   KIND_MULT_NEST64 = 19,
   KIND_MULTT_NEST64 = 20,
   KIND_MULT_NEST32 = 21,
-  KIND_MULT_NESTDF = 22
+  KIND_MULT_NESTDF = 22,
+  KIND_MULTT_NEST32 = 23,
+  KIND_MULTT_NESTDF = 24
 };
-constexpr int kKinds = 23;
+constexpr int kKinds = 25;
 
 template <typename T>
 static const T* gscale(const sgmev_op* op);
@@ -887,6 +889,18 @@ static bool nest_mults(sgmev_op* op, int prec) {
   return (prec == SGMEV_FP64 || op->mat_mode != 2) && nest_ready(op);
 }
 
+// The FP32 and float-float multTranspose: nested up to 8,192 data points, where it also saves building
+// the materialised products (d = 3..10, level 5..7, 1,000 points: 18-28 against 25-54 us in FP32 and
+// 18-36 against 31-214 us in float-float; 16,000 points: 27-77 against 25-62 and 31-131 against 32-218;
+// above that the materialised kernels win), and float-float on grids that the materialised kernels
+// do not take up to 10^8 subspaces x points (d=6 level 7, 64,000 points: 422 against 441 us).
+static bool nest_multts(sgmev_op* op, int prec) {
+  if (!nest_mults(op, prec)) return false;
+  if (prec == SGMEV_FP64 || op->m <= 8192) return true;
+  return prec == SGMEV_DF64 && static_cast<double>(op->nest.n_sub) * op->m <= 1e8 &&
+         !(op->sub_ok && op->mat_multt && subspace_mat_fits(op->sub, true) && mat_ready(op));
+}
+
 // Inputs: a64 [n] where nest_mults(); otherwise per precision FP64 a64; FP32 a32; DF64 (a32, a32lo) —
 // all padded to npad.
 // out64 / out32 [mpad] (zero beyond m) = B a over data range [j_begin, j_end).
@@ -949,18 +963,22 @@ static int dev_mult(sgmev_op* op, int prec, const double* a64, const float* a32,
   return SGMEV_OK;
 }
 
-// out64[g_begin..g_end) = B^T v (+ scale * add); inputs FP64 v64, FP32 v32, DF64 (v32, v32lo)
+// out64[g_begin..g_end) = B^T v (+ scale * add); inputs v64 [m] where nest_multts() (FP32: v32 where it is
+// not null), otherwise FP64 v64, FP32 v32, DF64 (v32, v32lo), padded to mpad
 static int dev_multt(sgmev_op* op, int prec, const double* v64, const float* v32,
                      const float* v32lo, double* out64, int64_t g_begin, int64_t g_end,
-                     const double* add, double scale) {
+                     const double* add, double scale, int64_t out_end = -1) {
   if (g_end <= g_begin) return SGMEV_OK;
   Plan p;
   const int64_t valid = std::min(op->n, g_end);
-  if (prec == SGMEV_FP64 && nest_ready(op)) {
+  if (nest_multts(op, prec)) {
     int launches = 0;
-    const long ev = prof_begin(op, KIND_MULTT_NEST64);
-    SGMEV_CUDA(nest_multt64(op->nest, op->stream, NestDense{op->xt64, op->li64, op->mpad}, op->m, v64,
-                            op->npad, out64, add, scale, op->num_sms, &launches));
+    const long ev = prof_begin(op, prec == SGMEV_FP64   ? KIND_MULTT_NEST64
+                                   : prec == SGMEV_FP32 ? KIND_MULTT_NEST32
+                                                        : KIND_MULTT_NESTDF);
+    SGMEV_CUDA(nest_multt(op->nest, op->stream, prec, NestDense{op->xt64, op->li64, op->mpad}, op->m, v64,
+                          prec == SGMEV_FP32 ? v32 : nullptr, out_end < 0 ? op->npad : out_end, out64, add, scale, op->num_sms,
+                          &launches));
     prof_end(op, ev);
     op->launches += launches;
   } else if (prec == SGMEV_FP64) {
@@ -1035,8 +1053,9 @@ static int dev_system(sgmev_op* op, int prec, const double* a64, double* out64, 
   } else if (prec == SGMEV_DF64) {
     if (!nested) SGMEV_TRY(dev_convert(op, a64, op->npad, op->npad, nullptr, op->a32, op->a32lo));
     SGMEV_TRY(dev_mult(op, prec, a64, op->a32, op->a32lo, op->v64, nullptr, 0, op->mpad));
-    SGMEV_TRY(dev_convert(op, op->v64, op->mpad, op->mpad, nullptr, op->v32, op->v32lo));
-    SGMEV_TRY(dev_multt(op, prec, nullptr, op->v32, op->v32lo, out64, 0, op->npad, a64, lm));
+    if (!nest_multts(op, prec))
+      SGMEV_TRY(dev_convert(op, op->v64, op->mpad, op->mpad, nullptr, op->v32, op->v32lo));
+    SGMEV_TRY(dev_multt(op, prec, op->v64, op->v32, op->v32lo, out64, 0, op->npad, a64, lm));
   } else {
     SGMEV_TRY(dev_mult(op, prec, a64, nullptr, nullptr, op->v64, nullptr, 0, op->mpad));
     SGMEV_TRY(dev_multt(op, prec, op->v64, nullptr, nullptr, out64, 0, op->npad, a64, lm));
@@ -1683,15 +1702,24 @@ static int multt_common(sgmev_op* op, const double* src_dev, const double* src_h
                                  cudaMemcpyHostToDevice, op->stream));
     src = op->out64;
   }
-  SGMEV_TRY(dev_convert(op, src, op->m, op->mpad, prec == SGMEV_FP64 ? op->v64 : nullptr,
-                        prec == SGMEV_FP64 ? nullptr : op->v32,
-                        prec == SGMEV_DF64 ? op->v32lo : nullptr));
+  const bool nested = nest_multts(op, prec);
+  if (!nested)
+    SGMEV_TRY(dev_convert(op, src, op->m, op->mpad, prec == SGMEV_FP64 ? op->v64 : nullptr,
+                          prec == SGMEV_FP64 ? nullptr : op->v32,
+                          prec == SGMEV_DF64 ? op->v32lo : nullptr));
   const int64_t tile_pts = multt_tile_pts(op, prec);
   const int64_t gb = (start / tile_pts) * tile_pts;
   const int64_t ge = std::min(op->npad, round_up(end, tile_pts));
   double* tmp = op->cg + 7 * op->npad;  // spare CG slot as result staging
-  SGMEV_TRY(dev_multt(op, prec, op->v64, op->v32, op->v32lo, tmp, gb, ge, nullptr, 0.0));
-  if (result_host) {
+  const bool direct = nested && result_dev && start == 0 && end == op->n;
+  if (nested)
+    SGMEV_TRY(dev_multt(op, prec, src, nullptr, nullptr, direct ? result_dev : tmp, gb, ge, nullptr, 0.0,
+                        direct ? op->n : op->npad));
+  else
+    SGMEV_TRY(dev_multt(op, prec, op->v64, op->v32, op->v32lo, tmp, gb, ge, nullptr, 0.0));
+  if (direct) {
+    // the nested kernels wrote the caller's device vector
+  } else if (result_host) {
     if (end > start)
       SGMEV_CUDA(cudaMemcpyAsync(result_host + start, tmp + start, sizeof(double) * (end - start),
                                  cudaMemcpyDeviceToHost, op->stream));

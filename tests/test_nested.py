@@ -196,3 +196,11 @@ def test_fp32_and_df64_mult_match_fp64(dim, level, rounds, m, precision, unit, b
     assert np.abs(out - outr).max() <= (4 * dim + n) * unit * big * np.abs(alpha).sum()
     op.mult(alpha, part, m // 3, m - m // 4)
     np.testing.assert_array_equal(part[m // 3:m - m // 4], out[m // 3:m - m // 4])
+    v, outt, outtr, again = rng.standard_normal(m), np.zeros(n), np.zeros(n), np.zeros(n)
+    op.multTranspose(v, outt)
+    ref.multTranspose(v, outtr)
+    assert np.abs(outt - outtr).max() <= (4 * dim + m) * unit * big * np.abs(v).sum()
+    op.multTranspose(v, again)
+    np.testing.assert_array_equal(again, outt)
+    kind = sg.SGMEV_KERNEL_MULTT_NEST32 if precision == "float" else sg.SGMEV_KERNEL_MULTT_NESTDF
+    assert m > 8192 or op.profileRead(kind)[0] == 2
