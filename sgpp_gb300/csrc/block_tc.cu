@@ -27,6 +27,7 @@
 #include <vector>
 
 #include "block_tc.h"
+#include "cg_cluster.cuh"
 #include "devmem.h"
 #include "tc_ptx.cuh"
 
@@ -563,7 +564,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1) block_mult_kernel(
     const int2* __restrict__ gslots, const uint16_t* __restrict__ coef, int n_groups, int n_slots, int64_t mpad, int64_t m, int n_tiles,
     int tiles, int gpp, int teams, int stages, int loads, int win, uint32_t tmem_cols, uint16_t* __restrict__ qtiles,
     double* __restrict__ out64, int* __restrict__ status, int f16, const float* __restrict__ scales,
-    float pscale, float qfac) {
+    float pscale, float qfac, const double* __restrict__ stop) {
+  if (stop && *stop != 0.0) return;  // a step enqueued ahead of the solve's end
   extern __shared__ __align__(1024) unsigned char smem[];
   const int smem_stages = TMEM_A ? 0 : stages;
   unsigned char* st = smem;
@@ -705,7 +707,8 @@ __global__ void __launch_bounds__(kMaxThreads, 1) block_multt_kernel(
     const uint32_t* __restrict__ pc, const BlockHeader* __restrict__ gheader,
     const int2* __restrict__ gslots, const uint16_t* __restrict__ qtiles, int n_groups, int n_slots, int64_t mpad, int n_tiles, int gpc,
     int streams, int teams, int stages, int loads, int win, uint32_t tmem_cols, int64_t rows,
-    double* __restrict__ part, int* __restrict__ status, int f16) {
+    double* __restrict__ part, int* __restrict__ status, int f16, const double* __restrict__ stop) {
+  if (stop && *stop != 0.0) return;
   extern __shared__ __align__(1024) unsigned char smem[];
   unsigned char* st = smem;
   unsigned char* lb = st + static_cast<size_t>(stages) * kStageBytes;
@@ -968,9 +971,8 @@ namespace sgmev {
 namespace {
 
 // ---- CG on 16 columns -------------------------------------------------------------------------
-// Vectors are column-major [16][np]; every dot product reduces in a fixed order (a shared-memory
-// tree per block, then the kBlockDotBlocks block sums in block order), so iterations are
-// reproducible bit for bit. Scalars (BlockCgScalars offsets) stay on the device.
+// Vectors are column-major [16][np]; every dot product reduces in a fixed order, so iterations are
+// reproducible bit for bit. Scalars (kSc* offsets) stay on the device.
 constexpr int kDotT = 256;
 
 __device__ __forceinline__ double block_tree_sum(double v, double* sh) {
@@ -983,12 +985,6 @@ __device__ __forceinline__ double block_tree_sum(double v, double* sh) {
   const double r = sh[0];
   __syncthreads();
   return r;
-}
-
-__device__ __forceinline__ double sum_parts(const double* __restrict__ part, int k) {
-  double s = 0.0;
-  for (int b = 0; b < kBlockDotBlocks; ++b) s += part[k * kBlockDotBlocks + b];
-  return s;
 }
 
 __global__ void __launch_bounds__(kDotT) bcg_dot_kernel(const double* __restrict__ a,
@@ -1006,84 +1002,62 @@ __global__ void __launch_bounds__(kDotT) bcg_dot_kernel(const double* __restrict
   if (threadIdx.x == 0) part[k * kBlockDotBlocks + blockIdx.x] = v;
 }
 
-// d = r, e = 0, partial r.r
-__global__ void __launch_bounds__(kDotT) bcg_init_kernel(const double* __restrict__ r,
-                                                         double* __restrict__ d,
-                                                         double* __restrict__ e, int64_t np,
-                                                         double* __restrict__ part) {
-  __shared__ double sh[kDotT];
+// The last of the 16 clusters to get here reports how many columns take another step
+__device__ __forceinline__ void bcg_report(double* sc, bool next, double* host) {
+  unsigned int* count = reinterpret_cast<unsigned int*>(sc + kScCount);  // [0] active, [1] arrived
+  if (next) atomicAdd(count, 1u);
+  __threadfence();
+  if (atomicAdd(count + 1, 1u) == kBlockRhs - 1) {
+    __threadfence();
+    const unsigned int active = atomicExch(count, 0u);
+    count[1] = 0u;
+    sc[kScStop] = active == 0u ? 1.0 : 0.0;
+    *reinterpret_cast<volatile double*>(host) = static_cast<double>(active);
+  }
+}
+
+// one cluster per column (cg_cluster.cuh)
+__global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads) bcg_init_kernel(
+    const double* __restrict__ r, double* __restrict__ d, double* __restrict__ e, int64_t np,
+    double* __restrict__ sc, double* __restrict__ host) {
+  __shared__ CgShared sh;
   const int k = blockIdx.y;
   const int64_t o = static_cast<int64_t>(k) * np;
   double v = 0.0;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * kDotT + threadIdx.x; i < np;
-       i += static_cast<int64_t>(gridDim.x) * kDotT) {
+  for (int64_t i = cg_first(); i < np; i += kCgStride) {
     const double ri = r[o + i];
     d[o + i] = ri;
     e[o + i] = 0.0;
-    v += ri * ri;
+    v = fma(ri, ri, v);
   }
-  v = block_tree_sum(v, sh);
-  if (threadIdx.x == 0) part[k * kBlockDotBlocks + blockIdx.x] = v;
-}
-
-// delta (slot 0) = delta_0 = the summed partials
-__global__ void bcg_set_delta_kernel(const double* __restrict__ part, double* __restrict__ sc) {
-  const int k = threadIdx.x;
-  if (k < kBlockRhs) {
-    const double v = sum_parts(part, k);
+  v = cg_cluster_sum(v, sh, 0);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
     sc[kScDelta + k] = v;
     sc[kScDelta0 + k] = v;
+    bcg_report(sc, v > sc[kScTol2 + k] * v, host);
   }
+  cg_cluster_end();
 }
 
-// alpha = delta / d.q on active columns; e += alpha d, r -= alpha q; partial r.r
-__global__ void __launch_bounds__(kDotT) bcg_update_kernel(
-    double* __restrict__ e, double* __restrict__ r, const double* __restrict__ d,
-    const double* __restrict__ q, int64_t np, const double* __restrict__ part_dq,
-    const double* __restrict__ sc, int cur, double* __restrict__ part_rr) {
-  __shared__ double sh[kDotT];
+__global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads) bcg_step_kernel(
+    double* __restrict__ e, double* __restrict__ r, double* __restrict__ d,
+    const double* __restrict__ q, int64_t np, double* __restrict__ sc, double* __restrict__ host) {
+  if (sc[kScStop] != 0.0) return;
+  __shared__ CgShared sh;
   const int k = blockIdx.y;
-  const double delta = sc[kScDelta + cur * kBlockRhs + k];
-  const double dq = sum_parts(part_dq, k);
-  const bool active = delta > sc[kScTol2 + k] * sc[kScDelta0 + k] && dq != 0.0;
-  const double alpha = active ? delta / dq : 0.0;
   const int64_t o = static_cast<int64_t>(k) * np;
-  double v = 0.0;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * kDotT + threadIdx.x; i < np;
-       i += static_cast<int64_t>(gridDim.x) * kDotT) {
-    double ri = r[o + i];
-    if (active) {
-      e[o + i] = fma(alpha, d[o + i], e[o + i]);
-      ri = fma(-alpha, q[o + i], ri);
-      r[o + i] = ri;
-    }
-    v += ri * ri;
-  }
-  v = block_tree_sum(v, sh);
-  if (threadIdx.x == 0) part_rr[k * kBlockDotBlocks + blockIdx.x] = v;
-}
-
-// beta = delta_new / delta; d = r + beta d on active columns; delta_new into the other slot
-__global__ void __launch_bounds__(kDotT) bcg_direction_kernel(
-    const double* __restrict__ r, double* __restrict__ d, int64_t np,
-    const double* __restrict__ part_dq, const double* __restrict__ part_rr,
-    double* __restrict__ sc, int cur) {
-  const int k = blockIdx.y;
-  const double delta = sc[kScDelta + cur * kBlockRhs + k];
-  const double dq = sum_parts(part_dq, k);
-  const bool active = delta > sc[kScTol2 + k] * sc[kScDelta0 + k] && dq != 0.0;
-  const double dnew = sum_parts(part_rr, k);
-  const double beta = active ? dnew / delta : 0.0;
-  const int64_t o = static_cast<int64_t>(k) * np;
-  if (active) {
-    for (int64_t i = static_cast<int64_t>(blockIdx.x) * kDotT + threadIdx.x; i < np;
-         i += static_cast<int64_t>(gridDim.x) * kDotT)
-      d[o + i] = fma(beta, d[o + i], r[o + i]);
-  }
+  const double delta = sc[kScDelta + k], delta0 = sc[kScDelta0 + k];
+  const bool take = delta > sc[kScTol2 + k] * delta0;
+  double dq, alpha, rr;
+  cg_column_step(np, d + o, q + o, e + o, r + o, delta, take, false, sh, &dq, &alpha, &rr);
+  cg_cluster_end();  // every block has read the column's scalars
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    // a column whose step was not taken keeps its delta (and stays inactive); d.q = 0 ends it
-    sc[kScDelta + (cur ^ 1) * kBlockRhs + k] = active ? dnew : delta;
-    sc[kScStalled + k] = (!active && dq == 0.0) ? 1.0 : 0.0;
+    // a column whose step was not taken keeps its delta (and stays as it is); d.q = 0 ends it
+    const double now = take && dq != 0.0 ? rr : delta;
+    sc[kScDelta + k] = now;
+    if (dq == 0.0) sc[kScTol2 + k] = HUGE_VAL;
+    if (take) sc[kScSteps + k] += 1.0;
+    bcg_report(sc, now > sc[kScTol2 + k] * delta0, host);
   }
 }
 
@@ -1095,19 +1069,14 @@ cudaError_t block_dot(cudaStream_t s, const double* a, const double* b, int64_t 
 }
 
 cudaError_t block_cg_init(cudaStream_t s, const double* r, double* d, double* e, int64_t np,
-                          double* part, double* sc) {
-  bcg_init_kernel<<<dim3(kBlockDotBlocks, kBlockRhs), kDotT, 0, s>>>(r, d, e, np, part);
-  bcg_set_delta_kernel<<<1, 32, 0, s>>>(part, sc);
+                          double* sc, double* host) {
+  bcg_init_kernel<<<dim3(kCgCtas, kBlockRhs), kCgThreads, 0, s>>>(r, d, e, np, sc, host);
   return cudaGetLastError();
 }
 
 cudaError_t block_cg_step(cudaStream_t s, double* e, double* r, double* d, const double* q,
-                          int64_t np, double* part_dq, double* part_rr, double* sc, int cur) {
-  bcg_dot_kernel<<<dim3(kBlockDotBlocks, kBlockRhs), kDotT, 0, s>>>(d, q, np, part_dq);
-  bcg_update_kernel<<<dim3(kBlockDotBlocks, kBlockRhs), kDotT, 0, s>>>(e, r, d, q, np, part_dq,
-                                                                       sc, cur, part_rr);
-  bcg_direction_kernel<<<dim3(kBlockDotBlocks, kBlockRhs), kDotT, 0, s>>>(r, d, np, part_dq,
-                                                                          part_rr, sc, cur);
+                          int64_t np, double* sc, double* host) {
+  bcg_step_kernel<<<dim3(kCgCtas, kBlockRhs), kCgThreads, 0, s>>>(e, r, d, q, np, sc, host);
   return cudaGetLastError();
 }
 
@@ -1373,11 +1342,25 @@ cudaError_t block_mult(BlockPlan& b, cudaStream_t s, const double* p, int64_t np
   e = set_smem_cap(kern, smem);
   if (e != cudaSuccess) return e;
   const int n_tiles = static_cast<int>(b.mpad / kBlockTile);
-  const unsigned ctas = static_cast<unsigned>(cdiv(n_tiles, sh.mult_tiles));
+  // tiles per CTA: up to the shape's, the count whose waves of CTAs carry the fewest tiles (a CTA's
+  // setup and first loads count as half a tile). 472 tiles (60,007 points): 59 CTAs of 8 took
+  // 110 us, 118 of 4 take 63 us; 8,192 tiles (2^20 points): 6 tiles in 9 waves instead of 8 in 7.
+  // At least as many as the MMA window, whose stages then feed different accumulators.
+  int tiles = sh.mult_tiles;
+  double best = 0.0;
+  const int t_min = std::min(sh.mult_tiles, sh.window);
+  for (int t = t_min; t <= sh.mult_tiles; ++t) {
+    const double cost = static_cast<double>(cdiv(cdiv(n_tiles, t), num_sms)) * (t + 0.5);
+    if (t == t_min || cost < best) {
+      best = cost;
+      tiles = t;
+    }
+  }
+  const unsigned ctas = static_cast<unsigned>(cdiv(n_tiles, tiles));
   kern<<<ctas, (kTeamWarps * sh.teams + 2) * 32, smem, s>>>(
-      b.pc, b.gheader, b.gslots, b.coef, b.n_groups, b.n_slots, b.mpad, b.m, n_tiles, sh.mult_tiles,
+      b.pc, b.gheader, b.gslots, b.coef, b.n_groups, b.n_slots, b.mpad, b.m, n_tiles, tiles,
       gpp, sh.teams, sh.stages, sh.loads, std::min(sh.window, sh.stages), cols, b.qtiles, out64, b.status,
-      b.f16 ? 1 : 0, b.scales, std::ldexp(1.0f, b.pexp), std::ldexp(1.0f, -(b.qshift + b.pexp)));
+      b.f16 ? 1 : 0, b.scales, std::ldexp(1.0f, b.pexp), std::ldexp(1.0f, -(b.qshift + b.pexp)), b.stop);
   return cudaGetLastError();
 }
 
@@ -1440,7 +1423,7 @@ cudaError_t block_multt(BlockPlan& b, cudaStream_t s, const double* v, int64_t n
                        smem, s>>>(
       b.pc, b.gheader, b.gslots, b.qtiles, b.n_groups, b.n_slots, b.mpad, n_tiles, gpc,
       streams, sh.teams, sh.stages, sh.loads, std::min(sh.window, sh.stages), cols, b.rows, b.part, b.status,
-      b.f16 ? 1 : 0);
+      b.f16 ? 1 : 0, b.stop);
   e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   block_finish_kernel<<<grid_for(b.rows * kBlockRhs, num_sms), 256, 0, s>>>(

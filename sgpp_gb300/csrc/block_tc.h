@@ -56,6 +56,7 @@ struct BlockShape {
 };
 
 struct BlockPlan {
+  const double* stop = nullptr;  // device flag: when it is not 0 the products are skipped
   int n_groups = 0;
   int n_slots = 0;            // subspaces, in group order
   int64_t rows = 0;           // n_groups * 128
@@ -110,20 +111,21 @@ cudaError_t block_status(BlockPlan& b, cudaStream_t s, int* host_status);
 bool block_shape_ok(const BlockShape& sh, int smem_cap);
 
 // CG on 16 columns (column-major [16][np] vectors; independent systems sharing the operator).
-// Scalars on the device, at these offsets of `sc` (kBlockScalars doubles): delta in two slots
-// (the iteration's and the next one's), delta_0 of the solve, the squared relative tolerance of
-// each column, and a flag per column whose last step had d.q = 0. Dot products go through
-// `part` arrays of kBlockRhs * kBlockDotBlocks doubles.
+// Scalars on the device, at these offsets of `sc` (kBlockScalars doubles, zeroed before the first
+// solve): per column delta, delta_0 of the solve, the squared relative tolerance (a column takes steps
+// while delta > tol2 * delta_0; a step with d.q = 0 sets it to infinity) and the steps taken over all
+// solves; then the stop flag (no column takes steps any more) and two counters of the kernels.
 constexpr int kBlockDotBlocks = 64;
-constexpr int kScDelta = 0, kScDelta0 = 32, kScTol2 = 48, kScStalled = 64, kBlockScalars = 80;
+constexpr int kScDelta = 0, kScDelta0 = 16, kScTol2 = 32, kScSteps = 48, kScStop = 64, kScCount = 65,
+              kBlockScalars = 72;
 // part[k * kBlockDotBlocks + b]: per-block sums of a_k . b_k
 cudaError_t block_dot(cudaStream_t s, const double* a, const double* b, int64_t np, double* part);
-// d = r, e = 0, delta = delta_0 = r.r (slot 0)
+// d = r, e = 0, delta = delta_0 = r.r; *host (page-locked) = columns that take a step
 cudaError_t block_cg_init(cudaStream_t s, const double* r, double* d, double* e, int64_t np,
-                          double* part, double* sc);
-// one CG step on every active column (delta > tol2 * delta_0), q = A d given; reads delta from
-// slot `cur` and writes the new one to slot cur ^ 1
+                          double* sc, double* host);
+// one CG step on every column that takes steps, q = A d given; nothing once the stop flag is set.
+// *host (page-locked) = columns that take another step
 cudaError_t block_cg_step(cudaStream_t s, double* e, double* r, double* d, const double* q,
-                          int64_t np, double* part_dq, double* part_rr, double* sc, int cur);
+                          int64_t np, double* sc, double* host);
 
 }  // namespace sgmev

@@ -226,11 +226,13 @@ struct NestMultArgs {
   int64_t n;
   const void* coef;  // coefficients in position order, or nullptr: gathered while they are staged
   int warps;         // warps of a CTA that take tiles; the others only help to stage
+  const double* stop;  // device flag: when it is not 0 the product is skipped
 };
 
 template <typename V, int MD, bool MOD>
 __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
     nest_mult_kernel(const __grid_constant__ NestMultArgs a) {
+  if (a.stop && *a.stop != 0.0) return;
   constexpr int D = MD > 0 ? MD : 1, kV = sizeof(V), R = kPts<V>;
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x, all = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = a.warps;
@@ -501,6 +503,7 @@ struct NestMulttArgs {
   int n_ent, dim, nq_max, sums, streams;
   double* rows;
   int* bad;
+  const double* stop;
 };
 __device__ __forceinline__ void read_entry(float& r, const NestMulttArgs& a, int64_t k) { r = a.tab_hi[k]; }
 __device__ __forceinline__ void read_entry(double& r, const NestMulttArgs& a, int64_t k) { r = a.tab64[k]; }
@@ -509,6 +512,7 @@ __device__ __forceinline__ void read_entry(ff& r, const NestMulttArgs& a, int64_
 template <typename V, typename VIN>
 __global__ void __launch_bounds__(256) nest_multt_kernel(const __grid_constant__ NestMulttArgs a,
                                                          const VIN* __restrict__ v) {
+  if (a.stop && *a.stop != 0.0) return;
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nth >> 5;
   const int chunk = blockIdx.x / a.streams, stream = blockIdx.x - chunk * a.streams;
@@ -826,6 +830,7 @@ cudaError_t mult(NestPlan& p, cudaStream_t s, NestConfig& c, const NestDense& de
   a.out64 = out64;
   a.part = part;
   a.out_end = out_end;
+  a.stop = p.stop;
   a.dense = dense;
   a.inv = p.inv;
   a.alpha = alpha;
@@ -920,6 +925,7 @@ cudaError_t multt(NestPlan& p, cudaStream_t s, std::vector<int>& streams, const 
   a.n_ent = p.n_ent;
   a.dim = p.dim;
   a.bad = p.bad;
+  a.stop = p.stop;
   a.rows = p.rows;
   int64_t cs_at = 0;
   for (size_t k = 0; k < p.classes.size(); ++k) {

@@ -20,6 +20,7 @@ struct NestConfig {  // launch of the mult in one precision, fixed on its first 
 };
 
 struct NestPlan {
+  const double* stop = nullptr;  // device flag: when it is not 0 the products are skipped
   bool ok = false;
   bool mod = false;
   int dim = 0, n_sub = 0, n_ent = 0;

@@ -26,6 +26,7 @@
 #include "nest.h"
 #include "subspace.h"
 #include "block_tc.h"
+#include "cg_cluster.cuh"
 
 namespace sgmev {
 
@@ -57,6 +58,7 @@ constexpr int kReduceBlocks = 1216;  // 8 x 152 SMs
 constexpr int kDotBlocks = 304;
 constexpr int kDotThreads = 256;
 constexpr int kCgSlots = 10;
+constexpr int64_t kClusterVector = 262144;  // CG vectors whose steps run on one cluster (2 MB each)
 
 static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 static inline int64_t round_up(int64_t a, int64_t b) { return ceil_div(a, b) * b; }
@@ -116,6 +118,7 @@ struct sgmev_op {
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_start = nullptr, ev_stop = nullptr;
+  cudaEvent_t ev_cg[2] = {nullptr, nullptr};  // steps of the CG loop
   cudaEvent_t ev_switch = nullptr;  // orders a new stream after the work of the previous one
   double last_seconds = -1.0;
   int64_t launches = 0;
@@ -496,6 +499,31 @@ __global__ void xpby_dev_kernel(int64_t n, const double* __restrict__ r,
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x)
     d[i] = fma(beta, d[i], r[i]);
+}
+
+// The step of a short column on one cluster (cg_cluster.cuh): alpha, x, r, beta and d as the kernels
+// above, scal[5] = the loop stops after this step, and {delta_new, d.q} into page-locked memory. A
+// step enqueued ahead of a stop does nothing.
+__global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads) cg_step_kernel(
+    int64_t n, double* __restrict__ d, const double* __restrict__ q, double* __restrict__ x,
+    double* __restrict__ r, double* __restrict__ scal, double delta_0, double* __restrict__ host) {
+  if (scal[5] != 0.0) return;
+  __shared__ CgShared sh;
+  const double delta = scal[0];
+  double dq, alpha, rr;
+  cg_column_step(n, d, q, x, r, delta, true, true, sh, &dq, &alpha, &rr);
+  cg_cluster_end();  // every block has read delta
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    scal[1] = delta;
+    scal[0] = rr;
+    scal[2] = dq;
+    scal[3] = alpha;
+    scal[4] = rr / delta;
+    scal[5] = dq == 0.0 || !(rr > delta_0) || !(rr > 0.0) ? 1.0 : 0.0;
+    volatile double* h = host;
+    h[0] = rr;
+    h[1] = dq;
+  }
 }
 
 // z = a * b (elementwise)
@@ -1032,7 +1060,10 @@ static int dev_convert(sgmev_op* op, const double* in, int64_t n, int64_t npad, 
 }
 
 // out64[npad] = B^T (B a) + lm * a, a given as padded FP64 device vector [npad]
-static int dev_system(sgmev_op* op, int prec, const double* a64, double* out64, double lm) {
+// (nested products leave out64 beyond n as it was when n_only is set)
+static int dev_system(sgmev_op* op, int prec, const double* a64, double* out64, double lm,
+                      bool n_only = false) {
+  const int64_t out_end = n_only ? op->n : op->npad;
   const bool nested = nest_mults(op, prec);
   if (prec == SGMEV_FP32) {
     const bool fused = op->fused_system && !op->use_half && op->sub_ok && op->mat_multt &&
@@ -1049,16 +1080,16 @@ static int dev_system(sgmev_op* op, int prec, const double* a64, double* out64, 
       return SGMEV_OK;
     }
     SGMEV_TRY(dev_mult(op, prec, a64, op->a32, nullptr, nullptr, op->v32, 0, op->mpad));
-    SGMEV_TRY(dev_multt(op, prec, nullptr, op->v32, nullptr, out64, 0, op->npad, a64, lm));
+    SGMEV_TRY(dev_multt(op, prec, nullptr, op->v32, nullptr, out64, 0, op->npad, a64, lm, out_end));
   } else if (prec == SGMEV_DF64) {
     if (!nested) SGMEV_TRY(dev_convert(op, a64, op->npad, op->npad, nullptr, op->a32, op->a32lo));
     SGMEV_TRY(dev_mult(op, prec, a64, op->a32, op->a32lo, op->v64, nullptr, 0, op->mpad));
     if (!nest_multts(op, prec))
       SGMEV_TRY(dev_convert(op, op->v64, op->mpad, op->mpad, nullptr, op->v32, op->v32lo));
-    SGMEV_TRY(dev_multt(op, prec, op->v64, op->v32, op->v32lo, out64, 0, op->npad, a64, lm));
+    SGMEV_TRY(dev_multt(op, prec, op->v64, op->v32, op->v32lo, out64, 0, op->npad, a64, lm, out_end));
   } else {
     SGMEV_TRY(dev_mult(op, prec, a64, nullptr, nullptr, op->v64, nullptr, 0, op->mpad));
-    SGMEV_TRY(dev_multt(op, prec, op->v64, nullptr, nullptr, out64, 0, op->npad, a64, lm));
+    SGMEV_TRY(dev_multt(op, prec, op->v64, nullptr, nullptr, out64, 0, op->npad, a64, lm, out_end));
   }
   return SGMEV_OK;
 }
@@ -1242,6 +1273,8 @@ static void release(sgmev_op* op) {
   if (op->ev_start) cudaEventDestroy(op->ev_start);
   if (op->ev_stop) cudaEventDestroy(op->ev_stop);
   if (op->ev_switch) cudaEventDestroy(op->ev_switch);
+  for (cudaEvent_t e : op->ev_cg)
+    if (e) cudaEventDestroy(e);
   if (op->own_stream) cudaStreamDestroy(op->own_stream);
   (void)cudaGetLastError();
 }
@@ -1500,6 +1533,7 @@ SGMEV_API int sgmev_create(sgmev_op** out, int dim, int64_t n_grid, const double
   CREATE_CUDA(cudaEventCreate(&op->ev_start));
   CREATE_CUDA(cudaEventCreate(&op->ev_stop));
   CREATE_CUDA(cudaEventCreateWithFlags(&op->ev_switch, cudaEventDisableTiming));
+  for (cudaEvent_t& e : op->ev_cg) CREATE_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   op->host_scalar = static_cast<double*>(pinned_block());
   if (!op->host_scalar) return bail(fail(SGMEV_ERR_OOM, "pinned host block"));
   CREATE_TRY(dalloc(op->stream, &op->dot_part, kDotBlocks));
@@ -1827,7 +1861,7 @@ SGMEV_API int sgmev_system_apply_device(sgmev_op* op, const double* d_alpha, dou
 static int cg_core(sgmev_op* op, int prec, const double* rhs, double* x, double lm,
                    int64_t imax, double eps, bool reuse, int64_t* iters, double* delta_final) {
   using namespace sgmev;
-  const int64_t np = op->npad;
+  const int64_t np = op->npad, n = op->n;
   double* r = op->cg + 2 * np;
   double* d = op->cg + 3 * np;
   double* q = op->cg + 4 * np;
@@ -1860,7 +1894,8 @@ static int cg_core(sgmev_op* op, int prec, const double* rhs, double* x, double 
     return SGMEV_OK;
   };
   // delta_new = r.r (the update kernel without steps)
-  cg_update_kernel<<<kDotBlocks, kDotThreads, 0, op->stream>>>(np, d, q, x, r, 0, 1,
+  SGMEV_CUDA(cudaMemsetAsync(sc + 5, 0, sizeof(double), op->stream));
+  cg_update_kernel<<<kDotBlocks, kDotThreads, 0, op->stream>>>(n, d, q, x, r, 0, 1,
                                                                  op->dot_part, sc);
   op->launches += 1;
   SGMEV_CUDA(cudaGetLastError());
@@ -1868,31 +1903,81 @@ static int cg_core(sgmev_op* op, int prec, const double* rhs, double* x, double 
   double delta_new = host[0];
   if (!reuse) delta_0 = delta_new * eps2;
   int64_t it = 0;
-  while (it < imax && delta_new > delta_0 && delta_new > 0.0) {
-    SGMEV_TRY(dev_system(op, prec, d, q, lm));
-    cg_alpha_kernel<<<kDotBlocks, kDotThreads, 0, op->stream>>>(d, q, np, op->dot_part, sc);
+  // one step with the kernels of any length; every 50 iterations with the true residual
+  // (ConjugateGradients.cpp:99-104)
+  auto step = [&]() -> int {
+    SGMEV_TRY(dev_system(op, prec, d, q, lm, true));
+    cg_alpha_kernel<<<kDotBlocks, kDotThreads, 0, op->stream>>>(d, q, n, op->dot_part, sc);
     op->launches += 1;
     if (it % 50 == 0 && it > 0) {
-      // the true residual every 50 iterations (ConjugateGradients.cpp:99-104)
-      axpy_dev_kernel<<<vec_blocks(np), 256, 0, op->stream>>>(np, sc, d, x);
-      SGMEV_TRY(dev_system(op, prec, x, t, lm));
-      sub_kernel<<<vec_blocks(np), 256, 0, op->stream>>>(np, rhs, t, r);
-      cg_update_kernel<<<kDotBlocks, kDotThreads, 0, op->stream>>>(np, d, q, x, r, 0, 1,
+      axpy_dev_kernel<<<vec_blocks(n), 256, 0, op->stream>>>(n, sc, d, x);
+      SGMEV_TRY(dev_system(op, prec, x, t, lm, true));
+      sub_kernel<<<vec_blocks(n), 256, 0, op->stream>>>(n, rhs, t, r);
+      cg_update_kernel<<<kDotBlocks, kDotThreads, 0, op->stream>>>(n, d, q, x, r, 0, 1,
                                                                      op->dot_part, sc);
       op->launches += 3;
     } else {
-      cg_update_kernel<<<kDotBlocks, kDotThreads, 0, op->stream>>>(np, d, q, x, r, 1, 0,
+      cg_update_kernel<<<kDotBlocks, kDotThreads, 0, op->stream>>>(n, d, q, x, r, 1, 0,
                                                                      op->dot_part, sc);
       op->launches += 1;
     }
-    xpby_dev_kernel<<<vec_blocks(np), 256, 0, op->stream>>>(np, r, sc, d);
+    xpby_dev_kernel<<<vec_blocks(n), 256, 0, op->stream>>>(n, r, sc, d);
     op->launches += 1;
     SGMEV_CUDA(cudaGetLastError());
-    SGMEV_TRY(read_scalars());
-    // d.q == 0: alpha was 0, so x and r did not move; stop as the reference does before a step
-    if (host[2] == 0.0) break;
-    delta_new = host[0];
-    ++it;
+    return read_scalars();
+  };
+  auto running = [&] { return it < imax && delta_new > delta_0 && delta_new > 0.0; };
+  // Up to kClusterVector entries a step's vector work is one cluster's, and the host enqueues a step
+  // before it reads the previous one's delta, so that the device never waits for it: a step beyond the
+  // stop finds scal[5] set and skips its products and updates. Not across the true residual's steps, and
+  // not where the mult would run all the same (the materialised and on-the-fly ones do).
+  if (n <= kClusterVector) {
+    const bool ahead = nest_mults(op, prec);
+    struct StopScope {
+      sgmev_op* o;
+      StopScope(sgmev_op* op_, const double* flag) : o(op_) { o->nest.stop = o->sub.stop = flag; }
+      ~StopScope() { o->nest.stop = o->sub.stop = nullptr; }
+    };
+    auto enqueue = [&](int64_t k) -> int {
+      StopScope scope(op, sc + 5);
+      SGMEV_TRY(dev_system(op, prec, d, q, lm, true));
+      cg_step_kernel<<<kCgCtas, kCgThreads, 0, op->stream>>>(n, d, q, x, r, sc, delta_0, host + 4 * (k & 1));
+      op->launches += 1;
+      SGMEV_CUDA(cudaGetLastError());
+      SGMEV_CUDA(cudaEventRecord(op->ev_cg[k & 1], op->stream));
+      return SGMEV_OK;
+    };
+    int64_t queued = 0;  // steps enqueued
+    while (running()) {
+      if (it % 50 == 0 && it > 0) {
+        SGMEV_TRY(step());
+        queued = it + 1;
+        if (host[2] == 0.0) break;
+        delta_new = host[0];
+      } else {
+        if (queued == it) {
+          SGMEV_TRY(enqueue(it));
+          ++queued;
+        }
+        if (ahead && queued < imax && queued % 50 != 0) {
+          SGMEV_TRY(enqueue(queued));
+          ++queued;
+        }
+        SGMEV_CUDA(cudaEventSynchronize(op->ev_cg[it & 1]));
+        const volatile double* h = host + 4 * (it & 1);
+        // d.q == 0: alpha was 0, so x and r did not move; stop as the reference does before a step
+        if (h[1] == 0.0) break;
+        delta_new = h[0];
+      }
+      ++it;
+    }
+  } else {
+    while (running()) {
+      SGMEV_TRY(step());
+      if (host[2] == 0.0) break;
+      delta_new = host[0];
+      ++it;
+    }
   }
   SGMEV_CUDA(cudaGetLastError());
   *iters = it;
@@ -2281,7 +2366,7 @@ static int fit_block_common(sgmev_op* op, const double* y, bool y_dev, double la
   DevBuf buf(op->stream);
   const size_t vec = static_cast<size_t>(K) * np;
   const size_t parts = static_cast<size_t>(K) * kBlockDotBlocks;
-  SGMEV_CUDA(dev_malloc(&buf.p, sizeof(double) * (8 * vec + 2 * parts + kBlockScalars), op->stream));
+  SGMEV_CUDA(dev_malloc(&buf.p, sizeof(double) * (8 * vec + parts + kBlockScalars), op->stream));
   double* b = static_cast<double*>(buf.p);
   double* x = b + vec;
   double* rr = x + vec;
@@ -2291,8 +2376,7 @@ static int fit_block_common(sgmev_op* op, const double* y, bool y_dev, double la
   double* q = d + vec;
   double* t = q + vec;
   double* part_a = t + vec;
-  double* part_b = part_a + parts;
-  double* sc = part_b + parts;
+  double* sc = part_a + parts;
   SGMEV_CUDA(cudaMemsetAsync(sc, 0, sizeof(double) * kBlockScalars, op->stream));
   SGMEV_TRY(begin_timed(op));
   // b_k = B^T y_k with the FP64-accurate df64 products (generateb per column)
@@ -2307,8 +2391,7 @@ static int fit_block_common(sgmev_op* op, const double* y, bool y_dev, double la
                         0.0));
   }
   SGMEV_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * vec, op->stream));
-  std::vector<double> host(3 * K + parts), rho(K, 0.0), rho0(K, 0.0), tol2(K, 0.0);
-  std::vector<int64_t> col_it(K, 0);
+  std::vector<double> host(std::max<size_t>(parts, K)), rho(K, 0.0), rho0(K, 0.0), tol2(K, 0.0);
   std::vector<char> done(K, 0);
   auto block_norms = [&](const double* v, std::vector<double>& out) -> int {
     SGMEV_CUDA(block_dot(op->stream, v, v, np, part_a));
@@ -2352,40 +2435,31 @@ static int fit_block_common(sgmev_op* op, const double* y, bool y_dev, double la
     SGMEV_CUDA(cudaMemcpyAsync(sc + kScTol2, tol2.data(), sizeof(double) * K, cudaMemcpyHostToDevice,
                                op->stream));
     SGMEV_CUDA(cudaMemcpyAsync(r, rr, sizeof(double) * vec, cudaMemcpyDeviceToDevice, op->stream));
-    SGMEV_CUDA(block_cg_init(op->stream, r, d, e, np, part_a, sc));
-    op->launches += 2;
-    int cur = 0;
-    int64_t steps = 0;
-    while (total_it < max_iterations) {
-      SGMEV_CUDA(cudaMemcpyAsync(host.data(), sc + kScDelta + cur * K, sizeof(double) * K,
-                                 cudaMemcpyDeviceToHost, op->stream));
-      SGMEV_CUDA(cudaMemcpyAsync(host.data() + K, sc + kScDelta0, sizeof(double) * K,
-                                 cudaMemcpyDeviceToHost, op->stream));
-      SGMEV_CUDA(cudaMemcpyAsync(host.data() + 2 * K, sc + kScStalled, sizeof(double) * K,
-                                 cudaMemcpyDeviceToHost, op->stream));
-      SGMEV_CUDA(cudaStreamSynchronize(op->stream));
-      int active = 0;
-      bool stalled = false;
-      for (int k = 0; k < K; ++k) {
-        if (host[2 * K + k] != 0.0 && tol2[k] != HUGE_VAL) {
-          tol2[k] = HUGE_VAL;  // d.q = 0: the column cannot move (the reference stops there too)
-          stalled = true;
-        }
-        if (host[k] > tol2[k] * host[K + k]) {
-          ++active;
-          ++col_it[k];
-        }
+    // The host enqueues a step before it reads how many columns the previous one leaves active; a
+    // step beyond the last finds the stop flag set and skips its products and updates.
+    double* slots = op->host_scalar;  // page-locked: columns that take the next step, by parity
+    SGMEV_CUDA(block_cg_init(op->stream, r, d, e, np, sc, slots + 1));
+    SGMEV_CUDA(cudaEventRecord(op->ev_cg[1], op->stream));
+    op->launches += 1;
+    struct StopScope {
+      sgmev_op* o;
+      StopScope(sgmev_op* op_, const double* flag) : o(op_) { o->blk.stop = flag; }
+      ~StopScope() { o->blk.stop = nullptr; }
+    } stop_scope(op, sc + kScStop);
+    int64_t steps = 0, queued = 0;
+    while (true) {
+      if (total_it + queued - steps < max_iterations) {
+        SGMEV_TRY(block_system(op, d, q, lm));
+        SGMEV_CUDA(block_cg_step(op->stream, e, r, d, q, np, sc, slots + (queued & 1)));
+        SGMEV_CUDA(cudaEventRecord(op->ev_cg[queued & 1], op->stream));
+        op->launches += 1;
+        ++queued;
       }
-      if (stalled)
-        SGMEV_CUDA(cudaMemcpyAsync(sc + kScTol2, tol2.data(), sizeof(double) * K,
-                                   cudaMemcpyHostToDevice, op->stream));
-      if (active == 0) break;
-      SGMEV_TRY(block_system(op, d, q, lm));
-      SGMEV_CUDA(block_cg_step(op->stream, e, r, d, q, np, part_a, part_b, sc, cur));
-      op->launches += 3;
-      cur ^= 1;
-      ++total_it;
+      // what the step before number `steps` (for 0: the start) left
+      SGMEV_CUDA(cudaEventSynchronize(op->ev_cg[(steps + 1) & 1]));
+      if (*static_cast<const volatile double*>(slots + ((steps + 1) & 1)) == 0.0 || queued == steps) break;
       ++steps;
+      ++total_it;
     }
     axpy_kernel<<<vec_blocks(static_cast<int64_t>(vec)), 256, 0, op->stream>>>(
         static_cast<int64_t>(vec), 1.0, e, x);
@@ -2401,10 +2475,12 @@ static int fit_block_common(sgmev_op* op, const double* y, bool y_dev, double la
                                  op->stream));
   SGMEV_TRY(end_timed(op, true));
   SGMEV_TRY(block_check(op));
-  for (int k = 0; k < K; ++k) {
-    if (iterations) iterations[k] = col_it[k];
-    if (residuals) residuals[k] = rho[k];
+  if (iterations) {
+    SGMEV_CUDA(cudaMemcpyAsync(host.data(), sc + kScSteps, sizeof(double) * K, cudaMemcpyDeviceToHost, op->stream));
+    SGMEV_CUDA(cudaStreamSynchronize(op->stream));
+    for (int k = 0; k < K; ++k) iterations[k] = static_cast<int64_t>(host[k]);
   }
+  if (residuals) std::copy(rho.begin(), rho.end(), residuals);
   return SGMEV_OK;
 }
 

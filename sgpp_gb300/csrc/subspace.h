@@ -29,6 +29,8 @@ inline cudaError_t set_smem_cap(Kernel kern, size_t need) {
 // offset + sum_t ((i_t - 1) / 2) * stride_t. Positions without a grid point (adaptive grids)
 // carry alpha = 0 and are ignored on output.
 struct SubPlan {
+  // device flag: when it is not 0 the FP16 and float-float materialised multTranspose is skipped
+  const double* stop = nullptr;
   int dim = 0;
   int n_sub = 0;
   int64_t total = 0;      // positions

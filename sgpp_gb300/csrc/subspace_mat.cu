@@ -492,7 +492,8 @@ __global__ void __launch_bounds__(kMatThreads, 2) mat_multt_half_kernel(
     const int4* __restrict__ sact, int n_sub, int s_pad, int cmax, int total,
     const float* __restrict__ v, int64_t n_tiles, const uint4* __restrict__ pp,
     const typename PairCells<CW>::T* __restrict__ cp, double* __restrict__ rows, int streams,
-    double unscale) {
+    double unscale, const double* __restrict__ stop) {
+  if (stop && *stop != 0.0) return;
   using PC = PairCells<CW>;
   using CT = typename PC::T;
   constexpr int A = kPairAheadMultT;
@@ -629,7 +630,8 @@ __global__ void __launch_bounds__(kMatThreads, 2) mat_multt_half_banked_kernel(
     const int4* __restrict__ sact, int n_sub, int s_pad, int cmax, int total,
     const float* __restrict__ v, int64_t n_tiles, const uint4* __restrict__ pp,
     const typename PairCells<CW>::T* __restrict__ cp, double* __restrict__ rows, int streams,
-    double unscale) {
+    double unscale, const double* __restrict__ stop) {
+  if (stop && *stop != 0.0) return;
   using PC = PairCells<CW>;
   using CT = typename PC::T;
   constexpr int A = kPairAheadMultT;
@@ -729,7 +731,8 @@ __global__ void __launch_bounds__(kMatThreads, 3) mat_multt_half_lean_kernel(
     const int4* __restrict__ sact, int n_sub, int s_pad, int cmax, int total,
     const float* __restrict__ v, int64_t n_tiles, const uint4* __restrict__ pp,
     const typename PairCells<CW>::T* __restrict__ cp, double* __restrict__ rows, int streams,
-    double unscale) {
+    double unscale, const double* __restrict__ stop) {
+  if (stop && *stop != 0.0) return;
   using PC = PairCells<CW>;
   using CT = typename PC::T;
   constexpr int A = 2;
@@ -921,7 +924,8 @@ __global__ void __launch_bounds__(kMatThreads, 1) mat_multt_df_kernel(
     const int4* __restrict__ sact, int n_sub, int s_pad, int cmax, int total,
     const float* __restrict__ vh, const float* __restrict__ vl, int64_t n_tiles,
     const float4* __restrict__ phi, const float4* __restrict__ plo,
-    const CW* __restrict__ cm, double* __restrict__ rows) {
+    const CW* __restrict__ cm, double* __restrict__ rows, const double* __restrict__ stop) {
+  if (stop && *stop != 0.0) return;
   extern __shared__ __align__(16) unsigned char smem[];
   const int tid = threadIdx.x, nth = blockDim.x;
   double* s_sum = reinterpret_cast<double*>(smem);  // [cmax][blockDim] (SACC)
@@ -1400,7 +1404,7 @@ cudaError_t launch_multt_df(const SubPlan& p, cudaStream_t s, int64_t mpad, cons
   *rows = std::min<int64_t>(std::max(1, per_sm) * static_cast<int64_t>(num_sms), std::min<int64_t>(p.row_cap, std::max<int64_t>(nt, 1)));
   kern<<<static_cast<unsigned>(*rows), nth, sm, s>>>(
       p.sact, p.n_sub, static_cast<int>(p.s_pad), p.cmax, static_cast<int>(p.total), vh, vl, nt,
-      p.pmat, p.pmat_lo, static_cast<const CW*>(p.cmat), p.rows);
+      p.pmat, p.pmat_lo, static_cast<const CW*>(p.cmat), p.rows, p.stop);
   return cudaGetLastError();
 }
 
@@ -1491,18 +1495,18 @@ cudaError_t launch_mat_multt(const SubPlan& p, cudaStream_t s, int64_t mpad, con
     // two banks take the shared memory of the single bank with its float-float sums
     // three CTAs per SM while their FP32 cell sums leave room for three (else the kernels above)
     if (p.multt_ctas == 3 && sizeof(float) * static_cast<size_t>(p.cmax) * nth <= 72 * 1024)
-      return go_lean(mat_multt_half_lean_kernel<CW>, pm, cm, un);
-    if (p.multt_banks == 2 && sacc) return go(mat_multt_half_banked_kernel<CW>, pm, cm, un);
+      return go_lean(mat_multt_half_lean_kernel<CW>, pm, cm, un, p.stop);
+    if (p.multt_banks == 2 && sacc) return go(mat_multt_half_banked_kernel<CW>, pm, cm, un, p.stop);
     switch (p.multt_batch) {
       case 2:
-        return sacc ? go(mat_multt_half_kernel<CW, true, 2>, pm, cm, un)
-                    : go(mat_multt_half_kernel<CW, false, 2>, pm, cm, un);
+        return sacc ? go(mat_multt_half_kernel<CW, true, 2>, pm, cm, un, p.stop)
+                    : go(mat_multt_half_kernel<CW, false, 2>, pm, cm, un, p.stop);
       case 4:
-        return sacc ? go(mat_multt_half_kernel<CW, true, 4>, pm, cm, un)
-                    : go(mat_multt_half_kernel<CW, false, 4>, pm, cm, un);
+        return sacc ? go(mat_multt_half_kernel<CW, true, 4>, pm, cm, un, p.stop)
+                    : go(mat_multt_half_kernel<CW, false, 4>, pm, cm, un, p.stop);
       default:
-        return sacc ? go(mat_multt_half_kernel<CW, true, 1>, pm, cm, un)
-                    : go(mat_multt_half_kernel<CW, false, 1>, pm, cm, un);
+        return sacc ? go(mat_multt_half_kernel<CW, true, 1>, pm, cm, un, p.stop)
+                    : go(mat_multt_half_kernel<CW, false, 1>, pm, cm, un, p.stop);
     }
   } else {
     const float4* pm = p.pmat;
