@@ -11,6 +11,8 @@ std::mutex g_mu;
 std::vector<cudaMemPool_t> g_pools;  // per device: the library's own pool (nullptr: not made yet)
 std::vector<void*> g_pinned;         // recycled pinned blocks
 constexpr size_t kPinnedBytes = 64;
+constexpr size_t kKeptStreams = 32;
+std::vector<std::vector<cudaStream_t>> g_streams;  // per device: idle streams of past operators
 
 // The library allocates from a pool of its own, not from the device's default pool: its release
 // threshold is raised so that freed blocks stay for the next operator, and raising it on the
@@ -63,6 +65,44 @@ cudaError_t dev_malloc(void** p, size_t bytes, cudaStream_t s) {
 
 void dev_free(void* p, cudaStream_t s) {
   if (p) cudaFreeAsync(p, s);
+}
+
+cudaStream_t stream_acquire() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (dev < static_cast<int>(g_streams.size()) && !g_streams[dev].empty()) {
+      cudaStream_t s = g_streams[dev].back();  // the one most recently in use
+      g_streams[dev].pop_back();
+      return s;
+    }
+  }
+  cudaStream_t s = nullptr;
+  if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  return s;
+}
+
+void stream_release(cudaStream_t s) {
+  if (!s) return;
+  int dev = 0;
+  if (cudaStreamGetDevice(s, &dev) == cudaSuccess) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (static_cast<int>(g_streams.size()) <= dev) g_streams.resize(dev + 1);
+    if (g_streams[dev].size() < kKeptStreams) {
+      g_streams[dev].push_back(s);
+      return;
+    }
+  } else {
+    (void)cudaGetLastError();
+  }
+  cudaStreamDestroy(s);
 }
 
 void* pinned_block() {

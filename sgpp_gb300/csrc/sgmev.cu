@@ -139,6 +139,7 @@ struct sgmev_op {
   int algo = 2;          // FP32 products: 0 dense, 1 subspace, 2 auto (params "algo")
   SubPlan sub;           // subspace tables of the current grid
   bool sub_ok = false;   // sub is built and chosen for the FP32 products
+  bool sub_tried = false;  // sub_ok is decided for the current grid (sub_ready())
   // nested subspace plan of the FP64 products, built on the first of them from the eval arrays
   sgmev::NestPlan nest;
   bool nest_failed = false;  // the current grid is not one the nested kernels take
@@ -856,6 +857,32 @@ static int64_t multt_tile_pts(const sgmev_op* op, int prec) {
 // ---------------------------------------------------------------------------------------
 // device-side products on padded device vectors
 // ---------------------------------------------------------------------------------------
+// subspace tables for the materialised and on-the-fly FP32 and float-float products, built when a
+// product first asks for them: used when chosen ("algo") and cheaper than the dense kernels by the
+// instruction count per data point (one basis function per subspace, ~8 per active dimension and ~10
+// per subspace, against 3 per dimension for every grid point)
+static bool sub_ready(sgmev_op* op, std::string* why = nullptr) {
+  using namespace sgmev;
+  if (op->sub_tried) return op->sub_ok;
+  op->sub_tried = true;
+  if (op->algo == 0 || op->n < 1) return false;
+  std::string reason;
+  if (!subspace_build(&op->sub, op->dim, op->n, op->h_level_pow2.data(), op->h_index.data(), op->stream,
+                      &reason)) {
+    if (why) *why = reason;
+    return false;
+  }
+  op->sub.mod = op->mod;
+  op->sub.multt_batch = op->multt_batch;
+  op->sub.multt_banks = op->multt_banks;
+  op->sub.multt_ctas = op->multt_ctas;
+  const double dense_cost = 3.0 * op->dim * static_cast<double>(op->n);
+  const double sub_cost = 8.0 * static_cast<double>(op->sub.act_work) + 10.0 * op->sub.n_sub;
+  op->sub_ok = op->algo == 1 || sub_cost * 1.5 < dense_cost;
+  if (!op->sub_ok) subspace_free(&op->sub);
+  return op->sub_ok;
+}
+
 // Materialised FP32 subspace products: built on the first FP32 product after the grid was
 // staged, when the "materialize" knob allows it and they fit (auto: at most half of the free
 // device memory and 64 GiB); a failed build falls back to the on-the-fly kernels for this grid.
@@ -926,7 +953,7 @@ static bool nest_multts(sgmev_op* op, int prec) {
   if (!nest_mults(op, prec)) return false;
   if (prec == SGMEV_FP64 || op->m <= 8192) return true;
   return prec == SGMEV_DF64 && static_cast<double>(op->nest.n_sub) * op->m <= 1e8 &&
-         !(op->sub_ok && op->mat_multt && subspace_mat_fits(op->sub, true) && mat_ready(op));
+         !(sub_ready(op) && op->mat_multt && subspace_mat_fits(op->sub, true) && mat_ready(op));
 }
 
 // Inputs: a64 [n] where nest_mults(); otherwise per precision FP64 a64; FP32 a32; DF64 (a32, a32lo) —
@@ -954,14 +981,14 @@ static int dev_mult(sgmev_op* op, int prec, const double* a64, const float* a32,
     SGMEV_TRY(run_mult<double>(op, op->xt64, op->li64, a64, j_begin, j_end, &p));
     if (out64) SGMEV_TRY((run_reduce<double, double>(op, (int)p.nsplit, op->mpad, j_begin, valid, total, out64, nullptr, 0.0)));
     if (out32) SGMEV_TRY((run_reduce<double, float>(op, (int)p.nsplit, op->mpad, j_begin, valid, total, out32, nullptr, 0.0)));
-  } else if (prec == SGMEV_DF64 && op->sub_ok && out64 && !out32 && mat_ready(op) &&
+  } else if (prec == SGMEV_DF64 && sub_ready(op) && out64 && !out32 && mat_ready(op) &&
              subspace_mat_fits(op->sub, true)) {
     const long ev = prof_begin(op, KIND_MULT_MATDF);
     SGMEV_CUDA(subspace_mult_mat_df(op->sub, op->stream, op->mpad, op->m, a32, a32lo, out64,
                                     j_begin, j_end, op->num_sms));
     prof_end(op, ev);
     op->launches += 2;
-  } else if (prec == SGMEV_DF64 && op->sub_ok && !op->mod && out64 && !out32) {
+  } else if (prec == SGMEV_DF64 && sub_ready(op) && !op->mod && out64 && !out32) {
     const long ev = prof_begin(op, KIND_MULT_SUBDF);
     SGMEV_CUDA(subspace_mult_df(op->sub, op->stream, op->xt32, op->xt32lo, op->mpad, op->m, a32,
                                 a32lo, out64, j_begin, j_end, op->num_sms));
@@ -971,13 +998,13 @@ static int dev_mult(sgmev_op* op, int prec, const double* a64, const float* a32,
     SGMEV_TRY(run_mult_df(op, a32, a32lo, j_begin, j_end, &p));
     if (out64) SGMEV_TRY((run_reduce<float2, double>(op, (int)p.nsplit, op->mpad, j_begin, valid, total, out64, nullptr, 0.0)));
     if (out32) SGMEV_TRY((run_reduce<float2, float>(op, (int)p.nsplit, op->mpad, j_begin, valid, total, out32, nullptr, 0.0)));
-  } else if (op->sub_ok && mat_ready(op)) {
+  } else if (sub_ready(op) && mat_ready(op)) {
     const long ev = prof_begin(op, op->use_half ? KIND_MULT_MAT16 : KIND_MULT_MAT32);
     SGMEV_CUDA(subspace_mult_mat(op->sub, op->stream, op->xt32, op->mpad, op->m, a32, out32, out64,
                                  j_begin, j_end, op->num_sms, op->use_half));
     prof_end(op, ev);
     op->launches += 2;
-  } else if (op->sub_ok && !op->mod) {
+  } else if (sub_ready(op) && !op->mod) {
     const long ev = prof_begin(op, KIND_MULT_SUB32);
     SGMEV_CUDA(subspace_mult(op->sub, op->stream, op->xt32, op->mpad, op->m, a32, out32, out64,
                              j_begin, j_end, op->num_sms));
@@ -1012,7 +1039,7 @@ static int dev_multt(sgmev_op* op, int prec, const double* v64, const float* v32
   } else if (prec == SGMEV_FP64) {
     SGMEV_TRY(run_multt<double>(op, op->xt64, v64, op->li64, g_begin, g_end, &p));
     SGMEV_TRY((run_reduce<double, double>(op, (int)p.nsplit, op->npad, g_begin, valid, g_end, out64, add, scale)));
-  } else if (prec == SGMEV_DF64 && op->sub_ok && op->mat_multt && mat_ready(op) &&
+  } else if (prec == SGMEV_DF64 && sub_ready(op) && op->mat_multt && mat_ready(op) &&
              subspace_mat_fits(op->sub, true)) {
     // the subspace sums produce every grid entry at once (the range is a subset of them)
     const long ev = prof_begin(op, KIND_MULTT_MATDF);
@@ -1020,7 +1047,7 @@ static int dev_multt(sgmev_op* op, int prec, const double* v64, const float* v32
                                      add, scale, op->num_sms));
     prof_end(op, ev);
     op->launches += 3;
-  } else if (prec == SGMEV_DF64 && op->sub_ok && !op->mod && subspace_owner_fits(op->sub, true)) {
+  } else if (prec == SGMEV_DF64 && sub_ready(op) && !op->mod && subspace_owner_fits(op->sub, true)) {
     // the subspace sums produce every grid entry at once (the range is a subset of them)
     const long ev = prof_begin(op, KIND_MULTT_SUBDF);
     SGMEV_CUDA(subspace_multt_df(op->sub, op->stream, op->xt32, op->xt32lo, op->mpad, op->m, v32,
@@ -1030,14 +1057,14 @@ static int dev_multt(sgmev_op* op, int prec, const double* v64, const float* v32
   } else if (prec == SGMEV_DF64) {
     SGMEV_TRY(run_multt_df(op, v32, v32lo, g_begin, g_end, &p));
     SGMEV_TRY((run_reduce<float2, double>(op, (int)p.nsplit, op->npad, g_begin, valid, g_end, out64, add, scale)));
-  } else if (op->sub_ok && op->mat_multt && mat_ready(op)) {
+  } else if (sub_ready(op) && op->mat_multt && mat_ready(op)) {
     // the subspace sums produce every grid entry at once (the range is a subset of them)
     const long ev = prof_begin(op, op->use_half ? KIND_MULTT_MAT16 : KIND_MULTT_MAT32);
     SGMEV_CUDA(subspace_multt_mat(op->sub, op->stream, op->xt32, op->mpad, op->m, v32, op->npad,
                                   out64, add, scale, op->num_sms, op->use_half));
     prof_end(op, ev);
     op->launches += 3;
-  } else if (op->sub_ok && !op->mod) {
+  } else if (sub_ready(op) && !op->mod) {
     // the subspace scatter produces every grid entry at once (the range is a subset of it)
     const long ev = prof_begin(op, KIND_MULTT_SUB32);
     SGMEV_CUDA(subspace_multt(op->sub, op->stream, op->xt32, op->mpad, op->m, v32, op->npad,
@@ -1066,7 +1093,7 @@ static int dev_system(sgmev_op* op, int prec, const double* a64, double* out64, 
   const int64_t out_end = n_only ? op->n : op->npad;
   const bool nested = nest_mults(op, prec);
   if (prec == SGMEV_FP32) {
-    const bool fused = op->fused_system && !op->use_half && op->sub_ok && op->mat_multt &&
+    const bool fused = op->fused_system && !op->use_half && sub_ready(op) && op->mat_multt &&
                        mat_ready(op) && subspace_system_mat_fits(op->sub);
     if (fused || !nested)
       SGMEV_TRY(dev_convert(op, a64, op->npad, op->npad, nullptr, op->a32, nullptr));
@@ -1147,16 +1174,18 @@ static int64_t part_need_elems(const sgmev_op* op) {
 static int check_grid(int dim, int64_t n, const double* level_pow2, const double* index) {
   for (int64_t k = 0; k < n * dim; ++k) {
     const double L = level_pow2[k], I = index[k];
-    if (!(L >= 2.0) || L > 1099511627776.0 || std::floor(L) != L) {
-      return fail(SGMEV_ERR_UNSUPPORTED,
-                  "level entry " + std::to_string(k) + " is not 2^l with l >= 1 (hat basis "
-                  "without boundary only)");
-    }
-    const double lg = std::log2(L);
-    if (std::floor(lg) != lg) {
+    uint64_t bits;
+    std::memcpy(&bits, &L, sizeof(bits));
+    // a finite power of two has no mantissa bits
+    if (!(L >= 2.0) || L > 1099511627776.0 || (bits & ((uint64_t(1) << 52) - 1)) != 0) {
+      if (!(L >= 2.0) || L > 1099511627776.0 || std::floor(L) != L)
+        return fail(SGMEV_ERR_UNSUPPORTED,
+                    "level entry " + std::to_string(k) + " is not 2^l with l >= 1 (hat basis "
+                    "without boundary only)");
       return fail(SGMEV_ERR_UNSUPPORTED, "level entry " + std::to_string(k) + " is not a power of two");
     }
-    if (!(I >= 1.0) || !(I < L) || std::floor(I) != I || std::fmod(I, 2.0) != 1.0) {
+    if (!(I >= 1.0) || !(I < L) || static_cast<double>(static_cast<int64_t>(I)) != I ||
+        (static_cast<int64_t>(I) & 1) == 0) {
       return fail(SGMEV_ERR_UNSUPPORTED,
                   "index entry " + std::to_string(k) + " is not an odd integer in (0, 2^l)");
     }
@@ -1207,11 +1236,12 @@ static int stage_grid(sgmev_op* op, int64_t n, const double* level_pow2, const d
   e = cudaStreamSynchronize(op->stream);
   dev_free(d_l, op->stream);
   dev_free(d_i, op->stream);
-  if (e != cudaSuccess) return fail(SGMEV_ERR_CUDA, std::string("stage grid: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) return fail(SGMEV_ERR_CUDA, std::string("stage data and grid: ") + cudaGetErrorString(e));
   // subspace tables for the FP32 products: used when chosen ("algo") and cheaper by the
   // instruction count per data point (one basis function per subspace, ~8 per active dimension
   // and ~10 per subspace, against 3 per dimension for every grid point)
   op->sub_ok = false;
+  op->sub_tried = false;
   op->mat_failed = false;
   op->mat_block_only = false;
   block_free(&op->blk);
@@ -1222,20 +1252,9 @@ static int stage_grid(sgmev_op* op, int64_t n, const double* level_pow2, const d
   op->nest_failed = false;
   op->h_level_pow2.assign(level_pow2, level_pow2 + n * op->dim);
   op->h_index.assign(index, index + n * op->dim);
-  if (op->algo != 0 && n > 0) {
+  if (op->algo == 1 && n > 0) {  // asked for: refused here when the grid is not one for it
     std::string why;
-    if (subspace_build(&op->sub, op->dim, n, level_pow2, index, op->stream, &why)) {
-      op->sub.mod = op->mod;
-      op->sub.multt_batch = op->multt_batch;
-      op->sub.multt_banks = op->multt_banks;
-      op->sub.multt_ctas = op->multt_ctas;
-      const double dense_cost = 3.0 * op->dim * static_cast<double>(n);
-      const double sub_cost = 8.0 * static_cast<double>(op->sub.act_work) + 10.0 * op->sub.n_sub;
-      op->sub_ok = op->algo == 1 || sub_cost * 1.5 < dense_cost;
-      if (!op->sub_ok) subspace_free(&op->sub);
-    } else if (op->algo == 1) {
-      return fail(SGMEV_ERR_UNSUPPORTED, "algo \"subspace\": " + why);
-    }
+    if (!sub_ready(op, &why)) return fail(SGMEV_ERR_UNSUPPORTED, "algo \"subspace\": " + why);
   }
   // output vector and split partials depend on npad
   SGMEV_TRY(dalloc(op->stream, &op->out64, static_cast<size_t>(std::max(op->npad, op->mpad))));
@@ -1260,6 +1279,8 @@ static void release(sgmev_op* op) {
   // the op's own stream covers all of the op's work.
   if (op->stream) cudaStreamSynchronize(op->stream);
   if (op->own_stream && op->own_stream != op->stream) cudaStreamSynchronize(op->own_stream);
+  // everything is idle: free on the op's own stream, which goes back with the memory
+  if (op->own_stream) op->stream = op->blk.stream = op->sub.stream = op->nest.stream = op->own_stream;
   block_free(&op->blk);
   subspace_free(&op->sub);
   nest_free(&op->nest);
@@ -1275,7 +1296,7 @@ static void release(sgmev_op* op) {
   if (op->ev_switch) cudaEventDestroy(op->ev_switch);
   for (cudaEvent_t e : op->ev_cg)
     if (e) cudaEventDestroy(e);
-  if (op->own_stream) cudaStreamDestroy(op->own_stream);
+  stream_release(op->own_stream);
   (void)cudaGetLastError();
 }
 
@@ -1528,7 +1549,8 @@ SGMEV_API int sgmev_create(sgmev_op** out, int dim, int64_t n_grid, const double
   CREATE_CUDA(cudaGetDevice(&op->device));
   CREATE_CUDA(cudaDeviceGetAttribute(&op->num_sms, cudaDevAttrMultiProcessorCount, op->device));
   op->target_ctas = static_cast<int64_t>(op->num_sms) * 4;
-  CREATE_CUDA(cudaStreamCreateWithFlags(&op->own_stream, cudaStreamNonBlocking));
+  op->own_stream = stream_acquire();
+  if (!op->own_stream) return bail(fail(SGMEV_ERR_CUDA, "stream for the operator"));
   op->stream = op->own_stream;
   CREATE_CUDA(cudaEventCreate(&op->ev_start));
   CREATE_CUDA(cudaEventCreate(&op->ev_stop));
@@ -1584,13 +1606,12 @@ SGMEV_API int sgmev_create(sgmev_op** out, int dim, int64_t n_grid, const double
       cudaMemcpyAsync(op->host_scalar, flag, sizeof(unsigned int), cudaMemcpyDeviceToHost,
                       op->stream);
     }
-    cudaError_t e = cudaStreamSynchronize(op->stream);
     dev_free(d_rows, op->stream);
     dev_free(d_bb, op->stream);
-    if (e != cudaSuccess) return bail(fail(SGMEV_ERR_CUDA, std::string("stage data: ") + cudaGetErrorString(e)));
-    if (op->mod) op->in_cube = *reinterpret_cast<const unsigned int*>(op->host_scalar) == 0;
   }
+  // (waits for the stream: the caller's buffers are free once this returns)
   CREATE_TRY(stage_grid(op, n_grid, level_pow2, index));
+  if (op->mod) op->in_cube = *reinterpret_cast<const unsigned int*>(op->host_scalar) == 0;
 #undef CREATE_CUDA
 #undef CREATE_TRY
   *out = op;
@@ -2165,7 +2186,7 @@ static int fit_common(sgmev_op* op, int mode, const double* y, bool y_on_device,
         sgmev_op* o;
         // ModLinear products reach 2^(active dimensions): FP16 holds them up to 15
         explicit HalfScope(sgmev_op* op_) : o(op_) {
-          o->use_half = o->inner_half && (!o->mod || o->sub.na_max <= 15);
+          o->use_half = o->inner_half && (!o->mod || (sub_ready(o) && o->sub.na_max <= 15));
         }
         ~HalfScope() { o->use_half = false; }
       } half_scope(op);
@@ -2254,8 +2275,8 @@ static int block_ready(sgmev_op* op) {
   // The block products are packed from the materialised products. Where the materialised
   // kernels do not take the grid (their coefficients live in shared memory: grids with many
   // subspaces of many cells), the products are built only for the packing and freed after it.
-  const bool block_only = op->sub_ok && !mat_ready(op) && block_materialize(op);
-  if (!op->sub_ok || (!block_only && !mat_ready(op))) {
+  const bool block_only = sub_ready(op) && !mat_ready(op) && block_materialize(op);
+  if (!sub_ready(op) || (!block_only && !mat_ready(op))) {
     op->blk_failed = true;
     op->blk_err = "they stream the materialised subspace products (params \"algo\": \"subspace\", "
                   "\"materialize\": not \"off\"), which this operator does not have";

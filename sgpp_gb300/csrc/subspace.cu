@@ -26,8 +26,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <map>
 #include <type_traits>
+#include <unordered_map>
 #include <vector>
 
 #include "devmem.h"
@@ -1056,21 +1056,35 @@ bool subspace_build(SubPlan* p, int dim, int64_t n, const double* level_pow2, co
     *err = "subspace kernels need 1 <= dim <= 16 and a non-empty grid";
     return false;
   }
-  // group grid points by level vector
-  std::map<std::vector<int>, std::vector<int64_t>> groups;
+  // group grid points by level vector (dim <= 16 levels of 5 bits: two words)
+  struct Key {
+    uint64_t a, b;
+    bool operator==(const Key& o) const { return a == o.a && b == o.b; }
+  };
+  struct Hash {
+    size_t operator()(const Key& k) const { return (k.a * 0x9E3779B97F4A7C15ull) ^ (k.b * 0xC2B2AE3D27D4EB4Full + (k.a >> 29)); }
+  };
+  std::unordered_map<Key, int, Hash> ids;
+  std::vector<std::pair<std::vector<int>, std::vector<int64_t>>> list;
   std::vector<int> lv(dim);
   for (int64_t g = 0; g < n; ++g) {
+    Key key{0, 0};
     for (int t = 0; t < dim; ++t) {
-      int e = 0;
-      std::frexp(level_pow2[g * dim + t], &e);
-      lv[t] = e - 1;  // 2^l
-      if (lv[t] < 1 || lv[t] > 20) {
+      uint64_t bits;
+      std::memcpy(&bits, &level_pow2[g * dim + t], sizeof(bits));  // 2^l (checked by the caller)
+      const int l = static_cast<int>((bits >> 52) & 0x7FF) - 1023;
+      if (l < 1 || l > 20) {
         *err = "subspace kernels need levels in [1, 20]";
         return false;
       }
+      lv[t] = l;
+      (t < 8 ? key.a : key.b) |= static_cast<uint64_t>(l) << (5 * (t & 7));
     }
-    groups[lv].push_back(g);
+    const auto it = ids.emplace(key, static_cast<int>(list.size()));
+    if (it.second) list.emplace_back(lv, std::vector<int64_t>());
+    list[it.first->second].second.push_back(g);
   }
+  std::sort(list.begin(), list.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
   std::vector<int4> desc, sinfo, act, sact;
   std::vector<uint32_t> base;
   int64_t cmax = 0;
@@ -1078,8 +1092,8 @@ bool subspace_build(SubPlan* p, int dim, int64_t n, const double* level_pow2, co
   int64_t act_work = 0;
   // subspaces in order of their number of active (level > 1) dimensions, so that neighbouring
   // threads of the owner-computes kernels run the same number of evaluations
-  std::vector<const std::pair<const std::vector<int>, std::vector<int64_t>>*> order;
-  for (const auto& kv : groups) order.push_back(&kv);
+  std::vector<const std::pair<std::vector<int>, std::vector<int64_t>>*> order;
+  for (const auto& kv : list) order.push_back(&kv);
   auto n_active = [](const std::vector<int>& l) {
     return static_cast<int>(std::count_if(l.begin(), l.end(), [](int v) { return v > 1; }));
   };
@@ -1146,7 +1160,7 @@ bool subspace_build(SubPlan* p, int dim, int64_t n, const double* level_pow2, co
     offset += size;
   }
   p->dim = dim;
-  p->n_sub = static_cast<int>(groups.size());
+  p->n_sub = static_cast<int>(list.size());
   p->total = offset;
   p->h_pos = pos;
   p->h_sub.clear();
