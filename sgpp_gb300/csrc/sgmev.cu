@@ -134,8 +134,10 @@ struct sgmev_op {
   // the products were built only to pack the block products (the materialised kernels do not take
   // this grid) and are gone: the other products run on the on-the-fly kernels
   bool mat_block_only = false;
-  bool inner_half = true;   // inner solves of mixed fits use the FP16 products ("inner_products")
-  bool use_half = false;    // set while such an inner solve runs
+  // inner solves of mixed fits use the FP16 products ("inner_products"): 0 no, 1 yes, 2 where they are
+  // the faster choice (the default)
+  int inner_half = 2;
+  bool use_half = false;    // set while an inner solve on the FP16 products runs
   int algo = 2;          // FP32 products: 0 dense, 1 subspace, 2 auto (params "algo")
   SubPlan sub;           // subspace tables of the current grid
   bool sub_ok = false;   // sub is built and chosen for the FP32 products
@@ -941,7 +943,7 @@ static bool nest_ready(sgmev_op* op) {
 }
 
 static bool nest_mults(sgmev_op* op, int prec) {
-  return (prec == SGMEV_FP64 || op->mat_mode != 2) && nest_ready(op);
+  return (prec == SGMEV_FP64 || (op->mat_mode != 2 && !op->use_half)) && nest_ready(op);
 }
 
 // The FP32 and float-float multTranspose: nested up to 8,192 data points, where it also saves building
@@ -954,6 +956,25 @@ static bool nest_multts(sgmev_op* op, int prec) {
   if (prec == SGMEV_FP64 || op->m <= 8192) return true;
   return prec == SGMEV_DF64 && static_cast<double>(op->nest.n_sub) * op->m <= 1e8 &&
          !(sub_ready(op) && op->mat_multt && subspace_mat_fits(op->sub, true) && mat_ready(op));
+}
+
+// Whether the inner solves of a mixed fit run on the FP16 products, both of them: a nested FP32 mult
+// beside the FP16 multTranspose is no symmetric operator, and the solutions it left had the residual
+// asked for but up to three times the error. On the nested FP32 mult and the FP32 multTranspose
+// (nested or materialised) an iteration's products take less time than on the FP16 ones on every
+// grid measured (d = 3..12, level 4..7, 1,000 to 256,000 points: 16,000 points 44-114 against 53-207 us,
+// 256,000 points 79-514 against 131-631 us) except where the FP16 mult fills its 16 warps of 64
+// subspaces in one pass and its cells are nibbles: d=10 level 5 138 against 128 us at 64,000 points,
+// 1.14 against 0.92 ms at 2^20; at 16,000 points 69 against 75.
+static bool inner_on_half(sgmev_op* op) {
+  using namespace sgmev;
+  if (op->inner_half == 0) return false;
+  // ModLinear products reach 2^(active dimensions): FP16 holds them up to 15
+  if (!sub_ready(op) || (op->mod && op->sub.na_max > 15) || !op->mat_multt) return false;
+  if (op->inner_half == 2 && op->mat_mode != 2 && nest_ready(op) &&
+      !(op->m > 32768 && op->sub.n_sub > 704 && op->sub.n_sub <= 1024 && op->sub.cmax <= 16))
+    return false;
+  return mat_ready(op);
 }
 
 // Inputs: a64 [n] where nest_mults(); otherwise per precision FP64 a64; FP32 a32; DF64 (a32, a32lo) —
@@ -1486,7 +1507,7 @@ SGMEV_API int sgmev_create(sgmev_op** out, int dim, int64_t n_grid, const double
   op->mat_mode = mat == "off" ? 0 : (mat == "on" ? 2 : 1);
   op->mat_multt = mat_t != "off";
   op->fused_system = sys_p == "fused";
-  op->inner_half = inner_p != "float";
+  op->inner_half = inner_p == "float" ? 0 : inner_p == "half" ? 1 : 2;
   op->mod = basis == "modlinear";
   {
     const std::string it = json_string(params_json, "inner_tol");
@@ -2179,17 +2200,20 @@ static int fit_common(sgmev_op* op, int mode, const double* y, bool y_on_device,
       if (rnorm2 <= epsilon * epsilon * r0 || rnorm2 == 0.0 || total_it >= max_iterations) break;
       int64_t it = 0;
       double dres = 0.0;
-      const double want = std::max(eps_inner, epsilon * std::sqrt(r0 / rnorm2) * 0.5);
+      // The reduction that ends the refinement: on FP32 products it is solved for where one solve
+      // reaches it, with room for the inner operator's own error, because the looser inner tolerance
+      // would leave a residual anywhere up to epsilon. The less exact FP16 products take one more
+      // solve there, and the residuals it leaves (4e-9 at epsilon 1e-8) are the accuracy to keep.
+      const bool half = inner_on_half(op);
+      const double last = (half ? 0.5 : 0.4) * epsilon * std::sqrt(r0 / rnorm2);
+      const double want = half ? std::max(eps_inner, last) : last > 0.1 * eps_inner ? last : eps_inner;
       // the inner solve may use the FP16 copy of the materialised products: the outer residual
       // is FP64-accurate, so the refinement still converges to the FP64 solution
       struct HalfScope {
         sgmev_op* o;
-        // ModLinear products reach 2^(active dimensions): FP16 holds them up to 15
-        explicit HalfScope(sgmev_op* op_) : o(op_) {
-          o->use_half = o->inner_half && (!o->mod || (sub_ready(o) && o->sub.na_max <= 15));
-        }
+        HalfScope(sgmev_op* op_, bool half_) : o(op_) { o->use_half = half_; }
         ~HalfScope() { o->use_half = false; }
-      } half_scope(op);
+      } half_scope(op, half);
       if (op->precond) {
         SGMEV_TRY(pcg_core(op, SGMEV_FP32, rr, dx, lm, max_iterations - total_it,
                            std::min(want, 0.5), &it));
