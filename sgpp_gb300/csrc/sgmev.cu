@@ -1067,14 +1067,14 @@ static int dev_multt(sgmev_op* op, int prec, const double* v64, const float* v32
     SGMEV_CUDA(subspace_multt_mat_df(op->sub, op->stream, op->mpad, v32, v32lo, op->npad, out64,
                                      add, scale, op->num_sms));
     prof_end(op, ev);
-    op->launches += 3;
+    op->launches += 2;
   } else if (prec == SGMEV_DF64 && sub_ready(op) && !op->mod && subspace_owner_fits(op->sub, true)) {
     // the subspace sums produce every grid entry at once (the range is a subset of them)
     const long ev = prof_begin(op, KIND_MULTT_SUBDF);
     SGMEV_CUDA(subspace_multt_df(op->sub, op->stream, op->xt32, op->xt32lo, op->mpad, op->m, v32,
                                  v32lo, op->npad, out64, add, scale, op->num_sms));
     prof_end(op, ev);
-    op->launches += 3;
+    op->launches += 2;
   } else if (prec == SGMEV_DF64) {
     SGMEV_TRY(run_multt_df(op, v32, v32lo, g_begin, g_end, &p));
     SGMEV_TRY((run_reduce<float2, double>(op, (int)p.nsplit, op->npad, g_begin, valid, g_end, out64, add, scale)));
@@ -1084,14 +1084,14 @@ static int dev_multt(sgmev_op* op, int prec, const double* v64, const float* v32
     SGMEV_CUDA(subspace_multt_mat(op->sub, op->stream, op->xt32, op->mpad, op->m, v32, op->npad,
                                   out64, add, scale, op->num_sms, op->use_half));
     prof_end(op, ev);
-    op->launches += 3;
+    op->launches += 2;
   } else if (sub_ready(op) && !op->mod) {
     // the subspace scatter produces every grid entry at once (the range is a subset of it)
     const long ev = prof_begin(op, KIND_MULTT_SUB32);
     SGMEV_CUDA(subspace_multt(op->sub, op->stream, op->xt32, op->mpad, op->m, v32, op->npad,
                               out64, add, scale, op->num_sms));
     prof_end(op, ev);
-    op->launches += 3;
+    op->launches += 2;
   } else {
     SGMEV_TRY(run_multt<float>(op, op->xt32, v32, op->li32, g_begin, g_end, &p));
     SGMEV_TRY((run_reduce<float, double>(op, (int)p.nsplit, op->npad, g_begin, valid, g_end, out64, add, scale)));

@@ -423,7 +423,7 @@ __global__ void __launch_bounds__(kMulttThreads) sub_multt_kernel(
 // [cell][thread] so that a warp's 32 updates hit 32 different banks. The points of a tile are
 // staged in shared memory as rows (x_0 .. x_{d-1}, v) and read by all threads at once (broadcast).
 // After each tile a thread adds its cells into the CTA's FP64 row of the partial matrix (its cells
-// belong to it alone, so the update order is fixed); sum_rows_kernel adds the rows in CTA order.
+// belong to it alone, so the update order is fixed); finish_rows_kernel adds the rows in a fixed order.
 // Every step has a fixed order, so the result is the same bit for bit from run to run.
 // Points with a coordinate outside the open interval (0, 1) see only zero hats; the staging step
 // gives them v = 0 and coordinates 0.5, which keeps the cell arithmetic inside the subspace with no
@@ -830,19 +830,21 @@ __global__ void __launch_bounds__(kActOwnThreads, 2) sub_multt_act_kernel(
   }
 }
 
-// sums[k] = sum over rows b in order of rows[b][k] (k < total)
-// sums[k] = sum over rows b of rows[b][k] (k < total) in a fixed order: a block of 32 x 8 threads
-// takes 32 positions; thread (x, y) adds rows y, y + 8, y + 16, ... in order (four loads in
-// flight), and the 8 partial sums are then added in y order
+// out[inv[k]] = sum over rows b of rows[b][k] (+ scale_add * add[inv[k]]) for the positions k of grid
+// points, and zero in [n, npad). The sums in a fixed order: a block of 32 x 8 threads takes 32
+// positions; thread (x, y) adds rows y, y + 8, y + 16, ... in order (four loads in flight), and the 8
+// partial sums are then added in y order.
 constexpr int kSumRowGroups = 8;
 
-__global__ void __launch_bounds__(32 * kSumRowGroups) sum_rows_kernel(
-    const double* __restrict__ rows, int nrows, int64_t total, double* __restrict__ sums) {
-  __shared__ double part[kSumRowGroups][32];
+__global__ void __launch_bounds__(32 * kSumRowGroups) finish_rows_kernel(
+    const double* __restrict__ rows, int nrows, int64_t total, const int* __restrict__ inv, int64_t n,
+    int64_t npad, const double* __restrict__ add, double scale_add, double* __restrict__ out) {
+  __shared__ double part[kSumRowGroups][33];
   const int64_t k = static_cast<int64_t>(blockIdx.x) * 32 + threadIdx.x;
   const int y = threadIdx.y;
+  const int g = k < total ? inv[k] : -1;
   double a = 0.0;
-  if (k < total) {
+  if (g >= 0) {
     int b = y;
     for (; b + 3 * kSumRowGroups < nrows; b += 4 * kSumRowGroups) {
       const double r0 = rows[static_cast<int64_t>(b) * total + k];
@@ -858,26 +860,13 @@ __global__ void __launch_bounds__(32 * kSumRowGroups) sum_rows_kernel(
   }
   part[y][threadIdx.x] = a;
   __syncthreads();
-  if (y == 0 && k < total) {
+  if (y == 0 && g >= 0) {
     double r = part[0][threadIdx.x];
-    for (int g = 1; g < kSumRowGroups; ++g) r += part[g][threadIdx.x];
-    sums[k] = r;
+    for (int b = 1; b < kSumRowGroups; ++b) r += part[b][threadIdx.x];
+    out[g] = add ? fma(scale_add, add[g], r) : r;
   }
-}
-
-// out[g] (g < n; zero in [n, npad)) = sums[pos[g]] (+ scale_add * add[g])
-__global__ void gather_sums_kernel(const double* __restrict__ sums, const int* __restrict__ pos,
-                                   int64_t n, int64_t npad, const double* __restrict__ add,
-                                   double scale_add, double* __restrict__ out) {
-  for (int64_t g = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; g < npad;
-       g += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    double r = 0.0;
-    if (g < n) {
-      r = sums[pos[g]];
-      if (add) r = fma(scale_add, add[g], r);
-    }
-    out[g] = r;
-  }
+  const int64_t first = n + static_cast<int64_t>(blockIdx.x) * blockDim.x * blockDim.y + y * 32 + threadIdx.x;
+  for (int64_t i = first; i < npad; i += static_cast<int64_t>(gridDim.x) * blockDim.x * blockDim.y) out[i] = 0.0;
 }
 
 __global__ void maxabs_kernel(const float* __restrict__ v, int64_t m, unsigned int* __restrict__ out) {
@@ -995,7 +984,7 @@ size_t own_smem(const SubPlan& p, int dim, bool df) {
 template <int DIM, bool DF>
 cudaError_t launch_multt_own(const SubPlan& p, cudaStream_t s, const float* xh, const float* xl,
                              int64_t mpad, int64_t m, const float* vh, const float* vl,
-                             int num_sms) {
+                             int num_sms, int64_t* nrows) {
   auto kern = sub_multt_own_kernel<DIM, DF>;
   const size_t sm = own_smem(p, DIM, DF);
   const int nth = own_threads(p, DF);
@@ -1011,10 +1000,7 @@ cudaError_t launch_multt_own(const SubPlan& p, cudaStream_t s, const float* xh, 
   kern<<<static_cast<unsigned>(rows), nth, sm, s>>>(p.desc, p.sinfo, p.n_sub, p.cmax,
                                                     static_cast<int>(p.total), xh, xl, mpad, m, vh,
                                                     vl, nt, p.rows);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  sum_rows_kernel<<<static_cast<unsigned>((p.total + 31) / 32), dim3(32, kSumRowGroups), 0, s>>>(
-      p.rows, static_cast<int>(rows), p.total, reinterpret_cast<double*>(p.acc));
+  *nrows = rows;
   return cudaGetLastError();
 }
 
@@ -1025,7 +1011,7 @@ size_t act_own_smem(const SubPlan& p, int dim) {
 
 template <int DIM>
 cudaError_t launch_multt_act(const SubPlan& p, cudaStream_t s, const float* xt, int64_t mpad,
-                             int64_t m, const float* v, int num_sms) {
+                             int64_t m, const float* v, int num_sms, int64_t* nrows) {
   auto kern = sub_multt_act_kernel<DIM>;
   const size_t sm = act_own_smem(p, DIM);
   const int nth = own_threads(p, false);
@@ -1039,10 +1025,7 @@ cudaError_t launch_multt_act(const SubPlan& p, cudaStream_t s, const float* xt, 
   kern<<<static_cast<unsigned>(rows), nth, sm, s>>>(p.act, p.sact, p.n_sub, p.cmax,
                                                     static_cast<int>(p.total), xt, mpad, m, v, nt,
                                                     p.rows);
-  e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  sum_rows_kernel<<<static_cast<unsigned>((p.total + 31) / 32), dim3(32, kSumRowGroups), 0, s>>>(
-      p.rows, static_cast<int>(rows), p.total, reinterpret_cast<double*>(p.acc));
+  *nrows = rows;
   return cudaGetLastError();
 }
 
@@ -1159,6 +1142,8 @@ bool subspace_build(SubPlan* p, int dim, int64_t n, const double* level_pow2, co
     }
     offset += size;
   }
+  std::vector<int> inv(static_cast<size_t>(offset), -1);
+  for (int64_t g = 0; g < n; ++g) inv[pos[g]] = static_cast<int>(g);
   p->dim = dim;
   p->n_sub = static_cast<int>(list.size());
   p->total = offset;
@@ -1191,6 +1176,7 @@ bool subspace_build(SubPlan* p, int dim, int64_t n, const double* level_pow2, co
             alloc(&p->rows, sizeof(double) * p->row_cap * offset) &&
             alloc(&p->base, sizeof(uint32_t) * base.size()) &&
             alloc(&p->pos, sizeof(int) * pos.size()) &&
+            alloc(&p->inv, sizeof(int) * offset) &&
             alloc(&p->asub, sizeof(float) * offset) &&
             alloc(&p->asub2, sizeof(float2) * offset) &&
             alloc(&p->acc, sizeof(unsigned long long) * offset) &&
@@ -1201,7 +1187,8 @@ bool subspace_build(SubPlan* p, int dim, int64_t n, const double* level_pow2, co
        put(p->act, act.data(), sizeof(int4) * act.size()) &&
        put(p->sact, sact.data(), sizeof(int4) * sact.size()) &&
        put(p->base, base.data(), sizeof(uint32_t) * base.size()) &&
-       put(p->pos, pos.data(), sizeof(int) * pos.size());
+       put(p->pos, pos.data(), sizeof(int) * pos.size()) &&
+       put(p->inv, inv.data(), sizeof(int) * inv.size());
   if (!ok) {
     subspace_free(p);
     *err = "subspace plan allocation failed";
@@ -1219,7 +1206,7 @@ bool subspace_build(SubPlan* p, int dim, int64_t n, const double* level_pow2, co
 void subspace_free(SubPlan* p) {
   const cudaStream_t st = p->stream;
   void* ptrs[] = {p->desc, p->sinfo, p->act,  p->sact,    p->pmat,  p->pmat_lo, p->pmat16,
-                  p->cmat, p->cpair, p->rows, p->base, p->pos,  p->asub,    p->asub2,
+                  p->cmat, p->cpair, p->rows, p->base, p->pos,  p->inv,  p->asub,    p->asub2,
                   p->acc,  p->maxbits};
   for (void* q : ptrs) dev_free(q, st);
   *p = SubPlan{};
@@ -1259,10 +1246,8 @@ cudaError_t subspace_scatter_alpha_df(const SubPlan& p, cudaStream_t s, const fl
 
 cudaError_t subspace_finish_rows(const SubPlan& p, cudaStream_t s, int64_t nrows, int64_t npad,
                                  double* out64, const double* add, double scale_add) {
-  sum_rows_kernel<<<static_cast<unsigned>((p.total + 31) / 32), dim3(32, kSumRowGroups), 0, s>>>(
-      p.rows, static_cast<int>(nrows), p.total, reinterpret_cast<double*>(p.acc));
-  gather_sums_kernel<<<static_cast<unsigned>(std::min<int64_t>(1216, (npad + 255) / 256)), 256, 0, s>>>(
-      reinterpret_cast<const double*>(p.acc), p.pos, p.n, npad, add, scale_add, out64);
+  finish_rows_kernel<<<static_cast<unsigned>((p.total + 31) / 32), dim3(32, kSumRowGroups), 0, s>>>(
+      p.rows, static_cast<int>(nrows), p.total, p.inv, p.n, npad, add, scale_add, out64);
   return cudaGetLastError();
 }
 
@@ -1308,16 +1293,6 @@ cudaError_t subspace_mult_df(const SubPlan& p, cudaStream_t s, const float* xh, 
   }
 }
 
-namespace {
-
-cudaError_t own_finish(const SubPlan& p, cudaStream_t s, int64_t npad, double* out64,
-                       const double* add, double scale_add) {
-  gather_sums_kernel<<<static_cast<unsigned>(std::min<int64_t>(1216, (npad + 255) / 256)), 256, 0, s>>>(
-      reinterpret_cast<const double*>(p.acc), p.pos, p.n, npad, add, scale_add, out64);
-  return cudaGetLastError();
-}
-}  // namespace
-
 bool subspace_owner_fits(const SubPlan& p, bool df) {
   const size_t sm = df ? own_smem(p, p.dim, true) : act_own_smem(p, p.dim);
   return p.n_sub > 0 && p.cmax > 0 && p.rows != nullptr && sm <= kOwnSmemBudget;
@@ -1327,11 +1302,12 @@ cudaError_t subspace_multt(const SubPlan& p, cudaStream_t s, const float* xt, in
                            int64_t m, const float* v32, int64_t npad, double* out64,
                            const double* add, double scale_add, int num_sms) {
   cudaError_t e = cudaSuccess;
+  int64_t nrows = 0;
   if (subspace_owner_fits(p, false)) {
     switch (p.dim) {
 #define F(D)                                                                                 \
   case D:                                                                                    \
-    e = launch_multt_act<D>(p, s, xt, mpad, m, v32, num_sms);                                \
+    e = launch_multt_act<D>(p, s, xt, mpad, m, v32, num_sms, &nrows);                        \
     break;
       SUB_DIMS(F)
 #undef F
@@ -1339,7 +1315,7 @@ cudaError_t subspace_multt(const SubPlan& p, cudaStream_t s, const float* xt, in
         return cudaErrorInvalidValue;
     }
     if (e != cudaSuccess) return e;
-    return own_finish(p, s, npad, out64, add, scale_add);
+    return subspace_finish_rows(p, s, nrows, npad, out64, add, scale_add);
   }
   if (p.total > kSubMaxPositions) return cudaErrorInvalidValue;  // (rejected at build)
   e = cudaMemsetAsync(p.maxbits, 0, sizeof(unsigned int), s);
@@ -1370,10 +1346,11 @@ cudaError_t subspace_multt_df(const SubPlan& p, cudaStream_t s, const float* xh,
                               int num_sms) {
   if (!subspace_owner_fits(p, true)) return cudaErrorInvalidValue;
   cudaError_t e = cudaSuccess;
+  int64_t nrows = 0;
   switch (p.dim) {
 #define F(D)                                                                   \
   case D:                                                                      \
-    e = launch_multt_own<D, true>(p, s, xh, xl, mpad, m, vh, vl, num_sms);     \
+    e = launch_multt_own<D, true>(p, s, xh, xl, mpad, m, vh, vl, num_sms, &nrows); \
     break;
     SUB_DIMS(F)
 #undef F
@@ -1381,7 +1358,7 @@ cudaError_t subspace_multt_df(const SubPlan& p, cudaStream_t s, const float* xh,
       return cudaErrorInvalidValue;
   }
   if (e != cudaSuccess) return e;
-  return own_finish(p, s, npad, out64, add, scale_add);
+  return subspace_finish_rows(p, s, nrows, npad, out64, add, scale_add);
 }
 
 }  // namespace sgmev

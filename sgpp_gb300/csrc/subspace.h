@@ -38,6 +38,7 @@ struct SubPlan {
   int4* desc = nullptr;   // [n_sub * dim] (bits(2^{l-1}), bits(2^l), stride, 0)
   uint32_t* base = nullptr;  // [n_sub] offset - sum_t bits(1.5*2^23) * stride_t (mod 2^32)
   int* pos = nullptr;     // [n] grid point -> position
+  int* inv = nullptr;     // [total] position -> grid point or -1
   float* asub = nullptr;  // [total] alpha in subspace order
   float2* asub2 = nullptr;  // [total] alpha as float-float pairs (df64 mult)
   unsigned long long* acc = nullptr;  // [total] fixed-point accumulators / FP64 sums (multT)

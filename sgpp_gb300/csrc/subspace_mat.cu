@@ -53,6 +53,16 @@ constexpr int kAhead = 4, kAheadDf = 2;
 static_assert(kGroups % kAhead == 0 && kGroups % kAheadDf == 0, "the ring must divide a tile");
 // multT: FP32 sums over this many tiles (1024 points) before they go into the FP64 row
 constexpr int kFlushTiles = 4;
+// multT: the points are dealt out to the streams in units of 128, one unit each up to two streams per
+// SM and two from there on (more rows of sums cost more than their shorter streams gain: a float-float
+// system product on 100,003 points 86 us with 391 streams, 93 with 782). In whole tiles of 256 points
+// 16,000 points reached 63 CTAs: FP32 multT at d=6 level 5 27.5 -> 21 us, float-float 35 -> 26.
+constexpr int kUnit = 128;
+int64_t most_streams(int64_t units, int num_sms) {
+  return std::max<int64_t>(1, std::min(units, std::max<int64_t>(2 * num_sms, units / 2)));
+}
+constexpr int kUnitGroups = kUnit / 4, kUnitPairs = kUnit / 8;
+static_assert(kUnitGroups % kAhead == 0 && kUnitGroups % kAheadDf == 0, "the ring must divide a unit");
 
 // Cell words: four points' cell indices in one word, a byte each (uint32_t, grids whose
 // subspaces have up to 256 cells) or a nibble each (uint16_t, up to 16 cells: 0.5 byte per entry
@@ -249,7 +259,7 @@ __global__ void __launch_bounds__(kMatThreads, 2) mat_mult_kernel(
 template <typename CW, bool SACC>
 __global__ void __launch_bounds__(kMatThreads, 2) mat_multt_kernel(
     const int4* __restrict__ sact, int n_sub, int s_pad, int cmax, int total,
-    const float* __restrict__ v, int64_t n_tiles, const float4* __restrict__ pm,
+    const float* __restrict__ v, int64_t n_units, const float4* __restrict__ pm,
     const CW* __restrict__ cm, double* __restrict__ rows, int streams) {
   using PT = float4;
   constexpr int A = kAhead;
@@ -272,8 +282,8 @@ __global__ void __launch_bounds__(kMatThreads, 2) mat_multt_kernel(
     for (int c = 0; c < info.y; ++c) acc[c * nth] = 0.0f;
     bool first = true;
     // the stream's tiles are contiguous and its ring runs over all of them
-    const int64_t g_begin = (stream * n_tiles / streams) * kGroups;
-    const int64_t g_end = ((stream + 1) * n_tiles / streams) * kGroups;
+    const int64_t g_begin = (stream * n_units / streams) * kUnitGroups;
+    const int64_t g_end = ((stream + 1) * n_units / streams) * kUnitGroups;
     if (g_begin < g_end) {
       const PT* src = pm + g_begin * s_pad + sid;
       const CW* csrc = cm + g_begin * s_pad + sid;
@@ -352,8 +362,8 @@ struct PairCells<uint32_t> {  // two byte words
 
 constexpr int kPairAheadMult = 2;   // pairs in flight per block: the 4 groups of the FP16 ring
 constexpr int kPairAheadMultT = 4;  // pairs in flight: 8 groups
-static_assert(kPairs % kPairAheadMult == 0 && kPairs % kPairAheadMultT == 0,
-              "the ring must divide a tile");
+static_assert(kPairs % kPairAheadMult == 0 && kUnitPairs % kPairAheadMultT == 0,
+              "the ring must divide a tile, or a unit");
 
 // mat_mult_kernel on the pair layout: a lane takes subspaces s and s + 32, two point groups per
 // ring slot. A CTA takes a contiguous range of tiles, and with one pass over the subspaces its
@@ -490,7 +500,7 @@ __global__ void __launch_bounds__(kMatThreads, 2) mat_mult_half_kernel(
 template <typename CW, bool SACC, int BATCH>
 __global__ void __launch_bounds__(kMatThreads, 2) mat_multt_half_kernel(
     const int4* __restrict__ sact, int n_sub, int s_pad, int cmax, int total,
-    const float* __restrict__ v, int64_t n_tiles, const uint4* __restrict__ pp,
+    const float* __restrict__ v, int64_t n_units, const uint4* __restrict__ pp,
     const typename PairCells<CW>::T* __restrict__ cp, double* __restrict__ rows, int streams,
     double unscale, const double* __restrict__ stop) {
   if (stop && *stop != 0.0) return;
@@ -514,8 +524,8 @@ __global__ void __launch_bounds__(kMatThreads, 2) mat_multt_half_kernel(
     for (int c = 0; c < info.y; ++c) acc[c * nth] = 0.0f;
     bool first = true;
     // the stream's tiles are contiguous, so the ring runs over all of them without restarting
-    const int64_t k_begin = (stream * n_tiles / streams) * kPairs;
-    const int64_t k_end = ((stream + 1) * n_tiles / streams) * kPairs;
+    const int64_t k_begin = (stream * n_units / streams) * kUnitPairs;
+    const int64_t k_end = ((stream + 1) * n_units / streams) * kUnitPairs;
     if (k_begin < k_end) {
       const uint4* src = pp + k_begin * s_pad + sid;
       const CT* csrc = cp + k_begin * s_pad + sid;
@@ -628,7 +638,7 @@ __global__ void __launch_bounds__(kMatThreads, 2) mat_multt_half_kernel(
 template <typename CW>
 __global__ void __launch_bounds__(kMatThreads, 2) mat_multt_half_banked_kernel(
     const int4* __restrict__ sact, int n_sub, int s_pad, int cmax, int total,
-    const float* __restrict__ v, int64_t n_tiles, const uint4* __restrict__ pp,
+    const float* __restrict__ v, int64_t n_units, const uint4* __restrict__ pp,
     const typename PairCells<CW>::T* __restrict__ cp, double* __restrict__ rows, int streams,
     double unscale, const double* __restrict__ stop) {
   if (stop && *stop != 0.0) return;
@@ -657,8 +667,8 @@ __global__ void __launch_bounds__(kMatThreads, 2) mat_multt_half_banked_kernel(
       b1[c * nth] = 0.0f;
       sum[c * nth] = 0.0f;
     }
-    const int64_t k_begin = (stream * n_tiles / streams) * kPairs;
-    const int64_t k_end = ((stream + 1) * n_tiles / streams) * kPairs;
+    const int64_t k_begin = (stream * n_units / streams) * kUnitPairs;
+    const int64_t k_end = ((stream + 1) * n_units / streams) * kUnitPairs;
     if (k_begin < k_end) {
       const uint4* src = pp + k_begin * s_pad + sid;
       const CT* csrc = cp + k_begin * s_pad + sid;
@@ -729,7 +739,7 @@ __global__ void __launch_bounds__(kMatThreads, 2) mat_multt_half_banked_kernel(
 template <typename CW>
 __global__ void __launch_bounds__(kMatThreads, 3) mat_multt_half_lean_kernel(
     const int4* __restrict__ sact, int n_sub, int s_pad, int cmax, int total,
-    const float* __restrict__ v, int64_t n_tiles, const uint4* __restrict__ pp,
+    const float* __restrict__ v, int64_t n_units, const uint4* __restrict__ pp,
     const typename PairCells<CW>::T* __restrict__ cp, double* __restrict__ rows, int streams,
     double unscale, const double* __restrict__ stop) {
   if (stop && *stop != 0.0) return;
@@ -750,8 +760,8 @@ __global__ void __launch_bounds__(kMatThreads, 3) mat_multt_half_lean_kernel(
     const uint32_t offset = static_cast<uint32_t>(info.x) - static_cast<uint32_t>(info.z);
     float* acc = s_acc + tid;
     for (int c = 0; c < info.y; ++c) acc[c * nth] = 0.0f;
-    const int64_t k_begin = (stream * n_tiles / streams) * kPairs;
-    const int64_t k_end = ((stream + 1) * n_tiles / streams) * kPairs;
+    const int64_t k_begin = (stream * n_units / streams) * kUnitPairs;
+    const int64_t k_end = ((stream + 1) * n_units / streams) * kUnitPairs;
     if (k_begin < k_end) {
       const uint4* src = pp + k_begin * s_pad + sid;
       const CT* csrc = cp + k_begin * s_pad + sid;
@@ -922,7 +932,7 @@ __global__ void __launch_bounds__(kMatThreads, 1) mat_mult_df_kernel(
 template <typename CW, bool SACC>
 __global__ void __launch_bounds__(kMatThreads, 1) mat_multt_df_kernel(
     const int4* __restrict__ sact, int n_sub, int s_pad, int cmax, int total,
-    const float* __restrict__ vh, const float* __restrict__ vl, int64_t n_tiles,
+    const float* __restrict__ vh, const float* __restrict__ vl, int64_t n_units,
     const float4* __restrict__ phi, const float4* __restrict__ plo,
     const CW* __restrict__ cm, double* __restrict__ rows, const double* __restrict__ stop) {
   if (stop && *stop != 0.0) return;
@@ -944,8 +954,8 @@ __global__ void __launch_bounds__(kMatThreads, 1) mat_multt_df_kernel(
     bool first = true;
     // the CTA's tiles are contiguous and the ring runs over all of them, instead of starting again
     // at each tile
-    const int64_t g_begin = (blockIdx.x * n_tiles / gridDim.x) * kGroups;
-    const int64_t g_end = ((blockIdx.x + 1) * n_tiles / gridDim.x) * kGroups;
+    const int64_t g_begin = (blockIdx.x * n_units / gridDim.x) * kUnitGroups;
+    const int64_t g_end = ((blockIdx.x + 1) * n_units / gridDim.x) * kUnitGroups;
     if (g_begin < g_end) {
       int64_t nxt = g_begin * s_pad + sid;
       float4 rh[kAheadDf], rl[kAheadDf];
@@ -1400,8 +1410,8 @@ cudaError_t launch_multt_df(const SubPlan& p, cudaStream_t s, int64_t mpad, cons
   int per_sm = 0;
   e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nth, sm);
   if (e != cudaSuccess) return e;
-  const int64_t nt = mpad / kOwnTile;
-  *rows = std::min<int64_t>(std::max(1, per_sm) * static_cast<int64_t>(num_sms), std::min<int64_t>(p.row_cap, std::max<int64_t>(nt, 1)));
+  const int64_t nt = mpad / kUnit;
+  *rows = std::min<int64_t>(std::max(1, per_sm) * static_cast<int64_t>(num_sms), std::min<int64_t>(p.row_cap, most_streams(nt, num_sms)));
   kern<<<static_cast<unsigned>(*rows), nth, sm, s>>>(
       p.sact, p.n_sub, static_cast<int>(p.s_pad), p.cmax, static_cast<int>(p.total), vh, vl, nt,
       p.pmat, p.pmat_lo, static_cast<const CW*>(p.cmat), p.rows, p.stop);
@@ -1457,12 +1467,12 @@ cudaError_t launch_mat_multt(const SubPlan& p, cudaStream_t s, int64_t mpad, con
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nth, sm);
     if (e != cudaSuccess) return e;
-    const int64_t nt = mpad / kOwnTile;
+    const int64_t nt = mpad / kUnit;
     // one CTA per (stream, pass): the resident CTAs split into passes, each stream a row
     const int64_t passes = (p.n_sub + nth - 1) / nth;
     const int64_t streams = std::max<int64_t>(
         1, std::min<int64_t>(std::max(1, per_sm) * static_cast<int64_t>(num_sms) / passes,
-                             std::min<int64_t>(p.row_cap, std::max<int64_t>(nt, 1))));
+                             std::min<int64_t>(p.row_cap, most_streams(nt, num_sms))));
     *rows = streams;
     kern<<<static_cast<unsigned>(streams * passes), nth, sm, s>>>(
         p.sact, p.n_sub, static_cast<int>(p.s_pad), p.cmax, static_cast<int>(p.total), v32, nt,
@@ -1477,11 +1487,11 @@ cudaError_t launch_mat_multt(const SubPlan& p, cudaStream_t s, int64_t mpad, con
     int per_sm = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, nth, sml);
     if (e != cudaSuccess) return e;
-    const int64_t nt = mpad / kOwnTile;
+    const int64_t nt = mpad / kUnit;
     const int64_t passes = (p.n_sub + nth - 1) / nth;
     const int64_t streams = std::max<int64_t>(
         1, std::min<int64_t>(std::max(1, per_sm) * static_cast<int64_t>(num_sms) / passes,
-                             std::min<int64_t>(p.row_cap, std::max<int64_t>(nt, 1))));
+                             std::min<int64_t>(p.row_cap, most_streams(nt, num_sms))));
     *rows = streams;
     kern<<<static_cast<unsigned>(streams * passes), nth, sml, s>>>(
         p.sact, p.n_sub, static_cast<int>(p.s_pad), p.cmax, static_cast<int>(p.total), v32, nt,
