@@ -11,7 +11,8 @@ std::mutex g_mu;
 std::vector<cudaMemPool_t> g_pools;  // per device: the library's own pool (nullptr: not made yet)
 std::vector<void*> g_pinned;         // recycled pinned blocks
 constexpr size_t kPinnedBytes = 64;
-constexpr size_t kKeptStreams = 32;
+constexpr size_t kKeptStreams = 32, kKeptBuffers = 16;
+std::vector<double*> g_buffers;  // idle pinned buffers
 std::vector<std::vector<cudaStream_t>> g_streams;  // per device: idle streams of past operators
 
 // The library allocates from a pool of its own, not from the device's default pool: its release
@@ -103,6 +104,35 @@ void stream_release(cudaStream_t s) {
     (void)cudaGetLastError();
   }
   cudaStreamDestroy(s);
+}
+
+double* pinned_buffer() {
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (!g_buffers.empty()) {
+      double* p = g_buffers.back();
+      g_buffers.pop_back();
+      return p;
+    }
+  }
+  double* p = nullptr;
+  if (cudaMallocHost(&p, kPinnedBuffer) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return nullptr;
+  }
+  return p;
+}
+
+void pinned_buffer_release(double* p) {
+  if (!p) return;
+  {
+    std::lock_guard<std::mutex> lk(g_mu);
+    if (g_buffers.size() < kKeptBuffers) {
+      g_buffers.push_back(p);
+      return;
+    }
+  }
+  cudaFreeHost(p);
 }
 
 void* pinned_block() {

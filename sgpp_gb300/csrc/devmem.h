@@ -29,6 +29,12 @@ void dev_free(void* p, cudaStream_t s);
 cudaStream_t stream_acquire();
 void stream_release(cudaStream_t s);
 
+// Pinned host buffers of kPinnedBuffer bytes, for small host vectors that the kernels read and write in
+// place (up to 16 idle ones are kept); nullptr when there is no memory for one
+constexpr size_t kPinnedBuffer = 96 * 1024;
+double* pinned_buffer();
+void pinned_buffer_release(double* p);
+
 // 64-byte pinned host blocks for scalars read back from the device
 void* pinned_block();
 void pinned_release(void* p);

@@ -204,3 +204,28 @@ def test_fp32_and_df64_mult_match_fp64(dim, level, rounds, m, precision, unit, b
     np.testing.assert_array_equal(again, outt)
     kind = sg.SGMEV_KERNEL_MULTT_NEST32 if precision == "float" else sg.SGMEV_KERNEL_MULTT_NESTDF
     assert m > 8192 or op.profileRead(kind)[0] == 2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,level,m", [(2, 3, 1), (2, 3, 8191), (2, 3, 8192), (2, 3, 8193),
+                                         (9, 4, 10766), (9, 4, 10767), (9, 4, 10768),
+                                         (6, 6, 1661), (6, 6, 1662), (6, 7, 5)])
+def test_host_vectors_read_in_place_and_copied(dim, level, m):
+    """Whole products of small host vectors against the same product asked for as two ranges, which
+    go through copies: results of up to 8,192 entries, up to 12,286 entries in all."""
+    grid = _grid(dim, level)
+    n = grid.getSize()
+    rng = np.random.default_rng(m)
+    op = _op(grid, _points(rng, m, dim, level), "auto")
+    alpha, v = rng.standard_normal(n), rng.standard_normal(m)
+    out, outt, parts, partst = np.zeros(m), np.zeros(n), np.zeros(m), np.zeros(n)
+    for _ in range(2):
+        op.mult(alpha, out)
+        op.multTranspose(v, outt)
+        for a, b in ((0, (m + 1) // 2), ((m + 1) // 2, m)):
+            op.mult(alpha, parts, a, b)
+        for a, b in ((0, (n + 1) // 2), ((n + 1) // 2, n)):
+            op.multTranspose(v, partst, a, b)
+        np.testing.assert_array_equal(out, parts)
+        np.testing.assert_array_equal(outt, partst)
+        alpha, v = -2.0 * alpha, 3.0 * v
