@@ -27,7 +27,7 @@
 #include <vector>
 
 #include "block_tc.h"
-#include "cg_cluster.cuh"
+#include "cg_ortho.cuh"
 #include "devmem.h"
 #include "tc_ptx.cuh"
 
@@ -1016,47 +1016,63 @@ __device__ __forceinline__ void bcg_report(double* sc, bool next, double* host) 
   }
 }
 
-// one cluster per column (cg_cluster.cuh)
+// One cluster per column (cg_cluster.cuh). The start of an inner solve for the residuals rr: from nothing
+// (`first`: e = 0, r = rr), else from e and r as the kept directions left them; a column that is done
+// (its tol2 is infinite) gets no correction.
 __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads) bcg_init_kernel(
-    const double* __restrict__ r, double* __restrict__ d, double* __restrict__ e, int64_t np,
-    double* __restrict__ sc, double* __restrict__ host) {
+    const double* __restrict__ rr, double* __restrict__ r, double* __restrict__ e, int64_t np,
+    double* __restrict__ sc, int first, double* __restrict__ host) {
   __shared__ CgShared sh;
   const int k = blockIdx.y;
   const int64_t o = static_cast<int64_t>(k) * np;
-  double v = 0.0;
+  const bool done = sc[kScTol2 + k] == HUGE_VAL;
+  double v0 = 0.0, v = 0.0;
   for (int64_t i = cg_first(); i < np; i += kCgStride) {
-    const double ri = r[o + i];
-    d[o + i] = ri;
-    e[o + i] = 0.0;
+    const double bi = rr[o + i];
+    if (first) r[o + i] = bi;
+    if (first || done) e[o + i] = 0.0;
+    const double ri = first ? bi : r[o + i];
+    v0 = fma(bi, bi, v0);
     v = fma(ri, ri, v);
   }
-  v = cg_cluster_sum(v, sh, 0);
+  v0 = cg_cluster_sum(v0, sh, 0);
+  v = cg_cluster_sum(v, sh, 1);
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     sc[kScDelta + k] = v;
-    sc[kScDelta0 + k] = v;
-    bcg_report(sc, v > sc[kScTol2 + k] * v, host);
+    sc[kScDelta0 + k] = v0;
+    sc[kScBest + k] = v;
+    sc[kScSince + k] = 0.0;
+    bcg_report(sc, v > sc[kScTol2 + k] * v0, host);
   }
   cg_cluster_end();
 }
 
 __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads) bcg_step_kernel(
-    double* __restrict__ e, double* __restrict__ r, double* __restrict__ d,
-    const double* __restrict__ q, int64_t np, double* __restrict__ sc, double* __restrict__ host) {
+    double* __restrict__ e, double* __restrict__ r, const double* __restrict__ d,
+    const double* __restrict__ q, int64_t np, double* __restrict__ sc, double* __restrict__ w,
+    double* __restrict__ host) {
   if (sc[kScStop] != 0.0) return;
   __shared__ CgShared sh;
   const int k = blockIdx.y;
   const int64_t o = static_cast<int64_t>(k) * np;
   const double delta = sc[kScDelta + k], delta0 = sc[kScDelta0 + k];
   const bool take = delta > sc[kScTol2 + k] * delta0;
-  double dq, alpha, rr;
-  cg_column_step(np, d + o, q + o, e + o, r + o, delta, take, false, sh, &dq, &alpha, &rr);
+  double dq, rr;
+  ortho_column_step(np, d + o, q + o, e + o, r + o, take, sh, &dq, &rr);
   cg_cluster_end();  // every block has read the column's scalars
   if (blockIdx.x == 0 && threadIdx.x == 0) {
-    // a column whose step was not taken keeps its delta (and stays as it is); d.q = 0 ends it
+    // a column whose step was not taken keeps its delta (and stays as it is), and so does its set of
+    // directions; d.q = 0 ends it, and so do 128 steps that bring no smaller residual, for this solve
+    w[k] = take ? dq : 0.0;
     const double now = take && dq != 0.0 ? rr : delta;
     sc[kScDelta + k] = now;
-    if (dq == 0.0) sc[kScTol2 + k] = HUGE_VAL;
-    if (take) sc[kScSteps + k] += 1.0;
+    if (take) {
+      sc[kScSteps + k] += 1.0;
+      const double since = now < sc[kScBest + k] ? 0.0 : sc[kScSince + k] + 1.0;
+      sc[kScSince + k] = since;
+      if (since == 0.0) sc[kScBest + k] = now;
+      if (dq == 0.0 || since >= 128.0) sc[kScTol2 + k] = HUGE_VAL;
+    }
     bcg_report(sc, now > sc[kScTol2 + k] * delta0, host);
   }
 }
@@ -1068,15 +1084,15 @@ cudaError_t block_dot(cudaStream_t s, const double* a, const double* b, int64_t 
   return cudaGetLastError();
 }
 
-cudaError_t block_cg_init(cudaStream_t s, const double* r, double* d, double* e, int64_t np,
-                          double* sc, double* host) {
-  bcg_init_kernel<<<dim3(kCgCtas, kBlockRhs), kCgThreads, 0, s>>>(r, d, e, np, sc, host);
+cudaError_t block_cg_init(cudaStream_t s, const double* rr, double* r, double* e, int64_t np, double* sc,
+                          bool first, double* host) {
+  bcg_init_kernel<<<dim3(kCgCtas, kBlockRhs), kCgThreads, 0, s>>>(rr, r, e, np, sc, first ? 1 : 0, host);
   return cudaGetLastError();
 }
 
-cudaError_t block_cg_step(cudaStream_t s, double* e, double* r, double* d, const double* q,
-                          int64_t np, double* sc, double* host) {
-  bcg_step_kernel<<<dim3(kCgCtas, kBlockRhs), kCgThreads, 0, s>>>(e, r, d, q, np, sc, host);
+cudaError_t block_cg_step(cudaStream_t s, double* e, double* r, const double* d, const double* q,
+                          int64_t np, double* sc, double* w, double* host) {
+  bcg_step_kernel<<<dim3(kCgCtas, kBlockRhs), kCgThreads, 0, s>>>(e, r, d, q, np, sc, w, host);
   return cudaGetLastError();
 }
 

@@ -52,22 +52,20 @@ __device__ __forceinline__ int64_t cg_first() {
 }
 constexpr int64_t kCgStride = static_cast<int64_t>(kCgCtas) * kCgThreads;
 
-// dq = d.q; alpha = take && dq != 0 ? delta / dq : 0; x += alpha d; r -= alpha q; rr = r.r;
-// d = r + (rr / delta) d where a step was taken (or `always`)
+// dq = d.q; alpha = dq != 0 ? delta / dq : 0; x += alpha d; r -= alpha q; rr = r.r; d = r + (rr / delta) d
 __device__ __forceinline__ void cg_column_step(int64_t n, double* __restrict__ d,
                                                const double* __restrict__ q,
                                                double* __restrict__ x, double* __restrict__ r,
-                                               double delta, bool take, bool always, CgShared& sh,
-                                               double* dq_out, double* alpha_out, double* rr_out) {
+                                               double delta, CgShared& sh, double* dq_out,
+                                               double* alpha_out, double* rr_out) {
   double acc = 0.0;
   for (int64_t i = cg_first(); i < n; i += kCgStride) acc = fma(d[i], q[i], acc);
   const double dq = cg_cluster_sum(acc, sh, 0);
-  take = take && dq != 0.0;
-  const double alpha = take ? delta / dq : 0.0;
+  const double alpha = dq != 0.0 ? delta / dq : 0.0;
   acc = 0.0;
   for (int64_t i = cg_first(); i < n; i += kCgStride) {
     double ri = r[i];
-    if (take) {
+    if (dq != 0.0) {
       x[i] = fma(alpha, d[i], x[i]);
       ri = fma(-alpha, q[i], ri);
       r[i] = ri;
@@ -75,10 +73,8 @@ __device__ __forceinline__ void cg_column_step(int64_t n, double* __restrict__ d
     acc = fma(ri, ri, acc);
   }
   const double rr = cg_cluster_sum(acc, sh, 1);
-  if (take || always) {
-    const double beta = rr / delta;
-    for (int64_t i = cg_first(); i < n; i += kCgStride) d[i] = fma(beta, d[i], r[i]);
-  }
+  const double beta = rr / delta;
+  for (int64_t i = cg_first(); i < n; i += kCgStride) d[i] = fma(beta, d[i], r[i]);
   *dq_out = dq;
   *alpha_out = alpha;
   *rr_out = rr;

@@ -27,6 +27,7 @@
 #include "subspace.h"
 #include "block_tc.h"
 #include "cg_cluster.cuh"
+#include "cg_ortho.cuh"
 
 namespace sgmev {
 
@@ -515,7 +516,7 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads) cg
   __shared__ CgShared sh;
   const double delta = scal[0];
   double dq, alpha, rr;
-  cg_column_step(n, d, q, x, r, delta, true, true, sh, &dq, &alpha, &rr);
+  cg_column_step(n, d, q, x, r, delta, sh, &dq, &alpha, &rr);
   cg_cluster_end();  // every block has read delta
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     scal[1] = delta;
@@ -2068,6 +2069,129 @@ static int cg_core(sgmev_op* op, int prec, const double* rhs, double* x, double 
   return SGMEV_OK;
 }
 
+struct DevBuf {  // stream-ordered scratch of one call
+  cudaStream_t s;
+  void* p = nullptr;
+  explicit DevBuf(cudaStream_t st) : s(st) {}
+  ~DevBuf() { sgmev::dev_free(p, s); }
+};
+
+// The kept directions of a mixed fit's inner solves (cg_ortho.cuh), `cols` columns of them: P, Q = A P,
+// their d.q and the dot products' scratch, in one buffer of the call.
+struct Directions {
+  DevBuf buf;
+  double *p = nullptr, *q = nullptr, *w = nullptr, *part = nullptr;
+  int64_t kept = 0, cap = 0;
+  explicit Directions(cudaStream_t s) : buf(s) {}
+};
+
+// Room for up to kOrthoKept directions, fewer on very large grids (512 MB) or when the device has no
+// room.
+static int directions_ready(sgmev_op* op, int cols, Directions* ks) {
+  using namespace sgmev;
+  const int64_t np = op->npad;
+  int64_t cap = ortho_cap(int64_t{512} << 20, cols, np);
+  for (;; cap = std::max<int64_t>(2, cap / 4)) {
+    const cudaError_t e = dev_malloc(&ks->buf.p, sizeof(double) * ortho_words(cap, cols, np), op->stream);
+    if (e == cudaSuccess) break;
+    (void)cudaGetLastError();
+    ks->buf.p = nullptr;
+    if (cap == 2) SGMEV_CUDA(e);
+  }
+  ks->p = static_cast<double*>(ks->buf.p);
+  ks->q = ks->p + cap * cols * np;
+  ks->w = ks->q + cap * cols * np;
+  ks->part = ks->w + cap * cols;
+  ks->cap = cap;
+  return SGMEV_OK;
+}
+
+// An inner solve of a mixed fit: (B^T B + lm I) x = rhs to eps |rhs| in operator precision `prec`, by CG
+// over the kept directions; the solves of a fit share them. rhs2 = rhs.rhs. *stalled: 128 steps in a row
+// brought no smaller residual, which is the rounding of the products rather than the problem's doing.
+static int inner_cg(sgmev_op* op, int prec, const double* rhs, double rhs2, double* x, double lm,
+                    int64_t imax, double eps, Directions* ks, int64_t* iters, bool* stalled) {
+  using namespace sgmev;
+  const int64_t np = op->npad, n = op->n;
+  double* r = op->cg + 2 * np;
+  double* sc = op->scal;
+  double* host = op->host_scalar;  // page-locked: {r.r, d.q} of a step, by parity
+  const double delta_0 = rhs2 * eps * eps;
+  double delta = rhs2;
+  SGMEV_CUDA(cudaMemsetAsync(sc + 5, 0, sizeof(double), op->stream));
+  if (ks->kept == 0) {
+    SGMEV_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * np, op->stream));
+    SGMEV_CUDA(cudaMemcpyAsync(r, rhs, sizeof(double) * np, cudaMemcpyDeviceToDevice, op->stream));
+  } else {
+    // the solution in the span of the kept directions, and what it leaves
+    SGMEV_CUDA(ortho_combine(op->stream, 1, n, np, ks->kept, ks->p, rhs, ks->p, ks->w, ks->part, 1.0,
+                             nullptr, x, sc + 5));
+    SGMEV_CUDA(ortho_combine(op->stream, 1, n, np, ks->kept, nullptr, nullptr, ks->q, ks->w, ks->part,
+                             -1.0, rhs, r, sc + 5));
+    op->launches += 3;
+    SGMEV_TRY(dev_dot(op, r, r, n, &delta));
+  }
+  int64_t it = 0, best_it = 0, next = ks->kept;  // next: the direction after the last one formed
+  double best = delta;
+  auto slot = [&](int64_t k) { return std::min(k, ks->cap - 1); };
+  auto direction = [&]() -> int {
+    double* d = ks->p + slot(next) * np;
+    const int64_t k = std::min(next, ks->cap);
+    if (k == 0)
+      SGMEV_CUDA(cudaMemcpyAsync(d, r, sizeof(double) * np, cudaMemcpyDeviceToDevice, op->stream));
+    else
+      SGMEV_CUDA(ortho_combine(op->stream, 1, n, np, k, ks->q, r, ks->p, ks->w, ks->part, -1.0, r, d,
+                               sc + 5));
+    op->launches += k == 0 ? 0 : 2;
+    ++next;
+    return SGMEV_OK;
+  };
+  struct StopScope {
+    sgmev_op* o;
+    StopScope(sgmev_op* op_, const double* flag) : o(op_) { o->nest.stop = o->sub.stop = flag; }
+    ~StopScope() { o->nest.stop = o->sub.stop = nullptr; }
+  };
+  // Step k and the direction after it. As in cg_core the host enqueues a step before it reads the
+  // previous one's residual where a step beyond the stop costs nothing.
+  const bool ahead = nest_mults(op, prec) && !op->use_half;
+  auto enqueue = [&](int64_t k) -> int {
+    const int64_t at = slot(next - 1);
+    double* d = ks->p + at * np;
+    double* q = ks->q + at * np;
+    {
+      StopScope scope(op, sc + 5);
+      SGMEV_TRY(dev_system(op, prec, d, q, lm, true));
+    }
+    ortho_step_kernel<<<kCgCtas, kCgThreads, 0, op->stream>>>(n, d, q, x, r, sc, ks->w + at, delta_0,
+                                                              host + 4 * (k & 1));
+    op->launches += 1;
+    SGMEV_CUDA(cudaGetLastError());
+    SGMEV_CUDA(cudaEventRecord(op->ev_cg[k & 1], op->stream));
+    return direction();
+  };
+  auto running = [&] { return it < imax && delta > delta_0 && delta > 0.0 && it - best_it < 128; };
+  int64_t queued = 0;
+  if (running()) SGMEV_TRY(direction());
+  while (running()) {
+    if (queued == it) SGMEV_TRY(enqueue(queued++));
+    if (ahead && queued < imax) SGMEV_TRY(enqueue(queued++));
+    SGMEV_CUDA(cudaEventSynchronize(op->ev_cg[it & 1]));
+    const volatile double* h = host + 4 * (it & 1);
+    if (h[1] == 0.0) break;  // d.q == 0: nothing moved
+    delta = h[0];
+    ++it;
+    if (delta < best) {
+      best = delta;
+      best_it = it;
+    }
+  }
+  SGMEV_CUDA(cudaGetLastError());
+  ks->kept = std::min(ks->kept + it, ks->cap);
+  *stalled = it - best_it >= 128;
+  *iters = it;
+  return SGMEV_OK;
+}
+
 // 1/diag(B^T B + lm I) into CG slot 9 (Jacobi preconditioner), from one FP32 squared-hat
 // multTranspose with v = 1: diag_i = sum_j prod_t hat_t(x_j)^2. Cached until the grid or lm changes.
 static int dev_precond(sgmev_op* op, double lm) {
@@ -2224,6 +2348,8 @@ static int fit_common(sgmev_op* op, int mode, const double* y, bool y_on_device,
     double* dx = op->cg + 7 * np;
     if (!reuse) SGMEV_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * np, op->stream));
     double rnorm2 = 0.0, r0 = 0.0;
+    bool stalled = false;
+    Directions kept(op->stream);
     const double eps_inner = op->inner_tol;
     if (op->precond) SGMEV_TRY(dev_precond(op, lm));
     for (int outer = 0; outer < 64; ++outer) {
@@ -2241,13 +2367,12 @@ static int fit_common(sgmev_op* op, int mode, const double* y, bool y_on_device,
       if (rnorm2 <= epsilon * epsilon * r0 || rnorm2 == 0.0 || total_it >= max_iterations) break;
       int64_t it = 0;
       double dres = 0.0;
-      // The reduction that ends the refinement: on FP32 products it is solved for where one solve
-      // reaches it, with room for the inner operator's own error, because the looser inner tolerance
-      // would leave a residual anywhere up to epsilon. The less exact FP16 products take one more
-      // solve there, and the residuals it leaves (4e-9 at epsilon 1e-8) are the accuracy to keep.
+      // The reduction that ends the refinement is solved for where one more solve reaches it, with
+      // room for the inner operator's own error: the plain inner tolerance would leave a residual
+      // anywhere up to epsilon. No solve asks for less than what rounded products can give.
       const bool half = inner_on_half(op);
-      const double last = (half ? 0.5 : 0.4) * epsilon * std::sqrt(r0 / rnorm2);
-      const double want = half ? std::max(eps_inner, last) : last > 0.1 * eps_inner ? last : eps_inner;
+      const double last = 0.3 * epsilon * std::sqrt(r0 / rnorm2);
+      const double want = std::max(1e-5, last > 0.1 * eps_inner ? last : eps_inner);
       // the inner solve may use the FP16 copy of the materialised products: the outer residual
       // is FP64-accurate, so the refinement still converges to the FP64 solution
       struct HalfScope {
@@ -2258,6 +2383,10 @@ static int fit_common(sgmev_op* op, int mode, const double* y, bool y_on_device,
       if (op->precond) {
         SGMEV_TRY(pcg_core(op, SGMEV_FP32, rr, dx, lm, max_iterations - total_it,
                            std::min(want, 0.5), &it));
+      } else if (!stalled) {
+        if (outer == 0) SGMEV_TRY(directions_ready(op, 1, &kept));
+        SGMEV_TRY(inner_cg(op, SGMEV_FP32, rr, rnorm2, dx, lm, max_iterations - total_it,
+                           std::min(want, 0.5), &kept, &it, &stalled));
       } else {
         SGMEV_TRY(cg_core(op, SGMEV_FP32, rr, dx, lm, max_iterations - total_it,
                           std::min(want, 0.5), false, &it, &dres));
@@ -2388,13 +2517,6 @@ static int block_system(sgmev_op* op, const double* d, double* q, double lm) {
   return SGMEV_OK;
 }
 
-struct DevBuf {  // stream-ordered scratch of one call
-  cudaStream_t s;
-  void* p = nullptr;
-  explicit DevBuf(cudaStream_t st) : s(st) {}
-  ~DevBuf() { sgmev::dev_free(p, s); }
-};
-
 static int block_products_common(sgmev_op* op, bool transpose, const double* in, double* out) {
   using namespace sgmev;
   SGMEV_TRY(check_op(op));
@@ -2448,19 +2570,19 @@ static int fit_block_common(sgmev_op* op, const double* y, bool y_dev, double la
   const int K = kBlockRhs;
   const int64_t np = op->npad;
   const double lm = static_cast<double>(op->m) * lambda;
-  // b, x, outer residual rr, inner solution e, inner residual r, direction d, product q, temp t
+  // b, x, outer residual rr, inner solution e, inner residual r, temp t
   DevBuf buf(op->stream);
   const size_t vec = static_cast<size_t>(K) * np;
   const size_t parts = static_cast<size_t>(K) * kBlockDotBlocks;
-  SGMEV_CUDA(dev_malloc(&buf.p, sizeof(double) * (8 * vec + parts + kBlockScalars), op->stream));
+  SGMEV_CUDA(dev_malloc(&buf.p, sizeof(double) * (6 * vec + parts + kBlockScalars), op->stream));
+  Directions ks(op->stream);
+  SGMEV_TRY(directions_ready(op, K, &ks));
   double* b = static_cast<double*>(buf.p);
   double* x = b + vec;
   double* rr = x + vec;
   double* e = rr + vec;
   double* r = e + vec;
-  double* d = r + vec;
-  double* q = d + vec;
-  double* t = q + vec;
+  double* t = r + vec;
   double* part_a = t + vec;
   double* sc = part_a + parts;
   SGMEV_CUDA(cudaMemsetAsync(sc, 0, sizeof(double) * kBlockScalars, op->stream));
@@ -2512,33 +2634,54 @@ static int fit_block_common(sgmev_op* op, const double* y, bool y_dev, double la
       all_done = all_done && done[k];
       const double inner_tol =
           op->block_inner_tol > 0.0 ? op->block_inner_tol : (op->block_f16 ? 1e-4 : 1e-3);
-      const double want = std::min(0.5, std::max(inner_tol,
-                                                 epsilon * std::sqrt(rho0[k] / std::max(rho[k], 1e-300)) * 0.5));
+      // the last reduction as in fit_common; the BF16 operands are too coarse for more than inner_tol
+      const double last = 0.3 * epsilon * std::sqrt(rho0[k] / std::max(rho[k], 1e-300));
+      const double want = std::min(
+          0.5, std::max(1e-5, op->block_f16 && last > 0.1 * inner_tol ? last : std::max(inner_tol, last)));
       tol2[k] = done[k] ? HUGE_VAL : want * want;
     }
     if (all_done || total_it >= max_iterations) break;
-    // inner block CG on A e = rr with the BF16 tensor-core products, e = 0 at the start
+    // Inner CG on A e = rr per column with the tensor-core products, each column on its own kept
+    // directions, which the outer iterations share: first its part in their span, then steps.
     SGMEV_CUDA(cudaMemcpyAsync(sc + kScTol2, tol2.data(), sizeof(double) * K, cudaMemcpyHostToDevice,
                                op->stream));
-    SGMEV_CUDA(cudaMemcpyAsync(r, rr, sizeof(double) * vec, cudaMemcpyDeviceToDevice, op->stream));
+    SGMEV_CUDA(cudaMemsetAsync(sc + kScStop, 0, sizeof(double), op->stream));
+    const double* stop = sc + kScStop;
+    const bool first = ks.kept == 0;
+    if (!first) {
+      SGMEV_CUDA(ortho_combine(op->stream, K, op->n, np, ks.kept, ks.p, rr, ks.p, ks.w, ks.part, 1.0,
+                               nullptr, e, stop));
+      SGMEV_CUDA(ortho_combine(op->stream, K, op->n, np, ks.kept, nullptr, nullptr, ks.q, ks.w, ks.part,
+                               -1.0, rr, r, stop));
+      op->launches += 3;
+    }
     // The host enqueues a step before it reads how many columns the previous one leaves active; a
     // step beyond the last finds the stop flag set and skips its products and updates.
     double* slots = op->host_scalar;  // page-locked: columns that take the next step, by parity
-    SGMEV_CUDA(block_cg_init(op->stream, r, d, e, np, sc, slots + 1));
+    SGMEV_CUDA(block_cg_init(op->stream, rr, r, e, np, sc, first, slots + 1));
     SGMEV_CUDA(cudaEventRecord(op->ev_cg[1], op->stream));
     op->launches += 1;
     struct StopScope {
       sgmev_op* o;
       StopScope(sgmev_op* op_, const double* flag) : o(op_) { o->blk.stop = flag; }
       ~StopScope() { o->blk.stop = nullptr; }
-    } stop_scope(op, sc + kScStop);
+    } stop_scope(op, stop);
     int64_t steps = 0, queued = 0;
     while (true) {
       if (total_it + queued - steps < max_iterations) {
+        // a direction conjugate to the kept ones, into the next slot (the last one once all are full)
+        const int64_t next = ks.kept + queued, k = std::min(next, ks.cap), at = std::min(next, ks.cap - 1);
+        double* d = ks.p + at * static_cast<int64_t>(vec);
+        double* q = ks.q + at * static_cast<int64_t>(vec);
+        if (k == 0)
+          SGMEV_CUDA(cudaMemcpyAsync(d, r, sizeof(double) * vec, cudaMemcpyDeviceToDevice, op->stream));
+        else
+          SGMEV_CUDA(ortho_combine(op->stream, K, op->n, np, k, ks.q, r, ks.p, ks.w, ks.part, -1.0, r, d,
+                                   stop));
         SGMEV_TRY(block_system(op, d, q, lm));
-        SGMEV_CUDA(block_cg_step(op->stream, e, r, d, q, np, sc, slots + (queued & 1)));
+        SGMEV_CUDA(block_cg_step(op->stream, e, r, d, q, np, sc, ks.w + at * K, slots + (queued & 1)));
         SGMEV_CUDA(cudaEventRecord(op->ev_cg[queued & 1], op->stream));
-        op->launches += 1;
+        op->launches += k == 0 ? 1 : 3;
         ++queued;
       }
       // what the step before number `steps` (for 0: the start) left
@@ -2547,11 +2690,12 @@ static int fit_block_common(sgmev_op* op, const double* y, bool y_dev, double la
       ++steps;
       ++total_it;
     }
+    ks.kept = std::min(ks.kept + steps, ks.cap);
     axpy_kernel<<<vec_blocks(static_cast<int64_t>(vec)), 256, 0, op->stream>>>(
         static_cast<int64_t>(vec), 1.0, e, x);
     op->launches += 1;
     SGMEV_TRY(block_check(op));
-    if (steps == 0) break;  // no column could take a step: further refinement cannot move
+    if (steps == 0 && first) break;  // no column could take a step: further refinement cannot move
   }
   for (int k = 0; k < K; ++k)
     if (op->n > 0)

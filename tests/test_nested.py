@@ -229,3 +229,57 @@ def test_host_vectors_read_in_place_and_copied(dim, level, m):
         np.testing.assert_array_equal(out, parts)
         np.testing.assert_array_equal(outt, partst)
         alpha, v = -2.0 * alpha, 3.0 * v
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", [sg.SGMEV_SOLVE_MIXED, sg.SGMEV_SOLVE_MIXED_NATIVE64])
+@pytest.mark.parametrize("dim,level,m,lam,inner", [
+    (1, 1, 5, 1e-3, None),       # one direction spans everything
+    (2, 3, 1, 1e-3, None), (3, 4, 700, 1e-4, None), (3, 4, 700, 1e-4, "1e-9"),
+    (4, 6, 3000, 1e-7, None),    # more steps than directions are kept
+    (2, 11, 2000, 1e-5, None),   # dot products in two pieces
+    (5, 5, 40000, 1e-4, "0.3")])  # many short solves
+def test_fits_on_kept_directions_reach_their_residual(dim, level, m, lam, inner, mode):
+    grid = _grid(dim, level)
+    n = grid.getSize()
+    rng = np.random.default_rng(dim * level)
+    x = rng.beta(2.0, 4.0, (m, dim))
+    y = np.sin(4.0 * x.sum(axis=1)) + 0.1 * rng.standard_normal(m)
+    op = sg.OperationMultiEvalCuda(grid, x, sg.SGMEV_FP64, {"inner_tol": inner} if inner else {})
+    eps = 1e-8
+    alpha, its, _ = op.fit(y, lam, 20000, eps, mode=mode)
+    ref = _op(grid, x, "dense")
+    b, pred, a = np.zeros(n), np.zeros(m), np.zeros(n)
+    ref.multTranspose(y, b)
+    ref.mult(alpha, pred)
+    ref.multTranspose(pred, a)
+    # the fit's own criterion, and a relative 1e-11 of the terms for the two evaluations of it
+    r = b - a - lam * m * alpha
+    assert np.linalg.norm(r) <= eps * np.linalg.norm(b) + 1e-11 * (np.linalg.norm(a) + np.linalg.norm(b))
+    assert 0 < its < 20000
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,level,m,lam", [(2, 3, 40, 1e-3), (4, 5, 3000, 1e-4), (4, 5, 3000, 1e-7)])
+def test_block_fits_on_kept_directions_reach_their_residuals(dim, level, m, lam):
+    """Columns that end at different steps, a zero one and two equal ones; more steps than are kept."""
+    grid = _grid(dim, level)
+    n, K = grid.getSize(), sg.SGMEV_BLOCK_RHS
+    rng = np.random.default_rng(m)
+    x = rng.beta(2.0, 4.0, (m, dim))
+    y = np.stack([np.sin((k + 1.0) * x.sum(axis=1)) + 0.1 * rng.standard_normal(m) for k in range(K)])
+    y[3], y[5] = 0.0, y[4]
+    op = sg.OperationMultiEvalCuda(grid, x, sg.SGMEV_FP64, {"algo": "subspace"})
+    eps = 1e-8
+    alpha, its, _ = op.fitBlock(y, lam, 20000, eps)
+    ref = _op(grid, x, "dense")
+    for k in range(K):
+        b, pred, a = np.zeros(n), np.zeros(m), np.zeros(n)
+        ref.multTranspose(y[k], b)
+        ref.mult(alpha[k], pred)
+        ref.multTranspose(pred, a)
+        r = b - a - lam * m * alpha[k]
+        # the fit's own criterion, and a relative 1e-11 of the terms for the two evaluations of it
+        assert np.linalg.norm(r) <= eps * np.linalg.norm(b) + 1e-11 * (np.linalg.norm(a) + np.linalg.norm(b))
+        assert (its[k] > 0) == (k != 3) and its[k] < 20000
+    assert np.all(alpha[3] == 0.0)
