@@ -1040,7 +1040,7 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads) bc
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     sc[kScDelta + k] = v;
     sc[kScDelta0 + k] = v0;
-    sc[kScBest + k] = v;
+    sc[kScMark + k] = v;
     sc[kScSince + k] = 0.0;
     bcg_report(sc, v > sc[kScTol2 + k] * v0, host);
   }
@@ -1050,7 +1050,7 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads) bc
 __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads) bcg_step_kernel(
     double* __restrict__ e, double* __restrict__ r, const double* __restrict__ d,
     const double* __restrict__ q, int64_t np, double* __restrict__ sc, double* __restrict__ w,
-    double* __restrict__ host) {
+    int recurrence, double* __restrict__ host) {
   if (sc[kScStop] != 0.0) return;
   __shared__ CgShared sh;
   const int k = blockIdx.y;
@@ -1062,16 +1062,18 @@ __global__ void __cluster_dims__(kCgCtas, 1, 1) __launch_bounds__(kCgThreads) bc
   cg_cluster_end();  // every block has read the column's scalars
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     // a column whose step was not taken keeps its delta (and stays as it is), and so does its set of
-    // directions; d.q = 0 ends it, and so do 128 steps that bring no smaller residual, for this solve
+    // directions; d.q = 0 ends it, and so does standing still, for this solve
     w[k] = take ? dq : 0.0;
     const double now = take && dq != 0.0 ? rr : delta;
     sc[kScDelta + k] = now;
     if (take) {
       sc[kScSteps + k] += 1.0;
-      const double since = now < sc[kScBest + k] ? 0.0 : sc[kScSince + k] + 1.0;
+      const double since = ortho_progress(now, sc[kScMark + k]) ? 0.0 : sc[kScSince + k] + 1.0;
       sc[kScSince + k] = since;
-      if (since == 0.0) sc[kScBest + k] = now;
-      if (dq == 0.0 || since >= 128.0) sc[kScTol2 + k] = HUGE_VAL;
+      if (since == 0.0) sc[kScMark + k] = now;
+      if (dq == 0.0 ||
+          (!recurrence && ortho_stands_still(static_cast<int64_t>(since), sc[kScMark + k], delta0)))
+        sc[kScTol2 + k] = HUGE_VAL;
     }
     bcg_report(sc, now > sc[kScTol2 + k] * delta0, host);
   }
@@ -1091,8 +1093,9 @@ cudaError_t block_cg_init(cudaStream_t s, const double* rr, double* r, double* e
 }
 
 cudaError_t block_cg_step(cudaStream_t s, double* e, double* r, const double* d, const double* q,
-                          int64_t np, double* sc, double* w, double* host) {
-  bcg_step_kernel<<<dim3(kCgCtas, kBlockRhs), kCgThreads, 0, s>>>(e, r, d, q, np, sc, w, host);
+                          int64_t np, double* sc, double* w, bool recurrence, double* host) {
+  bcg_step_kernel<<<dim3(kCgCtas, kBlockRhs), kCgThreads, 0, s>>>(e, r, d, q, np, sc, w,
+                                                                  recurrence ? 1 : 0, host);
   return cudaGetLastError();
 }
 

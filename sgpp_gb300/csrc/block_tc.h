@@ -115,10 +115,10 @@ bool block_shape_ok(const BlockShape& sh, int smem_cap);
 // zeroed before the first solve): per column delta, delta_0 = rhs.rhs of the solve, the squared relative
 // tolerance (a column takes steps while delta > tol2 * delta_0; a step with d.q = 0 sets it to infinity)
 // and the steps taken over all solves; then the stop flag (no column takes steps any more), two counters
-// of the kernels, and per column the smallest delta and the steps since.
+// of the kernels, and per column the progress mark and the steps since (cg_ortho.cuh).
 constexpr int kBlockDotBlocks = 64;
 constexpr int kScDelta = 0, kScDelta0 = 16, kScTol2 = 32, kScSteps = 48, kScStop = 64, kScCount = 65,
-              kScBest = 72, kScSince = 88, kBlockScalars = 104;
+              kScMark = 72, kScSince = 88, kBlockScalars = 104;
 // part[k * kBlockDotBlocks + b]: per-block sums of a_k . b_k
 cudaError_t block_dot(cudaStream_t s, const double* a, const double* b, int64_t np, double* part);
 // The start of a solve for rr: `first` r = rr and e = 0, else r and e hold what the kept directions gave;
@@ -126,8 +126,8 @@ cudaError_t block_dot(cudaStream_t s, const double* a, const double* b, int64_t 
 cudaError_t block_cg_init(cudaStream_t s, const double* rr, double* r, double* e, int64_t np, double* sc,
                           bool first, double* host);
 // one step along d on every column that takes steps, q = A d given; nothing once the stop flag is set.
-// w[16] = d.q, 0 for a column that took none; *host (page-locked) = columns that take another step
+// w[16] = d.q, 0 for a column that took none; `recurrence`: no column ends for standing still; *host (page-locked) = columns that take another step
 cudaError_t block_cg_step(cudaStream_t s, double* e, double* r, const double* d, const double* q,
-                          int64_t np, double* sc, double* w, double* host);
+                          int64_t np, double* sc, double* w, bool recurrence, double* host);
 
 }  // namespace sgmev

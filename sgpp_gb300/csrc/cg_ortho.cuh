@@ -26,6 +26,22 @@ constexpr int kOrthoEntries = 64;  // entries per block of ortho_apply_kernel, o
 constexpr int kOrthoPieces = 16;   // pieces of a vector in ortho_dot_kernel, at most
 constexpr int64_t kOrthoPiece = 16384;
 
+// A solve's progress (squares): `mark`, the residual after the last step that took 30 % off it since the
+// mark before, and `since`, the steps from there.
+__host__ __device__ inline bool ortho_progress(double delta, double mark) { return delta < 0.5 * mark; }
+// Whether a solve ends for want of it. Kept directions reach the floor that the products' rounding sets and
+// creep from there (16 columns, d = 4 level 5, lambda 1e-5: 3,112 steps instead of 794 of the recurrence);
+// once three digits are gained another refinement is the cheaper way on.
+__host__ __device__ inline bool ortho_stands_still(int64_t since, double mark, double rhs) {
+  return since >= (mark <= 1e-6 * rhs ? 32 : 128);
+}
+// Whether a fit goes on with the two-term recurrence (one direction kept, no standing still), as it always
+// converges: a solve of 128 steps or more took less than a digit off the true residual (squares). Where far
+// more steps are needed than directions are kept that can happen.
+inline bool ortho_gives_up(int64_t steps, double before, double after) {
+  return steps >= 128 && !(after <= 0.01 * before);
+}
+
 // pieces of a dot product of length n
 inline int ortho_pieces(int64_t n) {
   const int64_t p = (n + kOrthoPiece - 1) / kOrthoPiece;

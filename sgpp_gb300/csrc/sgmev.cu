@@ -2107,10 +2107,9 @@ static int directions_ready(sgmev_op* op, int cols, Directions* ks) {
 }
 
 // An inner solve of a mixed fit: (B^T B + lm I) x = rhs to eps |rhs| in operator precision `prec`, by CG
-// over the kept directions; the solves of a fit share them. rhs2 = rhs.rhs. *stalled: 128 steps in a row
-// brought no smaller residual, which is the rounding of the products rather than the problem's doing.
+// over the kept directions, which the solves of a fit share. rhs2 = rhs.rhs.
 static int inner_cg(sgmev_op* op, int prec, const double* rhs, double rhs2, double* x, double lm,
-                    int64_t imax, double eps, Directions* ks, int64_t* iters, bool* stalled) {
+                    int64_t imax, double eps, Directions* ks, int64_t* iters) {
   using namespace sgmev;
   const int64_t np = op->npad, n = op->n;
   double* r = op->cg + 2 * np;
@@ -2131,8 +2130,8 @@ static int inner_cg(sgmev_op* op, int prec, const double* rhs, double rhs2, doub
     op->launches += 3;
     SGMEV_TRY(dev_dot(op, r, r, n, &delta));
   }
-  int64_t it = 0, best_it = 0, next = ks->kept;  // next: the direction after the last one formed
-  double best = delta;
+  int64_t it = 0, mark_it = 0, next = ks->kept;  // next: the direction after the last one formed
+  double mark = delta;
   auto slot = [&](int64_t k) { return std::min(k, ks->cap - 1); };
   auto direction = [&]() -> int {
     double* d = ks->p + slot(next) * np;
@@ -2169,7 +2168,10 @@ static int inner_cg(sgmev_op* op, int prec, const double* rhs, double rhs2, doub
     SGMEV_CUDA(cudaEventRecord(op->ev_cg[k & 1], op->stream));
     return direction();
   };
-  auto running = [&] { return it < imax && delta > delta_0 && delta > 0.0 && it - best_it < 128; };
+  auto running = [&] {
+    return it < imax && delta > delta_0 && delta > 0.0 &&
+           (ks->cap == 1 || !ortho_stands_still(it - mark_it, mark, rhs2));
+  };
   int64_t queued = 0;
   if (running()) SGMEV_TRY(direction());
   while (running()) {
@@ -2180,14 +2182,13 @@ static int inner_cg(sgmev_op* op, int prec, const double* rhs, double rhs2, doub
     if (h[1] == 0.0) break;  // d.q == 0: nothing moved
     delta = h[0];
     ++it;
-    if (delta < best) {
-      best = delta;
-      best_it = it;
+    if (ortho_progress(delta, mark)) {
+      mark = delta;
+      mark_it = it;
     }
   }
   SGMEV_CUDA(cudaGetLastError());
   ks->kept = std::min(ks->kept + it, ks->cap);
-  *stalled = it - best_it >= 128;
   *iters = it;
   return SGMEV_OK;
 }
@@ -2348,7 +2349,8 @@ static int fit_common(sgmev_op* op, int mode, const double* y, bool y_on_device,
     double* dx = op->cg + 7 * np;
     if (!reuse) SGMEV_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * np, op->stream));
     double rnorm2 = 0.0, r0 = 0.0;
-    bool stalled = false;
+    int64_t last_it = 0;
+    double last_rnorm2 = 0.0;
     Directions kept(op->stream);
     const double eps_inner = op->inner_tol;
     if (op->precond) SGMEV_TRY(dev_precond(op, lm));
@@ -2366,7 +2368,6 @@ static int fit_common(sgmev_op* op, int mode, const double* y, bool y_on_device,
       res = rnorm2;
       if (rnorm2 <= epsilon * epsilon * r0 || rnorm2 == 0.0 || total_it >= max_iterations) break;
       int64_t it = 0;
-      double dres = 0.0;
       // The reduction that ends the refinement is solved for where one more solve reaches it, with
       // room for the inner operator's own error: the plain inner tolerance would leave a residual
       // anywhere up to epsilon. No solve asks for less than what rounded products can give.
@@ -2383,13 +2384,16 @@ static int fit_common(sgmev_op* op, int mode, const double* y, bool y_on_device,
       if (op->precond) {
         SGMEV_TRY(pcg_core(op, SGMEV_FP32, rr, dx, lm, max_iterations - total_it,
                            std::min(want, 0.5), &it));
-      } else if (!stalled) {
-        if (outer == 0) SGMEV_TRY(directions_ready(op, 1, &kept));
-        SGMEV_TRY(inner_cg(op, SGMEV_FP32, rr, rnorm2, dx, lm, max_iterations - total_it,
-                           std::min(want, 0.5), &kept, &it, &stalled));
       } else {
-        SGMEV_TRY(cg_core(op, SGMEV_FP32, rr, dx, lm, max_iterations - total_it,
-                          std::min(want, 0.5), false, &it, &dres));
+        if (outer == 0)
+          SGMEV_TRY(directions_ready(op, 1, &kept));
+        else if (ortho_gives_up(last_it, last_rnorm2, rnorm2))
+          kept.cap = 1;
+        if (kept.cap == 1) kept.kept = 0;
+        SGMEV_TRY(inner_cg(op, SGMEV_FP32, rr, rnorm2, dx, lm, max_iterations - total_it,
+                           std::min(want, 0.5), &kept, &it));
+        last_it = it;
+        last_rnorm2 = rnorm2;
       }
       total_it += it;
       SGMEV_TRY(dev_axpy(op, np, 1.0, dx, x));
@@ -2614,7 +2618,7 @@ static int fit_block_common(sgmev_op* op, const double* y, bool y_dev, double la
     op->launches += 1;
     return SGMEV_OK;
   };
-  int64_t total_it = 0;
+  int64_t total_it = 0, steps = 0;
   for (int outer = 0; outer < 64; ++outer) {
     if (outer == 0) {
       SGMEV_CUDA(cudaMemcpyAsync(rr, b, sizeof(double) * vec, cudaMemcpyDeviceToDevice, op->stream));
@@ -2626,8 +2630,13 @@ static int fit_block_common(sgmev_op* op, const double* y, bool y_dev, double la
         op->launches += 1;
       }
     }
+    const std::vector<double> before = rho;
     SGMEV_TRY(block_norms(rr, rho));
     if (outer == 0) rho0 = rho;
+    for (int k = 0; k < K && outer > 0; ++k)
+      if (!done[k] && ortho_gives_up(steps, before[k], rho[k])) ks.cap = 1;
+    if (ks.cap == 1) ks.kept = 0;
+    const bool recurrence = ks.cap == 1;
     bool all_done = true;
     for (int k = 0; k < K; ++k) {
       done[k] = done[k] || rho[k] <= epsilon * epsilon * rho0[k] || rho[k] == 0.0;
@@ -2666,7 +2675,8 @@ static int fit_block_common(sgmev_op* op, const double* y, bool y_dev, double la
       StopScope(sgmev_op* op_, const double* flag) : o(op_) { o->blk.stop = flag; }
       ~StopScope() { o->blk.stop = nullptr; }
     } stop_scope(op, stop);
-    int64_t steps = 0, queued = 0;
+    int64_t queued = 0;
+    steps = 0;
     while (true) {
       if (total_it + queued - steps < max_iterations) {
         // a direction conjugate to the kept ones, into the next slot (the last one once all are full)
@@ -2679,7 +2689,8 @@ static int fit_block_common(sgmev_op* op, const double* y, bool y_dev, double la
           SGMEV_CUDA(ortho_combine(op->stream, K, op->n, np, k, ks.q, r, ks.p, ks.w, ks.part, -1.0, r, d,
                                    stop));
         SGMEV_TRY(block_system(op, d, q, lm));
-        SGMEV_CUDA(block_cg_step(op->stream, e, r, d, q, np, sc, ks.w + at * K, slots + (queued & 1)));
+        SGMEV_CUDA(block_cg_step(op->stream, e, r, d, q, np, sc, ks.w + at * K, recurrence,
+                                 slots + (queued & 1)));
         SGMEV_CUDA(cudaEventRecord(op->ev_cg[queued & 1], op->stream));
         op->launches += k == 0 ? 1 : 3;
         ++queued;
