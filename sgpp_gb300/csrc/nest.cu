@@ -683,9 +683,14 @@ bool nest_build(NestPlan* p, int dim, int64_t n, const double* level_pow2, const
 }
 
 void nest_free(NestPlan* p) {
-  void* ptrs[] = {p->block, p->rows, p->tab64, p->tab_hi, p->xcell};
+  void* ptrs[] = {p->block, p->rows[0], p->rows[1], p->rows[2], p->tab64, p->tab_hi, p->xcell};
   for (void* q : ptrs) dev_free(q, p->stream);
   *p = NestPlan{};
+}
+
+bool nest_built(const NestPlan& p, int precision, bool transpose) {
+  return p.ok && (precision == SGMEV_FP64 ? p.tab64 != nullptr : p.tab_hi != nullptr) &&
+         (!transpose || !p.streams[precision].empty());
 }
 
 namespace {
@@ -874,7 +879,7 @@ cudaError_t nest_mult(NestPlan& p, cudaStream_t s, int precision, const NestDens
 
 namespace {
 template <typename V, typename VIN>
-cudaError_t multt(NestPlan& p, cudaStream_t s, std::vector<int>& streams, const NestDense& dense,
+cudaError_t multt(NestPlan& p, cudaStream_t s, std::vector<int>& streams, double*& rows, const NestDense& dense,
                   int64_t m, const VIN* v, int64_t npad, double* out, const double* add, double scale,
                   int num_sms, int* launches) {
   constexpr bool kF64 = std::is_same<V, double>::value;
@@ -898,14 +903,8 @@ cudaError_t multt(NestPlan& p, cudaStream_t s, std::vector<int>& streams, const 
           1, std::min<int64_t>({resident / c.chunks, n_tiles, (int64_t(1) << 25) / c.row_len}))));
       elems += st.back() * c.row_len;
     }
-    if (elems > p.row_elems) {
-      dev_free(p.rows, s);
-      p.rows = nullptr;
-      p.row_elems = 0;
-      e = dev_malloc(&p.rows, sizeof(double) * elems, s);
-      if (e != cudaSuccess) return e;
-      p.row_elems = elems;
-    }
+    e = dev_malloc(&rows, sizeof(double) * elems, s);
+    if (e != cudaSuccess) return e;
     streams = st;
   }
   if (npad > p.n) {
@@ -926,7 +925,7 @@ cudaError_t multt(NestPlan& p, cudaStream_t s, std::vector<int>& streams, const 
   a.dim = p.dim;
   a.bad = p.bad;
   a.stop = p.stop;
-  a.rows = p.rows;
+  a.rows = rows;
   int64_t cs_at = 0;
   for (size_t k = 0; k < p.classes.size(); ++k) {
     const NestClass& c = p.classes[k];
@@ -956,12 +955,13 @@ cudaError_t nest_multt(NestPlan& p, cudaStream_t s, int precision, const NestDen
                        const double* v64, const float* v32, int64_t npad, double* out,
                        const double* add, double scale, int num_sms, int* launches) {
   std::vector<int>& st = p.streams[precision];
+  double*& rows = p.rows[precision];
   if (precision == SGMEV_FP64)
-    return multt<double>(p, s, st, dense, m, v64, npad, out, add, scale, num_sms, launches);
+    return multt<double>(p, s, st, rows, dense, m, v64, npad, out, add, scale, num_sms, launches);
   if (precision == SGMEV_DF64)
-    return multt<ff>(p, s, st, dense, m, v64, npad, out, add, scale, num_sms, launches);
-  if (v32) return multt<float>(p, s, st, dense, m, v32, npad, out, add, scale, num_sms, launches);
-  return multt<float>(p, s, st, dense, m, v64, npad, out, add, scale, num_sms, launches);
+    return multt<ff>(p, s, st, rows, dense, m, v64, npad, out, add, scale, num_sms, launches);
+  if (v32) return multt<float>(p, s, st, rows, dense, m, v32, npad, out, add, scale, num_sms, launches);
+  return multt<float>(p, s, st, rows, dense, m, v64, npad, out, add, scale, num_sms, launches);
 }
 
 }  // namespace sgmev

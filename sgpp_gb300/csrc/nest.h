@@ -35,8 +35,7 @@ struct NestPlan {
   int *lmax = nullptr, *inv = nullptr, *clev = nullptr, *ccell = nullptr, *tinv = nullptr;
   NestOp4 *windows = nullptr, *prog = nullptr, *chunks = nullptr;
   NestOp2 *cq = nullptr, *cs = nullptr, *cwarp = nullptr;
-  double* rows = nullptr;  // multTranspose: partial rows, per class [streams][row_len]
-  int64_t row_elems = 0;
+  double* rows[3] = {nullptr, nullptr, nullptr};  // multTranspose: partial rows, per class [streams][row_len]
   void* coef = nullptr;    // [total] coefficients in position order, in the product's precision
   int* bad = nullptr;      // flags of values that are not finite, one per block
   // tables of the data, built on the first product
@@ -50,6 +49,8 @@ struct NestPlan {
 bool nest_build(NestPlan* p, int dim, int64_t n, const double* level_pow2, const double* index,
                 bool mod, int num_sms, cudaStream_t stream, std::string* err);
 void nest_free(NestPlan* p);
+// whether the product needs nothing more to be built (a product under stream capture must not)
+bool nest_built(const NestPlan& p, int precision, bool transpose);
 
 // The dense form of the operands, for coefficients or vectors that are not finite: such a value
 // times a hat of 0 is NaN at every point outside the function's support, as in the dense kernels.

@@ -858,6 +858,14 @@ static int64_t multt_tile_pts(const sgmev_op* op, int prec) {
   return kBlock * Blocking<float>::multt_r(op->dim);
 }
 
+// Whether the op's stream is being captured into a graph: what a product would build on first use
+// (plans, tables, rows) cannot be built then, and it runs on the kernels that need nothing.
+static bool capturing(const sgmev_op* op) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(op->stream, &st) != cudaSuccess) (void)cudaGetLastError();
+  return st != cudaStreamCaptureStatusNone;
+}
+
 // ---------------------------------------------------------------------------------------
 // device-side products on padded device vectors
 // ---------------------------------------------------------------------------------------
@@ -868,6 +876,7 @@ static int64_t multt_tile_pts(const sgmev_op* op, int prec) {
 static bool sub_ready(sgmev_op* op, std::string* why = nullptr) {
   using namespace sgmev;
   if (op->sub_tried) return op->sub_ok;
+  if (capturing(op)) return false;
   op->sub_tried = true;
   if (op->algo == 0 || op->n < 1) return false;
   std::string reason;
@@ -894,6 +903,7 @@ static bool mat_ready(sgmev_op* op) {
   using namespace sgmev;
   if (op->mat_block_only) return false;
   if (op->sub.pmat) return true;
+  if (capturing(op)) return false;
   if (op->mat_mode == 0 || op->mat_failed || !subspace_mat_fits(op->sub, false)) return false;
   // ModLinear products are built for data in the cube (the cell of a boundary-adjacent function
   // is clamped there); data outside it stays on the dense kernels, which extrapolate
@@ -945,7 +955,8 @@ static bool nest_ready(sgmev_op* op) {
 }
 
 static bool nest_mults(sgmev_op* op, int prec) {
-  return (prec == SGMEV_FP64 || (op->mat_mode != 2 && !op->use_half)) && nest_ready(op);
+  if (prec != SGMEV_FP64 && (op->mat_mode == 2 || op->use_half)) return false;
+  return sgmev::nest_built(op->nest, prec, false) || (!capturing(op) && nest_ready(op));
 }
 
 // The FP32 and float-float multTranspose: nested up to 8,192 data points, where it also saves building
@@ -954,7 +965,7 @@ static bool nest_mults(sgmev_op* op, int prec) {
 // above that the materialised kernels win), and float-float on grids that the materialised kernels
 // do not take up to 10^8 subspaces x points (d=6 level 7, 64,000 points: 422 against 441 us).
 static bool nest_multts(sgmev_op* op, int prec) {
-  if (!nest_mults(op, prec)) return false;
+  if (!nest_mults(op, prec) || (!sgmev::nest_built(op->nest, prec, true) && capturing(op))) return false;
   if (prec == SGMEV_FP64 || op->m <= 8192) return true;
   return prec == SGMEV_DF64 && static_cast<double>(op->nest.n_sub) * op->m <= 1e8 &&
          !(sub_ready(op) && op->mat_multt && subspace_mat_fits(op->sub, true) && mat_ready(op));

@@ -283,3 +283,38 @@ def test_block_fits_on_kept_directions_reach_their_residuals(dim, level, m, lam)
         assert np.linalg.norm(r) <= eps * np.linalg.norm(b) + 1e-11 * (np.linalg.norm(a) + np.linalg.norm(b))
         assert (its[k] > 0) == (k != 3) and its[k] < 20000
     assert np.all(alpha[3] == 0.0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("built", [False, True])
+@pytest.mark.parametrize("precision,unit", [("double", EPS), ("float", 2.0 ** -24), ("df64", 2.0 ** -44)])
+def test_products_captured_into_a_graph(precision, unit, built):
+    """A first product under capture runs on kernels that build nothing, a later one as outside."""
+    torch = pytest.importorskip("torch")
+    grid = _grid(4, 4)
+    n, m, dim = grid.getSize(), 3000, 4
+    rng = np.random.default_rng(1)
+    op = _op(grid, _points(rng, m, dim, 5), "auto", precision)
+    a, v = torch.from_numpy(rng.standard_normal(n)).cuda(), torch.from_numpy(rng.standard_normal(m)).cuda()
+    out = [torch.zeros(k, dtype=torch.float64, device="cuda") for k in (m, n)]
+    stream = torch.cuda.Stream()
+    op.setStream(stream.cuda_stream)
+
+    def products():
+        op.multDevice(a.data_ptr(), out[0].data_ptr())
+        op.multTransposeDevice(v.data_ptr(), out[1].data_ptr())
+
+    if built:
+        products()
+        torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        products()
+    graph.replay()
+    torch.cuda.synchronize()
+    got = [o.clone() for o in out]
+    products()
+    torch.cuda.synchronize()
+    for g, o, x, k in zip(got, out, (a, v), (n, m)):
+        bound = 0.0 if built else (6 * dim + k) * unit * float(x.abs().sum())
+        assert float((g - o).abs().max()) <= bound
