@@ -4,11 +4,13 @@
 //   staging   data rows -> dim-major FP64 and FP32 copies, grid (2^l, i) -> interleaved pairs
 //   plans     per precision: CTA tile shapes and the 2-D split (tiles x chunks) sized so that
 //             every launch has at least `target_ctas` CTAs on the 152 SMs
-//   products  mult / multT = one tile kernel writing partials + one fixed-order reduce kernel
-//   system    B^T(B a) + lambda*M*a: mult, reduce into the M-vector, multT, reduce (+ lambda term)
-//   fit       conjugate gradients with every vector on the device; scalars come back to the
-//             host once per dot product to drive the loop exactly like
-//             solver/src/sgpp/solver/sle/ConjugateGradients.cpp:22-151
+//   products  the nested kernels (nest.cu) for FP64, FP32 and float-float mult and for multT in FP64
+//             and on small data sets; the materialised ones (subspace_mat.cu) for the other multT;
+//             dense tile kernels + a fixed-order reduce where neither takes the grid or the data
+//   system    B^T(B a) + lambda*M*a: mult into the M-vector, multT (+ lambda term)
+//   fit       conjugate gradients with every vector on the device: plain, in the steps of
+//             solver/src/sgpp/solver/sle/ConjugateGradients.cpp:22-151, or mixed, iterative
+//             refinement around inner solves that keep their directions (cg_ortho.cuh)
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -404,8 +406,8 @@ __global__ void xpby_kernel(int64_t n, const double* __restrict__ r, double beta
 // ---- CG with its scalars on the device ---------------------------------------------------
 // scal[0] delta_new, [1] delta_old, [2] d.q, [3] alpha, [4] beta; a ticket counter (scal + 8)
 // lets the last block of a launch add the partials. Every sum has the thread mapping and the
-// tree of dot_partial_kernel + dot_final_kernel, so the scalars are bit-identical to the
-// host-driven loop's.
+// tree of dot_partial_kernel + dot_final_kernel. Vectors beyond kClusterVector entries and the steps
+// with a true residual use these kernels, the others cg_step_kernel.
 __device__ __forceinline__ double block_tree_sum(double acc, double* s) {
   s[threadIdx.x] = acc;
   __syncthreads();
@@ -965,6 +967,7 @@ static bool nest_mults(sgmev_op* op, int prec) {
 // above that the materialised kernels win), and float-float on grids that the materialised kernels
 // do not take up to 10^8 subspaces x points (d=6 level 7, 64,000 points: 422 against 441 us).
 static bool nest_multts(sgmev_op* op, int prec) {
+  if (prec == SGMEV_FP32 && op->m > 8192) return false;  // (before the plan is built for nothing)
   if (!nest_mults(op, prec) || (!sgmev::nest_built(op->nest, prec, true) && capturing(op))) return false;
   if (prec == SGMEV_FP64 || op->m <= 8192) return true;
   return prec == SGMEV_DF64 && static_cast<double>(op->nest.n_sub) * op->m <= 1e8 &&
@@ -1979,8 +1982,8 @@ static int cg_core(sgmev_op* op, int prec, const double* rhs, double* x, double 
     op->launches += 1;
   }
   SGMEV_CUDA(cudaMemcpyAsync(d, r, sizeof(double) * np, cudaMemcpyDeviceToDevice, op->stream));
-  // the scalars live on the device (alpha and beta never visit the host); the host reads
-  // delta_new and d.q once per iteration for the stopping test
+  // the scalars live on the device (alpha and beta never visit the host); the host reads delta_new and
+  // d.q of a step for the stopping test, where it can after the next step is enqueued
   double* sc = op->scal;
   double* host = op->host_scalar;  // pinned: [0] delta_new, [1] delta_old, [2] d.q
   auto read_scalars = [&]() -> int {
@@ -2172,9 +2175,19 @@ static int inner_cg(sgmev_op* op, int prec, const double* rhs, double rhs2, doub
       StopScope scope(op, sc + 5);
       SGMEV_TRY(dev_system(op, prec, d, q, lm, true));
     }
+    op->launches += 1;
+    if (n <= kOrthoShort) {
+      ortho_short_kernel<<<kCgCtas, kCgThreads, 0, op->stream>>>(
+          static_cast<int>(n), static_cast<int>(np), ks->p, ks->q, ks->w, static_cast<int>(at),
+          static_cast<int>(std::min(next, ks->cap)), ks->p + slot(next) * np, x, r, sc, delta_0,
+          host + 4 * (k & 1));
+      ++next;
+      SGMEV_CUDA(cudaGetLastError());
+      SGMEV_CUDA(cudaEventRecord(op->ev_cg[k & 1], op->stream));
+      return SGMEV_OK;
+    }
     ortho_step_kernel<<<kCgCtas, kCgThreads, 0, op->stream>>>(n, d, q, x, r, sc, ks->w + at, delta_0,
                                                               host + 4 * (k & 1));
-    op->launches += 1;
     SGMEV_CUDA(cudaGetLastError());
     SGMEV_CUDA(cudaEventRecord(op->ev_cg[k & 1], op->stream));
     return direction();

@@ -238,6 +238,7 @@ def test_host_vectors_read_in_place_and_copied(dim, level, m):
     (2, 3, 1, 1e-3, None), (3, 4, 700, 1e-4, None), (3, 4, 700, 1e-4, "1e-9"),
     (4, 6, 3000, 1e-7, None),    # more steps than directions are kept
     (2, 11, 2000, 1e-5, None),   # dot products in two pieces
+    (1, 12, 3000, 1e-4, None), (7, 5, 3000, 1e-4, None),  # 4,095 and 4,159 entries: one cluster or not
     (5, 5, 40000, 1e-4, "0.3")])  # many short solves
 def test_fits_on_kept_directions_reach_their_residual(dim, level, m, lam, inner, mode):
     grid = _grid(dim, level)
