@@ -878,35 +878,42 @@ cudaError_t nest_mult(NestPlan& p, cudaStream_t s, int precision, const NestDens
 }
 
 namespace {
+// the multTranspose's streams and partial rows in the precision
+template <typename V>
+cudaError_t multt_rows(NestPlan& p, cudaStream_t s, int precision, int64_t m, int num_sms) {
+  if (!p.streams[precision].empty()) return cudaSuccess;
+  auto kern = nest_multt_kernel<V, double>;
+  const int64_t n_tiles = std::max<int64_t>(1, (m + kTile - 1) / kTile);
+  // as many streams as fit the SMs at once (at most 256 MB of rows); fixed from here on, and
+  // with them the order of every sum
+  std::vector<int> st;
+  int64_t elems = 0;
+  for (const NestClass& c : p.classes) {
+    const size_t sm = c.smem(sizeof(V), p.n_ent, p.dim);
+    cudaError_t e = set_smem_cap(kern, sm);
+    if (e == cudaSuccess && std::is_same<V, float>::value) e = set_smem_cap(nest_multt_kernel<float, float>, sm);
+    int per_sm = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, c.threads, sm);
+    if (e != cudaSuccess) return e;
+    const int64_t resident = std::min<int64_t>(4, std::max(1, per_sm)) * num_sms;
+    st.push_back(static_cast<int>(std::max<int64_t>(
+        1, std::min<int64_t>({resident / c.chunks, n_tiles, (int64_t(1) << 25) / c.row_len}))));
+    elems += st.back() * c.row_len;
+  }
+  const cudaError_t e = dev_malloc(&p.rows[precision], sizeof(double) * elems, s);
+  if (e == cudaSuccess) p.streams[precision] = st;
+  return e;
+}
+
 template <typename V, typename VIN>
-cudaError_t multt(NestPlan& p, cudaStream_t s, std::vector<int>& streams, double*& rows, const NestDense& dense,
-                  int64_t m, const VIN* v, int64_t npad, double* out, const double* add, double scale,
-                  int num_sms, int* launches) {
+cudaError_t multt(NestPlan& p, cudaStream_t s, int precision, const NestDense& dense, int64_t m, const VIN* v,
+                  int64_t npad, double* out, const double* add, double scale, int* launches) {
   constexpr bool kF64 = std::is_same<V, double>::value;
-  cudaError_t e = tables(p, s, dense, m, kF64, launches);
-  if (e != cudaSuccess) return e;
+  const std::vector<int>& streams = p.streams[precision];
+  double* rows = p.rows[precision];
+  cudaError_t e = cudaSuccess;
   auto kern = nest_multt_kernel<V, VIN>;
   const int64_t n_tiles = std::max<int64_t>(1, (m + kTile - 1) / kTile);
-  if (streams.empty()) {
-    // as many streams as fit the SMs at once (at most 256 MB of rows); fixed from here on, and
-    // with them the order of every sum
-    std::vector<int> st;
-    int64_t elems = 0;
-    for (const NestClass& c : p.classes) {
-      const size_t sm = c.smem(sizeof(V), p.n_ent, p.dim);
-      e = set_smem_cap(kern, sm);
-      int per_sm = 0;
-      if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, c.threads, sm);
-      if (e != cudaSuccess) return e;
-      const int64_t resident = std::min<int64_t>(4, std::max(1, per_sm)) * num_sms;
-      st.push_back(static_cast<int>(std::max<int64_t>(
-          1, std::min<int64_t>({resident / c.chunks, n_tiles, (int64_t(1) << 25) / c.row_len}))));
-      elems += st.back() * c.row_len;
-    }
-    e = dev_malloc(&rows, sizeof(double) * elems, s);
-    if (e != cudaSuccess) return e;
-    streams = st;
-  }
   if (npad > p.n) {
     e = cudaMemsetAsync(out + p.n, 0, sizeof(double) * (npad - p.n), s);
     if (e != cudaSuccess) return e;
@@ -951,17 +958,29 @@ cudaError_t multt(NestPlan& p, cudaStream_t s, std::vector<int>& streams, double
 }
 }  // namespace
 
+bool nest_prepare(NestPlan& p, cudaStream_t s, int precision, bool transpose, const NestDense& dense,
+                  int64_t m, int num_sms, int* launches) {
+  bool& refused = p.refused[transpose ? 1 : 0][precision];
+  if (refused) return false;
+  cudaError_t e = tables(p, s, dense, m, precision == SGMEV_FP64, launches);
+  if (e == cudaSuccess && transpose)
+    e = precision == SGMEV_FP64   ? multt_rows<double>(p, s, precision, m, num_sms)
+        : precision == SGMEV_DF64 ? multt_rows<ff>(p, s, precision, m, num_sms)
+                                  : multt_rows<float>(p, s, precision, m, num_sms);
+  if (e != cudaSuccess) (void)cudaGetLastError();
+  refused = e != cudaSuccess;
+  return !refused;
+}
+
 cudaError_t nest_multt(NestPlan& p, cudaStream_t s, int precision, const NestDense& dense, int64_t m,
                        const double* v64, const float* v32, int64_t npad, double* out,
-                       const double* add, double scale, int num_sms, int* launches) {
-  std::vector<int>& st = p.streams[precision];
-  double*& rows = p.rows[precision];
+                       const double* add, double scale, int* launches) {
   if (precision == SGMEV_FP64)
-    return multt<double>(p, s, st, rows, dense, m, v64, npad, out, add, scale, num_sms, launches);
+    return multt<double>(p, s, precision, dense, m, v64, npad, out, add, scale, launches);
   if (precision == SGMEV_DF64)
-    return multt<ff>(p, s, st, rows, dense, m, v64, npad, out, add, scale, num_sms, launches);
-  if (v32) return multt<float>(p, s, st, rows, dense, m, v32, npad, out, add, scale, num_sms, launches);
-  return multt<float>(p, s, st, rows, dense, m, v64, npad, out, add, scale, num_sms, launches);
+    return multt<ff>(p, s, precision, dense, m, v64, npad, out, add, scale, launches);
+  if (v32) return multt<float>(p, s, precision, dense, m, v32, npad, out, add, scale, launches);
+  return multt<float>(p, s, precision, dense, m, v64, npad, out, add, scale, launches);
 }
 
 }  // namespace sgmev

@@ -42,6 +42,7 @@ struct NestPlan {
   double* tab64 = nullptr;    // [n_ent][mpad], FP64 products
   float* tab_hi = nullptr;    // [2][n_ent][mpad], high and low parts, FP32 and float-float products
   uint32_t* xcell = nullptr;  // [dim][mpad]
+  bool refused[2][3] = {};  // by direction and precision: nest_prepare() found no memory
   cudaStream_t stream = nullptr;
 };
 
@@ -60,6 +61,11 @@ struct NestDense {
   int64_t mpad;
 };
 
+// Builds what a product of the precision needs beside the plan: the tables of the data and, for the
+// transpose, its partial rows. False when there is no memory for them (not tried again).
+bool nest_prepare(NestPlan& p, cudaStream_t s, int precision, bool transpose, const NestDense& dense,
+                  int64_t m, int num_sms, int* launches);
+
 // out32[j] and / or out64[j] = sum_g alpha_g phi_g(x_j) in the given precision (SGMEV_FP64, SGMEV_FP32,
 // SGMEV_DF64), j in [j_begin, j_end) and the rest of their tiles (32 points, 64 in FP32) up to
 // out_end, 0 beyond m; alpha [n] FP64;
@@ -73,6 +79,6 @@ cudaError_t nest_mult(NestPlan& p, cudaStream_t s, int precision, const NestDens
 // v64 [m], or v32 [m] (nullptr: v64) for SGMEV_FP32
 cudaError_t nest_multt(NestPlan& p, cudaStream_t s, int precision, const NestDense& dense, int64_t m,
                        const double* v64, const float* v32, int64_t npad, double* out,
-                       const double* add, double scale, int num_sms, int* launches);
+                       const double* add, double scale, int* launches);
 
 }  // namespace sgmev

@@ -956,9 +956,22 @@ static bool nest_ready(sgmev_op* op) {
   return true;
 }
 
+// Whether the product's tables and rows are there or could be built; without memory for them it runs as
+// on a grid that the plan does not take.
+static bool nest_prepared(sgmev_op* op, int prec, bool transpose) {
+  using namespace sgmev;
+  if (nest_built(op->nest, prec, transpose)) return true;
+  if (capturing(op) || !nest_ready(op)) return false;
+  int launches = 0;
+  const bool ok = nest_prepare(op->nest, op->stream, prec, transpose,
+                               NestDense{op->xt64, op->li64, op->mpad}, op->m, op->num_sms, &launches);
+  op->launches += launches;
+  return ok;
+}
+
 static bool nest_mults(sgmev_op* op, int prec) {
   if (prec != SGMEV_FP64 && (op->mat_mode == 2 || op->use_half)) return false;
-  return sgmev::nest_built(op->nest, prec, false) || (!capturing(op) && nest_ready(op));
+  return nest_prepared(op, prec, false);
 }
 
 // The FP32 and float-float multTranspose: nested up to 8,192 data points, where it also saves building
@@ -968,10 +981,12 @@ static bool nest_mults(sgmev_op* op, int prec) {
 // do not take up to 10^8 subspaces x points (d=6 level 7, 64,000 points: 422 against 441 us).
 static bool nest_multts(sgmev_op* op, int prec) {
   if (prec == SGMEV_FP32 && op->m > 8192) return false;  // (before the plan is built for nothing)
-  if (!nest_mults(op, prec) || (!sgmev::nest_built(op->nest, prec, true) && capturing(op))) return false;
-  if (prec == SGMEV_FP64 || op->m <= 8192) return true;
-  return prec == SGMEV_DF64 && static_cast<double>(op->nest.n_sub) * op->m <= 1e8 &&
-         !(sub_ready(op) && op->mat_multt && subspace_mat_fits(op->sub, true) && mat_ready(op));
+  if (!nest_mults(op, prec)) return false;
+  if (prec == SGMEV_DF64 && op->m > 8192 &&
+      (static_cast<double>(op->nest.n_sub) * op->m > 1e8 ||
+       (sub_ready(op) && op->mat_multt && subspace_mat_fits(op->sub, true) && mat_ready(op))))
+    return false;
+  return nest_prepared(op, prec, true);
 }
 
 // Whether the inner solves of a mixed fit run on the FP16 products, both of them: a nested FP32 mult
@@ -1069,7 +1084,7 @@ static int dev_multt(sgmev_op* op, int prec, const double* v64, const float* v32
                                    : prec == SGMEV_FP32 ? KIND_MULTT_NEST32
                                                         : KIND_MULTT_NESTDF);
     SGMEV_CUDA(nest_multt(op->nest, op->stream, prec, NestDense{op->xt64, op->li64, op->mpad}, op->m, v64,
-                          prec == SGMEV_FP32 ? v32 : nullptr, out_end < 0 ? op->npad : out_end, out64, add, scale, op->num_sms,
+                          prec == SGMEV_FP32 ? v32 : nullptr, out_end < 0 ? op->npad : out_end, out64, add, scale,
                           &launches));
     prof_end(op, ev);
     op->launches += launches;

@@ -319,3 +319,20 @@ def test_products_captured_into_a_graph(precision, unit, built):
     for g, o, x, k in zip(got, out, (a, v), (n, m)):
         bound = 0.0 if built else (6 * dim + k) * unit * float(x.abs().sum())
         assert float((g - o).abs().max()) <= bound
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,level", [(4, 4), (10, 5), (3, 9)])
+def test_single_precision_transposes_of_double_and_single_vectors(dim, level):
+    """A single-precision operator's own product (double vector), then its fit's inner products (single
+    vectors) on the same plan, and the product again."""
+    grid = _grid(dim, level)
+    n, m = grid.getSize(), 2000
+    rng = np.random.default_rng(5)
+    op = _op(grid, _points(rng, m, dim, 5), "auto", "float")
+    v, first, again = rng.standard_normal(m), np.zeros(n), np.zeros(n)
+    op.multTranspose(v, first)
+    _, its, _ = op.fit(v, 1e-2, 500, 1e-8, mode=sg.SGMEV_SOLVE_MIXED)
+    op.multTranspose(v, again)
+    assert 0 < its < 500
+    np.testing.assert_array_equal(first, again)
