@@ -438,8 +438,8 @@ def plain_fp64_fit(args, grid, x, d_y, stream, mixed_fits_per_sec, local_rank):
     op.close()
     t = statistics.median(times)
     return {"fits_per_sec": 1.0 / t, "ms_per_fit": t * 1e3, "cg_iterations": its,
-            "what": "SGMEV_SOLVE_PLAIN on a df64 operator (FP64-accurate float-float products "
-                    "streamed from the materialised subspace products), the reference's CG",
+            "what": "SGMEV_SOLVE_PLAIN on a df64 operator (FP64-accurate float-float products, "
+                    "nested mult and materialised multTranspose), the reference's CG",
             "speedup_mixed_vs_plain_fp64": mixed_fits_per_sec * t}
 
 
@@ -566,7 +566,13 @@ def run_ours(args):
                ("multT_matdf64", sg.SGMEV_KERNEL_MULTT_MATDF),
                ("system_mat32", sg.SGMEV_KERNEL_SYSTEM_MAT32),
                ("mult_mat16", sg.SGMEV_KERNEL_MULT_MAT16),
-               ("multT_mat16", sg.SGMEV_KERNEL_MULTT_MAT16))}
+               ("multT_mat16", sg.SGMEV_KERNEL_MULTT_MAT16),
+               ("mult_nest64", sg.SGMEV_KERNEL_MULT_NEST64),
+               ("multT_nest64", sg.SGMEV_KERNEL_MULTT_NEST64),
+               ("mult_nest32", sg.SGMEV_KERNEL_MULT_NEST32),
+               ("mult_nestdf64", sg.SGMEV_KERNEL_MULT_NESTDF),
+               ("multT_nest32", sg.SGMEV_KERNEL_MULTT_NEST32),
+               ("multT_nestdf64", sg.SGMEV_KERNEL_MULTT_NESTDF))}
     op.profile(False)
     alpha = d_alpha.cpu().numpy()
     err = float(np.abs(alpha - alpha_ref).max() / np.abs(alpha_ref).max())
@@ -602,8 +608,10 @@ def run_ours(args):
                                    "no subspace has more than 16 cells, else a byte) per padded "
                                    "point and padded subspace, plus the input and output vectors"}
     else:
-        achieved = work_per_op / avg / 1e12
-        is64 = dom.endswith("fp64") and not dom.endswith("df64")
+        # the nested kernels: a multiply-add per subspace and point
+        work = 2.0 * len(np.unique(lp, axis=0)) * m if "_nest" in dom else work_per_op
+        achieved = work / avg / 1e12
+        is64 = dom.endswith("fp64") or dom.endswith("nest64")
         peak = (peak64 if is64 else peak32) / 1e12
         roofline = {"bound": "fp64-vector" if is64 else "fp32-vector", "kernel": dom,
                     "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
@@ -611,7 +619,7 @@ def run_ours(args):
                     "avg_launch_ms": avg * 1e3,
                     "peak_source": "measured in this run: FMA chains on every SM (sgmev_fma_peak)",
                     "peaks_measured_tflops": {"fp32": peak32 / 1e12, "fp64": peak64 / 1e12},
-                    "flop_per_launch": work_per_op}
+                    "flop_per_launch": work}
 
     # mult GFLOP/s by the reference's count (6 N M d per op) of the dense kernels (the
     # STREAMING algorithm: every grid point for every data point), against the FMA peaks
@@ -674,8 +682,8 @@ def run_ours(args):
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "f16+f32+df64", "data": "synthetic",
             "config": bench_config(args.basis, n, m, args.epsilon, world),
-            "precision": "mixed: inner CG in FP32 arithmetic on FP16 copies of the materialised "
-                         "subspace products (2^-11 relative per product) with FP64 vectors; "
+            "precision": "mixed: inner CG (directions kept) in FP32 arithmetic on FP16 copies of the "
+                         "materialised subspace products (2^-11 relative per product) with FP64 vectors; "
                          "outer iterative-refinement residual with FP64-accurate float-float "
                          "(df64) products",
             "latency_ms": {"p50": p(0.5), "p99": p(0.99)},
@@ -744,7 +752,9 @@ def run_block(args):
     kst = {k: op.profileRead(kind) for k, kind in (("block_mult", sg.SGMEV_KERNEL_BLOCK_MULT),
                                                    ("block_multT", sg.SGMEV_KERNEL_BLOCK_MULTT),
                                                    ("mult_matdf64", sg.SGMEV_KERNEL_MULT_MATDF),
-                                                   ("multT_matdf64", sg.SGMEV_KERNEL_MULTT_MATDF))}
+                                                   ("multT_matdf64", sg.SGMEV_KERNEL_MULTT_MATDF),
+                                                   ("mult_nestdf64", sg.SGMEV_KERNEL_MULT_NESTDF),
+                                                   ("multT_nestdf64", sg.SGMEV_KERNEL_MULTT_NESTDF))}
     op.profile(False)
     alpha = d_a.cpu().numpy()
     ref, note = reference_alpha(args, x, y)
@@ -788,7 +798,7 @@ def run_block(args):
         "speedup_vs_16_single_fits": 16 * single_ms / step,
         "block_kernels": {"mult": {"launches": bm[0], "ms_avg": bm[1] / max(bm[0], 1) * 1e3},
                           "multT": {"launches": bt[0], "ms_avg": bt[1] / max(bt[0], 1) * 1e3}},
-        "df64_residual_ms": (kst["mult_matdf64"][1] + kst["multT_matdf64"][1]) * 1e3 / args.steps,
+        "df64_residual_ms": sum(v[1] for k, v in kst.items() if k.endswith("df64")) * 1e3 / args.steps,
         "launch_shape": tuned, "clocks": clocks,
     }
     print(json.dumps(line), flush=True)

@@ -87,15 +87,20 @@ SGMEV_API int sgmev_device_count(void);
  * inner correction solves of SGMEV_SOLVE_MIXED* fits (SGMEV_SOLVE_PLAIN is never preconditioned).
  * Jacobi (diag(B^T B) + lambda*M) doubled the iteration count on clustered (Gaussian-mixture) data,
  * where fine-level hats see few points, so it is off unless asked for.
- * "inner_tol": relative tolerance of the inner correction solves of mixed fits (default "1e-4").
- * "algo": "auto" (default), "dense" or "subspace" — how the FP32 products are evaluated: dense
+ * "inner_tol": relative tolerance of the inner correction solves of mixed fits (default "1e-4"; none
+ * asks for less than 1e-5, which is what the rounded products can give).
+ * "algo": "auto" (default), "dense" or "subspace" — how the products are evaluated: dense
  * (every grid point for every data point, the STREAMING algorithm) or subspace-skipping (one basis
- * function per subspace and data point, as the reference's DEFAULT operator; grids of dim <= 16
- * with at most 24,576 subspace positions); "auto" takes subspace when it needs fewer instructions.
+ * function per subspace and data point, as the reference's DEFAULT operator). "auto" takes the nested
+ * form of the latter where a grid has it (dim <= 32, level <= 20, at most 512 points per subspace) and
+ * otherwise the subspace kernels (dim <= 16, at most 24,576 subspace positions) when they need fewer
+ * instructions than the dense ones; "subspace" always takes either.
  * "materialize": "auto" (default), "on" or "off" — whether the subspace FP32 products keep
  * p_s(x_j) for every data point and subspace in device memory (built on the first
  * FP32 product) and streams it, instead of evaluating the hats on every call; "auto" does so when
- * it takes at most half of the free device memory and 64 GiB. The products are kept as
+ * it takes at most half of the free device memory and 64 GiB. With "auto" the mult runs nested where
+ * it can and needs none of this, and so does the multTranspose up to 8,192 data points; "on" keeps both
+ * on the materialised products. The products are kept as
  * float-float pairs with their cell index (8 bytes and a byte, or a nibble when no subspace has
  * more than 16 cells; grids whose subspaces have at most 256 cells), so the df64 (FP64-accurate)
  * products stream them too, beside an FP16 copy with its own copy of the cell indices for the
@@ -103,9 +108,10 @@ SGMEV_API int sgmev_device_count(void);
  * (default) or "off" — whether multTranspose streams them as well as mult. "system_product":
  * "separate" (default) or "fused" — FP32 system products B^T (B a) on the materialised products
  * as the mult and multTranspose kernels or in one fused pass. "inner_products":
- * "half" (default) or "float" — the inner FP32 solves of mixed fits stream an FP16 copy of the
- * products (2.5-3 bytes per entry instead of 4.5-5; the FP64-accurate outer residual keeps the result
- * exact to the fit's tolerance).
+ * "half" or "float" — the inner solves of mixed fits stream an FP16 copy of the products (2.5-3 bytes
+ * per entry) in both directions, or use the FP32 products in both; by default whichever is faster for
+ * the grid and the number of points. The FP64-accurate outer residual keeps the result exact to the
+ * fit's tolerance either way.
  * "multt_batch": "1" (default), "2" or "4" — points per read-modify-write round of the owner's
  * cell sums in the FP16 multTranspose (the same bits for each; a launch-shape choice of the
  * autotuner, sgpp_gb300.autotune). "multt_banks": "1" (default) or "2" — banks of cell sums per

@@ -74,9 +74,10 @@ def _keep(keep_alpha, r: "Request") -> bool:
 def request_footprint(grid: "sg.Grid", m: int) -> int:
     """Device bytes one request's operator and fit hold, as the pool server budgets them: the data
     staged dim-major in FP64, FP32 and FP32 low parts (points padded to 1024), the grid arrays,
-    the CG vectors, and the materialised subspace products (P_hi, P_lo, the FP16 copy and the
-    cells, 12 bytes per padded point and padded subspace while they are built, at most 64 GiB, the
-    library's own cap)."""
+    the CG vectors and the kept search directions (two vectors each, 128 of them, at most 512 MiB),
+    the nested kernels' tables (16 bytes per padded point and 1-D level), and the materialised
+    subspace products (P_hi, P_lo, the FP16 copy and the cells, 12 bytes per padded point and padded
+    subspace while they are built, at most 64 GiB, the library's own cap)."""
     d, n = grid.getDimension(), grid.getSize()
     mpad = -(-max(m, 1) // 1024) * 1024
     npad = -(-max(n, 1) // 512) * 512
@@ -95,7 +96,13 @@ def request_footprint(grid: "sg.Grid", m: int) -> int:
             pass
     s_pad = -(-n_sub // 32) * 32
     products = min(mpad * s_pad * 12, 64 << 30)
-    return int(mpad * d * 16 + npad * d * 32 + 12 * npad * 8 + 4 * mpad * 8 + products)
+    levels = 20 * d if n else 0  # the nested plan's limit
+    if n:
+        lp, _ = grid.getStorage().getLevelIndexArraysForEval()
+        levels = int(np.log2(np.asarray(lp).reshape(n, d).max(axis=0)).sum())
+    directions = min(128 * npad * 16, 512 << 20)
+    return int(mpad * d * 20 + npad * d * 32 + 12 * npad * 8 + 4 * mpad * 8 + directions
+               + mpad * min(levels, 20 * d) * 16 + products)
 
 
 class FitServer:
