@@ -214,7 +214,8 @@ SGMEV_API int sgmev_system_apply_device(sgmev_op* op, const double* d_alpha, dou
  *   SGMEV_SOLVE_PLAIN  — CG with the op's own precision kernels (FP64 op: the plain FP64 path).
  *   SGMEV_SOLVE_MIXED  — iterative refinement: the outer residual b - A alpha (and b) with the
  *                        FP64-accurate df64 kernels, the inner correction solves by CG with
- *                        FP32 kernels and FP64 vectors (Jacobi-preconditioned with
+ *                        FP32 kernels and FP64 vectors, every search direction kept over the
+ *                        solves of the fit (up to 128; or Jacobi-preconditioned with
  *                        diag(B^T B) + lambda*M if params say "precond": "jacobi"); stops when
  *                        ||b - A alpha||^2 <= epsilon^2 * ||b - A alpha_0||^2 (true residual).
  *   SGMEV_SOLVE_MIXED_NATIVE64 — the same with native FP64 kernels for the residual.
@@ -297,8 +298,9 @@ SGMEV_API int sgmev_mult_transpose_block(sgmev_op* op, const double* source, dou
  * (datadriven/src/sgpp/datadriven/algorithm/SystemMatrixLeastSquaresIdentity.cpp:32-56) solved
  * as ConjugateGradients::solve would (solver/src/sgpp/solver/sle/ConjugateGradients.cpp:22-151),
  * by mixed-precision iterative refinement: b_k = B^T y_k and the outer residuals b_k - A alpha_k
- * with the FP64-accurate df64 products, the inner correction solves as one block CG over the 16
- * columns on the BF16 tensor-core products (each column its own CG scalars); a column stops when
+ * with the FP64-accurate df64 products, the inner correction solves by CG on all 16
+ * columns at once on the tensor-core products (each column its own scalars and kept directions, up to
+ * 128 of them and 512 MB in all); a column stops when
  * ||b_k - A alpha_k||^2 <= epsilon^2 ||b_k||^2. y: [16 x n_data] column-major; alpha: [16 x n_grid]
  * out (cold start); iterations[16]: inner CG steps of each column; residuals[16]: the final
  * ||b_k - A alpha_k||^2 (either may be NULL).
