@@ -326,7 +326,12 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
       if (l[t] > 1) c = (c << (l[t] - 1)) | ((static_cast<int>(index[g * dim + t]) - 1) / 2);
     cell_of[g] = c;
     const Place& pl = place[node_of[g]];
-    inv[pl.base + (c >> pl.hs) * pl.hi + ((c >> pl.ms) & pl.mm) * pl.mid + (c & pl.lm)] = static_cast<int>(g);
+    int& at = inv[pl.base + (c >> pl.hs) * pl.hi + ((c >> pl.ms) & pl.mm) * pl.mid + (c & pl.lm)];
+    if (at >= 0) {  // a position holds one grid point; the dense kernels add both
+      *err = "nested kernels: a grid point occurs twice";
+      return false;
+    }
+    at = static_cast<int>(g);
   }
   // ---- multTranspose program: subspaces by cell count, then tree order, in chunks ----
   std::vector<int> subs;

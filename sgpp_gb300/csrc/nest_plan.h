@@ -125,7 +125,7 @@ struct NestTables {
 
 // False (and a reason) when the grid is not one that the kernels take: dim <= 32, levels up to 20, at
 // most 512 cells per subspace (multTranspose keeps them in shared memory), a table row and a chunk
-// that fit shared memory.
+// that fit shared memory, no grid point twice.
 bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, const double* index,
                std::string* err);
 

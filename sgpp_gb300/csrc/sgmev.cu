@@ -1306,7 +1306,8 @@ static int stage_grid(sgmev_op* op, int64_t n, const double* level_pow2, const d
   op->h_index.assign(index, index + n * op->dim);
   if (op->algo == 1 && n > 0) {  // asked for: refused here when the grid is not one for it
     std::string why;
-    if (!sub_ready(op, &why)) return fail(SGMEV_ERR_UNSUPPORTED, "algo \"subspace\": " + why);
+    if (!sub_ready(op, &why) && !why.empty())
+      return fail(SGMEV_ERR_UNSUPPORTED, "algo \"subspace\": " + why);
   }
   // output vector and split partials depend on npad
   SGMEV_TRY(dalloc(op->stream, &op->out64, static_cast<size_t>(std::max(op->npad, op->mpad))));

@@ -1143,7 +1143,13 @@ bool subspace_build(SubPlan* p, int dim, int64_t n, const double* level_pow2, co
     offset += size;
   }
   std::vector<int> inv(static_cast<size_t>(offset), -1);
-  for (int64_t g = 0; g < n; ++g) inv[pos[g]] = static_cast<int>(g);
+  for (int64_t g = 0; g < n; ++g) {
+    if (inv[pos[g]] >= 0) {  // a position holds one grid point; the dense kernels add both
+      err->clear();
+      return false;
+    }
+    inv[pos[g]] = static_cast<int>(g);
+  }
   p->dim = dim;
   p->n_sub = static_cast<int>(list.size());
   p->total = offset;

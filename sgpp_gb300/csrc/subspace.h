@@ -99,7 +99,8 @@ constexpr int64_t kSubMaxTotal = int64_t(1) << 27;
 
 // Build the plan from the eval arrays (host, [n x dim] 2^l and i). Returns false (and leaves
 // the plan empty) when the grid has more than kSubMaxTotal positions, a subspace that the
-// owner-computes multTranspose cannot hold (beyond kSubMaxPositions), or dim is not templated.
+// owner-computes multTranspose cannot hold (beyond kSubMaxPositions), or dim is not templated; and, with
+// an empty reason, when a grid point occurs twice (the dense kernels serve such grids).
 bool subspace_build(SubPlan* p, int dim, int64_t n, const double* level_pow2,
                     const double* index, cudaStream_t stream, std::string* err);
 void subspace_free(SubPlan* p);

@@ -101,12 +101,46 @@ def test_grids_the_plan_does_not_take(lib):
                                np.zeros(1).ctypes.data) == 1
 
 
+def _twice():
+    """A storage that holds the point (1, 1; level 2, 1) twice."""
+    level = np.array([[1, 1], [2, 1], [2, 1], [2, 1], [1, 2]], np.int32)
+    index = np.array([[1, 1], [1, 1], [3, 1], [1, 1], [1, 3]], np.int32)
+    return sg.Grid.fromArrays(level, index)
+
+
+def test_grids_with_a_point_twice_are_refused_by_the_plan(lib):
+    lp, ix = _twice().getStorage().getLevelIndexArraysForEval()
+    x, one = np.full((1, 2), 0.3), np.ones(5)
+    assert lib.sgmev_nest_host(2, 5, lp.ctypes.data, ix.ctypes.data, 0, 1, x.ctypes.data,
+                               one.ctypes.data, one.ctypes.data, np.zeros(1).ctypes.data,
+                               np.zeros(5).ctypes.data) == 1
+
+
 # ---- GPU -------------------------------------------------------------------------------------------
 def _op(grid, x, algo, precision="double"):
     cfg = sg.OperationMultipleEvalConfiguration(
         sg.OperationMultipleEvalType.STREAMING, sg.OperationMultipleEvalSubType.CUDA,
         parameters={"precision": precision, "algo": algo})
     return sg.createOperationMultipleEval(grid, x, cfg)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [50, 9000])
+@pytest.mark.parametrize("algo", ["auto", "dense", "subspace"])
+@pytest.mark.parametrize("precision,unit", [("double", EPS), ("float", 2.0 ** -24), ("df64", 2.0 ** -44)])
+def test_both_copies_of_a_grid_point_count(precision, unit, algo, m):
+    grid = _twice()
+    rng = np.random.default_rng(1)
+    x = rng.random((m, 2))
+    alpha, v = np.arange(1.0, 6.0), rng.random(m) + 0.5
+    op = _op(grid, x, algo, precision)
+    out, outt = np.zeros(m), np.full(5, -9.0)
+    op.mult(alpha, out)
+    op.multTranspose(v, outt)
+    ref, reft, _, _ = _dense(grid, x, alpha, v)
+    # a hat of level 2 is good to 4 roundings of 1, a product to 10, and one per addend
+    assert np.all(np.abs(out - ref) <= 15 * unit * np.abs(alpha).sum())
+    assert np.all(np.abs(outt - reft) <= (10 + m) * unit * np.abs(v).sum())
 
 
 @pytest.mark.gpu
