@@ -136,6 +136,9 @@ __device__ __forceinline__ double to_double(double v) { return v; }
 __device__ __forceinline__ double to_double(ff v) {
   return static_cast<double>(v.h) + static_cast<double>(v.l);
 }
+__device__ __forceinline__ bool is_finite(float v) { return isfinite(v); }
+__device__ __forceinline__ bool is_finite(double v) { return isfinite(v); }
+__device__ __forceinline__ bool is_finite(ff v) { return isfinite(v.h); }
 // asynchronous copies into shared memory: `bytes` (4 or 8) of a thread's own column
 template <int BYTES>
 __device__ __forceinline__ void copy_async(void* dst, const void* src) {
@@ -180,18 +183,32 @@ __device__ double dense_value(const NestDense& d, int dim, int64_t g, int64_t j)
   for (int t = 1; t < dim; ++t) p = h_next<MOD>(p, d.xt[t * d.mpad + j], d.li[g * dim + t]);
   return p;
 }
+__device__ double dense_value(const NestDense& d, int dim, int64_t g, int64_t j) {
+  return d.mod ? dense_value<true>(d, dim, g, j) : dense_value<false>(d, dim, g, j);
+}
+
+// a value as the product's arithmetic holds it
+template <typename V>
+__device__ __forceinline__ double held(double v) {
+  V r;
+  set_val(r, v);
+  return to_double(r);
+}
 
 // NaN when a non-finite coefficient meets a hat of 0 at point j, else 0
-template <bool MOD>
+template <typename V>
 __device__ __noinline__ double mult_poison(const NestDense& d, int dim, int64_t n,
                                            const double* alpha, int64_t j) {
   double r = 0.0;
   for (int64_t g = 0; g < n; ++g) {
-    const double a = alpha[g];
-    if (!isfinite(a) && isnan(a * dense_value<MOD>(d, dim, g, j))) r = a - a;
+    const double a = held<V>(alpha[g]);
+    if (!isfinite(a) && isnan(a * dense_value(d, dim, g, j))) r = a - a;
   }
   return r;
 }
+__device__ __forceinline__ void add_poison(float& s, double v) { s += static_cast<float>(v); }
+__device__ __forceinline__ void add_poison(double& s, double v) { s += v; }
+__device__ __forceinline__ void add_poison(ff& s, double v) { s.h += static_cast<float>(v); }
 
 // R adjacent data points per thread (two in FP32, one in the wider arithmetics), a warp at a time over
 // a contiguous range of 32 R-point tiles; the points' table rows and cells in shared memory
@@ -229,7 +246,9 @@ struct NestMultArgs {
   const double* stop;  // device flag: when it is not 0 the product is skipped
 };
 
-template <typename V, int MD, bool MOD>
+// SPREAD: coefficients that are not finite spread as in the dense kernels. A variant of its own: as a
+// branch of one kernel it cost the grids that need no look 1 to 2 %.
+template <typename V, int MD, bool SPREAD>
 __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
     nest_mult_kernel(const __grid_constant__ NestMultArgs a) {
   if (a.stop && *a.stop != 0.0) return;
@@ -246,7 +265,7 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
   V* s_coef = reinterpret_cast<V*>(s_x - tid + a.dim * nth);
   const int w_begin = blockIdx.y * a.n_windows / gridDim.y;
   const int w_end = (blockIdx.y + 1) * a.n_windows / gridDim.y;
-  bool poison = false;  // FP64: a coefficient that is not finite (the same in every thread)
+  bool poison = false;  // a coefficient that is not finite (the same in every thread)
   auto stage = [&](const NestOp4& w) {
     for (int k = w.x + tid; k < w.y; k += all) s_prog[k - w.x] = a.prog[k];
     bool finite = true;
@@ -254,19 +273,20 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
 #pragma unroll 4
       for (int k = w.z + tid; k < w.w; k += all) {
         const V v = static_cast<const V*>(a.coef)[k];
-        finite = finite && isfinite(to_double(v));
+        if constexpr (SPREAD) finite = finite && is_finite(v);
         s_coef[k - w.z] = v;
       }
     } else {
 #pragma unroll 4
       for (int k = w.z + tid; k < w.w; k += all) {
         const int g = a.inv[k];
-        const double v = g >= 0 ? a.alpha[g] : 0.0;
-        finite = finite && isfinite(v);
-        set_val(s_coef[k - w.z], v);
+        V v;
+        set_val(v, g >= 0 ? a.alpha[g] : 0.0);
+        if constexpr (SPREAD) finite = finite && is_finite(v);
+        s_coef[k - w.z] = v;
       }
     }
-    if constexpr (std::is_same<V, double>::value) poison = __syncthreads_or(!finite) || poison;
+    if constexpr (SPREAD) poison = __syncthreads_or(!finite) || poison;
     else __syncthreads();
   };
   // the warps' tile ranges are contiguous and as equal as can be; every warp of the CTA runs the same
@@ -475,9 +495,7 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
     for (int r = 0; r < R; ++r) {
       const int64_t k = j + r;
       const bool real = k < a.m;
-      if constexpr (std::is_same<V, double>::value) {
-        if (poison && real) acc[r] += mult_poison<MOD>(a.dense, a.dim, a.n, a.alpha, k);
-      }
+      if (SPREAD && poison && real) add_poison(acc[r], mult_poison<V>(a.dense, a.dim, a.n, a.alpha, k));
       if (gridDim.y > 1) {
         reinterpret_cast<V*>(a.part)[blockIdx.y * mpad + k] = acc[r];
       } else {
@@ -504,6 +522,7 @@ struct NestMulttArgs {
   double* rows;
   int* bad;
   const double* stop;
+  bool spread;  // values that are not finite spread as in the dense kernels
 };
 __device__ __forceinline__ void read_entry(float& r, const NestMulttArgs& a, int64_t k) { r = a.tab_hi[k]; }
 __device__ __forceinline__ void read_entry(double& r, const NestMulttArgs& a, int64_t k) { r = a.tab64[k]; }
@@ -539,10 +558,10 @@ __global__ void __launch_bounds__(256) nest_multt_kernel(const __grid_constant__
     for (int t = warp; t < a.dim; t += nw) s_x[lane * lay.xs + t] = a.xcell[t * a.mpad + j0 + lane];
     if (warp == nw - 1) {  // the root: v_j H_1 (the same warp reads H_1 itself)
       const double vj = j0 + lane < a.m ? static_cast<double>(v[j0 + lane]) : 0.0;
-      nonfinite = nonfinite || !isfinite(vj);
       V h1, vv;
       read_entry(h1, a, j0 + lane);
       set_val(vv, vj);
+      nonfinite = nonfinite || !is_finite(vv);
       s_p[lane * lay.qs] = mul(vv, h1);
       s_c[lane * lay.cs] = 0;
       set_val(s_t[lane * lay.es + a.n_ent], 1.0);
@@ -576,29 +595,31 @@ __global__ void __launch_bounds__(256) nest_multt_kernel(const __grid_constant__
   }
   double* row = a.rows + stream * a.row_len + at.y + lane;
   for (int c = 0; c < own_cells; ++c) row[32 * c] = to_double(own_acc[32 * c]);
-  const int any = __syncthreads_or(std::is_same<V, double>::value && nonfinite);
+  const int any = __syncthreads_or(a.spread && nonfinite);
   if (tid == 0) a.bad[blockIdx.x] = any;
 }
 
 // NaN when a non-finite v_j meets a hat of 0 of grid point g, else 0
-template <bool MOD>
+template <typename V, typename VIN>
 __device__ __noinline__ double multt_poison(const NestDense& d, int dim, int64_t m,
-                                            const double* v, int64_t g) {
+                                            const VIN* v, int64_t g) {
   double r = 0.0;
-  for (int64_t j = 0; j < m; ++j)
-    if (!isfinite(v[j]) && isnan(v[j] * dense_value<MOD>(d, dim, g, j))) r = v[j] - v[j];
+  for (int64_t j = 0; j < m; ++j) {
+    const double vj = held<V>(static_cast<double>(v[j]));
+    if (!isfinite(vj) && isnan(vj * dense_value(d, dim, g, j))) r = vj - vj;
+  }
   return r;
 }
 
 // out[g] = sum over the streams' rows in a fixed order (+ scale add[g]): a block of 32 x 8 threads
 // takes 32 positions; thread (x, y) adds rows y, y + 8, ... in order, then the 8 sums in y order
 constexpr int kSumGroups = 8;
-template <bool MOD>
+template <typename V, typename VIN>
 __global__ void __launch_bounds__(32 * kSumGroups) nest_finish_kernel(
     const double* __restrict__ rows, int nrows, int64_t row_len, const int* __restrict__ tinv,
     const double* __restrict__ add, double scale, double* __restrict__ out,
     const int* __restrict__ bad, NestDense dense, int dim, int64_t m,
-    const double* __restrict__ v) {
+    const VIN* __restrict__ v) {
   __shared__ double part[kSumGroups][33];
   const int64_t k = static_cast<int64_t>(blockIdx.x) * 32 + threadIdx.x;
   const int y = threadIdx.y, tid = y * 32 + threadIdx.x;
@@ -615,7 +636,7 @@ __global__ void __launch_bounds__(32 * kSumGroups) nest_finish_kernel(
   if (y == 0 && g >= 0) {
     double r = part[0][threadIdx.x];
     for (int b = 1; b < kSumGroups; ++b) r += part[b][threadIdx.x];
-    if (poison) r += multt_poison<MOD>(dense, dim, m, v, g);
+    if (poison) r += multt_poison<V>(dense, dim, m, v, g);
     out[g] = add ? fma(scale, add[g], r) : r;
   }
 }
@@ -632,6 +653,9 @@ bool nest_build(NestPlan* p, int dim, int64_t n, const double* level_pow2, const
   p->n = n;
   p->mod = mod;
   p->n_sub = h.n_sub;
+  p->n_act = h.n_act;
+  p->cells = h.cells;
+  p->cmax = h.cmax;
   p->n_ent = h.n_ent;
   p->lists = h.list_begin;
   p->list_cells = h.list_cells;
@@ -765,10 +789,10 @@ cudaError_t mult_config(const NestPlan& p, NestConfig* c, Kern kern, int64_t m, 
   return cudaSuccess;
 }
 
-template <typename V, int MD, bool MOD>
+template <typename V, int MD, bool SPREAD>
 cudaError_t launch_mult(NestPlan& p, cudaStream_t s, NestConfig& c, NestMultArgs& a, int64_t mpad,
                         int64_t part_bytes, int64_t tiles, int num_sms) {
-  auto kern = nest_mult_kernel<V, MD, MOD>;
+  auto kern = nest_mult_kernel<V, MD, SPREAD>;
   if (c.threads == 0) {
     const cudaError_t e = mult_config<V>(p, &c, kern, a.m, mpad, part_bytes, num_sms);
     if (e != cudaSuccess) {
@@ -792,24 +816,25 @@ cudaError_t launch_mult(NestPlan& p, cudaStream_t s, NestConfig& c, NestMultArgs
   return cudaGetLastError();
 }
 
-template <typename V, bool MOD>
+template <typename V, bool SPREAD>
 cudaError_t launch_mult_dim(NestPlan& p, cudaStream_t s, NestConfig& c, NestMultArgs& a,
                             int64_t mpad, int64_t part_bytes, int64_t tiles, int num_sms) {
   switch (p.dim) {
 #define F(D) \
   case D:    \
-    return launch_mult<V, D, MOD>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
+    return launch_mult<V, D, SPREAD>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
     F(1) F(2) F(3) F(4) F(5) F(6) F(7) F(8) F(9) F(10) F(11) F(12) F(13) F(14) F(15) F(16)
 #undef F
     default:
-      return launch_mult<V, 0, MOD>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
+      return launch_mult<V, 0, SPREAD>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
   }
 }
 
 template <typename V, typename TP>
 cudaError_t mult(NestPlan& p, cudaStream_t s, NestConfig& c, const NestDense& dense, int64_t m,
                  const double* alpha, float* out32, double* out64, int64_t j_begin, int64_t j_end,
-                 int64_t out_end, void* part, int64_t part_bytes, int num_sms, int* launches) {
+                 int64_t out_end, void* part, int64_t part_bytes, int num_sms, bool spread,
+                 int* launches) {
   constexpr bool kF64 = std::is_same<V, double>::value;
   cudaError_t e = tables(p, s, dense, m, kF64, launches);
   if (e != cudaSuccess) return e;
@@ -840,11 +865,9 @@ cudaError_t mult(NestPlan& p, cudaStream_t s, NestConfig& c, const NestDense& de
   a.inv = p.inv;
   a.alpha = alpha;
   a.n = p.n;
-  // (MOD only changes the dense form that non-finite FP64 coefficients are checked against)
-  if constexpr (kF64)
-    e = p.mod ? launch_mult_dim<V, true>(p, s, c, a, dense.mpad, part_bytes, a.n_tiles, num_sms)
-              : launch_mult_dim<V, false>(p, s, c, a, dense.mpad, part_bytes, a.n_tiles, num_sms);
-  else
+  if (kF64 || spread)
+    e = launch_mult_dim<V, true>(p, s, c, a, dense.mpad, part_bytes, a.n_tiles, num_sms);
+  else if constexpr (!kF64)
     e = launch_mult_dim<V, false>(p, s, c, a, dense.mpad, part_bytes, a.n_tiles, num_sms);
   if (e != cudaSuccess) return e;
   *launches += c.restage ? 2 : 1;
@@ -865,15 +888,15 @@ cudaError_t mult(NestPlan& p, cudaStream_t s, NestConfig& c, const NestDense& de
 cudaError_t nest_mult(NestPlan& p, cudaStream_t s, int precision, const NestDense& dense, int64_t m,
                       const double* alpha, float* out32, double* out64, int64_t j_begin,
                       int64_t j_end, int64_t out_end, void* part, int64_t part_bytes, int num_sms,
-                      int* launches) {
+                      bool spread, int* launches) {
   NestConfig& c = p.config[precision];
   switch (precision) {
     case SGMEV_FP64:
-      return mult<double, double>(p, s, c, dense, m, alpha, out32, out64, j_begin, j_end, out_end, part, part_bytes, num_sms, launches);
+      return mult<double, double>(p, s, c, dense, m, alpha, out32, out64, j_begin, j_end, out_end, part, part_bytes, num_sms, spread, launches);
     case SGMEV_FP32:
-      return mult<float, float>(p, s, c, dense, m, alpha, out32, out64, j_begin, j_end, out_end, part, part_bytes, num_sms, launches);
+      return mult<float, float>(p, s, c, dense, m, alpha, out32, out64, j_begin, j_end, out_end, part, part_bytes, num_sms, spread, launches);
     default:
-      return mult<ff, float2>(p, s, c, dense, m, alpha, out32, out64, j_begin, j_end, out_end, part, part_bytes, num_sms, launches);
+      return mult<ff, float2>(p, s, c, dense, m, alpha, out32, out64, j_begin, j_end, out_end, part, part_bytes, num_sms, spread, launches);
   }
 }
 
@@ -907,8 +930,7 @@ cudaError_t multt_rows(NestPlan& p, cudaStream_t s, int precision, int64_t m, in
 
 template <typename V, typename VIN>
 cudaError_t multt(NestPlan& p, cudaStream_t s, int precision, const NestDense& dense, int64_t m, const VIN* v,
-                  int64_t npad, double* out, const double* add, double scale, int* launches) {
-  constexpr bool kF64 = std::is_same<V, double>::value;
+                  int64_t npad, double* out, const double* add, double scale, bool spread, int* launches) {
   const std::vector<int>& streams = p.streams[precision];
   double* rows = p.rows[precision];
   cudaError_t e = cudaSuccess;
@@ -932,6 +954,7 @@ cudaError_t multt(NestPlan& p, cudaStream_t s, int precision, const NestDense& d
   a.dim = p.dim;
   a.bad = p.bad;
   a.stop = p.stop;
+  a.spread = spread;
   a.rows = rows;
   int64_t cs_at = 0;
   for (size_t k = 0; k < p.classes.size(); ++k) {
@@ -945,11 +968,8 @@ cudaError_t multt(NestPlan& p, cudaStream_t s, int precision, const NestDense& d
     a.streams = streams[k];
     a.row_len = c.row_len;
     kern<<<static_cast<unsigned>(streams[k] * c.chunks), c.threads, c.smem(sizeof(V), p.n_ent, p.dim), s>>>(a, v);
-    // (non-finite values are looked after in FP64 only, and only there the basis matters)
-    const double* v64 = kF64 ? reinterpret_cast<const double*>(v) : nullptr;
-    auto fin = p.mod ? nest_finish_kernel<true> : nest_finish_kernel<false>;
-    fin<<<static_cast<unsigned>((c.row_len + 31) / 32), dim3(32, kSumGroups), 0, s>>>(
-        a.rows, streams[k], c.row_len, p.tinv + c.row_begin, add, scale, out, p.bad, dense, p.dim, m, v64);
+    nest_finish_kernel<V, VIN><<<static_cast<unsigned>((c.row_len + 31) / 32), dim3(32, kSumGroups), 0, s>>>(
+        a.rows, streams[k], c.row_len, p.tinv + c.row_begin, add, scale, out, p.bad, dense, p.dim, m, v);
     a.rows += streams[k] * c.row_len;
     cs_at += static_cast<int64_t>(c.chunks) * c.threads;
     *launches += 2;
@@ -974,13 +994,13 @@ bool nest_prepare(NestPlan& p, cudaStream_t s, int precision, bool transpose, co
 
 cudaError_t nest_multt(NestPlan& p, cudaStream_t s, int precision, const NestDense& dense, int64_t m,
                        const double* v64, const float* v32, int64_t npad, double* out,
-                       const double* add, double scale, int* launches) {
+                       const double* add, double scale, bool spread, int* launches) {
   if (precision == SGMEV_FP64)
-    return multt<double>(p, s, precision, dense, m, v64, npad, out, add, scale, launches);
+    return multt<double>(p, s, precision, dense, m, v64, npad, out, add, scale, spread, launches);
   if (precision == SGMEV_DF64)
-    return multt<ff>(p, s, precision, dense, m, v64, npad, out, add, scale, launches);
-  if (v32) return multt<float>(p, s, precision, dense, m, v32, npad, out, add, scale, launches);
-  return multt<float>(p, s, precision, dense, m, v64, npad, out, add, scale, launches);
+    return multt<ff>(p, s, precision, dense, m, v64, npad, out, add, scale, spread, launches);
+  if (v32) return multt<float>(p, s, precision, dense, m, v32, npad, out, add, scale, spread, launches);
+  return multt<float>(p, s, precision, dense, m, v64, npad, out, add, scale, spread, launches);
 }
 
 }  // namespace sgmev

@@ -25,6 +25,8 @@ struct NestPlan {
   bool mod = false;
   int dim = 0, n_sub = 0, n_ent = 0;
   int64_t n = 0, total = 0;
+  int64_t n_act = 0, cells = 0;  // see NestTables
+  int cmax = 0;
   std::vector<NestClass> classes;
   std::vector<int> lists, list_cells, list_words;  // see NestTables
   int h_entry[32] = {0}, h_lmax[32] = {0};
@@ -54,11 +56,13 @@ void nest_free(NestPlan* p);
 bool nest_built(const NestPlan& p, int precision, bool transpose);
 
 // The dense form of the operands, for coefficients or vectors that are not finite: such a value
-// times a hat of 0 is NaN at every point outside the function's support, as in the dense kernels.
+// times a hat of 0 is NaN at every point outside the function's support, as in the dense kernels
+// (products with `spread` set; the others, like the subspace kernels, meet a value only in its cell).
 struct NestDense {
   const double* xt;
   const double2* li;
   int64_t mpad;
+  bool mod;  // ModLinear
 };
 
 // Builds what a product of the precision needs beside the plan: the tables of the data and, for the
@@ -73,12 +77,12 @@ bool nest_prepare(NestPlan& p, cudaStream_t s, int precision, bool transpose, co
 cudaError_t nest_mult(NestPlan& p, cudaStream_t s, int precision, const NestDense& dense, int64_t m,
                       const double* alpha, float* out32, double* out64, int64_t j_begin,
                       int64_t j_end, int64_t out_end, void* part, int64_t part_bytes, int num_sms,
-                      int* launches);
+                      bool spread, int* launches);
 
 // out[g] (g < n; zero in [n, npad)) = sum_j v_j phi_g(x_j) (+ scale * add[g]) in the given precision;
 // v64 [m], or v32 [m] (nullptr: v64) for SGMEV_FP32
 cudaError_t nest_multt(NestPlan& p, cudaStream_t s, int precision, const NestDense& dense, int64_t m,
                        const double* v64, const float* v32, int64_t npad, double* out,
-                       const double* add, double scale, int* launches);
+                       const double* add, double scale, bool spread, int* launches);
 
 }  // namespace sgmev

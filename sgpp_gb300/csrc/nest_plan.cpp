@@ -338,6 +338,11 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
   for (int id : order)
     if (real[id]) subs.push_back(id);
   std::stable_sort(subs.begin(), subs.end(), [&](int a, int b) { return excess[a] > excess[b]; });
+  for (int id : subs) {
+    p->cells += int64_t(1) << excess[id];
+    p->cmax = std::max(p->cmax, 1 << excess[id]);
+    for (int a = id; parent[a] >= 0; a = parent[a]) ++p->n_act;
+  }
   std::vector<NestOp4> chunks;
   std::vector<NestOp2> cq, cs, cwarp;
   std::vector<int> clev, ccell, local(n_nodes, -1), depth(n_nodes, 0);

@@ -871,10 +871,16 @@ static bool capturing(const sgmev_op* op) {
 // ---------------------------------------------------------------------------------------
 // device-side products on padded device vectors
 // ---------------------------------------------------------------------------------------
-// subspace tables for the materialised and on-the-fly FP32 and float-float products, built when a
-// product first asks for them: used when chosen ("algo") and cheaper than the dense kernels by the
+// Whether the subspace tables are used: when chosen ("algo") or cheaper than the dense kernels by the
 // instruction count per data point (one basis function per subspace, ~8 per active dimension and ~10
-// per subspace, against 3 per dimension for every grid point)
+// per subspace, against 3 per dimension for every grid point).
+static bool sub_cheaper(const sgmev_op* op, int n_sub, int64_t n_act) {
+  return op->algo == 1 || (8.0 * static_cast<double>(n_act) + 10.0 * n_sub) * 1.5 <
+                              3.0 * op->dim * static_cast<double>(op->n);
+}
+
+// subspace tables for the materialised and on-the-fly FP32 and float-float products, built when a
+// product first asks for them
 static bool sub_ready(sgmev_op* op, std::string* why = nullptr) {
   using namespace sgmev;
   if (op->sub_tried) return op->sub_ok;
@@ -891,9 +897,7 @@ static bool sub_ready(sgmev_op* op, std::string* why = nullptr) {
   op->sub.multt_batch = op->multt_batch;
   op->sub.multt_banks = op->multt_banks;
   op->sub.multt_ctas = op->multt_ctas;
-  const double dense_cost = 3.0 * op->dim * static_cast<double>(op->n);
-  const double sub_cost = 8.0 * static_cast<double>(op->sub.act_work) + 10.0 * op->sub.n_sub;
-  op->sub_ok = op->algo == 1 || sub_cost * 1.5 < dense_cost;
+  op->sub_ok = sub_cheaper(op, op->sub.n_sub, op->sub.act_work);
   if (!op->sub_ok) subspace_free(&op->sub);
   return op->sub_ok;
 }
@@ -956,6 +960,29 @@ static bool nest_ready(sgmev_op* op) {
   return true;
 }
 
+static sgmev::NestDense nest_dense(const sgmev_op* op) {
+  return sgmev::NestDense{op->xt64, op->li64, op->mpad, op->mod};
+}
+
+// Whether values that are not finite spread in a nested product as in the dense kernels: in FP64, and
+// in FP32 and float-float on the grids that the subspace kernels leave to the dense ones (small ones, more
+// than 16 dimensions, ModLinear ones without materialised products).
+static bool nest_spreads(const sgmev_op* op, int prec, bool transpose) {
+  using namespace sgmev;
+  if (prec == SGMEV_FP64) return true;
+  SubPlan p;  // the shape that the tables would have
+  p.dim = op->dim;
+  p.n_sub = op->nest.n_sub;
+  p.cmax = op->nest.cmax;
+  p.total = op->nest.cells;
+  if (op->dim > 16 || !sub_cheaper(op, p.n_sub, op->nest.n_act)) return true;
+  if (p.total > kSubMaxTotal || (p.total > kSubMaxPositions && !subspace_owner_fits(p, false))) return true;
+  if (op->mat_mode != 0 && (!transpose || op->mat_multt) && subspace_mat_fits(p, false) &&
+      (prec == SGMEV_FP32 || subspace_mat_fits(p, true)))
+    return false;
+  return op->mod || (prec == SGMEV_DF64 && transpose && !subspace_owner_fits(p, true));
+}
+
 // Whether the product's tables and rows are there or could be built; without memory for them it runs as
 // on a grid that the plan does not take.
 static bool nest_prepared(sgmev_op* op, int prec, bool transpose) {
@@ -963,8 +990,8 @@ static bool nest_prepared(sgmev_op* op, int prec, bool transpose) {
   if (nest_built(op->nest, prec, transpose)) return true;
   if (capturing(op) || !nest_ready(op)) return false;
   int launches = 0;
-  const bool ok = nest_prepare(op->nest, op->stream, prec, transpose,
-                               NestDense{op->xt64, op->li64, op->mpad}, op->m, op->num_sms, &launches);
+  const bool ok = nest_prepare(op->nest, op->stream, prec, transpose, nest_dense(op), op->m, op->num_sms,
+                               &launches);
   op->launches += launches;
   return ok;
 }
@@ -1024,9 +1051,9 @@ static int dev_mult(sgmev_op* op, int prec, const double* a64, const float* a32,
     const long ev = prof_begin(op, prec == SGMEV_FP64   ? KIND_MULT_NEST64
                                    : prec == SGMEV_FP32 ? KIND_MULT_NEST32
                                                         : KIND_MULT_NESTDF);
-    SGMEV_CUDA(nest_mult(op->nest, op->stream, prec, NestDense{op->xt64, op->li64, op->mpad}, op->m,
-                         a64, out32, out64, j_begin, j_end, std::min(out_end, op->mpad), op->part,
-                         static_cast<int64_t>(op->part_bytes), op->num_sms, &launches));
+    SGMEV_CUDA(nest_mult(op->nest, op->stream, prec, nest_dense(op), op->m, a64, out32, out64, j_begin, j_end,
+                         std::min(out_end, op->mpad), op->part, static_cast<int64_t>(op->part_bytes),
+                         op->num_sms, nest_spreads(op, prec, false), &launches));
     prof_end(op, ev);
     op->launches += launches;
   } else if (prec == SGMEV_FP64) {
@@ -1083,9 +1110,9 @@ static int dev_multt(sgmev_op* op, int prec, const double* v64, const float* v32
     const long ev = prof_begin(op, prec == SGMEV_FP64   ? KIND_MULTT_NEST64
                                    : prec == SGMEV_FP32 ? KIND_MULTT_NEST32
                                                         : KIND_MULTT_NESTDF);
-    SGMEV_CUDA(nest_multt(op->nest, op->stream, prec, NestDense{op->xt64, op->li64, op->mpad}, op->m, v64,
+    SGMEV_CUDA(nest_multt(op->nest, op->stream, prec, nest_dense(op), op->m, v64,
                           prec == SGMEV_FP32 ? v32 : nullptr, out_end < 0 ? op->npad : out_end, out64, add, scale,
-                          &launches));
+                          nest_spreads(op, prec, true), &launches));
     prof_end(op, ev);
     op->launches += launches;
   } else if (prec == SGMEV_FP64) {

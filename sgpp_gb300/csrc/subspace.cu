@@ -1301,7 +1301,7 @@ cudaError_t subspace_mult_df(const SubPlan& p, cudaStream_t s, const float* xh, 
 
 bool subspace_owner_fits(const SubPlan& p, bool df) {
   const size_t sm = df ? own_smem(p, p.dim, true) : act_own_smem(p, p.dim);
-  return p.n_sub > 0 && p.cmax > 0 && p.rows != nullptr && sm <= kOwnSmemBudget;
+  return p.n_sub > 0 && p.cmax > 0 && sm <= kOwnSmemBudget;
 }
 
 cudaError_t subspace_multt(const SubPlan& p, cudaStream_t s, const float* xt, int64_t mpad,

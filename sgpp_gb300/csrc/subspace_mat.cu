@@ -1230,7 +1230,7 @@ int mat_mult_window(int cmax, int64_t s_pad) {
 
 bool subspace_mat_fits(const SubPlan& p, bool df) {
   const int64_t s_pad = (p.n_sub + 31) / 32 * 32;
-  if (!(p.n_sub > 0 && p.cmax > 0 && p.cmax <= kMatMaxCells && p.rows != nullptr)) return false;
+  if (!(p.n_sub > 0 && p.cmax > 0 && p.cmax <= kMatMaxCells)) return false;
   if (df)
     return mat_mult_df_smem(p.cmax, s_pad) <= kMatSmemBudget &&
            mat_multt_df_smem(p.cmax, s_pad) <= kMatSmemBudget;

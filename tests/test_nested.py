@@ -204,6 +204,58 @@ def test_values_that_are_not_finite_spread_as_in_the_dense_kernels(value):
             np.testing.assert_array_equal(np.isinf(a), np.isinf(b))
 
 
+def _not_finite(grid, x, algo, precision, value, at_grid, at_data):
+    n, m = grid.getSize(), x.shape[0]
+    rng = np.random.default_rng(4)
+    alpha, v = rng.standard_normal(n), rng.standard_normal(m)
+    alpha[at_grid], v[at_data] = value, value
+    op = _op(grid, x, algo, precision)
+    a, b = np.zeros(m), np.zeros(n)
+    op.mult(alpha, a)
+    op.multTranspose(v, b)
+    return a, b
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("basis", ["linear", "modlinear"])
+@pytest.mark.parametrize("precision", ["float", "df64"])
+@pytest.mark.parametrize("dim,level,rounds,m", [(1, 3, 0, 200), (2, 4, 0, 200), (4, 2, 0, 9000), (3, 3, 2, 500),
+                                                (17, 2, 0, 300)])
+def test_values_that_are_not_finite_on_grids_left_to_the_dense_kernels(dim, level, rounds, m, precision, basis):
+    """FP32 and float-float on small grids and beyond 16 dimensions: NaN for every point outside the
+    support, as the dense kernels answer there."""
+    grid = _grid(dim, level, basis, rounds)
+    rng = np.random.default_rng(3)
+    x = rng.random((m, dim))
+    x[1::5] = np.round(x[1::5] * 2 ** level) / 2 ** level
+    if basis == "linear":
+        x[7, 0], x[9, dim - 1] = np.nan, -0.5
+    # (1e39: not finite as FP32)
+    for value, at_grid, at_data in ((np.nan, 0, 3), (np.inf, grid.getSize() - 1, 9), (-np.inf, 1, m - 1),
+                                    (1e39, 2, 5)):
+        got = _not_finite(grid, x, "auto", precision, value, at_grid, at_data)
+        want = _not_finite(grid, x, "dense", precision, value, at_grid, at_data)
+        for a, b in zip(got, want):
+            np.testing.assert_array_equal(np.isnan(a), np.isnan(b))
+            np.testing.assert_array_equal(np.isinf(a), np.isinf(b))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["float", "df64"])
+def test_values_that_are_not_finite_on_grids_of_the_subspace_kernels(precision):
+    """There a coefficient only meets the points of its support, and a value the functions of its cells."""
+    grid = _grid(5, 5)
+    n, m = grid.getSize(), 3000
+    x = np.random.default_rng(2).random((m, 5))
+    at_grid = int(np.argmax(grid.getStorage().level[:, 1]))
+    a, b = _not_finite(grid, x, "auto", precision, np.nan, at_grid, 11)
+    one, unit = np.zeros(n), np.zeros(m)
+    one[at_grid] = unit[11] = 1.0
+    ref, reft, _, _ = _dense(grid, x, one, unit)
+    np.testing.assert_array_equal(np.isnan(a), ref != 0.0)
+    np.testing.assert_array_equal(np.isnan(b), reft != 0.0)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("basis", ["linear", "modlinear"])
 @pytest.mark.parametrize("precision,unit", [("float", 2.0 ** -24), ("df64", 2.0 ** -44)])
