@@ -1738,6 +1738,8 @@ SGMEV_API int sgmev_set_stream(sgmev_op* op, void* stream) {
     SGMEV_CUDA(cudaEventRecord(op->ev_switch, op->stream));
     SGMEV_CUDA(cudaStreamWaitEvent(next, op->ev_switch, 0));
     op->stream = next;
+    // the plans free their memory on the stream they hold: never on one that the caller has taken back
+    op->sub.stream = op->nest.stream = op->blk.stream = next;
   }
   return SGMEV_OK;
 }

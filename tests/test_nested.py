@@ -1,5 +1,7 @@
 """The nested subspace products: the plan's two programs on the host (every index checked) against
 the dense evaluation, and the FP64 kernels against the dense ones on the GPU."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -438,3 +440,41 @@ def test_single_precision_transposes_of_double_and_single_vectors(dim, level):
     op.multTranspose(v, again)
     assert 0 < its < 500
     np.testing.assert_array_equal(first, again)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", ["double", "float", "df64"])
+def test_plans_follow_the_operator_to_another_stream(precision):
+    """Plans and tables built by products on a stream that is destroyed before the next grid is staged."""
+    torch = pytest.importorskip("torch")
+    torch.cuda.init()
+    rt = torch.cuda.cudart()
+    grid = _grid(4, 4)
+    m = 9000
+    rng = np.random.default_rng(8)
+    x = rng.random((m, 4))
+    op = _op(grid, x, "auto", precision)
+    first, second = ctypes.c_void_p(0), ctypes.c_void_p(0)
+    assert int(rt.cudaStreamCreate(ctypes.addressof(first))) == 0
+    assert int(rt.cudaStreamCreate(ctypes.addressof(second))) == 0
+    op.setStream(first.value)
+    for _ in range(2):
+        n = grid.getSize()
+        alpha, v = rng.standard_normal(n), rng.standard_normal(m)
+        out, outt = np.zeros(m), np.zeros(n)
+        op.mult(alpha, out)
+        op.multTranspose(v, outt)
+        op.fit(v, 1e-3, 100, 1e-6, mode=sg.SGMEV_SOLVE_MIXED)
+        ref, reft, _, _ = _dense(grid, x, alpha, v)
+        unit = {"double": EPS, "float": 2.0 ** -24, "df64": 2.0 ** -44}[precision]
+        assert np.abs(out - ref).max() <= 100 * unit * np.abs(alpha).sum()
+        assert np.abs(outt - reft).max() <= 100 * unit * np.abs(v).sum()
+        if first.value:
+            op.setStream(second.value)
+            op.synchronize()
+            assert int(rt.cudaStreamDestroy(first.value)) == 0
+            first.value = None
+        grid.getGenerator().refine(sg.SurplusRefinementFunctor(alpha, 5, 0.0))
+        op.prepare()
+    op.close()
+    assert int(rt.cudaStreamDestroy(second.value)) == 0
