@@ -10,7 +10,8 @@ themselves with CUDA events (sgmev_profile), and the parameters are set on the l
 (sgmev_set_params) instead of rebuilding it, so a search costs a few seconds.
 
 Tunables:
-  multT16   "multt_banks"            banks of cell sums per owner of the FP16 multTranspose (2: two
+  multT16   (operators whose mixed fits run the FP16 products, see "inner_products")
+            "multt_banks"            banks of cell sums per owner of the FP16 multTranspose (2: two
                                      independent read-modify-write chains)
             "multt_ctas"             its CTAs per SM (3: FP32 cell sums only, two loads in flight)
   block     "block_window", "block_mult_a", "block_mult_tiles", "block_stages",
@@ -108,8 +109,12 @@ def store_cache(cache: dict, path: Optional[str] = None) -> None:
     os.replace(tmp, path)
 
 
+class KernelNotUsed(sg.OperationException):
+    """The operator does not launch the kernel: there is nothing to tune."""
+
+
 def _evaluate(op, kernel: str, m: int, n: int, repeats: int) -> float:
-    """Median seconds of the operation the kernel serves, on the live operator."""
+    """Mean seconds of a launch of the kernel, on the live operator."""
     rng = np.random.default_rng(11)
     if kernel == "multT16":
         # the FP16 multTranspose runs inside the inner solves of a mixed fit: time those launches
@@ -119,7 +124,10 @@ def _evaluate(op, kernel: str, m: int, n: int, repeats: int) -> float:
         op.fit(y, 1e-4, 8 * repeats, 1e-30, mode=sg.SGMEV_SOLVE_MIXED)
         cnt, sec = op.profileRead(sg.SGMEV_KERNEL_MULTT_MAT16)
         op.profile(False)
-        return sec / max(cnt, 1)
+        if cnt == 0:
+            raise KernelNotUsed("autotune: the inner solves of this operator's fits do not run the FP16 "
+                                "multTranspose (\"inner_products\": \"half\" makes them)")
+        return sec / cnt
     a = rng.standard_normal((sg.SGMEV_BLOCK_RHS, n))
     v = rng.standard_normal((sg.SGMEV_BLOCK_RHS, m))
     op.multBlock(a)
@@ -136,12 +144,14 @@ def _evaluate(op, kernel: str, m: int, n: int, repeats: int) -> float:
 
 def tune(op, grid, m: int, kernel: str, repeats: int = 3, log=None) -> Tuple[dict, float]:
     """Grid search of `kernel`'s tunables on the live operator; leaves the best combination set
-    on it and returns (params, seconds)."""
+    on it and returns (params, seconds). KernelNotUsed when the operator does not launch it."""
     best, best_t = None, float("inf")
     for combo in combinations(TUNABLES[kernel]):
         try:
             op.setParams(combo)
             t = _evaluate(op, kernel, m, grid.getSize(), repeats)
+        except KernelNotUsed:
+            raise
         except sg.OperationException as e:
             if log:
                 log({"kernel": kernel, "params": combo, "error": str(e)})
@@ -156,29 +166,42 @@ def tune(op, grid, m: int, kernel: str, repeats: int = 3, log=None) -> Tuple[dic
     return best, best_t
 
 
+def _measured(entry: dict) -> bool:
+    """An entry of 0 ms was searched on an operator that did not launch the kernel."""
+    return entry.get("ms", 1.0) > 0.0
+
+
 def tuned_params(grid, m: int, kernels: Sequence[str] = ("multT16", "block"),
                  path: Optional[str] = None) -> dict:
     """The cached choices for this device and problem shape (empty where none was tuned)."""
     cache = load_cache(path)
     out = {}
     for k in kernels:
-        out.update(cache.get(shape_key(k, grid, m), {}).get("params", {}))
+        entry = cache.get(shape_key(k, grid, m), {})
+        if _measured(entry):
+            out.update(entry.get("params", {}))
     return out
 
 
 def tune_and_cache(op, grid, m: int, kernels: Sequence[str] = ("multT16", "block"),
                    path: Optional[str] = None, log=None, force: bool = False) -> dict:
     """Tune the kernels not yet cached for this shape (all of them with force), set the choices on
-    the operator and store them; returns the parameters set."""
+    the operator and store them; returns the parameters set. Kernels that the operator does not launch
+    are passed over."""
     cache = load_cache(path)
     chosen = {}
     for k in kernels:
         key = shape_key(k, grid, m)
-        if key in cache and not force:
+        if key in cache and _measured(cache[key]) and not force:
             params = cache[key]["params"]
             op.setParams(params)
         else:
-            params, t = tune(op, grid, m, k, log=log)
+            try:
+                params, t = tune(op, grid, m, k, log=log)
+            except KernelNotUsed as e:
+                if log:
+                    log({"kernel": k, "skipped": str(e)})
+                continue
             cache[key] = {"params": params, "ms": t * 1e3}
         chosen.update(params)
     store_cache(cache, path)
@@ -200,7 +223,8 @@ def main() -> int:
     cfg = sg.OperationMultipleEvalConfiguration(sg.OperationMultipleEvalType.STREAMING,
                                                 sg.OperationMultipleEvalSubType.CUDA,
                                                 parameters={"algo": "subspace",
-                                                            "materialize": "on"})
+                                                            "materialize": "on",
+                                                            "inner_products": "half"})
     op = sg.createOperationMultipleEval(grid, x, cfg)
     kernels = ["multT16", "block"] if args.kernel == "all" else [args.kernel]
     chosen = tune_and_cache(op, grid, args.points, kernels, force=args.force,

@@ -80,3 +80,37 @@ def test_tune_and_cache_reuses_the_cached_choice(tmp_path, monkeypatch):
     again = autotune.tune_and_cache(op, g, 64, ["multT16"], path=path)
     assert again == first and len(calls) == n_calls
     assert autotune.tuned_params(g, 64, ["multT16"], path=path) == first
+
+
+class _WithoutHalf:
+    """An operator whose fits run no FP16 multTranspose."""
+
+    def __init__(self):
+        self.params = {"multt_banks": "as it was"}
+
+    def setParams(self, p):
+        self.params = dict(p)
+
+    def fit(self, y, lam, imax, epsilon, mode):
+        return np.zeros(1), imax, 0.0
+
+    def profile(self, enable=True):
+        pass
+
+    def profileRead(self, kind):
+        return 0, 0.0
+
+
+def test_kernels_that_never_ran_are_not_tuned(tmp_path):
+    path = str(tmp_path / "c.json")
+    g = sg.Grid.createLinearGrid(2)
+    g.getGenerator().regular(2)
+    with pytest.raises(sg.OperationException, match="do not run"):
+        autotune.tune(_WithoutHalf(), g, 64, "multT16")
+    # a choice stored at 0 ms is not one either
+    key = autotune.shape_key("multT16", g, 64)
+    autotune.store_cache({key: {"params": {"multt_banks": "2"}, "ms": 0.0}}, path)
+    log = []
+    assert autotune.tune_and_cache(_WithoutHalf(), g, 64, ["multT16"], path=path, log=log.append) == {}
+    assert "skipped" in log[-1]
+    assert autotune.tuned_params(g, 64, ["multT16"], path=path) == {}
