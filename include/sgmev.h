@@ -94,7 +94,8 @@ SGMEV_API int sgmev_device_count(void);
  * function per subspace and data point, as the reference's DEFAULT operator). "auto" takes the nested
  * form of the latter where a grid has it (dim <= 32, level <= 20, at most 512 points per subspace) and
  * otherwise the subspace kernels (dim <= 16, at most 24,576 subspace positions) when they need fewer
- * instructions than the dense ones; "subspace" always takes either.
+ * instructions than the dense ones; "subspace" always takes either, and with "materialize": "off" the
+ * subspace kernels that evaluate the hats on every call for the FP32 and float-float products.
  * "materialize": "auto" (default), "on" or "off" — whether the subspace FP32 products keep
  * p_s(x_j) for every data point and subspace in device memory (built on the first
  * FP32 product) and streams it, instead of evaluating the hats on every call; "auto" does so when

@@ -34,6 +34,12 @@ KINDS = {("mult", "float", "dense"): sg.SGMEV_KERNEL_MULT_FP32,
          ("multT", "double", "dense"): sg.SGMEV_KERNEL_MULTT_FP64,
          ("mult", "df64", "dense"): sg.SGMEV_KERNEL_MULT_DF64,
          ("multT", "df64", "dense"): sg.SGMEV_KERNEL_MULTT_DF64,
+         ("mult", "float", "nested"): sg.SGMEV_KERNEL_MULT_NEST32,
+         ("multT", "float", "nested"): sg.SGMEV_KERNEL_MULTT_NEST32,
+         ("mult", "double", "nested"): sg.SGMEV_KERNEL_MULT_NEST64,
+         ("multT", "double", "nested"): sg.SGMEV_KERNEL_MULTT_NEST64,
+         ("mult", "df64", "nested"): sg.SGMEV_KERNEL_MULT_NESTDF,
+         ("multT", "df64", "nested"): sg.SGMEV_KERNEL_MULTT_NESTDF,
          ("mult", "df64", "subspace"): sg.SGMEV_KERNEL_MULT_SUBDF,
          ("multT", "df64", "subspace"): sg.SGMEV_KERNEL_MULTT_SUBDF}
 
@@ -50,8 +56,11 @@ def main() -> int:
     ap.add_argument("--report", choices=["mult16", "multT16"], default="mult16",
                     help="with --kernel fit: which kernel's launches to report")
     ap.add_argument("--precision", choices=["float", "double", "df64"], default="float")
-    ap.add_argument("--algo", choices=["dense", "subspace", "materialized"], default="dense",
-                    help="materialized: subspace products kept in device memory (float-float, "
+    ap.add_argument("--algo", choices=["dense", "subspace", "materialized", "nested"],
+                    default="dense",
+                    help="subspace: hats evaluated on every call; nested: one program over the tree of "
+                         "subspaces (in double also under the other two subspace forms; the transpose in "
+                         "float and df64 up to 8192 points); materialized: subspace products kept in device memory (float-float, "
                          "with an FP16 copy for the inner solves of --kernel fit)")
     ap.add_argument("--dim", type=int, default=10)
     ap.add_argument("--level", type=int, default=5)
@@ -63,6 +72,7 @@ def main() -> int:
     args = ap.parse_args()
 
     mat = args.algo == "materialized"
+    materialize = {"materialized": "on", "nested": "auto"}.get(args.algo, "off")
     rng = np.random.default_rng(7)
     grid = sg.Grid.createLinearGrid(args.dim)
     grid.getGenerator().regular(args.level)
@@ -72,8 +82,9 @@ def main() -> int:
                                                 sg.OperationMultipleEvalSubType.CUDA,
                                                 parameters={
                                                     "precision": args.precision,
-                                                    "algo": "subspace" if mat else args.algo,
-                                                    "materialize": "on" if mat else "off",
+                                                    "algo": {"materialized": "subspace",
+                                                             "nested": "auto"}.get(args.algo, args.algo),
+                                                    "materialize": materialize,
                                                     "materialize_multt": "on" if mat else "off",
                                                     "system_product": "fused",
                                                     **dict(kv.split("=", 1) for kv in args.param)})
@@ -105,7 +116,7 @@ def main() -> int:
     op.profile(True)
     for _ in range(args.launches):
         run()
-    algo = "dense" if args.precision == "double" else args.algo
+    algo = "nested" if args.precision == "double" and args.algo != "dense" else args.algo
     if args.kernel == "fit":
         kind = sg.SGMEV_KERNEL_MULT_MAT16 if args.report == "mult16" else sg.SGMEV_KERNEL_MULTT_MAT16
     elif args.kernel.startswith("block"):

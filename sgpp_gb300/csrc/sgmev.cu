@@ -940,7 +940,7 @@ static bool mat_ready(sgmev_op* op) {
 
 // The nested subspace kernels serve the FP64 products, and the FP32 and float-float mult, of every grid
 // whose plan they take, unless "algo" is "dense" or, for the latter two, "materialize" is "on" (which
-// asks for the materialised products). FP64: about 1.3 instructions of the FP64 pipe per subspace and
+// asks for the materialised products) or "off" with "algo" "subspace" (for the on-the-fly ones). FP64: about 1.3 instructions of the FP64 pipe per subspace and
 // data point against 3 d per grid point and data point, and a subspace has at least one grid point;
 // smallest measured, 351 points and 3,000 data points: a host system product 279 -> 97 us. FP32 and
 // float-float mult against the materialised ones, d = 3..10, level 5..7, 1,000 to 256,000 points:
@@ -997,7 +997,8 @@ static bool nest_prepared(sgmev_op* op, int prec, bool transpose) {
 }
 
 static bool nest_mults(sgmev_op* op, int prec) {
-  if (prec != SGMEV_FP64 && (op->mat_mode == 2 || op->use_half)) return false;
+  if (prec != SGMEV_FP64 && (op->mat_mode == 2 || op->use_half || (op->algo == 1 && op->mat_mode == 0)))
+    return false;
   return nest_prepared(op, prec, false);
 }
 

@@ -478,3 +478,26 @@ def test_plans_follow_the_operator_to_another_stream(precision):
         op.prepare()
     op.close()
     assert int(rt.cudaStreamDestroy(second.value)) == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision,unit", [("float", 2.0 ** -24), ("df64", 2.0 ** -44)])
+def test_subspace_without_materialised_products_evaluates_on_the_fly(precision, unit):
+    grid = _grid(4, 5)
+    n, m = grid.getSize(), 3000
+    rng = np.random.default_rng(6)
+    x = rng.random((m, 4))
+    op = sg.createOperationMultipleEval(grid, x, sg.OperationMultipleEvalConfiguration(
+        sg.OperationMultipleEvalType.STREAMING, sg.OperationMultipleEvalSubType.CUDA,
+        parameters={"precision": precision, "algo": "subspace", "materialize": "off"}))
+    op.profile(True)
+    alpha, v, out, outt = rng.standard_normal(n), rng.standard_normal(m), np.zeros(m), np.zeros(n)
+    op.mult(alpha, out)
+    op.multTranspose(v, outt)
+    kinds = {"float": (sg.SGMEV_KERNEL_MULT_SUB32, sg.SGMEV_KERNEL_MULTT_SUB32),
+             "df64": (sg.SGMEV_KERNEL_MULT_SUBDF, sg.SGMEV_KERNEL_MULTT_SUBDF)}[precision]
+    assert [op.profileRead(k)[0] for k in kinds] == [1, 1]
+    ref, reft, _, _ = _dense(grid, x, alpha, v)
+    # a hat of level 5 is good to 2^5 roundings of 1; sums of at most m addends
+    assert np.abs(out - ref).max() <= (4 * 32 + 70) * unit * np.abs(alpha).max() * 70
+    assert np.abs(outt - reft).max() <= (4 * 32 + m) * unit * np.abs(v).sum()
