@@ -1,6 +1,7 @@
 """The nested subspace products: the plan's two programs on the host (every index checked) against
 the dense evaluation, and the FP64 kernels against the dense ones on the GPU."""
 import ctypes
+import time
 
 import numpy as np
 import pytest
@@ -116,6 +117,34 @@ def test_grids_with_a_point_twice_are_refused_by_the_plan(lib):
     assert lib.sgmev_nest_host(2, 5, lp.ctypes.data, ix.ctypes.data, 0, 1, x.ctypes.data,
                                one.ctypes.data, one.ctypes.data, np.zeros(1).ctypes.data,
                                np.zeros(5).ctypes.data) == 1
+
+
+def _sparse(dim, excess):
+    """Eval arrays of a grid with one point in every subspace of at most 2^excess cells."""
+    rows = np.zeros((1, 0))
+    for _ in range(dim):
+        rows = np.concatenate([np.column_stack([rows[rows.sum(axis=1) + k <= excess],
+                                                np.full((rows.sum(axis=1) + k <= excess).sum(), k)])
+                               for k in range(excess + 1)])
+    return np.ascontiguousarray(2.0 ** (rows + 1)), np.ones(rows.shape)
+
+
+def _plan_seconds(lib, lp, ix):
+    n, dim = lp.shape
+    none, one, out = np.zeros((0, dim)), np.ones(n), np.zeros(n)
+    t = time.process_time()
+    rc = lib.sgmev_nest_host(dim, n, lp.ctypes.data, ix.ctypes.data, 0, 0, none.ctypes.data, one.ctypes.data,
+                             none.ctypes.data, none.ctypes.data, out.ctypes.data)
+    assert rc == 0
+    return time.process_time() - t
+
+
+def test_plans_take_time_in_proportion_to_the_grid(lib):
+    """24,310 and 92,378 subspaces with thousands of windows, both mostly of 512 cells: building every list
+    again for every count of windows took 3.9 times as long per subspace with the larger number."""
+    small = min(_plan_seconds(lib, *_sparse(8, 9)) for _ in range(3))
+    large = min(_plan_seconds(lib, *_sparse(10, 9)) for _ in range(3))
+    assert large / 92378 < 2.5 * small / 24310
 
 
 # ---- GPU -------------------------------------------------------------------------------------------
