@@ -258,6 +258,10 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
       if (inner(c)) add_q(c);
   }
   q_coef.push_back(total);
+  if (total > kNestMaxPositions) {
+    *err = "nested kernels: too many coefficient positions";
+    return false;
+  }
   // windows: runs of inner nodes whose coefficients and program fit shared memory together; a list
   // for S CTAs per tile of points asks for a multiple of S of them, with about the same work each
   const int n_q = static_cast<int>(qops.size());
@@ -270,6 +274,10 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
     q_head[q] = 1 + (g.y - g.x + 3) / 4;
     q_words[q] = 2 + (qops[q].y >= 0 ? qops[q].z - qops[q].y : 0);
     least_words += q_words[q] + (opens(q, 0) ? q_head[q] : 0);
+  }
+  if (least_words > kNestMaxWords) {
+    *err = "nested kernels: too many subspaces";
+    return false;
   }
   // the end of window number `made` that begins with node q0, with `want` of them asked for
   auto window_end = [&](int q0, int64_t cap, int64_t want, int64_t made, int64_t* done) {
@@ -430,6 +438,10 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
       }
       c.sums = std::max(c.sums, sums);
       c.row_len += sums;
+      if (row_total + c.row_len > kNestMaxPositions) {
+        *err = "nested kernels: too many cell sums";
+        return false;
+      }
       c.nq = std::max(c.nq, static_cast<int>(need.size()));
       for (int a : need) local[a] = -1;
       at += cnt;

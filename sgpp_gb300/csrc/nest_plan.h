@@ -65,6 +65,10 @@ constexpr int kNestMacroDim = 16;
 constexpr int kNestBlockCells = 6144;  // most coefficients of one inner node's block
 constexpr int kNestLeaves = 256;       // most leaves of one inner node's record
 constexpr int kNestProgram = 640;      // most words (16 bytes) of a window's program
+// positions are 32-bit, and a subspace takes up to 512 of them whatever its number of grid points: 1 GB of
+// coefficients in FP64 at most; and the ten lists' programs together stay below 3 GB
+constexpr int64_t kNestMaxPositions = int64_t(1) << 27;
+constexpr int64_t kNestMaxWords = int64_t(1) << 24;
 // window lists: at most cap coefficients per window, for so many CTAs sharing a tile of points
 constexpr int kNestLists = 10;
 NEST_HD constexpr int nest_list_cap(int list) { return list < kNestLists / 2 ? 18432 : 6144; }
@@ -127,7 +131,7 @@ struct NestTables {
 
 // False (and a reason) when the grid is not one that the kernels take: dim <= 32, levels up to 20, at
 // most 512 cells per subspace (multTranspose keeps them in shared memory), a table row and a chunk
-// that fit shared memory, no grid point twice.
+// that fit shared memory, no grid point twice, positions and words within the limits above.
 bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, const double* index,
                std::string* err);
 

@@ -18,6 +18,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -888,8 +889,14 @@ static bool sub_ready(sgmev_op* op, std::string* why = nullptr) {
   op->sub_tried = true;
   if (op->algo == 0 || op->n < 1) return false;
   std::string reason;
-  if (!subspace_build(&op->sub, op->dim, op->n, op->h_level_pow2.data(), op->h_index.data(), op->stream,
-                      &reason)) {
+  bool built = false;
+  try {
+    built = subspace_build(&op->sub, op->dim, op->n, op->h_level_pow2.data(), op->h_index.data(), op->stream,
+                           &reason);
+  } catch (const std::bad_alloc&) {
+    reason = "no host memory for the subspace tables";
+  }
+  if (!built) {
     if (why) *why = reason;
     return false;
   }
@@ -952,12 +959,13 @@ static bool nest_ready(sgmev_op* op) {
   if (op->nest.ok) return true;
   if (op->algo == 0 || op->nest_failed || op->n < 1 || (op->mod && !op->in_cube)) return false;
   std::string why;
-  if (!nest_build(&op->nest, op->dim, op->n, op->h_level_pow2.data(), op->h_index.data(), op->mod,
-                  op->num_sms, op->stream, &why)) {
+  try {
+    op->nest_failed = !nest_build(&op->nest, op->dim, op->n, op->h_level_pow2.data(), op->h_index.data(),
+                                  op->mod, op->num_sms, op->stream, &why);
+  } catch (const std::bad_alloc&) {  // host memory for the plan
     op->nest_failed = true;
-    return false;
   }
-  return true;
+  return !op->nest_failed;
 }
 
 static sgmev::NestDense nest_dense(const sgmev_op* op) {

@@ -147,6 +147,16 @@ def test_plans_take_time_in_proportion_to_the_grid(lib):
     assert large / 92378 < 2.5 * small / 24310
 
 
+def test_plans_with_more_positions_than_indices_are_refused(lib):
+    """497,420 points, one in each subspace, on 1.9e8 positions."""
+    lp, ix = _sparse(13, 9)
+    n = lp.shape[0]
+    none, one, out = np.zeros((0, 13)), np.ones(n), np.zeros(n)
+    assert (np.prod(lp, axis=1) / 2 ** 13).sum() > 2 ** 27
+    assert lib.sgmev_nest_host(13, n, lp.ctypes.data, ix.ctypes.data, 0, 0, none.ctypes.data, one.ctypes.data,
+                               none.ctypes.data, none.ctypes.data, out.ctypes.data) == 1
+
+
 # ---- GPU -------------------------------------------------------------------------------------------
 def _op(grid, x, algo, precision="double"):
     cfg = sg.OperationMultipleEvalConfiguration(
