@@ -509,7 +509,9 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
 // ---- multTranspose -----------------------------------------------------------------------------
 // CTA (stream, chunk): chunk's subspaces over the stream's contiguous range of tiles. Phase A: lane
 // = point, a warp per inner node, one depth of the tree after the other. Phase B: thread =
-// subspace, points in order, sums in the thread's own cells.
+// subspace, points in order, sums in the thread's own cells. LONG: FP32 streams of more than 1,024
+// points, which a plain FP32 sum would round by up to 2^-12 (8,192 points in one: 1.2e-4 off at worst); a
+// variant of its own, as the branch in the other one made that 2 to 4 us slower (d=10 level 5, 34 us).
 struct NestMulttArgs {
   const NestOp4* chunks;
   const NestOp2 *cq, *cs, *cwarp;
@@ -528,7 +530,7 @@ __device__ __forceinline__ void read_entry(float& r, const NestMulttArgs& a, int
 __device__ __forceinline__ void read_entry(double& r, const NestMulttArgs& a, int64_t k) { r = a.tab64[k]; }
 __device__ __forceinline__ void read_entry(ff& r, const NestMulttArgs& a, int64_t k) { r = ff{a.tab_hi[k], a.tab_lo[k]}; }
 
-template <typename V, typename VIN>
+template <typename V, typename VIN, bool LONG>
 __global__ void __launch_bounds__(256) nest_multt_kernel(const __grid_constant__ NestMulttArgs a,
                                                          const VIN* __restrict__ v) {
   if (a.stop && *a.stop != 0.0) return;
@@ -588,13 +590,27 @@ __global__ void __launch_bounds__(256) nest_multt_kernel(const __grid_constant__
         mac(r, s_p[i * lay.qs + own.x], s_t[i * lay.es + own_e]);
         *acc = r;
       }
-      // float-float sums are settled every 1,024 points
+      // every 1,024 points float-float sums are settled, and FP32 ones of LONG streams go into the FP64 row
       if (std::is_same<V, ff>::value && ((tile - t_begin) & 31) == 31)
         for (int c = 0; c < own_cells; ++c) settle(own_acc[32 * c]);
+      if constexpr (LONG) {
+        if (((tile - t_begin) & 31) == 31 && tile + 1 < t_end) {
+          double* row = a.rows + stream * a.row_len + at.y + lane;
+          for (int c = 0; c < own_cells; ++c) {
+            const double s = to_double(own_acc[32 * c]);
+            row[32 * c] = tile >= t_begin + 32 ? row[32 * c] + s : s;
+            own_acc[32 * c] = V{};
+          }
+        }
+      }
     }
   }
   double* row = a.rows + stream * a.row_len + at.y + lane;
-  for (int c = 0; c < own_cells; ++c) row[32 * c] = to_double(own_acc[32 * c]);
+  for (int c = 0; c < own_cells; ++c) {
+    const double s = to_double(own_acc[32 * c]);
+    if constexpr (LONG) row[32 * c] = t_end - t_begin > 32 ? row[32 * c] + s : s;
+    else row[32 * c] = s;
+  }
   const int any = __syncthreads_or(a.spread && nonfinite);
   if (tid == 0) a.bad[blockIdx.x] = any;
 }
@@ -905,7 +921,7 @@ namespace {
 template <typename V>
 cudaError_t multt_rows(NestPlan& p, cudaStream_t s, int precision, int64_t m, int num_sms) {
   if (!p.streams[precision].empty()) return cudaSuccess;
-  auto kern = nest_multt_kernel<V, double>;
+  auto kern = nest_multt_kernel<V, double, false>;
   const int64_t n_tiles = std::max<int64_t>(1, (m + kTile - 1) / kTile);
   // as many streams as fit the SMs at once (at most 256 MB of rows); fixed from here on, and
   // with them the order of every sum
@@ -914,7 +930,11 @@ cudaError_t multt_rows(NestPlan& p, cudaStream_t s, int precision, int64_t m, in
   for (const NestClass& c : p.classes) {
     const size_t sm = c.smem(sizeof(V), p.n_ent, p.dim);
     cudaError_t e = set_smem_cap(kern, sm);
-    if (e == cudaSuccess && std::is_same<V, float>::value) e = set_smem_cap(nest_multt_kernel<float, float>, sm);
+    if constexpr (std::is_same<V, float>::value) {
+      if (e == cudaSuccess) e = set_smem_cap(nest_multt_kernel<float, float, false>, sm);
+      if (e == cudaSuccess) e = set_smem_cap(nest_multt_kernel<float, double, true>, sm);
+      if (e == cudaSuccess) e = set_smem_cap(nest_multt_kernel<float, float, true>, sm);
+    }
     int per_sm = 0;
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, c.threads, sm);
     if (e != cudaSuccess) return e;
@@ -934,7 +954,6 @@ cudaError_t multt(NestPlan& p, cudaStream_t s, int precision, const NestDense& d
   const std::vector<int>& streams = p.streams[precision];
   double* rows = p.rows[precision];
   cudaError_t e = cudaSuccess;
-  auto kern = nest_multt_kernel<V, VIN>;
   const int64_t n_tiles = std::max<int64_t>(1, (m + kTile - 1) / kTile);
   if (npad > p.n) {
     e = cudaMemsetAsync(out + p.n, 0, sizeof(double) * (npad - p.n), s);
@@ -967,6 +986,9 @@ cudaError_t multt(NestPlan& p, cudaStream_t s, int precision, const NestDense& d
     a.sums = c.sums;
     a.streams = streams[k];
     a.row_len = c.row_len;
+    auto kern = nest_multt_kernel<V, VIN, false>;
+    if constexpr (std::is_same<V, float>::value)
+      if ((n_tiles + streams[k] - 1) / streams[k] > 32) kern = nest_multt_kernel<V, VIN, true>;
     kern<<<static_cast<unsigned>(streams[k] * c.chunks), c.threads, c.smem(sizeof(V), p.n_ent, p.dim), s>>>(a, v);
     nest_finish_kernel<V, VIN><<<static_cast<unsigned>((c.row_len + 31) / 32), dim3(32, kSumGroups), 0, s>>>(
         a.rows, streams[k], c.row_len, p.tinv + c.row_begin, add, scale, out, p.bad, dense, p.dim, m, v);

@@ -540,3 +540,24 @@ def test_subspace_without_materialised_products_evaluates_on_the_fly(precision, 
     # a hat of level 5 is good to 2^5 roundings of 1; sums of at most m addends
     assert np.abs(out - ref).max() <= (4 * 32 + 70) * unit * np.abs(alpha).max() * 70
     assert np.abs(outt - reft).max() <= (4 * 32 + m) * unit * np.abs(v).sum()
+
+
+@pytest.mark.gpu
+def test_fp32_transposes_sum_at_most_1024_points_in_fp32():
+    """230,230 subspaces leave one stream of points per block; all 8,192 points at the centre, where only
+    the coarsest function is not 0, with a value that a long FP32 sum rounds down every time."""
+    lp, _ = _sparse(20, 6)
+    grid = sg.Grid.fromArrays(np.log2(lp).astype(np.int32), np.ones(lp.shape, np.int32))
+    n, m = grid.getSize(), 8192
+    op = _op(grid, np.full((m, 20), 0.5), "auto", "float")
+    op.profile(True)
+    value = 0.5 + 2.0 ** -13 - 2.0 ** -19
+    out = np.zeros(n)
+    op.multTranspose(np.full(m, value), out)
+    assert op.profileRead(sg.SGMEV_KERNEL_MULTT_NEST32)[0] == 1
+    root = int(np.argmin(lp.sum(axis=1)))
+    # sums of up to 1,024 values stay below 513: each addition rounds by at most half an ulp, 2^-16 below
+    # 512, against addends of 0.5; a sum over all points loses 1.2e-4
+    assert abs(out[root] - m * value) <= 2.0 ** -15 * m * value
+    out[root] = 0.0
+    assert np.all(out == 0.0)
