@@ -88,7 +88,8 @@ SGMEV_API int sgmev_device_count(void);
  * Jacobi (diag(B^T B) + lambda*M) doubled the iteration count on clustered (Gaussian-mixture) data,
  * where fine-level hats see few points, so it is off unless asked for.
  * "inner_tol": relative tolerance of the inner correction solves of mixed fits (default "1e-4"; none
- * asks for less than 1e-5, which is what the rounded products can give).
+ * asks for less than 1e-5, which is what the rounded products can give, or less than "inner_tol" where
+ * that is smaller).
  * "algo": "auto" (default), "dense" or "subspace" — how the products are evaluated: dense
  * (every grid point for every data point, the STREAMING algorithm) or subspace-skipping (one basis
  * function per subspace and data point, as the reference's DEFAULT operator). "auto" takes the nested

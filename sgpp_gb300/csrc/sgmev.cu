@@ -2458,10 +2458,11 @@ static int fit_common(sgmev_op* op, int mode, const double* y, bool y_on_device,
       int64_t it = 0;
       // The reduction that ends the refinement is solved for where one more solve reaches it, with
       // room for the inner operator's own error: the plain inner tolerance would leave a residual
-      // anywhere up to epsilon. No solve asks for less than what rounded products can give.
+      // anywhere up to epsilon. No solve asks for less than what rounded products can give, unless the
+      // caller does ("inner_tol").
       const bool half = inner_on_half(op);
       const double last = 0.3 * epsilon * std::sqrt(r0 / rnorm2);
-      const double want = std::max(1e-5, last > 0.1 * eps_inner ? last : eps_inner);
+      const double want = std::max(std::min(1e-5, eps_inner), last > 0.1 * eps_inner ? last : eps_inner);
       // the inner solve may use the FP16 copy of the materialised products: the outer residual
       // is FP64-accurate, so the refinement still converges to the FP64 solution
       struct HalfScope {
@@ -2734,7 +2735,7 @@ static int fit_block_common(sgmev_op* op, const double* y, bool y_dev, double la
       // the last reduction as in fit_common; the BF16 operands are too coarse for more than inner_tol
       const double last = 0.3 * epsilon * std::sqrt(rho0[k] / std::max(rho[k], 1e-300));
       const double want = std::min(
-          0.5, std::max(1e-5, op->block_f16 && last > 0.1 * inner_tol ? last : std::max(inner_tol, last)));
+          0.5, std::max(std::min(1e-5, inner_tol), op->block_f16 && last > 0.1 * inner_tol ? last : std::max(inner_tol, last)));
       tol2[k] = done[k] ? HUGE_VAL : want * want;
     }
     if (all_done || total_it >= max_iterations) break;

@@ -388,6 +388,24 @@ def test_fits_on_kept_directions_reach_their_residual(dim, level, m, lam, inner,
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("inner,solves", [(None, 2), ("1e-7", 1)])
+def test_inner_tolerances_below_the_default_floor_are_honoured(inner, solves):
+    """To 1e-5 by default, so that a fit to 2e-6 takes two inner solves; asked for more, one."""
+    grid = _grid(3, 4)
+    rng = np.random.default_rng(12)
+    x = rng.random((2000, 3))
+    y = np.sin(4.0 * x.sum(axis=1)) + 0.1 * rng.standard_normal(2000)
+    op = sg.OperationMultiEvalCuda(grid, x, sg.SGMEV_FP64, {"inner_tol": inner} if inner else {})
+    op.profile(True)
+    _, _, residual = op.fit(y, 1e-2, 1000, 2e-6, mode=sg.SGMEV_SOLVE_MIXED)
+    b = np.zeros(grid.getSize())
+    op.multTranspose(y, b)
+    assert residual <= (2e-6 * np.linalg.norm(b)) ** 2 * (1 + 1e-6)
+    # a residual product after every solve (the first one starts from 0)
+    assert op.profileRead(sg.SGMEV_KERNEL_MULT_NESTDF)[0] == solves
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("dim,level,m,lam", [(5, 5, 3000, 1e-7), (6, 4, 3000, 1e-8)])
 def test_solves_that_fill_the_kept_directions_take_fewer_steps_than_the_recurrence(dim, level, m, lam):
     """Inner solves that end for standing still with every slot taken, and others that start from what
