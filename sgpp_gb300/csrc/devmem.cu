@@ -64,6 +64,17 @@ cudaError_t dev_malloc(void** p, size_t bytes, cudaStream_t s) {
   return e;
 }
 
+size_t dev_available() {
+  size_t free_b = 0, total_b = 0;
+  cudaMemPool_t pool = library_pool();
+  uint64_t reserved = 0, used = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || !pool ||
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+    (void)cudaGetLastError();
+  return free_b + static_cast<size_t>(reserved > used ? reserved - used : 0);
+}
+
 void dev_free(void* p, cudaStream_t s) {
   if (p) cudaFreeAsync(p, s);
 }

@@ -18,6 +18,8 @@ inline cudaError_t dev_malloc(T** p, size_t bytes, cudaStream_t s) {
   return dev_malloc(reinterpret_cast<void**>(p), bytes, s);
 }
 
+// bytes that dev_malloc could give out on the current device: free ones and the pool's own unused blocks
+size_t dev_available();
 // cudaFreeAsync on `s` (nullptr is accepted); the memory is reused once `s` reaches this point
 void dev_free(void* p, cudaStream_t s);
 

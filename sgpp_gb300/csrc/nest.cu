@@ -660,8 +660,9 @@ __global__ void __launch_bounds__(32 * kSumGroups) nest_finish_kernel(
 }  // namespace
 
 bool nest_build(NestPlan* p, int dim, int64_t n, const double* level_pow2, const double* index,
-                bool mod, int num_sms, cudaStream_t stream, std::string* err) {
+                bool mod, int num_sms, cudaStream_t stream, std::string* err, size_t* need) {
   nest_free(p);
+  *need = 0;
   p->stream = stream;
   NestTables h;
   if (!nest_plan(&h, dim, n, level_pow2, index, err)) return false;
@@ -712,6 +713,7 @@ bool nest_build(NestPlan* p, int dim, int64_t n, const double* level_pow2, const
           cudaSuccess) {  // (pageable source: the copy has taken the data when it returns)
     (void)cudaGetLastError();
     nest_free(p);
+    *need = o_bad + sizeof(int) * flags;
     *err = "nested plan allocation failed";
     return false;
   }
@@ -739,12 +741,16 @@ cudaError_t tables(NestPlan& p, cudaStream_t s, const NestDense& d, int64_t m, b
                    int* launches) {
   if (f64 ? p.tab64 != nullptr : p.tab_hi != nullptr) return cudaSuccess;
   cudaError_t e = cudaSuccess;
-  if (!p.xcell) e = dev_malloc(&p.xcell, sizeof(uint32_t) * p.dim * d.mpad, s);
-  if (e != cudaSuccess) return e;
-  const int64_t n = p.n_ent * d.mpad;
-  if (f64) e = dev_malloc(&p.tab64, sizeof(double) * n, s);
-  else e = dev_malloc(&p.tab_hi, 2 * sizeof(float) * n, s);
-  if (e != cudaSuccess) return e;
+  const int64_t n = p.n_ent * d.mpad, cells = sizeof(uint32_t) * p.dim * d.mpad;
+  const bool first = !p.xcell;
+  if (first) e = dev_malloc(&p.xcell, cells, s);
+  if (e == cudaSuccess) e = f64 ? dev_malloc(&p.tab64, sizeof(double) * n, s) : dev_malloc(&p.tab_hi, 2 * sizeof(float) * n, s);
+  if (e != cudaSuccess) {
+    p.need = sizeof(double) * n + (first ? cells : 0);
+    if (first) dev_free(p.xcell, s);
+    if (first) p.xcell = nullptr;
+    return e;
+  }
   const unsigned blocks = static_cast<unsigned>((d.mpad + 127) / 128);
   auto kern = f64 ? (p.mod ? nest_table_kernel<true, true, false> : nest_table_kernel<false, true, false>)
                   : (p.mod ? nest_table_kernel<true, false, true> : nest_table_kernel<false, false, true>);
@@ -945,6 +951,7 @@ cudaError_t multt_rows(NestPlan& p, cudaStream_t s, int precision, int64_t m, in
   }
   const cudaError_t e = dev_malloc(&p.rows[precision], sizeof(double) * elems, s);
   if (e == cudaSuccess) p.streams[precision] = st;
+  else p.need = sizeof(double) * elems;
   return e;
 }
 

@@ -45,12 +45,13 @@ struct NestPlan {
   float* tab_hi = nullptr;    // [2][n_ent][mpad], high and low parts, FP32 and float-float products
   uint32_t* xcell = nullptr;  // [dim][mpad]
   bool refused[2][3] = {};  // by direction and precision: nest_prepare() found no memory
+  size_t need = 0;          // for so many bytes
   cudaStream_t stream = nullptr;
 };
 
-// False (and a reason) when nest_plan does not take the grid or memory is short.
+// False (and a reason) when nest_plan does not take the grid, or with *need bytes where device memory is short.
 bool nest_build(NestPlan* p, int dim, int64_t n, const double* level_pow2, const double* index,
-                bool mod, int num_sms, cudaStream_t stream, std::string* err);
+                bool mod, int num_sms, cudaStream_t stream, std::string* err, size_t* need);
 void nest_free(NestPlan* p);
 // whether the product needs nothing more to be built (a product under stream capture must not)
 bool nest_built(const NestPlan& p, int precision, bool transpose);
@@ -66,7 +67,8 @@ struct NestDense {
 };
 
 // Builds what a product of the precision needs beside the plan: the tables of the data and, for the
-// transpose, its partial rows. False when there is no memory for them (not tried again).
+// transpose, its partial rows. False when there is no memory for them, `need` bytes (not tried again
+// while `refused` is set).
 bool nest_prepare(NestPlan& p, cudaStream_t s, int precision, bool transpose, const NestDense& dense,
                   int64_t m, int num_sms, int* launches);
 

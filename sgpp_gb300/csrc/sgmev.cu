@@ -18,6 +18,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <iterator>
 #include <new>
 #include <string>
 #include <vector>
@@ -150,6 +151,7 @@ struct sgmev_op {
   // nested subspace plan of the FP64 products, built on the first of them from the eval arrays
   sgmev::NestPlan nest;
   bool nest_failed = false;  // the current grid is not one the nested kernels take
+  size_t nest_need = 0;      // bytes that a nested plan, its tables or rows were refused for
   std::vector<double> h_level_pow2, h_index;
   // BF16 tensor-core products with 16 right-hand sides (built on the first block call)
   sgmev::BlockPlan blk;
@@ -961,7 +963,7 @@ static bool nest_ready(sgmev_op* op) {
   std::string why;
   try {
     op->nest_failed = !nest_build(&op->nest, op->dim, op->n, op->h_level_pow2.data(), op->h_index.data(),
-                                  op->mod, op->num_sms, op->stream, &why);
+                                  op->mod, op->num_sms, op->stream, &why, &op->nest_need);
   } catch (const std::bad_alloc&) {  // host memory for the plan
     op->nest_failed = true;
   }
@@ -1001,7 +1003,18 @@ static bool nest_prepared(sgmev_op* op, int prec, bool transpose) {
   const bool ok = nest_prepare(op->nest, op->stream, prec, transpose, nest_dense(op), op->m, op->num_sms,
                                &launches);
   op->launches += launches;
+  if (!ok) op->nest_need = std::max(op->nest_need, op->nest.need);
   return ok;
+}
+
+// At the start of a call: what was refused for want of memory is asked for again once there is enough.
+// (Within a call the answer stays: its products and what they are given have to agree.)
+static void nest_again(sgmev_op* op) {
+  using namespace sgmev;
+  if (op->nest_need == 0 || capturing(op) || dev_available() < op->nest_need) return;
+  op->nest_need = 0;
+  op->nest_failed = false;
+  for (auto& d : op->nest.refused) std::fill(std::begin(d), std::end(d), false);
 }
 
 static bool nest_mults(sgmev_op* op, int prec) {
@@ -1023,6 +1036,13 @@ static bool nest_multts(sgmev_op* op, int prec) {
        (sub_ready(op) && op->mat_multt && subspace_mat_fits(op->sub, true) && mat_ready(op))))
     return false;
   return nest_prepared(op, prec, true);
+}
+
+// Builds what the products of the precision will read, in both directions.
+static void products_ready(sgmev_op* op, int prec) {
+  using namespace sgmev;
+  const bool mult = nest_mults(op, prec), transpose = nest_multts(op, prec);
+  if (prec != SGMEV_FP64 && (!mult || (!transpose && op->mat_multt)) && sub_ready(op)) (void)mat_ready(op);
 }
 
 // Whether the inner solves of a mixed fit run on the FP16 products, both of them: a nested FP32 mult
@@ -1338,6 +1358,7 @@ static int stage_grid(sgmev_op* op, int64_t n, const double* level_pow2, const d
   subspace_free(&op->sub);
   nest_free(&op->nest);
   op->nest_failed = false;
+  op->nest_need = 0;
   op->h_level_pow2.assign(level_pow2, level_pow2 + n * op->dim);
   op->h_index.assign(index, index + n * op->dim);
   if (op->algo == 1 && n > 0) {  // asked for: refused here when the grid is not one for it
@@ -1821,6 +1842,7 @@ static int mult_common(sgmev_op* op, const double* alpha_dev_or_null, const doub
                        double* result_dev, double* result_host, int64_t start, int64_t end) {
   using namespace sgmev;
   const int prec = op->precision;
+  nest_again(op);
   const bool nested = nest_mults(op, prec), whole = start == 0 && end == op->m;
   double* small = nested && whole && alpha_host && result_host ? small_buffer(op, op->n, op->m) : nullptr;
   SGMEV_TRY(begin_timed(op));
@@ -1871,6 +1893,7 @@ static int multt_common(sgmev_op* op, const double* src_dev, const double* src_h
                         double* result_dev, double* result_host, int64_t start, int64_t end) {
   using namespace sgmev;
   const int prec = op->precision;
+  nest_again(op);
   const bool nested = nest_multts(op, prec), whole = start == 0 && end == op->n;
   double* small = nested && whole && src_host && result_host ? small_buffer(op, op->m, op->n) : nullptr;
   SGMEV_TRY(begin_timed(op));
@@ -1969,6 +1992,7 @@ SGMEV_API int sgmev_mult_transpose_device(sgmev_op* op, const double* d_source,
 static int system_common(sgmev_op* op, const double* a_dev, const double* a_host, double* r_dev,
                          double* r_host, double lm) {
   using namespace sgmev;
+  nest_again(op);
   SGMEV_TRY(begin_timed(op));
   double* a = op->cg + 6 * op->npad;  // padded copy of the input
   double* r = op->cg + 7 * op->npad;
@@ -2410,6 +2434,7 @@ static int fit_common(sgmev_op* op, int mode, const double* y, bool y_on_device,
   double* b = op->cg;
   double* x = op->cg + np;
   const double lm = static_cast<double>(op->m) * lambda;
+  nest_again(op);
   SGMEV_TRY(begin_timed(op));
   // b = B^T y in FP64 (generateb)
   if (op->m > 0)
@@ -2474,10 +2499,13 @@ static int fit_common(sgmev_op* op, int mode, const double* y, bool y_on_device,
         SGMEV_TRY(pcg_core(op, SGMEV_FP32, rr, dx, lm, max_iterations - total_it,
                            std::min(want, 0.5), &it));
       } else {
-        if (outer == 0)
+        if (outer == 0) {
+          // what the products need has to be there before the directions take up to 512 MB
+          if (!half) products_ready(op, SGMEV_FP32);
+          products_ready(op, res_prec);
           SGMEV_TRY(directions_ready(op, 1, &kept));
-        else if (ortho_gives_up(last_it, last_rnorm2, rnorm2))
-          kept.cap = 1;
+        }
+        if (outer > 0 && ortho_gives_up(last_it, last_rnorm2, rnorm2)) kept.cap = 1;
         if (kept.cap == 1) kept.kept = 0;
         SGMEV_TRY(inner_cg(op, SGMEV_FP32, rr, rnorm2, dx, lm, max_iterations - total_it,
                            std::min(want, 0.5), &kept, &it));
@@ -2659,7 +2687,9 @@ static int fit_block_common(sgmev_op* op, const double* y, bool y_dev, double la
   SGMEV_TRY(check_op(op));
   if ((op->m > 0 && !y) || (op->n > 0 && !alpha)) return fail(SGMEV_ERR_INVALID, "NULL vector");
   if (!(epsilon > 0.0) || max_iterations < 0) return fail(SGMEV_ERR_INVALID, "bad epsilon/max_iterations");
+  nest_again(op);
   SGMEV_TRY(block_ready(op));
+  products_ready(op, SGMEV_DF64);  // (before the directions take up to 512 MB)
   const int K = kBlockRhs;
   const int64_t np = op->npad;
   const double lm = static_cast<double>(op->m) * lambda;

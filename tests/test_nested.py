@@ -1,6 +1,9 @@
 """The nested subspace products: the plan's two programs on the host (every index checked) against
 the dense evaluation, and the FP64 kernels against the dense ones on the GPU."""
 import ctypes
+import os
+import subprocess
+import sys
 import time
 
 import numpy as np
@@ -579,3 +582,38 @@ def test_fp32_transposes_sum_at_most_1024_points_in_fp32():
     assert abs(out[root] - m * value) <= 2.0 ** -15 * m * value
     out[root] = 0.0
     assert np.all(out == 0.0)
+
+
+SHORT_OF_MEMORY = """
+import sys
+sys.path.insert(0, {root!r})
+import numpy as np, torch
+import sgpp_gb300 as sg
+grid = sg.Grid.createLinearGrid(2)
+grid.getGenerator().regular(8)
+n, m = grid.getSize(), 1 << 24
+rng = np.random.default_rng(1)
+op = sg.createOperationMultipleEval(grid, rng.random((m, 2)), sg.OperationMultipleEvalConfiguration(
+    sg.OperationMultipleEvalType.STREAMING, sg.OperationMultipleEvalSubType.CUDA))
+alpha, first, second = rng.standard_normal(n), np.zeros(m), np.zeros(m)
+# the tables take 2.1 GB
+rest = torch.empty(torch.cuda.mem_get_info()[0] - (1 << 30), dtype=torch.uint8, device="cuda")
+op.profile(True)
+op.mult(alpha, first)
+assert op.profileRead(sg.SGMEV_KERNEL_MULT_NEST64)[0] == 0
+assert op.profileRead(sg.SGMEV_KERNEL_MULT_FP64)[0] == 1
+del rest
+torch.cuda.empty_cache()
+op.mult(alpha, second)
+assert op.profileRead(sg.SGMEV_KERNEL_MULT_NEST64)[0] == 1
+assert np.abs(first - second).max() <= (6 * 2 + n) * 2.0 ** -52 * np.abs(alpha).sum()
+"""
+
+
+@pytest.mark.gpu
+def test_tables_refused_for_want_of_memory_are_built_once_there_is_some():
+    pytest.importorskip("torch")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", SHORT_OF_MEMORY.format(root=root)], capture_output=True, text=True,
+                          timeout=300)
+    assert done.returncode == 0, done.stderr
