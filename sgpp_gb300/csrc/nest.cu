@@ -18,12 +18,14 @@
 // point; FP32 and float-float instruction issue (7 instructions per subspace and point in FP32, 28 in
 // float-float, at 0.55 of the issue rate with the 12 to 14 warps per SM that the tables leave room
 // for). Measured before and after:
-//   FP64, d=5 level 6 (252 subspaces), 65,536 points: mult 10,791 -> 36 us, multT 10,895 -> 60 us
+//   FP64, d=5 level 6 (252 subspaces), 65,536 points: mult 10,791 -> 36 us, multT 10,895 -> 57 us
 //   FP64, adaptive d=8 grid (4,024 points), 2^19 data points: B^T (B a) 199.1 -> 1.22 ms
-//   FP32, d=10 level 5 (1,001 subspaces), 262,147 points: mult 168 -> 92 us (materialised before)
+//   FP32, d=10 level 5 (1,001 subspaces), 262,147 points: mult 168 -> 94 us (materialised before)
 //   float-float, d=9 level 6 (2,002 subspaces), 40,961 points: mult 583 -> 109 us (hats on the fly)
 // The errors against 64-bit results, relative to their norm: FP64 mult 6.1e-16 before and after,
-// multT 6.2e-16 -> 4.4e-16; FP32 mult 1.2e-7 before and after; float-float 1.5e-13 -> 8e-15.
+// multT 6.2e-16 -> 4.4e-16; FP32 mult 1.1e-7 -> 1.0e-7 (0.6 to 1.1 times the stored products' over 18
+// grids; up to 1.3 where one tree is the whole grid); float-float 1.5e-13 -> 8e-15 (ModLinear 8e-15 -> 6e-15
+// to 1.2e-14).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -120,6 +122,25 @@ __device__ __forceinline__ void mac_all(float (&s)[2], const float (&t)[2], cons
       "fma.rn.f32x2 vs, vt, va, vs;\n\tmov.b64 {%0, %1}, vs;\n\t}"
       : "+f"(s[0]), "+f"(s[1]) : "f"(t[0]), "f"(t[1]), "f"(a[0]), "f"(a[1]));
 }
+// s += t * a with the rounding errors of s collected in c (FP32): the sums over inner nodes and over
+// groups are long, and without this the error was up to 1.46 times that of the stored products, which are
+// rounded once (adaptive d=8 level 4, ModLinear: 1.22e-7 of the norm, now 6.8e-8, stored 8.4e-8); it costs
+// 1 % (d=10 level 5, 262,147 points: 92.6 -> 93.7 us)
+template <typename V, int R>
+__device__ __forceinline__ void mac_kept(V (&s)[R], V (&)[R], const V (&t)[R], const V (&a)[R]) { mac_all(s, t, a); }
+__device__ __forceinline__ void mac_kept(float (&s)[2], float (&c)[2], const float (&t)[2], const float (&a)[2]) {
+  // n = t a + s; c += t a + (s - n), where s - n is exact unless n is far smaller than s
+  asm("{\n\t.reg .b64 vs, vt, va, vn, vd, vc, vm;\n\tmov.b64 vs, {%0, %1};\n\tmov.b64 vc, {%2, %3};\n\t"
+      "mov.b64 vt, {%4, %5};\n\tmov.b64 va, {%6, %7};\n\tmov.b64 vm, {%8, %8};\n\t"
+      "fma.rn.f32x2 vn, vt, va, vs;\n\tfma.rn.f32x2 vd, vn, vm, vs;\n\tfma.rn.f32x2 vd, vt, va, vd;\n\t"
+      "add.rn.f32x2 vc, vc, vd;\n\tmov.b64 {%0, %1}, vn;\n\tmov.b64 {%2, %3}, vc;\n\t}"
+      : "+f"(s[0]), "+f"(s[1]), "+f"(c[0]), "+f"(c[1])
+      : "f"(t[0]), "f"(t[1]), "f"(a[0]), "f"(a[1]), "f"(-1.0f));
+}
+// (a correction that is not finite belongs to a sum that is not)
+__device__ __forceinline__ float corrected(float s, float c) { return fabsf(c) <= 3.4e38f ? s + c : s; }
+__device__ __forceinline__ double corrected(double s, double) { return s; }
+__device__ __forceinline__ ff corrected(ff s, ff) { return s; }
 __device__ __forceinline__ float mul(float a, float b) { return a * b; }
 __device__ __forceinline__ double mul(double a, double b) { return a * b; }
 __device__ __forceinline__ ff mul(ff a, ff b) {
@@ -330,7 +351,7 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
         }
       }
     }
-    V acc[R] = {};
+    V acc[R] = {}, acc_c[R] = {};
     for (int w = w_begin; w < w_end; ++w) {
       const NestOp4 win = a.windows[w];
       if (!one) {
@@ -342,7 +363,7 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
       const NestOp4* const op_end = op + (win.y - win.x);
       while (op < op_end) {
         const NestOp4 head = *op++;
-        V pr[R], ar[R] = {};
+        V pr[R], ar[R] = {}, ar_c[R] = {};
         uint32_t cr[R] = {};
 #pragma unroll
         for (int r = 0; r < R; ++r) set_val(pr[r], 1.0);
@@ -398,6 +419,8 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
               }
             };
             auto tree = [&](const char* (&row)[R], int t1, V (&st)[R]) {
+              // (FP32: level-2 and level-3 children in a sum each, half the roundings of one chain)
+              V s2[R] = {};
 #pragma unroll
               for (int r = 0; r < R; ++r) st[r] = ld(row[r]);
 #pragma unroll
@@ -421,7 +444,12 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
                 }
 #pragma unroll
                 for (int r = 0; r < R; ++r) settle(sq[r]);
-                mac_all(st, T2[t], sq);
+                if constexpr (std::is_same<V, float>::value) mac_all(s2, T2[t], sq);
+                else mac_all(st, T2[t], sq);
+              }
+              if constexpr (std::is_same<V, float>::value) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) st[r] += s2[r];
               }
             };
             const char* row[R];
@@ -478,19 +506,18 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
             }
           }
 #pragma unroll
-          for (int r = 0; r < R; ++r) {
-            settle(sum[r]);
-            mac(ar[r], tq[r], sum[r]);
-          }
+          for (int r = 0; r < R; ++r) settle(sum[r]);
+          mac_kept(ar, ar_c, tq, sum);
         }
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-          settle(ar[r]);
-          mac(acc[r], pr[r], ar[r]);
-        }
+        for (int r = 0; r < R; ++r) settle(ar[r]);
+        mac_kept(acc, acc_c, pr, ar);
+        if constexpr (std::is_same<V, float>::value) mac_all(acc_c, pr, ar_c);
       }
     }
     if (!live) continue;
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = corrected(acc[r], acc_c[r]);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const int64_t k = j + r;

@@ -617,3 +617,28 @@ def test_tables_refused_for_want_of_memory_are_built_once_there_is_some():
     done = subprocess.run([sys.executable, "-c", SHORT_OF_MEMORY.format(root=root)], capture_output=True, text=True,
                           timeout=300)
     assert done.returncode == 0, done.stderr
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("basis", ["linear", "modlinear"])
+@pytest.mark.parametrize("dim,level,rounds", [(4, 4, 6), (8, 4, 3)])
+def test_fp32_mult_is_as_close_as_the_one_of_stored_products(dim, level, rounds, basis):
+    """60,001 points, so that a thread adds all subspaces of its point in FP32; stored products are rounded
+    to FP32 once. Errors against FP64 vary by some 10 % between coefficient vectors: the mean of three."""
+    grid = _grid(dim, level, basis, rounds)
+    n, m = grid.getSize(), 60001
+    rng = np.random.default_rng(m)
+    x = rng.random((m, dim))
+    stored = sg.createOperationMultipleEval(grid, x, sg.OperationMultipleEvalConfiguration(
+        sg.OperationMultipleEvalType.STREAMING, sg.OperationMultipleEvalSubType.CUDA,
+        parameters={"precision": "float", "algo": "subspace", "materialize": "on"}))
+    nested, exact = _op(grid, x, "auto", "float"), _op(grid, x, "auto")
+    errors = np.zeros(2)
+    for _ in range(3):
+        alpha, ref = rng.standard_normal(n), np.zeros(m)
+        exact.mult(alpha, ref)
+        for k, op in enumerate((nested, stored)):
+            out = np.zeros(m)
+            op.mult(alpha, out)
+            errors[k] += np.linalg.norm(out - ref) / np.linalg.norm(ref) / 3.0
+    assert errors[0] <= 1.1 * errors[1]
