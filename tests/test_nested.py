@@ -642,3 +642,27 @@ def test_fp32_mult_is_as_close_as_the_one_of_stored_products(dim, level, rounds,
             op.mult(alpha, out)
             errors[k] += np.linalg.norm(out - ref) / np.linalg.norm(ref) / 3.0
     assert errors[0] <= 1.1 * errors[1]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("basis", ["linear", "modlinear"])
+@pytest.mark.parametrize("precision,unit", [("float", 2.0 ** -24), ("df64", 2.0 ** -44)])
+@pytest.mark.parametrize("m", [33, 2000, 70001])
+@pytest.mark.parametrize("dim,level", [(3, 6), (9, 6), (12, 3), (16, 3)])
+def test_every_fp32_and_df64_result_against_its_own_addends(dim, level, m, precision, unit, basis):
+    """Each result within its own roundings: a result's addends are its subspaces' (mult), or its data
+    points', of which at most 1,024 are added in FP32 (multTranspose); and the error of the whole vector."""
+    grid = _grid(dim, level, basis)
+    n = grid.getSize()
+    rng = np.random.default_rng(m + dim)
+    x = _points(rng, m, dim, level + 1)
+    alpha, v = rng.standard_normal(n), rng.standard_normal(m)
+    op, ref = _op(grid, x, "auto", precision), _op(grid, x, "auto")
+    n_sub = len(np.unique(grid.getStorage().level, axis=0))
+    for product, values, size, addends in ((0, alpha, m, n_sub), (1, v, n, min(m, 1024))):
+        out, exact, own = np.zeros(size), np.zeros(size), np.zeros(size)
+        for o, a, into in ((op, values, out), (ref, values, exact), (ref, np.abs(values), own)):
+            (o.multTranspose if product else o.mult)(a, into)
+        # two roundings a factor (table entry and product) on either side of the sum
+        assert np.all(np.abs(out - exact) <= (4 * dim + addends) * unit * own)
+        assert np.linalg.norm(out - exact) <= (1e-6 if precision == "float" else 1e-12) * np.linalg.norm(exact)
