@@ -246,8 +246,8 @@ SGMEV_API double sgmev_get_duration(sgmev_op* op);
 
 /* Use `stream` (a cudaStream_t) for all following work of this op; NULL restores the op's own.
  * The new stream is made to wait (an event) for the work the op enqueued on the previous one, so
- * sgmev_synchronize and sgmev_destroy (which frees on the current stream) cover the op's work on
- * every stream it used. */
+ * sgmev_synchronize and sgmev_destroy cover the op's work on every stream it used (the latter waits for
+ * it and frees on the op's own stream). Staging a new grid frees on the current one. */
 SGMEV_API int sgmev_set_stream(sgmev_op* op, void* stream);
 
 /* Change launch-shape knobs of a live operator: params_json may hold only "multt_batch",

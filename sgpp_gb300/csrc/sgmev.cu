@@ -63,7 +63,10 @@ constexpr int kReduceBlocks = 1216;  // 8 x 152 SMs
 constexpr int kDotBlocks = 304;
 constexpr int kDotThreads = 256;
 constexpr int kCgSlots = 10;
-constexpr int64_t kClusterVector = 262144;  // CG vectors whose steps run on one cluster (2 MB each)
+// CG vectors whose steps run on one cluster (2 MB each) in plain fits. The inner solves of mixed fits take it
+// at any length: with their passes over the kept directions a step's vector work is 123 us beside 474 us of
+// products at 242,815 entries (d=9 level 7, 20,000 points), 398 beside 5,200 at 956,929 (d=12 level 7).
+constexpr int64_t kClusterVector = 262144;
 
 static inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 static inline int64_t round_up(int64_t a, int64_t b) { return ceil_div(a, b) * b; }
@@ -1047,12 +1050,20 @@ static void products_ready(sgmev_op* op, int prec) {
 
 // Whether the inner solves of a mixed fit run on the FP16 products, both of them: a nested FP32 mult
 // beside the FP16 multTranspose is no symmetric operator, and the solutions it left had the residual
-// asked for but up to three times the error. On the nested FP32 mult and the FP32 multTranspose
-// (nested or materialised) an iteration's products take less time than on the FP16 ones on every
-// grid measured (d = 3..12, level 4..7, 1,000 to 256,000 points: 16,000 points 44-114 against 53-207 us,
-// 256,000 points 79-514 against 131-631 us) except where the FP16 mult fills its 16 warps of 64
-// subspaces in one pass and its cells are nibbles: d=10 level 5 138 against 128 us at 64,000 points,
-// 1.14 against 0.92 ms at 2^20; at 16,000 points 69 against 75.
+// asked for but up to three times the error. FP16 gains where its mult fills its 16 warps of 64 subspaces
+// in one pass, its cells are nibbles and the points are many. An iteration's products, nested FP32 mult and
+// FP32 multTranspose against FP16 (us, at 16,384 / 65,536 / 2^20 points; subspaces in brackets):
+//   within the bounds     d=9 level 5 [715]   60:67    117:106  899:835
+//                         d=15 level 4 [816]  63:61    140:95   1,100:836
+//                         d=16 level 4 [969]  69:63    164:103  1,472:874
+//                         d=10 level 5 [1001] 75:81    150:124  1,149:916
+//   below and above them  d=8 level 5 [495]   50:57    93:91    568:540
+//                         d=14 level 4 [680]  68:57    112:90   1,008:790
+//                         d=11 level 5 [1365] 87:113   175:167  1,668:1,452
+//                         adaptive d=9 level 5 [1598, 32 cells]  117:187  247:289  2,860:2,888
+// and at 32,768 points 89:86, 93:74, 105:75 and 104:91 within. Whole fits differ by less, as FP32 often saves
+// a step: outside the bounds the FP32 fits are at most 6 % slower than FP16 ones (d=14 level 4), at 32,768
+// points and below within them at most 12 % (d=16 level 4), at most 2 % at level 5.
 static bool inner_on_half(sgmev_op* op) {
   using namespace sgmev;
   if (op->inner_half == 0) return false;
