@@ -27,6 +27,8 @@ CXX_FLAGS = ["-O3", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wall",
 
 CU_SOURCES = ["sgmev.cu", "dense_mod.cu", "peak.cu", "noalloc.cu", "batch.cu", "subspace.cu",
               "subspace_mat.cu", "nest.cu", "devmem.cu", "fitter.cu", "block_tc.cu"]
+# one object per dimension: a process loads the kernels of the dimensions that it uses
+PER_DIM = [("nest_mult.cu", f"NEST_MULT_DIM={d}") for d in range(17)]
 CPP_SOURCES = ["grid.cpp", "datasets.cpp", "nest_plan.cpp"]
 
 
@@ -58,12 +60,12 @@ def build(verbose: bool = False, ptxas_info: bool = False) -> str:
     headers = _headers()
     jobs = []
     objs = []
-    for src in CU_SOURCES:
+    for src, define in [(f, "") for f in CU_SOURCES] + PER_DIM:
         s = os.path.join(CSRC, src)
-        o = os.path.join(BUILD, src + ".o")
+        o = os.path.join(BUILD, src + define.replace("=", "_") + ".o")
         objs.append(o)
         if ptxas_info or _sources_newer(o, [s] + headers):
-            cmd = [nvcc, *ARCH, *NVCC_FLAGS, "-c", s, "-o", o]
+            cmd = [nvcc, *ARCH, *NVCC_FLAGS, *(["-D" + define] if define else []), "-c", s, "-o", o]
             if ptxas_info:
                 cmd.insert(1, "-Xptxas=-v")
             jobs.append(cmd)

@@ -36,7 +36,8 @@
 #include "../../include/sgmev.h"
 #include "devmem.h"
 #include "kernels.cuh"
-#include "nest.h"
+#include "nest_arith.cuh"
+#include "nest_mult.h"
 #include "subspace.h"
 
 namespace sgmev {
@@ -97,440 +98,6 @@ __global__ void nest_table_kernel(const double* __restrict__ xt, int64_t mpad, i
     }
   }
   put(0, h1p);
-}
-
-// ---- mult ----------------------------------------------------------------------------------------
-// The three arithmetics. A value of the float-float one is (h, l) as in kernels.cuh.
-__device__ __forceinline__ void set_val(float& r, double v) { r = static_cast<float>(v); }
-__device__ __forceinline__ void set_val(double& r, double v) { r = v; }
-__device__ __forceinline__ void set_val(ff& r, double v) {
-  r.h = static_cast<float>(v);
-  r.l = static_cast<float>(v - static_cast<double>(r.h));
-}
-// s += t * a
-__device__ __forceinline__ void mac(float& s, float t, float a) { s = fmaf(t, a, s); }
-__device__ __forceinline__ void mac(double& s, double t, double a) { s = fma(t, a, s); }
-__device__ __forceinline__ void mac(ff& s, ff t, ff a) { add_ff(s, mul_ff(t, a)); }
-template <typename V, int R>
-__device__ __forceinline__ void mac_all(V (&s)[R], const V (&t)[R], const V (&a)[R]) {
-#pragma unroll
-  for (int r = 0; r < R; ++r) mac(s[r], t[r], a[r]);
-}
-// two FP32 multiply-adds in one instruction
-__device__ __forceinline__ void mac_all(float (&s)[2], const float (&t)[2], const float (&a)[2]) {
-  asm("{\n\t.reg .b64 vs, vt, va;\n\tmov.b64 vs, {%0, %1};\n\tmov.b64 vt, {%2, %3};\n\tmov.b64 va, {%4, %5};\n\t"
-      "fma.rn.f32x2 vs, vt, va, vs;\n\tmov.b64 {%0, %1}, vs;\n\t}"
-      : "+f"(s[0]), "+f"(s[1]) : "f"(t[0]), "f"(t[1]), "f"(a[0]), "f"(a[1]));
-}
-// s += t * a with the rounding errors of s collected in c (FP32): the sums over inner nodes and over
-// groups are long, and without this the error was up to 1.46 times that of the stored products, which are
-// rounded once (adaptive d=8 level 4, ModLinear: 1.22e-7 of the norm, now 6.8e-8, stored 8.4e-8); it costs
-// 1 % (d=10 level 5, 262,147 points: 92.6 -> 93.7 us)
-template <typename V, int R>
-__device__ __forceinline__ void mac_kept(V (&s)[R], V (&)[R], const V (&t)[R], const V (&a)[R]) { mac_all(s, t, a); }
-__device__ __forceinline__ void mac_kept(float (&s)[2], float (&c)[2], const float (&t)[2], const float (&a)[2]) {
-  // n = t a + s; c += t a + (s - n), where s - n is exact unless n is far smaller than s
-  asm("{\n\t.reg .b64 vs, vt, va, vn, vd, vc, vm;\n\tmov.b64 vs, {%0, %1};\n\tmov.b64 vc, {%2, %3};\n\t"
-      "mov.b64 vt, {%4, %5};\n\tmov.b64 va, {%6, %7};\n\tmov.b64 vm, {%8, %8};\n\t"
-      "fma.rn.f32x2 vn, vt, va, vs;\n\tfma.rn.f32x2 vd, vn, vm, vs;\n\tfma.rn.f32x2 vd, vt, va, vd;\n\t"
-      "add.rn.f32x2 vc, vc, vd;\n\tmov.b64 {%0, %1}, vn;\n\tmov.b64 {%2, %3}, vc;\n\t}"
-      : "+f"(s[0]), "+f"(s[1]), "+f"(c[0]), "+f"(c[1])
-      : "f"(t[0]), "f"(t[1]), "f"(a[0]), "f"(a[1]), "f"(-1.0f));
-}
-// (a correction that is not finite belongs to a sum that is not)
-__device__ __forceinline__ float corrected(float s, float c) { return fabsf(c) <= 3.4e38f ? s + c : s; }
-__device__ __forceinline__ double corrected(double s, double) { return s; }
-__device__ __forceinline__ ff corrected(ff s, ff) { return s; }
-__device__ __forceinline__ float mul(float a, float b) { return a * b; }
-__device__ __forceinline__ double mul(double a, double b) { return a * b; }
-__device__ __forceinline__ ff mul(ff a, ff b) {
-  ff r = mul_ff(a, b);
-  renorm_ff(r);
-  return r;
-}
-// a finished sum, before it becomes a factor (mul_ff drops the product of the low parts)
-__device__ __forceinline__ void settle(float&) {}
-__device__ __forceinline__ void settle(double&) {}
-__device__ __forceinline__ void settle(ff& s) { renorm_ff(s); }
-__device__ __forceinline__ double to_double(float v) { return static_cast<double>(v); }
-__device__ __forceinline__ double to_double(double v) { return v; }
-__device__ __forceinline__ double to_double(ff v) {
-  return static_cast<double>(v.h) + static_cast<double>(v.l);
-}
-__device__ __forceinline__ bool is_finite(float v) { return isfinite(v); }
-__device__ __forceinline__ bool is_finite(double v) { return isfinite(v); }
-__device__ __forceinline__ bool is_finite(ff v) { return isfinite(v.h); }
-// asynchronous copies into shared memory: `bytes` (4 or 8) of a thread's own column
-template <int BYTES>
-__device__ __forceinline__ void copy_async(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
-                   static_cast<uint32_t>(__cvta_generic_to_shared(dst))), "l"(src), "n"(BYTES) : "memory");
-}
-__device__ __forceinline__ void prefetch_l2(const void* p) {
-  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-}
-template <typename V>
-__device__ __forceinline__ void prefetch_entry(const float* hi, const float* lo, const double* d, int64_t k) {
-  if constexpr (std::is_same<V, double>::value) {
-    prefetch_l2(d + k);
-  } else {
-    prefetch_l2(hi + k);
-    if constexpr (sizeof(V) == 8) prefetch_l2(lo + k);
-  }
-}
-// table entries of R adjacent points (k: the first one's index)
-__device__ __forceinline__ void load_entry(float (&r)[2], const float* hi, const float*, const double*, int64_t k) { copy_async<8>(r, hi + k); }
-__device__ __forceinline__ void load_entry(double (&r)[1], const float*, const float*, const double* d, int64_t k) { copy_async<8>(r, d + k); }
-__device__ __forceinline__ void load_entry(ff (&r)[1], const float* hi, const float* lo, const double*, int64_t k) {
-  copy_async<4>(&r[0].h, hi + k);
-  copy_async<4>(&r[0].l, lo + k);
-}
-
-// coefficients into position order (launches that stage them more than once)
-template <typename V>
-__global__ void nest_coef_kernel(const double* __restrict__ alpha, const int* __restrict__ inv,
-                                 int64_t total, V* __restrict__ coef) {
-  for (int64_t p = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; p < total;
-       p += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int g = inv[p];
-    set_val(coef[p], g >= 0 ? alpha[g] : 0.0);
-  }
-}
-
-// the dense value of grid point g's function at point j (0 exactly outside its support)
-template <bool MOD>
-__device__ double dense_value(const NestDense& d, int dim, int64_t g, int64_t j) {
-  double p = h_first<MOD>(d.xt[j], d.li[g * dim]);
-  for (int t = 1; t < dim; ++t) p = h_next<MOD>(p, d.xt[t * d.mpad + j], d.li[g * dim + t]);
-  return p;
-}
-__device__ double dense_value(const NestDense& d, int dim, int64_t g, int64_t j) {
-  return d.mod ? dense_value<true>(d, dim, g, j) : dense_value<false>(d, dim, g, j);
-}
-
-// a value as the product's arithmetic holds it
-template <typename V>
-__device__ __forceinline__ double held(double v) {
-  V r;
-  set_val(r, v);
-  return to_double(r);
-}
-
-// NaN when a non-finite coefficient meets a hat of 0 at point j, else 0
-template <typename V>
-__device__ __noinline__ double mult_poison(const NestDense& d, int dim, int64_t n,
-                                           const double* alpha, int64_t j) {
-  double r = 0.0;
-  for (int64_t g = 0; g < n; ++g) {
-    const double a = held<V>(alpha[g]);
-    if (!isfinite(a) && isnan(a * dense_value(d, dim, g, j))) r = a - a;
-  }
-  return r;
-}
-__device__ __forceinline__ void add_poison(float& s, double v) { s += static_cast<float>(v); }
-__device__ __forceinline__ void add_poison(double& s, double v) { s += v; }
-__device__ __forceinline__ void add_poison(ff& s, double v) { s.h += static_cast<float>(v); }
-
-// R adjacent data points per thread (two in FP32, one in the wider arithmetics), a warp at a time over
-// a contiguous range of 32 R-point tiles; the points' table rows and cells in shared memory
-// ([entry][thread][R], private to the thread, copied asynchronously), their level-2 and level-3
-// factors and cells in registers for the runs and trees (MD = dim, or 0 for more dimensions than
-// kNestMacroDim: then the plan has none). A window's coefficients and program are staged in shared
-// memory: a warp's 32 gathers from one row hit different banks or the same word, and the program's
-// loads are broadcasts (read through L1 they missed half the time beside this much shared memory,
-// and the FP32 kernel took 203 us instead of 128). blockIdx.y takes windows
-// [y windows / splits, (y + 1) windows / splits) of the list and, with several splits, writes its own
-// row of partial sums.
-template <typename V>
-constexpr int kPts = sizeof(V) == 4 ? 2 : 1;
-constexpr int kMultMaxThreads = 448;
-
-struct NestMultArgs {
-  const NestOp4 *windows, *prog;
-  int n_windows, words;  // windows of the list, words of the longest program
-  int n_ent, dim;
-  int entry[32], lmax[32];  // first table entry (level 2) and finest level of each dimension
-  const float *tab_hi, *tab_lo;
-  const double* tab64;
-  const uint32_t* xcell;
-  int64_t m, j_begin, n_tiles;
-  float* out32;
-  double* out64;
-  void* part;
-  int64_t out_end;  // outputs are written for j < out_end, zero beyond m
-  NestDense dense;
-  const int* inv;
-  const double* alpha;
-  int64_t n;
-  const void* coef;  // coefficients in position order, or nullptr: gathered while they are staged
-  int warps;         // warps of a CTA that take tiles; the others only help to stage
-  const double* stop;  // device flag: when it is not 0 the product is skipped
-};
-
-// SPREAD: coefficients that are not finite spread as in the dense kernels. A variant of its own: as a
-// branch of one kernel it cost the grids that need no look 1 to 2 %.
-template <typename V, int MD, bool SPREAD>
-__global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
-    nest_mult_kernel(const __grid_constant__ NestMultArgs a) {
-  if (a.stop && *a.stop != 0.0) return;
-  constexpr int D = MD > 0 ? MD : 1, kV = sizeof(V), R = kPts<V>;
-  extern __shared__ __align__(16) unsigned char smem[];
-  const int tid = threadIdx.x, all = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = a.warps;
-  const int nth = 32 * nw;
-  const int64_t mpad = a.dense.mpad;
-  using Col = V[R];
-  using ColX = uint32_t[R];
-  NestOp4* s_prog = reinterpret_cast<NestOp4*>(smem);
-  Col* s_tab = reinterpret_cast<Col*>(s_prog + a.words) + tid;
-  ColX* s_x = reinterpret_cast<ColX*>(s_tab - tid + a.n_ent * nth) + tid;
-  V* s_coef = reinterpret_cast<V*>(s_x - tid + a.dim * nth);
-  const int w_begin = blockIdx.y * a.n_windows / gridDim.y;
-  const int w_end = (blockIdx.y + 1) * a.n_windows / gridDim.y;
-  bool poison = false;  // a coefficient that is not finite (the same in every thread)
-  auto stage = [&](const NestOp4& w) {
-    for (int k = w.x + tid; k < w.y; k += all) s_prog[k - w.x] = a.prog[k];
-    bool finite = true;
-    if (a.coef) {
-#pragma unroll 4
-      for (int k = w.z + tid; k < w.w; k += all) {
-        const V v = static_cast<const V*>(a.coef)[k];
-        if constexpr (SPREAD) finite = finite && is_finite(v);
-        s_coef[k - w.z] = v;
-      }
-    } else {
-#pragma unroll 4
-      for (int k = w.z + tid; k < w.w; k += all) {
-        const int g = a.inv[k];
-        V v;
-        set_val(v, g >= 0 ? a.alpha[g] : 0.0);
-        if constexpr (SPREAD) finite = finite && is_finite(v);
-        s_coef[k - w.z] = v;
-      }
-    }
-    if constexpr (SPREAD) poison = __syncthreads_or(!finite) || poison;
-    else __syncthreads();
-  };
-  // the warps' tile ranges are contiguous and as equal as can be; every warp of the CTA runs the same
-  // number of rounds (the barriers of several windows), some of them on no tile
-  const int64_t warps = static_cast<int64_t>(gridDim.x) * nw, gw = static_cast<int64_t>(blockIdx.x) * nw + warp;
-  const int64_t t_begin = warp < nw ? gw * a.n_tiles / warps : 0;
-  const int64_t t_end = warp < nw ? (gw + 1) * a.n_tiles / warps : 0;
-  const int64_t rounds = (a.n_tiles + warps - 1) / warps;
-  const bool one = w_end - w_begin == 1;
-  if (one) stage(a.windows[w_begin]);
-  for (int64_t round = 0; round < rounds; ++round) {
-    const bool live = t_begin + round < t_end;
-    if (one && !live) break;
-    const int64_t j = a.j_begin + ((t_begin + round) * 32 + lane) * R;
-    V T2[D][R], T3[D][R];
-    uint32_t B2[D][R], B3[D][R];  // byte offsets of the points' cells of levels 2 and 3
-    if (live) {
-#pragma unroll 4
-      for (int t = 0; t < a.dim; ++t) copy_async<4 * R>(s_x[t * nth], a.xcell + t * mpad + j);
-#pragma unroll 4
-      for (int e = 0; e < a.n_ent; ++e)
-        load_entry(s_tab[e * nth], a.tab_hi, a.tab_lo, a.tab64, e * mpad + j);
-      // the warp's next tile into L2: it streams from HBM otherwise, a full latency per tile
-      if (t_begin + round + 1 < t_end && (lane & 15) == 0) {
-        const int64_t jn = j + 32 * R;
-        for (int e = 0; e < a.n_ent; ++e) prefetch_entry<V>(a.tab_hi, a.tab_lo, a.tab64, e * mpad + jn);
-      }
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      if constexpr (MD > 0) {
-#pragma unroll
-        for (int t = 0; t < MD; ++t) {
-          const int bits = a.lmax[t] - 1;
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const uint32_t x = s_x[t * nth][r];
-            T2[t][r] = bits >= 1 ? s_tab[a.entry[t] * nth][r] : V{};
-            B2[t][r] = bits >= 1 ? (x >> (bits - 1)) * kV : 0u;
-            T3[t][r] = bits >= 2 ? s_tab[(a.entry[t] + 1) * nth][r] : V{};
-            B3[t][r] = bits >= 2 ? (x >> (bits - 2)) * kV : 0u;
-          }
-        }
-      }
-    }
-    V acc[R] = {}, acc_c[R] = {};
-    for (int w = w_begin; w < w_end; ++w) {
-      const NestOp4 win = a.windows[w];
-      if (!one) {
-        __syncthreads();  // the previous window is no longer read
-        stage(win);
-      }
-      if (!live) continue;
-      const NestOp4* op = s_prog;
-      const NestOp4* const op_end = op + (win.y - win.x);
-      while (op < op_end) {
-        const NestOp4 head = *op++;
-        V pr[R], ar[R] = {}, ar_c[R] = {};
-        uint32_t cr[R] = {};
-#pragma unroll
-        for (int r = 0; r < R; ++r) set_val(pr[r], 1.0);
-        const int* facs = reinterpret_cast<const int*>(op);
-        for (int i = 0; i < head.y; ++i) {
-          const int f = facs[i];
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            pr[r] = mul(pr[r], s_tab[fac_e(f) * nth][r]);
-            cr[r] = (cr[r] << fac_k(f)) | (s_x[fac_t(f) * nth][r] >> fac_shift(f));
-          }
-        }
-        op += (head.y + 3) / 4;
-        for (int q = 0; q < head.x; ++q) {
-          const NestOp4 qo = op[0], qf = op[1];
-          op += 2;
-          uint32_t c[R];
-          V tq[R], sum[R] = {};
-#pragma unroll
-          for (int r = 0; r < R; ++r) {
-            tq[r] = s_tab[qf.x * nth][r];
-            c[r] = (cr[r] << qf.z) | (s_x[qf.y * nth][r] >> qf.w);
-          }
-          if (MD == 0 || qo.y >= 0) {
-            if (qo.x >= 0) {
-#pragma unroll
-              for (int r = 0; r < R; ++r) sum[r] = s_coef[qo.x + c[r]];
-            }
-            const NestOp4* const leaf_end = op + qo.y;
-#pragma unroll 2
-            for (; op < leaf_end; ++op) {
-              const NestOp4 lo = *op;
-              const int e = lo.y & 0xFFFF, t = lo.y >> 16;
-#pragma unroll
-              for (int r = 0; r < R; ++r)
-                mac(sum[r], s_tab[e * nth][r],
-                    s_coef[lo.x + ((c[r] << lo.z) | (s_x[t * nth][r] >> lo.w))]);
-            }
-          } else if constexpr (MD > 0) {
-            const int kind = -qo.y - 1, t0 = kind >> 2;
-            auto ld = [](const char* p) { return *reinterpret_cast<const V*>(p); };
-            // the value of a run and of a tree whose dimensions begin at t1, from their rows
-            auto run = [&](const char* (&row)[R], int t1, V (&sr)[R]) {
-#pragma unroll
-              for (int r = 0; r < R; ++r) sr[r] = ld(row[r]);
-#pragma unroll
-              for (int t = MD - 1; t >= 0; --t) {
-                if (t < t1) break;
-                V v[R];
-#pragma unroll
-                for (int r = 0; r < R; ++r) v[r] = ld(row[r] + B2[t][r] + kV * (1 + 2 * (MD - 1 - t)));
-                mac_all(sr, T2[t], v);
-              }
-            };
-            auto tree = [&](const char* (&row)[R], int t1, V (&st)[R]) {
-              // (FP32: level-2 and level-3 children in a sum each, half the roundings of one chain)
-              V s2[R] = {};
-#pragma unroll
-              for (int r = 0; r < R; ++r) st[r] = ld(row[r]);
-#pragma unroll
-              for (int t = MD - 1; t >= 0; --t) {
-                if (t < t1) break;
-                const int kt = MD - 1 - t, sec = kV * nest_tree_at(kt);
-                V sq[R], v[R];
-                const char* rq[R];
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                  rq[r] = row[r] + B2[t][r] * static_cast<uint32_t>(nest_run_row(kt));
-                  sq[r] = ld(rq[r] + sec);
-                  v[r] = ld(row[r] + B3[t][r] + (sec + kV * 2 * nest_run_row(kt)));
-                }
-                mac_all(st, T3[t], v);
-#pragma unroll
-                for (int u = MD - 1; u > t; --u) {
-#pragma unroll
-                  for (int r = 0; r < R; ++r) v[r] = ld(rq[r] + B2[u][r] + (sec + kV * (1 + 2 * (MD - 1 - u))));
-                  mac_all(sq, T2[u], v);
-                }
-#pragma unroll
-                for (int r = 0; r < R; ++r) settle(sq[r]);
-                if constexpr (std::is_same<V, float>::value) mac_all(s2, T2[t], sq);
-                else mac_all(st, T2[t], sq);
-              }
-              if constexpr (std::is_same<V, float>::value) {
-#pragma unroll
-                for (int r = 0; r < R; ++r) st[r] += s2[r];
-              }
-            };
-            const char* row[R];
-            if ((kind & 3) < 2) {
-#pragma unroll
-              for (int r = 0; r < R; ++r) row[r] = reinterpret_cast<const char*>(s_coef + qo.x + c[r] * qo.z);
-              if ((kind & 3) == 0) run(row, t0, sum);
-              else tree(row, t0, sum);
-            } else {
-              const V* cells = s_coef + qo.x;
-#pragma unroll
-              for (int r = 0; r < R; ++r) sum[r] = cells[c[r]];
-              cells += ((1 << qo.z) + 3) & ~3;
-              int tree_row = nest_tree_row(0), run_row = nest_run_row(0), tree_end = nest_tree_at(0);
-              for (int t = MD - 1; t >= t0; --t) {
-                const int bits = a.lmax[t] - 1;
-                const Col* te = s_tab + a.entry[t] * nth;
-                V v[R], tl[R];
-                uint32_t x[R];
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                  x[r] = s_x[t * nth][r];
-                  row[r] = reinterpret_cast<const char*>(cells + ((c[r] << 1) | (x[r] >> (bits - 1))) * tree_row);
-                  tl[r] = te[0][r];
-                }
-                tree(row, t + 1, v);
-#pragma unroll
-                for (int r = 0; r < R; ++r) settle(v[r]);
-                mac_all(sum, tl, v);
-                cells += (2 * tree_row) << qo.z;
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                  row[r] = reinterpret_cast<const char*>(cells + ((c[r] << 2) | (x[r] >> (bits - 2))) * run_row);
-                  tl[r] = te[nth][r];
-                }
-                run(row, t + 1, v);
-#pragma unroll
-                for (int r = 0; r < R; ++r) settle(v[r]);
-                mac_all(sum, tl, v);
-                cells += (4 * run_row) << qo.z;
-#pragma unroll
-                for (int r = 0; r < R; ++r) {
-                  v[r] = cells[(c[r] << 3) | (x[r] >> (bits - 3))];
-                  tl[r] = te[2 * nth][r];
-                }
-                mac_all(sum, tl, v);
-                cells += 8 << qo.z;
-                // the next dimension's row lengths (nest_tree_at, nest_tree_row and nest_run_row of k + 1)
-                tree_end += 2 * run_row + 4;
-                tree_row = ((tree_end + 3) & ~7) + 4;
-                const int k = MD - t;
-                run_row = 2 * k + ((k & 1) == 0 ? 2 : 4);
-              }
-            }
-          }
-#pragma unroll
-          for (int r = 0; r < R; ++r) settle(sum[r]);
-          mac_kept(ar, ar_c, tq, sum);
-        }
-#pragma unroll
-        for (int r = 0; r < R; ++r) settle(ar[r]);
-        mac_kept(acc, acc_c, pr, ar);
-        if constexpr (std::is_same<V, float>::value) mac_all(acc_c, pr, ar_c);
-      }
-    }
-    if (!live) continue;
-#pragma unroll
-    for (int r = 0; r < R; ++r) acc[r] = corrected(acc[r], acc_c[r]);
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int64_t k = j + r;
-      const bool real = k < a.m;
-      if (SPREAD && poison && real) add_poison(acc[r], mult_poison<V>(a.dense, a.dim, a.n, a.alpha, k));
-      if (gridDim.y > 1) {
-        reinterpret_cast<V*>(a.part)[blockIdx.y * mpad + k] = acc[r];
-      } else {
-        if (a.out32 && k < a.out_end) a.out32[k] = real ? static_cast<float>(to_double(acc[r])) : 0.0f;
-        if (a.out64 && k < a.out_end) a.out64[k] = real ? to_double(acc[r]) : 0.0;
-      }
-    }
-  }
 }
 
 // ---- multTranspose -----------------------------------------------------------------------------
@@ -787,98 +354,6 @@ cudaError_t tables(NestPlan& p, cudaStream_t s, const NestDense& d, int64_t m, b
   return cudaGetLastError();
 }
 
-// Threads per CTA, the window list and the CTAs that share a tile of points, once per operator (m
-// does not change). A CTA has as many warps as its shared memory holds table rows for (one CTA per
-// SM), or fewer when the tiles would not reach every SM. Of the lists, the one with the least cycles
-// by a model of the measured kernels: a round of a warp costs about 2,500 cycles for its table rows
-// and 75 (FP32, two points a thread), 150 (float-float) or 21 a warp of the SM (FP64, whose pipe the
-// warps share) per subspace; staging a window about 1,500 and a cycle per 40 bytes; several CTAs per
-// tile pay about 5,000 for the partial sums' pass.
-template <typename V, typename Kern>
-cudaError_t mult_config(const NestPlan& p, NestConfig* c, Kern kern, int64_t m, int64_t mpad,
-                        int64_t part_bytes, int num_sms) {
-  constexpr int64_t kV = sizeof(V), R = kPts<V>;
-  const int caps = kV == 4 ? 0 : kNestLists / 2;
-  const int64_t tiles = std::max<int64_t>(1, (m + 32 * R - 1) / (32 * R));
-  const int64_t row = 32 * R * (kV * p.n_ent + 4 * p.dim);  // table rows of a warp
-  const int64_t most = (kV == 4 ? 384 : kMultMaxThreads) / 32;
-  double best = 0.0;
-  int64_t warps = 1, window = 0;
-  for (int k = 0; k < kNestLists / 2; ++k) {
-    const int list = caps + k, n_windows = p.lists[list + 1] - p.lists[list];
-    const int64_t ctas = nest_list_ctas(list);
-    if (k > 0 && (n_windows < ctas || part_bytes < ctas * mpad * kV)) break;
-    const int64_t w = kV * p.list_cells[list] + static_cast<int64_t>(sizeof(NestOp4)) * p.list_words[list];
-    const int64_t fit = std::max<int64_t>(1, std::min<int64_t>({most, (static_cast<int64_t>(kNestMultSmem) - w) / row,
-                                                                std::max<int64_t>(2, (tiles * ctas + num_sms - 1) / num_sms)}));
-    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((tiles + fit - 1) / fit, num_sms / ctas));
-    const int64_t rounds = (tiles + blocks * fit - 1) / (blocks * fit);
-    const double per_sub = std::is_same<V, double>::value ? 21.0 * static_cast<double>(fit) : kV == 4 ? 75.0 : 150.0;
-    const double staged = 1500.0 + static_cast<double>(kV * p.list_cells[list]) / 40.0;
-    const int64_t per_cta = (n_windows + ctas - 1) / ctas;
-    const double cost = static_cast<double>(rounds) * (2500.0 + 20.0 * p.n_ent + per_sub * p.n_sub / static_cast<double>(ctas)) +
-                        static_cast<double>(per_cta > 1 ? rounds * per_cta : 1) * staged + (ctas > 1 ? 5000.0 : 0.0);
-    if (k == 0 || cost < best) {
-      best = cost;
-      c->list = list;
-      c->splits = static_cast<int>(ctas);
-      c->restage = per_cta > 1 && rounds > 1;
-      warps = fit;
-      window = w;
-    }
-  }
-  c->warps = static_cast<int>(warps);
-  c->threads = 32 * std::max(8, c->warps);
-  c->smem = static_cast<size_t>(window + row * warps);
-  cudaError_t e = set_smem_cap(kern, c->smem);
-  int per_sm = 0;
-  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, c->threads, c->smem);
-  if (e != cudaSuccess) return e;
-  c->ctas = std::max(1, per_sm) * num_sms;
-  return cudaSuccess;
-}
-
-template <typename V, int MD, bool SPREAD>
-cudaError_t launch_mult(NestPlan& p, cudaStream_t s, NestConfig& c, NestMultArgs& a, int64_t mpad,
-                        int64_t part_bytes, int64_t tiles, int num_sms) {
-  auto kern = nest_mult_kernel<V, MD, SPREAD>;
-  if (c.threads == 0) {
-    const cudaError_t e = mult_config<V>(p, &c, kern, a.m, mpad, part_bytes, num_sms);
-    if (e != cudaSuccess) {
-      c.threads = 0;
-      return e;
-    }
-  }
-  a.windows = p.windows + p.lists[c.list];
-  a.n_windows = p.lists[c.list + 1] - p.lists[c.list];
-  a.words = p.list_words[c.list];
-  a.warps = c.warps;
-  a.coef = nullptr;
-  if (c.restage) {
-    nest_coef_kernel<V><<<32, 512, 0, s>>>(a.alpha, p.inv, p.total, static_cast<V*>(p.coef));
-    a.coef = p.coef;
-  }
-  const int nw = c.warps;
-  const int64_t blocks = std::max<int64_t>(
-      1, std::min<int64_t>((tiles + nw - 1) / nw, c.ctas / c.splits));
-  kern<<<dim3(static_cast<unsigned>(blocks), static_cast<unsigned>(c.splits)), c.threads, c.smem, s>>>(a);
-  return cudaGetLastError();
-}
-
-template <typename V, bool SPREAD>
-cudaError_t launch_mult_dim(NestPlan& p, cudaStream_t s, NestConfig& c, NestMultArgs& a,
-                            int64_t mpad, int64_t part_bytes, int64_t tiles, int num_sms) {
-  switch (p.dim) {
-#define F(D) \
-  case D:    \
-    return launch_mult<V, D, SPREAD>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
-    F(1) F(2) F(3) F(4) F(5) F(6) F(7) F(8) F(9) F(10) F(11) F(12) F(13) F(14) F(15) F(16)
-#undef F
-    default:
-      return launch_mult<V, 0, SPREAD>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
-  }
-}
-
 template <typename V, typename TP>
 cudaError_t mult(NestPlan& p, cudaStream_t s, NestConfig& c, const NestDense& dense, int64_t m,
                  const double* alpha, float* out32, double* out64, int64_t j_begin, int64_t j_end,
@@ -914,10 +389,13 @@ cudaError_t mult(NestPlan& p, cudaStream_t s, NestConfig& c, const NestDense& de
   a.inv = p.inv;
   a.alpha = alpha;
   a.n = p.n;
-  if (kF64 || spread)
-    e = launch_mult_dim<V, true>(p, s, c, a, dense.mpad, part_bytes, a.n_tiles, num_sms);
-  else if constexpr (!kF64)
-    e = launch_mult_dim<V, false>(p, s, c, a, dense.mpad, part_bytes, a.n_tiles, num_sms);
+  static NestMultLaunch* const launch[kNestMacroDim + 1] = {
+      nest_mult_0,  nest_mult_1,  nest_mult_2,  nest_mult_3,  nest_mult_4,  nest_mult_5,
+      nest_mult_6,  nest_mult_7,  nest_mult_8,  nest_mult_9,  nest_mult_10, nest_mult_11,
+      nest_mult_12, nest_mult_13, nest_mult_14, nest_mult_15, nest_mult_16};
+  const int precision = kF64 ? SGMEV_FP64 : std::is_same<V, float>::value ? SGMEV_FP32 : SGMEV_DF64;
+  e = launch[p.dim <= kNestMacroDim ? p.dim : 0](p, s, precision, spread, c, a, dense.mpad, part_bytes,
+                                                  a.n_tiles, num_sms);
   if (e != cudaSuccess) return e;
   *launches += c.restage ? 2 : 1;
   if (c.splits > 1) {
