@@ -301,43 +301,52 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
     // the other from S on took 6 s for 230,230 subspaces, this 0.3 s); the kernels take any number.
     int64_t want = std::max((total + cap - 1) / cap, (least_words + kNestProgram - 1) / kNestProgram);
     want = std::max<int64_t>(1, (want + ctas - 1) / ctas) * ctas;
-    for (int tries = 0; tries < 32; ++tries) {
-      int64_t made = 0, done = 0;
-      for (int q = 0; q < n_q; ++made) q = window_end(q, cap, want, made, &done);
-      if (made <= want || want >= 2 * n_q) break;
-      want += std::max<int64_t>(1, (made - want) / (4 * ctas)) * ctas;
-    }
+    const size_t prog0 = p->prog.size(), win0 = p->windows.size();
     int64_t widest = 0, longest = 0, made = 0, done = 0;
-    p->list_begin.push_back(static_cast<int>(p->windows.size()));
-    for (int q = 0; q < n_q; ++made) {
-      const int p0 = static_cast<int>(p->prog.size()), q0 = q, c0 = static_cast<int>(q_coef[q0]);
-      const int q1 = window_end(q0, cap, want, made, &done);
-      size_t header = 0;
-      for (; q < q1; ++q) {
-        const NestOp4& o = qops[q];
-        const NestOp2& g = groups[q_group[q]];
-        const int nl = o.y >= 0 ? o.z - o.y : 0;
-        if (opens(q, q0)) {
-          header = p->prog.size();
-          p->prog.push_back(NestOp4{0, g.y - g.x, 0, 0});
-          for (int i = g.x; i < g.y; i += 4) {
-            auto f = [&](int k) { return k < g.y ? facs[k] : 0; };
-            p->prog.push_back(NestOp4{f(i), f(i + 1), f(i + 2), f(i + 3)});
+    auto build = [&] {
+      p->prog.resize(prog0);
+      p->windows.resize(win0);
+      widest = longest = made = done = 0;
+      for (int q = 0; q < n_q; ++made) {
+        const int p0 = static_cast<int>(p->prog.size()), q0 = q, c0 = static_cast<int>(q_coef[q0]);
+        const int q1 = window_end(q0, cap, want, made, &done);
+        size_t header = 0;
+        for (; q < q1; ++q) {
+          const NestOp4& o = qops[q];
+          const NestOp2& g = groups[q_group[q]];
+          const int nl = o.y >= 0 ? o.z - o.y : 0;
+          if (opens(q, q0)) {
+            header = p->prog.size();
+            p->prog.push_back(NestOp4{0, g.y - g.x, 0, 0});
+            for (int i = g.x; i < g.y; i += 4) {
+              auto f = [&](int k) { return k < g.y ? facs[k] : 0; };
+              p->prog.push_back(NestOp4{f(i), f(i + 1), f(i + 2), f(i + 3)});
+            }
+          }
+          ++p->prog[header].x;
+          p->prog.push_back(NestOp4{o.x >= 0 ? o.x - c0 : -1, o.y >= 0 ? nl : o.y, o.z, 0});
+          p->prog.push_back(NestOp4{fac_e(o.w), fac_t(o.w), fac_k(o.w), fac_shift(o.w)});
+          for (int i = 0; i < nl; ++i) {
+            const NestOp2& u = lops[o.y + i];
+            p->prog.push_back(NestOp4{u.x - c0, fac_e(u.y) | (fac_t(u.y) << 16), fac_k(u.y), fac_shift(u.y)});
           }
         }
-        ++p->prog[header].x;
-        p->prog.push_back(NestOp4{o.x >= 0 ? o.x - c0 : -1, o.y >= 0 ? nl : o.y, o.z, 0});
-        p->prog.push_back(NestOp4{fac_e(o.w), fac_t(o.w), fac_k(o.w), fac_shift(o.w)});
-        for (int i = 0; i < nl; ++i) {
-          const NestOp2& u = lops[o.y + i];
-          p->prog.push_back(NestOp4{u.x - c0, fac_e(u.y) | (fac_t(u.y) << 16), fac_k(u.y), fac_shift(u.y)});
-        }
+        const int p1 = static_cast<int>(p->prog.size());
+        widest = std::max(widest, q_coef[q] - q_coef[q0]);
+        longest = std::max<int64_t>(longest, p1 - p0);
+        p->windows.push_back(NestOp4{p0, p1, c0, static_cast<int>(q_coef[q])});
       }
-      const int p1 = static_cast<int>(p->prog.size());
-      widest = std::max(widest, q_coef[q] - q_coef[q0]);
-      longest = std::max<int64_t>(longest, p1 - p0);
-      p->windows.push_back(NestOp4{p0, p1, c0, static_cast<int>(q_coef[q])});
+    };
+    build();
+    if (made > want && want < 2 * n_q) {  // (count before the next one is built)
+      for (int tries = 0; tries < 32 && made > want && want < 2 * n_q; ++tries) {
+        want += std::max<int64_t>(1, (made - want) / (4 * ctas)) * ctas;
+        made = done = 0;
+        for (int q = 0; q < n_q; ++made) q = window_end(q, cap, want, made, &done);
+      }
+      build();
     }
+    p->list_begin.push_back(static_cast<int>(win0));
     p->list_cells.push_back(static_cast<int>(widest));
     p->list_words.push_back(static_cast<int>(longest));
   }
@@ -366,12 +375,12 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
   for (int id : subs) {
     p->cells += int64_t(1) << excess[id];
     p->cmax = std::max(p->cmax, 1 << excess[id]);
-    for (int a = id; parent[a] >= 0; a = parent[a]) ++p->n_act;
   }
   std::vector<NestOp4> chunks;
   std::vector<NestOp2> cq, cs, cwarp;
   std::vector<int> clev, ccell, local(n_nodes, -1), depth(n_nodes, 0);
   for (int id : order) depth[id] = parent[id] < 0 ? 0 : depth[parent[id]] + 1;
+  for (int id : subs) p->n_act += depth[id];
   std::vector<int64_t> tpos(n_nodes, -1);
   int64_t row_total = 0;
   for (size_t at = 0; at < subs.size();) {
