@@ -23,8 +23,8 @@
 //   FP32, d=10 level 5 (1,001 subspaces), 262,147 points: mult 168 -> 94 us (materialised before)
 //   float-float, d=9 level 6 (2,002 subspaces), 40,961 points: mult 583 -> 109 us (hats on the fly)
 // The errors against 64-bit results, relative to their norm: FP64 mult 6.1e-16 before and after,
-// multT 6.2e-16 -> 4.4e-16; FP32 mult 1.1e-7 -> 1.0e-7 (0.6 to 1.1 times the stored products' over 18
-// grids; up to 1.3 where one tree is the whole grid); float-float 1.5e-13 -> 8e-15 (ModLinear 8e-15 -> 6e-15
+// multT 6.2e-16 -> 4.4e-16; FP32 mult 1.1e-7 -> 1.1e-7 (0.7 to 1.06 times the stored products' over 32
+// grids); float-float 1.5e-13 -> 8e-15 (ModLinear 8e-15 -> 6e-15
 // to 1.2e-14).
 #include <cuda_runtime.h>
 
@@ -267,6 +267,7 @@ bool nest_build(NestPlan* p, int dim, int64_t n, const double* level_pow2, const
   p->n_act = h.n_act;
   p->cells = h.cells;
   p->cmax = h.cmax;
+  p->whole = h.whole;
   p->n_ent = h.n_ent;
   p->lists = h.list_begin;
   p->list_cells = h.list_cells;

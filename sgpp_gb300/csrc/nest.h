@@ -27,6 +27,7 @@ struct NestPlan {
   int64_t n = 0, total = 0;
   int64_t n_act = 0, cells = 0;  // see NestTables
   int cmax = 0;
+  bool whole = false;
   std::vector<NestClass> classes;
   std::vector<int> lists, list_cells, list_words;  // see NestTables
   int h_entry[32] = {0}, h_lmax[32] = {0};

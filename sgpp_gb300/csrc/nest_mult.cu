@@ -19,10 +19,13 @@
 namespace sgmev {
 namespace {
 
-// s += t * a with the rounding errors of s collected in c (FP32): the sums over inner nodes and over
-// groups are long, and without this the error was up to 1.46 times that of the stored products, which are
-// rounded once (adaptive d=8 level 4, ModLinear: 1.22e-7 of the norm, now 6.8e-8, stored 8.4e-8); it costs
-// 1 % (d=10 level 5, 262,147 points: 92.6 -> 93.7 us)
+// s += t * a with the rounding errors of s collected in c (FP32): the sums over groups and inner nodes, and
+// over the dimensions where one forest or tree is all of the grid (regular ones of level 3 and 4), are long,
+// and without this the error was up to 1.46 times that of the stored products, which are rounded once; now
+// 0.7 to 1.06 times over 28 regular and four refined grids (d=12 level 4: 1.42 -> 1.02, adaptive d=8 level 4
+// 1.43 -> 0.8). It costs 1 % (d=10 level 5, 262,147 points: 92.7 -> 93.8 us; 100 us with it in every forest and
+// tree of such a grid, where the ratio is 0.9 without) and 3 to 5 % where a block is all of the grid (d=8 level 4,
+// 262,144 points: 26.0 -> 26.9 us, 118 on stored products; d=16 level 3, whose kernel spills: 25.3 -> 29.1, 113).
 template <typename V, int R>
 __device__ __forceinline__ void mac_kept(V (&s)[R], V (&)[R], const V (&t)[R], const V (&a)[R]) { mac_all(s, t, a); }
 __device__ __forceinline__ void mac_kept(float (&s)[2], float (&c)[2], const float (&t)[2], const float (&a)[2]) {
@@ -103,8 +106,9 @@ __device__ __forceinline__ void add_poison(ff& s, double v) { s.h += static_cast
 constexpr int kMultMaxThreads = 448;
 
 // SPREAD: coefficients that are not finite spread as in the dense kernels. A variant of its own: as a
-// branch of one kernel it cost the grids that need no look 1 to 2 %.
-template <typename V, int MD, bool SPREAD>
+// branch of one kernel it cost the grids that need no look 1 to 2 %. WHOLE (FP32): one forest or tree is all of
+// the grid, whose sums then carry their errors too (a variant for the same reason: 7 % as a branch).
+template <typename V, int MD, bool SPREAD, bool WHOLE>
 __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
     nest_mult_kernel(const __grid_constant__ NestMultArgs a) {
   if (a.stop && *a.stop != 0.0) return;
@@ -239,6 +243,7 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
             }
           } else if constexpr (MD > 0) {
             const int kind = -qo.y - 1, t0 = kind >> 2;
+            V sum_c[R] = {};
             auto ld = [](const char* p) { return *reinterpret_cast<const V*>(p); };
             // the value of a run and of a tree whose dimensions begin at t1, from their rows
             auto run = [&](const char* (&row)[R], int t1, V (&sr)[R]) {
@@ -253,8 +258,8 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
                 mac_all(sr, T2[t], v);
               }
             };
-            auto tree = [&](const char* (&row)[R], int t1, V (&st)[R]) {
-              // (FP32: level-2 and level-3 children in a sum each, half the roundings of one chain)
+            // (`alone`, a constant where this is inlined: not one of a forest's, which adds them up)
+            auto tree = [&](const char* (&row)[R], int t1, V (&st)[R], bool alone) {
               V s2[R] = {};
 #pragma unroll
               for (int r = 0; r < R; ++r) st[r] = ld(row[r]);
@@ -279,10 +284,10 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
                 }
 #pragma unroll
                 for (int r = 0; r < R; ++r) settle(sq[r]);
-                if constexpr (std::is_same<V, float>::value) mac_all(s2, T2[t], sq);
+                if (WHOLE && alone) mac_kept(s2, sum_c, T2[t], sq);
                 else mac_all(st, T2[t], sq);
               }
-              if constexpr (std::is_same<V, float>::value) {
+              if constexpr (WHOLE) {
 #pragma unroll
                 for (int r = 0; r < R; ++r) st[r] += s2[r];
               }
@@ -292,7 +297,7 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
 #pragma unroll
               for (int r = 0; r < R; ++r) row[r] = reinterpret_cast<const char*>(s_coef + qo.x + c[r] * qo.z);
               if ((kind & 3) == 0) run(row, t0, sum);
-              else tree(row, t0, sum);
+              else tree(row, t0, sum, true);
             } else {
               const V* cells = s_coef + qo.x;
 #pragma unroll
@@ -310,10 +315,11 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
                   row[r] = reinterpret_cast<const char*>(cells + ((c[r] << 1) | (x[r] >> (bits - 1))) * tree_row);
                   tl[r] = te[0][r];
                 }
-                tree(row, t + 1, v);
+                tree(row, t + 1, v, false);
 #pragma unroll
                 for (int r = 0; r < R; ++r) settle(v[r]);
-                mac_all(sum, tl, v);
+                if (WHOLE) mac_kept(sum, sum_c, tl, v);
+                else mac_all(sum, tl, v);
                 cells += (2 * tree_row) << qo.z;
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
@@ -323,14 +329,16 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
                 run(row, t + 1, v);
 #pragma unroll
                 for (int r = 0; r < R; ++r) settle(v[r]);
-                mac_all(sum, tl, v);
+                if (WHOLE) mac_kept(sum, sum_c, tl, v);
+                else mac_all(sum, tl, v);
                 cells += (4 * run_row) << qo.z;
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                   v[r] = cells[(c[r] << 3) | (x[r] >> (bits - 3))];
                   tl[r] = te[2 * nth][r];
                 }
-                mac_all(sum, tl, v);
+                if (WHOLE) mac_kept(sum, sum_c, tl, v);
+                else mac_all(sum, tl, v);
                 cells += 8 << qo.z;
                 // the next dimension's row lengths (nest_tree_at, nest_tree_row and nest_run_row of k + 1)
                 tree_end += 2 * run_row + 4;
@@ -339,6 +347,7 @@ __global__ void __launch_bounds__(sizeof(V) == 4 ? 384 : kMultMaxThreads, 1)
                 run_row = 2 * k + ((k & 1) == 0 ? 2 : 4);
               }
             }
+            if constexpr (WHOLE) mac_all(ar_c, tq, sum_c);
           }
 #pragma unroll
           for (int r = 0; r < R; ++r) settle(sum[r]);
@@ -419,10 +428,10 @@ cudaError_t mult_config(const NestPlan& p, NestConfig* c, Kern kern, int64_t m, 
   return cudaSuccess;
 }
 
-template <typename V, int MD, bool SPREAD>
+template <typename V, int MD, bool SPREAD, bool WHOLE = false>
 cudaError_t launch_mult(NestPlan& p, cudaStream_t s, NestConfig& c, NestMultArgs& a, int64_t mpad,
                         int64_t part_bytes, int64_t tiles, int num_sms) {
-  auto kern = nest_mult_kernel<V, MD, SPREAD>;
+  auto kern = nest_mult_kernel<V, MD, SPREAD, WHOLE>;
   if (c.threads == 0) {
     const cudaError_t e = mult_config<V>(p, &c, kern, a.m, mpad, part_bytes, num_sms);
     if (e != cudaSuccess) {
@@ -454,9 +463,13 @@ cudaError_t NEST_MULT_NAME(NEST_MULT_DIM)(NestPlan& p, cudaStream_t s, int preci
                                           int num_sms) {
   constexpr int D = NEST_MULT_DIM;
   if (precision == SGMEV_FP64) return launch_mult<double, D, true>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
-  if (precision == SGMEV_FP32)
-    return spread ? launch_mult<float, D, true>(p, s, c, a, mpad, part_bytes, tiles, num_sms)
-                  : launch_mult<float, D, false>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
+  if (precision == SGMEV_FP32) {
+    // (grids whose values spread are mostly small: one variant, with everything)
+    constexpr bool kBlocks = D > 0;
+    if (spread) return launch_mult<float, D, true, kBlocks>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
+    if (p.whole) return launch_mult<float, D, false, kBlocks>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
+    return launch_mult<float, D, false>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
+  }
   return spread ? launch_mult<ff, D, true>(p, s, c, a, mpad, part_bytes, tiles, num_sms)
                 : launch_mult<ff, D, false>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
 }

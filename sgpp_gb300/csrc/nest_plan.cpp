@@ -242,6 +242,7 @@ bool nest_plan(NestTables* p, int dim, int64_t n, const double* level_pow2, cons
     }
     flush();
   };
+  p->whole = budget[root] > 0;
   groups.push_back(NestOp2{0, 0});
   add_q(root);  // the root by itself: its factor is H_1
   for (int id : order) {

@@ -108,6 +108,7 @@ struct NestTables {
   int64_t n = 0;
   int64_t n_act = 0, cells = 0;  // active dimensions and cells of all subspaces
   int cmax = 0;                  // most cells of a subspace
+  bool whole = false;            // one run, tree or forest is all of the grid
   std::vector<int> lmax;  // [dim] finest level per dimension
   // mult: per window list, windows (first and end word of the program, first and end position). The
   // program is a sequence of groups: a header (inner nodes, factors), the factors of the group's

@@ -621,7 +621,7 @@ def test_tables_refused_for_want_of_memory_are_built_once_there_is_some():
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("basis", ["linear", "modlinear"])
-@pytest.mark.parametrize("dim,level,rounds", [(4, 4, 6), (8, 4, 3)])
+@pytest.mark.parametrize("dim,level,rounds", [(4, 4, 6), (8, 4, 3), (8, 4, 0), (12, 3, 0)])
 def test_fp32_mult_is_as_close_as_the_one_of_stored_products(dim, level, rounds, basis):
     """60,001 points, so that a thread adds all subspaces of its point in FP32; stored products are rounded
     to FP32 once. Errors against FP64 vary by some 10 % between coefficient vectors: the mean of three."""
