@@ -645,6 +645,29 @@ def test_fp32_mult_is_as_close_as_the_one_of_stored_products(dim, level, rounds,
 
 
 @pytest.mark.gpu
+def test_fp32_transpose_is_as_close_as_the_one_of_stored_products():
+    """Many small factors of a product, each rounded to FP32 (1.22 times the stored products' error with v_j,
+    H_1 and their product rounded one by one). The mean of six vectors, within 15 %."""
+    grid = _grid(8, 6)
+    n, m = grid.getSize(), 8000
+    rng = np.random.default_rng(1)
+    x = rng.random((m, 8))
+    stored = sg.createOperationMultipleEval(grid, x, sg.OperationMultipleEvalConfiguration(
+        sg.OperationMultipleEvalType.STREAMING, sg.OperationMultipleEvalSubType.CUDA,
+        parameters={"precision": "float", "algo": "subspace", "materialize": "on"}))
+    nested, exact = _op(grid, x, "auto", "float"), _op(grid, x, "auto")
+    errors = np.zeros(2)
+    for _ in range(6):
+        v, ref = rng.standard_normal(m), np.zeros(n)
+        exact.multTranspose(v, ref)
+        for k, op in enumerate((nested, stored)):
+            out = np.zeros(n)
+            op.multTranspose(v, out)
+            errors[k] += np.linalg.norm(out - ref) / np.linalg.norm(ref) / 6.0
+    assert errors[0] <= 1.15 * errors[1]
+
+
+@pytest.mark.gpu
 def test_df64_mult_is_as_close_as_the_one_of_stored_products():
     """ModLinear, one tree of 16 dimensions: 1.4 times the stored products' error with one chain for all of
     its children. The mean of eight coefficient vectors, within a fifth."""
