@@ -424,7 +424,7 @@ cudaError_t nest_mult(NestPlan& p, cudaStream_t s, int precision, const NestDens
                       const double* alpha, float* out32, double* out64, int64_t j_begin,
                       int64_t j_end, int64_t out_end, void* part, int64_t part_bytes, int num_sms,
                       bool spread, int* launches) {
-  NestConfig& c = p.config[precision];
+  NestConfig& c = p.config[precision == SGMEV_FP32 && p.plain ? 3 : precision];  // (a kernel each)
   switch (precision) {
     case SGMEV_FP64:
       return mult<double, double>(p, s, c, dense, m, alpha, out32, out64, j_begin, j_end, out_end, part, part_bytes, num_sms, spread, launches);

@@ -21,6 +21,7 @@ struct NestConfig {  // launch of the mult in one precision, fixed on its first 
 
 struct NestPlan {
   const double* stop = nullptr;  // device flag: when it is not 0 the products are skipped
+  bool plain = false;            // FP32 mult of an inner solve: sums as they come where one block is the grid
   bool ok = false;
   bool mod = false;
   int dim = 0, n_sub = 0, n_ent = 0;
@@ -31,7 +32,7 @@ struct NestPlan {
   std::vector<NestClass> classes;
   std::vector<int> lists, list_cells, list_words;  // see NestTables
   int h_entry[32] = {0}, h_lmax[32] = {0};
-  NestConfig config[3];  // by precision (SGMEV_FP64, SGMEV_FP32, SGMEV_DF64)
+  NestConfig config[4];  // by precision (SGMEV_FP64, SGMEV_FP32, SGMEV_DF64); FP32 plain
   std::vector<int> streams[3];  // multTranspose: tile streams (rows of partial sums) of each class
   unsigned char* block = nullptr;  // device memory of the plan
   // device copies of NestTables

@@ -474,7 +474,7 @@ cudaError_t NEST_MULT_NAME(NEST_MULT_DIM)(NestPlan& p, cudaStream_t s, int preci
     // (grids whose values spread are mostly small: one variant, with everything)
     constexpr bool kBlocks = D > 0;
     if (spread) return launch_mult<float, D, true, kBlocks>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
-    if (p.whole) return launch_mult<float, D, false, kBlocks>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
+    if (p.whole && !p.plain) return launch_mult<float, D, false, kBlocks>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
     return launch_mult<float, D, false>(p, s, c, a, mpad, part_bytes, tiles, num_sms);
   }
   return spread ? launch_mult<ff, D, true>(p, s, c, a, mpad, part_bytes, tiles, num_sms)

@@ -2250,8 +2250,14 @@ static int inner_cg(sgmev_op* op, int prec, const double* rhs, double rhs2, doub
   };
   struct StopScope {
     sgmev_op* o;
-    StopScope(sgmev_op* op_, const double* flag) : o(op_) { o->nest.stop = o->sub.stop = flag; }
-    ~StopScope() { o->nest.stop = o->sub.stop = nullptr; }
+    StopScope(sgmev_op* op_, const double* flag) : o(op_) {
+      o->nest.stop = o->sub.stop = flag;
+      o->nest.plain = true;  // (the outer residual corrects what the products round)
+    }
+    ~StopScope() {
+      o->nest.stop = o->sub.stop = nullptr;
+      o->nest.plain = false;
+    }
   };
   // Step k and the direction after it. As in cg_core the host enqueues a step before it reads the
   // previous one's residual where a step beyond the stop costs nothing.

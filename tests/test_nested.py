@@ -742,3 +742,30 @@ def test_the_first_mult_of_a_process_loads_its_own_dimension_only():
         assert done.returncode == 0, done.stderr
         seconds.append(float(done.stdout))
     assert min(seconds) < 5e-3
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("fit_first", [False, True])
+@pytest.mark.parametrize("dim,level", [(6, 4), (12, 3)])
+def test_single_precision_products_and_fits_where_one_block_is_the_grid(dim, level, fit_first):
+    """The operator's own mult and its fits' inner one are two kernels there, each with its own launch."""
+    grid = _grid(dim, level)
+    n, m = grid.getSize(), 20000
+    rng = np.random.default_rng(9)
+    x, alpha = rng.random((m, dim)), rng.standard_normal(n)
+    y = np.sin(4.0 * x.sum(axis=1)) + 0.1 * rng.standard_normal(m)
+    op, ref = _op(grid, x, "auto", "float"), _op(grid, x, "auto")
+    fits, outs, exact = [], [], np.zeros(m)
+    for k in range(4):
+        if (k % 2 == 0) == fit_first:
+            fits.append(op.fit(y, 1e-3, 1000, 1e-8, mode=sg.SGMEV_SOLVE_MIXED))
+        else:
+            outs.append(np.zeros(m))
+            op.mult(alpha, outs[-1])
+    ref.mult(alpha, exact)
+    np.testing.assert_array_equal(outs[0], outs[1])
+    assert np.linalg.norm(outs[0] - exact) <= 1e-6 * np.linalg.norm(exact)
+    np.testing.assert_array_equal(fits[0][0], fits[1][0])
+    assert 0 < fits[0][1] < 1000
+    double = ref.fit(y, 1e-3, 1000, 1e-10, mode=sg.SGMEV_SOLVE_PLAIN)[0]
+    assert np.abs(fits[0][0] - double).max() <= 1e-5 * np.abs(double).max()
