@@ -23,7 +23,7 @@ namespace {
 // over the dimensions where one forest or tree is all of the grid (regular ones of level 3 and 4), are long,
 // and without this the error was up to 1.46 times that of the stored products, which are rounded once; now
 // 0.7 to 1.06 times over 28 regular and four refined grids (d=12 level 4: 1.42 -> 1.02, adaptive d=8 level 4
-// 1.43 -> 0.8). It costs 1 % (d=10 level 5, 262,147 points: 92.7 -> 93.8 us; 100 us with it in every forest and
+// 1.43 -> 0.8). It costs 1 to 2 % (d=10 level 5, 262,147 points: 92.8 -> 94.3 us; 100 us with it in every forest and
 // tree of such a grid, where the ratio is 0.9 without) and 3 to 5 % where a block is all of the grid (d=8 level 4,
 // 262,144 points: 26.0 -> 26.9 us, 118 on stored products; d=16 level 3, whose kernel spills: 25.3 -> 29.1, 113).
 template <typename V, int R>
